@@ -224,6 +224,11 @@ int s2c_rft_forward(const float* x, const float* F, float* out, int nf, int n_gr
  * other cases return "unsupported" (use s2c_rft_forward). */
 int s2c_rft_forward_t(const float* x, const float* Ft, float* out, int nf, int n_grid, int nspec,
                       void* stream);
+/* The product of scale * x (rounded to float32 first, as the reference's kernel * scaling,
+ * s2cnn/soft/s2_conv.py:41, so3_conv.py:47) in one pass: Ft, the transposed matrix, may be NULL; the
+ * tensor cores are used when it is given and n_grid is even (CUDA build), F otherwise. */
+int s2c_rft_forward_scaled(const float* x, const float* F, const float* Ft, float* out, int nf,
+                           int n_grid, int nspec, float scale, void* stream);
 /* gx[f, a] = sum_{s,c} g[s, f, c] F[a, s, c]: the autograd transpose of the einsum above (on the
  * tensor cores when n_grid is even). */
 int s2c_rft_backward(const float* g, const float* F, float* gx, int nf, int n_grid, int nspec,

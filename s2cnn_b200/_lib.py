@@ -10,6 +10,7 @@ from ctypes import c_char_p, c_double, c_float, c_int, c_long, c_size_t, c_void_
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 CUDA_LIB_PATH = os.path.join(_HERE, "lib", "libs2cnn_b200.so")
+HOST_PATH = os.path.join(_HERE, "lib", "s2cnn_host_ops.so")
 
 _P = c_void_p
 
@@ -66,6 +67,7 @@ _SIGNATURES = {
     "s2c_s2_mm_grady": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_rft_forward": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P]),
     "s2c_rft_forward_t": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P]),
+    "s2c_rft_forward_scaled": (c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_float, _P]),
     "s2c_rft_backward": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P]),
     "s2c_so3_integrate": (c_int, [_P, _P, c_long, c_int, c_int, _P]),
     "s2c_so3_integrate_backward": (c_int, [_P, _P, _P, c_long, c_int, c_int, _P]),
@@ -139,3 +141,23 @@ def cuda_lib():
             raise S2cError("s2cnn_b200: %s is not a CUDA build" % CUDA_LIB_PATH)
         _cuda_lib = lib
     return _cuda_lib
+
+
+_host_module = None
+
+
+def host_module():
+    """The native host path (host/host_ops.cpp), loaded once.  Raises if it has not been built."""
+    global _host_module
+    if _host_module is None:
+        if not os.path.exists(HOST_PATH):
+            raise S2cError("s2cnn_b200: native host path not found at %s - build it with "
+                           "`python -m s2cnn_b200.build`" % HOST_PATH)
+        import importlib.util
+        import torch  # noqa: F401  (its libraries must be loaded first)
+        spec = importlib.util.spec_from_file_location("s2cnn_host_ops", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_error_type(S2cError)
+        _host_module = mod
+    return _host_module

@@ -1,6 +1,7 @@
-"""Ahead-of-time build of the CUDA library (sm_100a only, no JIT, no fallback).
+"""Ahead-of-time build of the CUDA library (sm_100a only, no JIT, no fallback) and of the native host
+path that drives it.
 
-    python -m s2cnn_b200.build            # builds s2cnn_b200/lib/libs2cnn_b200.so
+    python -m s2cnn_b200.build            # builds s2cnn_b200/lib/{libs2cnn_b200,s2cnn_host_ops}.so
 
 Replaces the reference's run-time NVRTC path (s2cnn/utils/cuda.py:19-27): kernels are compiled
 once with nvcc for the B200 and loaded through the C ABI declared in include/s2cnn_b200.h.
@@ -15,6 +16,10 @@ SRC = os.path.join(PKG, "csrc", "lib.cu")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libs2cnn_b200.so")
 
+HOST_SRC = os.path.join(PKG, "host", "host_ops.cpp")
+HOST_NAME = "s2cnn_host_ops"
+HOST_PATH = os.path.join(LIB_DIR, HOST_NAME + ".so")
+
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared"]
 
@@ -25,15 +30,44 @@ def _sources():
         [os.path.join(os.path.dirname(PKG), "include", "s2cnn_b200.h")]
 
 
-def is_stale():
-    if not os.path.exists(LIB_PATH):
+def _older(path, sources):
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    return any(os.path.getmtime(s) > t for s in _sources())
+    t = os.path.getmtime(path)
+    return any(os.path.getmtime(s) > t for s in sources)
+
+
+def is_stale():
+    return _older(LIB_PATH, _sources())
+
+
+def build_host(force=False):
+    """Compile the native host path (checks, allocation, autograd rules: host/host_ops.cpp) against
+    the installed torch if it is missing or older than its source; returns its path."""
+    if not force and not _older(HOST_PATH, [HOST_SRC, os.path.join(os.path.dirname(PKG), "include", "s2cnn_b200.h")]):
+        return HOST_PATH
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    os.makedirs(LIB_DIR, exist_ok=True)
+    tmp = HOST_PATH + ".tmp%d" % os.getpid()
+    cmd = ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=" + HOST_NAME,
+           "-DTORCH_API_INCLUDE_EXTENSION_H"] + ["-isystem" + i for i in inc] + [HOST_SRC, "-o", tmp,
+           "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda", "-ldl"]
+    res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("host path build failed:\n" + res.stdout)
+    os.replace(tmp, HOST_PATH)
+    return HOST_PATH
 
 
 def build(force=False, verbose=False):
-    """Compile the library if it is missing or older than its sources; returns its path."""
+    """Compile the library and the host path if they are missing or older than their sources;
+    returns the library's path."""
+    build_host(force)
     if not force and not is_stale():
         return LIB_PATH
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"

@@ -90,9 +90,16 @@ inline int dev_current() {
 inline int dev_memset_async(void* p, int v, size_t bytes, stream_t s) {
   return cuda_check(cudaMemsetAsync(p, v, bytes, s), "memset");
 }
+// Per-device values the host looks up on every call, remembered after the first (0 = not yet known).
+constexpr int kMaxDevices = 64;
 inline int dev_smem_limit() {
-  int dev = dev_current(), v = 0;
-  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  static std::atomic<int> known[kMaxDevices];
+  const int dev = dev_current();
+  int v = dev < kMaxDevices ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (v == 0) {
+    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (dev < kMaxDevices) known[dev].store(v, std::memory_order_relaxed);
+  }
   return v;
 }
 
@@ -146,15 +153,25 @@ inline std::vector<TimingRec>& timing_recs() {   // guarded by timing_mutex()
   return r;
 }
 
-template <class K, class P>
-inline int launch_impl(K kernel, const char* kname, long grid, int block, size_t smem,
-                       stream_t stream, const P& p) {
+// The kernel is a template argument, so that the shared-memory limit it has been given on each device
+// is remembered per kernel: the attribute is set when a launch needs more than any launch before it
+// (cudaFuncSetAttribute on every launch was a tenth of the host time of a small call).
+template <auto kernel, class P>
+inline int launch_impl(const char* kname, long grid, int block, size_t smem, stream_t stream, const P& p) {
   if (grid <= 0) return S2C_OK;
   if (grid > 2147483647L) return fail(S2C_ERR_UNSUPPORTED, std::string(kname) + ": grid too large");
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return cuda_check(e, kname);
+    static std::atomic<int> granted[kMaxDevices];
+    const int dev = dev_current();
+    if (dev >= kMaxDevices || granted[dev].load(std::memory_order_acquire) < (int)smem) {
+      static std::mutex mu;
+      std::lock_guard<std::mutex> lock(mu);   // a smaller request must not undo a larger one
+      if (dev >= kMaxDevices || granted[dev].load(std::memory_order_relaxed) < (int)smem) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return cuda_check(e, kname);
+        if (dev < kMaxDevices) granted[dev].store((int)smem, std::memory_order_release);
+      }
+    }
   }
   TimingRec rec{kname, nullptr, nullptr};
   const bool timed = timing_on();
@@ -175,7 +192,7 @@ inline int launch_impl(K kernel, const char* kname, long grid, int block, size_t
 }  // namespace s2c
 
 #define S2C_LAUNCH(name, grid, block, smem, stream, params) \
-  s2c::launch_impl(name, #name, (long)(grid), (int)(block), (size_t)(smem), stream, params)
+  s2c::launch_impl<name>(#name, (long)(grid), (int)(block), (size_t)(smem), stream, params)
 
 namespace s2c {
 // ---- asynchronous bulk copy global -> shared (TMA, 1-D) completing on an mbarrier -------------

@@ -816,6 +816,20 @@ int s2c_s2_ifft(const float* x, float* out, int out_is_real, long nbatch, int b_
 // ---- spectral products ---------------------------------------------------------------------------
 #ifndef S2C_EMUL
 static __device__ int g_tc_err_flag;
+// its address on the current device, looked up once per device
+static int tc_err_flag(int** out) {
+  static std::atomic<int*> known[kMaxDevices];
+  const int dev = dev_current();
+  int* p = dev < kMaxDevices ? known[dev].load(std::memory_order_relaxed) : nullptr;
+  if (!p) {
+    void* q = nullptr;
+    S2C_TRY(cuda_check(cudaGetSymbolAddress(&q, g_tc_err_flag), "tensor-core status flag"));
+    p = (int*)q;
+    if (dev < kMaxDevices) known[dev].store(p, std::memory_order_relaxed);
+  }
+  *out = p;
+  return S2C_OK;
+}
 #endif
 
 #ifndef S2C_EMUL
@@ -830,9 +844,7 @@ static int so3_mm_tc_launch(int op, const float* a, const float* b, float* c, in
   p.run = 2 * (op == kTcFwd ? fi : op == kTcGradX ? fo : nb);
   if (p.run <= kTcKMax) { p.kblk = (p.run + 7) / 8 * 8; p.nblk = 1; }
   else { p.kblk = kTcKMax; p.nblk = (p.run + kTcKMax - 1) / kTcKMax; }
-  void* flag = nullptr;
-  S2C_TRY(cuda_check(cudaGetSymbolAddress(&flag, g_tc_err_flag), "tensor-core status flag"));
-  p.err = (int*)flag;
+  S2C_TRY(tc_err_flag(&p.err));
   // Few output tiles (the grad-y product: its rows are only (p, k)) leave most SMs idle: several
   // CTAs then share a tile, each contracting a slice of the outer index and adding its partial
   // result atomically into the zeroed output (float additions in arrival order).
@@ -852,8 +864,8 @@ static int so3_mm_tc_launch(int op, const float* a, const float* b, float* c, in
   const bool flush = chain_mmas > kTcChainMax;
   const bool vec = so3_mm_tc_vec16(op, nb, fi, fo);
 #define S2C_TC_LAUNCH2(OP, FL, NAME)                                                               \
-  (vec ? launch_impl(so3_mm_tc_kernel<OP, FL, true>, NAME, tiles, kTcThreads, kTcSmemBytes, st, p)  \
-       : launch_impl(so3_mm_tc_kernel<OP, FL, false>, NAME, tiles, kTcThreads, kTcSmemBytes, st, p))
+  (vec ? launch_impl<so3_mm_tc_kernel<OP, FL, true>>(NAME, tiles, kTcThreads, kTcSmemBytes, st, p)  \
+       : launch_impl<so3_mm_tc_kernel<OP, FL, false>>(NAME, tiles, kTcThreads, kTcSmemBytes, st, p))
 #define S2C_TC_LAUNCH(OP, NAME) (flush ? S2C_TC_LAUNCH2(OP, true, NAME) : S2C_TC_LAUNCH2(OP, false, NAME))
   if (op == kTcFwd) return S2C_TC_LAUNCH(kTcFwd, "so3_mm_tc_kernel");
   if (op == kTcGradX) return S2C_TC_LAUNCH(kTcGradX, "so3_mm_tc_gradx");
@@ -864,7 +876,7 @@ static int so3_mm_tc_launch(int op, const float* a, const float* b, float* c, in
 // on the tensor-core pipeline: the kernel-grid -> spectrum transforms and their transposes.
 static int plain_tc_launch(bool a_strided, const float* a, const float* b, float* c, long M, long N,
                            long K, long a_rs, long a_ps, long b_rs, long b_ps, long c_rs, long c_ps,
-                           stream_t st) {
+                           float a_scale, stream_t st) {
   MmTcParams p;
   p.a = a; p.b = b; p.c = c;
   p.nl = 1; p.nb = (int)M; p.fi = (int)(K / 2); p.fo = (int)(N / 2);
@@ -873,9 +885,8 @@ static int plain_tc_launch(bool a_strided, const float* a, const float* b, float
   else { p.kblk = kTcKMax; p.nblk = (p.run + kTcKMax - 1) / kTcKMax; }
   p.ksplit = 1;
   p.a_rs = a_rs; p.a_ps = a_ps; p.b_rs = b_rs; p.b_ps = b_ps; p.c_rs = c_rs; p.c_ps = c_ps;
-  void* flag = nullptr;
-  S2C_TRY(cuda_check(cudaGetSymbolAddress(&flag, g_tc_err_flag), "tensor-core status flag"));
-  p.err = (int*)flag;
+  p.a_scale = a_scale;
+  S2C_TRY(tc_err_flag(&p.err));
   const long tiles = ((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);
   const bool flush = (long)((p.run + 7) / 8) * 3 > kTcChainMax;
   // 16-byte loads need K a multiple of 4 and 16-byte aligned rows of every contiguous operand
@@ -965,28 +976,40 @@ int s2c_s2_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb, 
 }
 
 // ---- kernel-grid -> spectrum -----------------------------------------------------------------------
-int s2c_rft_forward(const float* x, const float* F, float* out, int nf, int ng, int ns, void* st) {
-  if (!x || !F || !out || nf < 1 || ng < 1 || ns < 1)
-    return fail(S2C_ERR_BAD_ARG, "s2c_rft_forward: bad argument");
+static int rft_forward_any(const float* x, const float* F, const float* Ft, float* out, int nf, int ng,
+                            int ns, float scale, stream_t st) {
+#ifndef S2C_EMUL
+  if (Ft && ng % 2 == 0)
+    // C[f][(s, c)] = sum_a (scale x[f][a]) Ft[(s, c)][a], written to out[s][f][c]
+    return plain_tc_launch(false, x, Ft, out, nf, 2L * ns, ng, ng, 2, ng, 2, 2, 2L * nf, scale, st);
+#endif
+  if (!F) return fail(S2C_ERR_UNSUPPORTED, "rft with the transposed matrix: needs the CUDA build and an even n_grid");
   RftFwdParams p;
   p.x = x; p.F = (const float2*)F; p.out = (float2*)out;
-  p.nf = nf; p.ng = ng; p.ns = ns;
+  p.nf = nf; p.ng = ng; p.ns = ns; p.scale = scale;
   p.tiles_f = (nf + kRftTF - 1) / kRftTF;
   const long tiles_s = (ns + kRftTS - 1) / kRftTS;
   const size_t sm = kRftTF * (kRftTA + 1) * 4 + kRftTA * kRftTS * 8;
-  return S2C_LAUNCH(rft_forward, p.tiles_f * tiles_s, 256, sm, as_stream(st), p);
+  return S2C_LAUNCH(rft_forward, p.tiles_f * tiles_s, 256, sm, st, p);
+}
+
+int s2c_rft_forward(const float* x, const float* F, float* out, int nf, int ng, int ns, void* st) {
+  if (!x || !F || !out || nf < 1 || ng < 1 || ns < 1)
+    return fail(S2C_ERR_BAD_ARG, "s2c_rft_forward: bad argument");
+  return rft_forward_any(x, F, nullptr, out, nf, ng, ns, 1.f, as_stream(st));
 }
 
 int s2c_rft_forward_t(const float* x, const float* Ft, float* out, int nf, int ng, int ns, void* st) {
   if (!x || !Ft || !out || nf < 1 || ng < 1 || ns < 1)
     return fail(S2C_ERR_BAD_ARG, "s2c_rft_forward_t: bad argument");
-#ifndef S2C_EMUL
-  if (ng % 2 == 0) {
-    // C[f][(s, c)] = sum_a x[f][a] Ft[(s, c)][a], written to out[s][f][c]
-    return plain_tc_launch(false, x, Ft, out, nf, 2L * ns, ng, ng, 2, ng, 2, 2, 2L * nf, as_stream(st));
-  }
-#endif
-  return fail(S2C_ERR_UNSUPPORTED, "s2c_rft_forward_t: needs the CUDA build and an even n_grid");
+  return rft_forward_any(x, nullptr, Ft, out, nf, ng, ns, 1.f, as_stream(st));
+}
+
+int s2c_rft_forward_scaled(const float* x, const float* F, const float* Ft, float* out, int nf, int ng,
+                           int ns, float scale, void* st) {
+  if (!x || !F || !out || nf < 1 || ng < 1 || ns < 1)
+    return fail(S2C_ERR_BAD_ARG, "s2c_rft_forward_scaled: bad argument");
+  return rft_forward_any(x, F, Ft, out, nf, ng, ns, scale, as_stream(st));
 }
 
 int s2c_rft_backward(const float* g, const float* F, float* gx, int nf, int ng, int ns, void* st) {
@@ -996,7 +1019,7 @@ int s2c_rft_backward(const float* g, const float* F, float* gx, int nf, int ng, 
   if (!g_force_general && ng % 2 == 0) {
     // gx[f][a] = sum_{(s, c)} g[s][f][c] F[a][(s, c)]: the row operand holds k = (s, c) as pairs
     // 2 nf floats apart
-    return plain_tc_launch(true, g, F, gx, nf, ng, 2L * ns, 2, 2L * nf, 2L * ns, 2, ng, 2, as_stream(st));
+    return plain_tc_launch(true, g, F, gx, nf, ng, 2L * ns, 2, 2L * nf, 2L * ns, 2, ng, 2, 1.f, as_stream(st));
   }
 #endif
   RftBwdParams p;

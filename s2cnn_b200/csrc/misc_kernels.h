@@ -15,6 +15,7 @@ struct RftFwdParams {
   float2* out;       // [ns][nf]
   int nf, ng, ns;
   int tiles_f;
+  float scale;       // x is multiplied by this (and rounded) while it is staged
 };
 constexpr int kRftTF = 32, kRftTS = 32, kRftTA = 32;
 
@@ -32,7 +33,7 @@ S2C_KERNEL(rft_forward, RftFwdParams) {
     for (int e = ctx.tid; e < kRftTF * kRftTA; e += ctx.nthr) {
       const int f = e / kRftTA, a = e - f * kRftTA;
       xs[f * (kRftTA + 1) + a] =
-          (f0 + f < p.nf && a0 + a < p.ng) ? p.x[(long)(f0 + f) * p.ng + a0 + a] : 0.f;
+          (f0 + f < p.nf && a0 + a < p.ng) ? p.x[(long)(f0 + f) * p.ng + a0 + a] * p.scale : 0.f;
     }
     for (int e = ctx.tid; e < kRftTA * kRftTS; e += ctx.nthr) {
       const int a = e / kRftTS, s = e - a * kRftTS;

@@ -15,8 +15,6 @@
 // (s2cnn/soft/so3_fft.py:64-112,158-202,246-443) and produce the same values.
 #pragma once
 
-#include <map>
-#include <mutex>
 #include <string>
 #include <type_traits>
 
@@ -757,21 +755,12 @@ __global__ void __launch_bounds__(kFusedMaxThreads) so3_fwd_fused(const FwdFused
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
   so3_fwd_fused_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
 }
-// name of an instantiation for the launch records, e.g. "so3_inv_fused<20>" (interned: the
-// records keep the pointer)
-inline const char* kernel_name_n(const char* base, int n) {
-  static std::mutex mu;
-  static std::map<std::pair<std::string, int>, std::string> names;
-  std::lock_guard<std::mutex> g(mu);
-  auto key = std::make_pair(std::string(base), n);
-  auto it = names.find(key);
-  if (it == names.end())
-    it = names.emplace(key, std::string(base) + "<" + std::to_string(n) + ">").first;
-  return it->second.c_str();
-}
+// name of an instantiation for the launch records, e.g. "so3_inv_fused<20>"
 #define S2C_LAUNCH_N(name, N, grid, block, smem, stream, params)                              \
-  s2c::launch_impl(name<N>, s2c::kernel_name_n(#name, N), (long)(grid), (int)(block),          \
-                   (size_t)(smem), stream, params)
+  ([&] {                                                                                      \
+    static const std::string kname = std::string(#name "<") + std::to_string(N) + ">";        \
+    return s2c::launch_impl<name<N>>(kname.c_str(), (long)(grid), (int)(block), (size_t)(smem), stream, params); \
+  }())
 #else
 #define S2C_LAUNCH_N(name, N, grid, block, smem, stream, params) \
   s2c::emu_launch<name##_impl<N>>(#name, (long)(grid), (int)(block), (size_t)(smem), params)

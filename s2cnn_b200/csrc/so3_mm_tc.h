@@ -83,6 +83,7 @@ struct MmTcParams {
   // element (column c, k) of b likewise, element (r, c) of the result at r * c_rs + (c / 2) * c_ps + c % 2;
   // nb = rows, fi = K / 2, fo = columns / 2, nl = 1
   long a_rs, a_ps, b_rs, b_ps, c_rs, c_ps;
+  float a_scale;    // kTcPlainCC: the row operand is multiplied by this (and rounded) while it is staged
 };
 
 // row / column geometry of one degree
@@ -552,7 +553,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
 #pragma unroll
       for (int q = 0; q < kSlots; ++q) {
         if ((live >> q) & 1u) {
-          split_store(stage, stage + kTcBufBytes, soA[q], ra[q]);
+          float4 va = ra[q];
+          if (OP == kTcPlainCC)   // (__fmul_rn: the product must not be contracted into the hi / lo split)
+            va = make_float4(__fmul_rn(va.x, p.a_scale), __fmul_rn(va.y, p.a_scale),
+                             __fmul_rn(va.z, p.a_scale), __fmul_rn(va.w, p.a_scale));
+          split_store(stage, stage + kTcBufBytes, soA[q], va);
           split_store(stage + 2 * kTcBufBytes, stage + 3 * kTcBufBytes, soB[q],
                       column_rows(rb[q], (oddB >> q) & 1u));
         }

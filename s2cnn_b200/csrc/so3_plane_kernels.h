@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(plane_threads(kPlaneRW), 2) so3_inv_plane(cons
   so3_inv_plane_impl<N, kPlaneRW>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
 }
 #define S2C_LAUNCH_PLANE(name, N, grid, stream, params)                                       \
-  s2c::launch_impl(name<N>, #name, (long)(grid), s2c::plane_threads(s2c::kPlaneRW),           \
+  s2c::launch_impl<name<N>>(#name, (long)(grid), s2c::plane_threads(s2c::kPlaneRW),           \
                    s2c::plane_smem_bytes(N, s2c::kPlaneRW), stream, params)
 #else
 #define S2C_LAUNCH_PLANE(name, N, grid, stream, params)                                       \

@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) so3_inv_wigner_r(const InvRow
   so3_inv_wigner_r_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
 }
 #define S2C_LAUNCH_ROWS(name, N, grid, stream, params)                                         \
-  s2c::launch_impl(name<N>, #name, (long)(grid), s2c::kRowsThreads, s2c::rows_smem_bytes<N>(), \
+  s2c::launch_impl<name<N>>(#name, (long)(grid), s2c::kRowsThreads, s2c::rows_smem_bytes<N>(), \
                    stream, params)
 #else
 #define S2C_LAUNCH_ROWS(name, N, grid, stream, params)                                         \

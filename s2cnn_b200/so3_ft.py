@@ -9,7 +9,7 @@ from functools import lru_cache
 import torch
 
 from .ops import cuda_ops
-from .s2_ft import _Rft, fourier_matrices
+from .s2_ft import fourier_matrices
 
 
 @lru_cache(maxsize=32)
@@ -28,6 +28,4 @@ def so3_rft(x, b, grid):
     """
     F, Ft = _setup_so3_ft(b, grid, device_type=x.device.type, device_index=x.device.index)
     assert x.size(-1) == F.size(0)
-    sz = x.size()
-    out = _Rft.apply(x.reshape(-1, x.size(-1)), F, Ft)
-    return out.view(-1, *sz[:-1], 2)
+    return cuda_ops().ag_rft(x, F, Ft)

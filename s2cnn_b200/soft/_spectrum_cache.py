@@ -1,30 +1,58 @@
-"""Per-module cache of the kernel's spectrum.
+"""Per-module caches around the transform of the kernel.
 
 ``S2Convolution`` / ``SO3Convolution`` transform ``kernel * scaling`` to the spectral domain in
-every forward pass (s2cnn/soft/s2_conv.py:41, so3_conv.py:47).  The result depends on the weights
-alone, so in inference it is the same tensor pass after pass; the cache keeps it while the
-parameter has not been written to (its version counter, storage and device are unchanged) and no
-gradient with respect to it is being recorded.  During training the transform runs every time, as
-autograd needs it in the graph.
+every forward pass (s2cnn/soft/s2_conv.py:41, so3_conv.py:47).
+
+* ``KernelSpectrumCache``: the result depends on the weights alone, so in inference it is the same
+  tensor pass after pass; the cache keeps it while the parameter has not been written to (its version
+  counter, storage and device are unchanged) and no gradient with respect to it is being recorded.
+  During training the transform runs every time, as autograd needs it in the graph.
+* ``FourierMatrices``: the Fourier matrices of the layer's grid, and the one of the gradient with the
+  layer's constant scaling multiplied in; the forward product scales the kernel while it reads it, so
+  neither ``kernel * scaling`` nor its gradient is a pass of its own.
+
+Each keeps one entry as a single tuple: replaced in one assignment, so a reader in another thread
+never sees half of one entry and half of another.  Copies and pickles of a module start empty.
 """
 import torch
 
 
-class KernelSpectrumCache:
+class _OneEntry:
     def __init__(self):
-        self._key = None
-        self._value = None
+        self._entry = None
 
+    def __deepcopy__(self, memo):
+        return type(self)()
+
+    def __reduce__(self):
+        return (type(self), ())
+
+    def clear(self):
+        self._entry = None
+
+
+class KernelSpectrumCache(_OneEntry):
     def get(self, kernel, transform):
         if torch.is_grad_enabled() and kernel.requires_grad:
             return transform(kernel)
-        key = (kernel._version, kernel.data_ptr(), kernel.device, tuple(kernel.shape))
-        if self._key != key:
+        key = (kernel._version, kernel.data_ptr(), kernel.device, kernel.shape)
+        entry = self._entry
+        if entry is None or entry[0] != key:
             with torch.no_grad():
-                self._value = transform(kernel)
-            self._key = key
-        return self._value
+                entry = (key, transform(kernel))
+            self._entry = entry
+        return entry[1]
 
-    def clear(self):
-        self._key = None
-        self._value = None
+
+class FourierMatrices(_OneEntry):
+    def get(self, setup, b, grid, scaling, device):
+        """``setup(b, grid, device_type, device_index)`` -> (F, Ft); returns (F, Ft, scaling, scaling * F),
+        the arguments of ``ag_rft``.  The grid (a tuple of hundreds of angles, costly to hash) is
+        compared by identity first."""
+        entry = self._entry
+        key = (b, scaling, device)
+        if entry is None or entry[0] is not grid or entry[1] != key:
+            F, Ft = setup(b, grid, device_type=device.type, device_index=device.index)
+            entry = (grid, key, (F, Ft, scaling, F * scaling))
+            self._entry = entry
+        return entry[2]

@@ -7,11 +7,11 @@ from torch.nn.modules import Module
 from torch.nn.parameter import Parameter
 
 from ..ops import cuda_ops
-from ..so3_ft import so3_rft
+from ..so3_ft import _setup_so3_ft
 from ..so3_mm import so3_mm
 from .so3_fft import SO3_fft_real, SO3_fft_real_relu, SO3_ifft_real_bias
 from .so3_integrate import so3_relu_integrate
-from ._spectrum_cache import KernelSpectrumCache
+from ._spectrum_cache import FourierMatrices, KernelSpectrumCache
 from ._recompute import fused_or_recompute
 
 
@@ -36,6 +36,12 @@ class SO3Convolution(Module):
         # the scaling stays outside the parameter (so3_conv.py:30-34)
         self.scaling = 1. / math.sqrt(len(self.grid) * self.nfeature_in * (self.b_out ** 3.) / (self.b_in ** 3.))
         self._spectrum_cache = KernelSpectrumCache()
+        self._fourier = FourierMatrices()
+
+    def _kernel_spectrum(self, kernel):
+        """so3_rft(kernel * scaling, b_out, grid)"""
+        return cuda_ops().ag_rft(kernel, *self._fourier.get(_setup_so3_ft, self.b_out, self.grid, self.scaling,
+                                                            kernel.device))
 
     def forward(self, x, relu_input=False, relu_integrate=False, input_spectrum=False,
                 relu_so3_fft=None, channel_scale=None, bias=None):
@@ -68,7 +74,7 @@ class SO3Convolution(Module):
                     x = torch.relu(x)
                 x = SO3_fft_real.apply(x, self.b_out)  # [l * m * n, batch, feature_in, complex]
         # [l * m * n, feature_in, feature_out, complex]; kept between calls while the weights stand still
-        y = self._spectrum_cache.get(self.kernel, lambda k: so3_rft(k * self.scaling, self.b_out, self.grid))
+        y = self._spectrum_cache.get(self.kernel, self._kernel_spectrum)
         if channel_scale is not None:
             y = y * channel_scale.view(1, 1, -1, 1)
         own_bias = self.bias if bias is None else bias

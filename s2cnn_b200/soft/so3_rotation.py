@@ -22,19 +22,6 @@ def _setup_so3_rotation(b, alpha, beta, gamma, device_type, device_index):
     return torch.from_numpy(U).to(torch.device(device_type, device_index))
 
 
-class _RotateSpectrum(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, U, b):
-        ctx.b = b
-        ctx.save_for_backward(U)
-        return cuda_ops().so3_rotate_spectrum(U, x, b, adjoint=False)
-
-    @staticmethod
-    def backward(ctx, g):
-        (U,) = ctx.saved_tensors
-        return cuda_ops().so3_rotate_spectrum(U, g.contiguous(), ctx.b, adjoint=True), None, None
-
-
 def so3_rotation(x, alpha, beta, gamma):
     """
     :param x: [..., beta, alpha, gamma] (..., 2b, 2b, 2b)
@@ -44,6 +31,6 @@ def so3_rotation(x, alpha, beta, gamma):
     U = _setup_so3_rotation(b, float(alpha), float(beta), float(gamma),
                             device_type=x.device.type, device_index=x.device.index)
     x = SO3_fft_real.apply(x)          # [l * m * n, ..., complex]
-    z = _RotateSpectrum.apply(x, U, b)
+    z = cuda_ops().ag_rotate_spectrum(x, U, b)
     z = SO3_ifft_real.apply(z)
     return z.contiguous().view(*x_size)
