@@ -110,7 +110,7 @@ inline int dev_smem_limit() {
     static __device__ __forceinline__ void run(const s2c::Ctx& ctx, const P& p,              \
                                                unsigned char* smem);                         \
   };                                                                                         \
-  __global__ void name(const P p) {                                                          \
+  static __global__ void name(const P p) {                                                        \
     extern __shared__ float4 s2c_dyn_smem[];                                                 \
     s2c::Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};        \
     name##_impl::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));                \
@@ -123,7 +123,7 @@ inline int dev_smem_limit() {
     static __device__ __forceinline__ void run(const s2c::Ctx& ctx, const P& p,              \
                                                unsigned char* smem);                         \
   };                                                                                         \
-  __global__ void __launch_bounds__(MAXT, MINB) name(const P p) {                            \
+  static __global__ void __launch_bounds__(MAXT, MINB) name(const P p) {                            \
     extern __shared__ float4 s2c_dyn_smem[];                                                 \
     s2c::Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};        \
     name##_impl::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));                \

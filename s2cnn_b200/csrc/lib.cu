@@ -1,6 +1,7 @@
 // C-ABI entry points of s2cnn_b200 (see include/s2cnn_b200.h) and the host-side dispatch that
-// sequences the kernels.  Single translation unit: nvcc -gencode arch=compute_100a,code=sm_100a
-// for the product; g++ -x c++ -DS2C_EMUL for the host-emulation build used by the CPU tests.
+// sequences the kernels.  nvcc -gencode arch=compute_100a,code=sm_100a for the product, the kernel
+// families with many instantiations compiled beside it from parts.cu (-DS2C_SPLIT); one translation unit
+// with g++ -x c++ -DS2C_EMUL for the host-emulation build used by the CPU tests.
 #include "../../include/s2cnn_b200.h"
 
 #include <algorithm>
@@ -845,31 +846,20 @@ static int so3_mm_tc_launch(int op, const float* a, const float* b, float* c, in
   if (p.run <= kTcKMax) { p.kblk = (p.run + 7) / 8 * 8; p.nblk = 1; }
   else { p.kblk = kTcKMax; p.nblk = (p.run + kTcKMax - 1) / kTcKMax; }
   S2C_TRY(tc_err_flag(&p.err));
-  // Few output tiles (the grad-y product: its rows are only (p, k)) leave most SMs idle: several
-  // CTAs then share a tile, each contracting a slice of the outer index and adding its partial
-  // result atomically into the zeroed output (float additions in arrival order).
-  p.ksplit = 1;
-  {
-    const long plain = so3_mm_tc_tiles(op, nl, nb, fi, fo);
-    if (op == kTcGradY && plain < 100 && nl > 1) p.ksplit = (int)std::min<long>(8, (148 + plain - 1) / plain);
-  }
-  if (p.ksplit > 1) {
-    const size_t out_bytes = (size_t)so3_nspec(nl) * fi * fo * sizeof(float2);
+  // The forward product always runs one CTA per tile: its rounding is then the same whatever the batch.
+  p.kper = op == kTcFwd ? kTcNoSplit : tc_pick_kper(op, nl, nb, fi, fo, p.nblk);
+  if (p.kper != kTcNoSplit) {
+    const size_t out_bytes = (size_t)so3_nspec(nl) * (op == kTcGradX ? (size_t)nb * fi : (size_t)fi * fo) * sizeof(float2);
     S2C_TRY(cuda_check(cudaMemsetAsync(c, 0, out_bytes, st), "so3_mm split-K output clear"));
   }
-  const long tiles = so3_mm_tc_tiles(op, nl, nb, fi, fo, p.ksplit);
-  // longest K loop of any CTA
-  const long lmax = 2 * nl - 1;
-  const long chain_mmas = ((lmax + p.ksplit - 1) / p.ksplit) * (long)((p.run + 7) / 8) * 3;
+  const long tiles = so3_mm_tc_tiles(op, nl, nb, fi, fo, p.nblk, p.kper);
+  // MMAs of the longest CTA
+  const long chain_mmas = 3 * (p.kper == kTcNoSplit ? (2L * nl - 1) * ((p.run + 7) / 8) : (long)p.kper * (p.kblk / 8));
   const bool flush = chain_mmas > kTcChainMax;
   const bool vec = so3_mm_tc_vec16(op, nb, fi, fo);
-#define S2C_TC_LAUNCH2(OP, FL, NAME)                                                               \
-  (vec ? launch_impl<so3_mm_tc_kernel<OP, FL, true>>(NAME, tiles, kTcThreads, kTcSmemBytes, st, p)  \
-       : launch_impl<so3_mm_tc_kernel<OP, FL, false>>(NAME, tiles, kTcThreads, kTcSmemBytes, st, p))
-#define S2C_TC_LAUNCH(OP, NAME) (flush ? S2C_TC_LAUNCH2(OP, true, NAME) : S2C_TC_LAUNCH2(OP, false, NAME))
-  if (op == kTcFwd) return S2C_TC_LAUNCH(kTcFwd, "so3_mm_tc_kernel");
-  if (op == kTcGradX) return S2C_TC_LAUNCH(kTcGradX, "so3_mm_tc_gradx");
-  return S2C_TC_LAUNCH(kTcGradY, "so3_mm_tc_grady");
+  if (op == kTcFwd) return launch_so3_mm_tc<kTcFwd>("so3_mm_tc_kernel", tiles, flush, vec, st, p);
+  if (op == kTcGradX) return launch_so3_mm_tc<kTcGradX>("so3_mm_tc_gradx", tiles, flush, vec, st, p);
+  return launch_so3_mm_tc<kTcGradY>("so3_mm_tc_grady", tiles, flush, vec, st, p);
 }
 
 // A plain real product C[r][c] = sum_k A[r][k] B[c][k] (M rows, N columns, K terms; N and K even)
@@ -883,18 +873,20 @@ static int plain_tc_launch(bool a_strided, const float* a, const float* b, float
   p.run = (int)K;
   if (p.run <= kTcKMax) { p.kblk = (p.run + 7) / 8 * 8; p.nblk = 1; }
   else { p.kblk = kTcKMax; p.nblk = (p.run + kTcKMax - 1) / kTcKMax; }
-  p.ksplit = 1;
   p.a_rs = a_rs; p.a_ps = a_ps; p.b_rs = b_rs; p.b_ps = b_ps; p.c_rs = c_rs; p.c_ps = c_ps;
   p.a_scale = a_scale;
   S2C_TRY(tc_err_flag(&p.err));
-  const long tiles = ((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);
-  const bool flush = (long)((p.run + 7) / 8) * 3 > kTcChainMax;
+  // (one degree, l = 0, with M rows and N columns in the spectral geometry; the forward transform has a
+  // short contraction and is not split)
+  p.kper = a_strided ? tc_pick_kper(kTcPlainSC, 1, (int)M, p.fi, p.fo, p.nblk) : kTcNoSplit;
+  if (p.kper != kTcNoSplit)
+    S2C_TRY(cuda_check(cudaMemsetAsync(c, 0, (size_t)M * N * sizeof(float), st), "rft split-K output clear"));
+  const long tiles = so3_mm_tc_tiles(kTcPlainSC, 1, (int)M, p.fi, p.fo, p.nblk, p.kper);
+  const bool flush = 3 * (p.kper == kTcNoSplit ? (K + 7) / 8 : (long)p.kper * (p.kblk / 8)) > kTcChainMax;
   // 16-byte loads need K a multiple of 4 and 16-byte aligned rows of every contiguous operand
   const bool vec = K % 4 == 0 && b_rs % 4 == 0 && (a_strided || a_rs % 4 == 0);
-  if (a_strided) return S2C_TC_LAUNCH(kTcPlainSC, "rft_tc_backward");
-  return S2C_TC_LAUNCH(kTcPlainCC, "rft_tc_forward");
-#undef S2C_TC_LAUNCH2
-#undef S2C_TC_LAUNCH
+  if (a_strided) return launch_so3_mm_tc<kTcPlainSC>("rft_tc_backward", tiles, flush, vec, st, p);
+  return launch_so3_mm_tc<kTcPlainCC>("rft_tc_forward", tiles, flush, vec, st, p);
 }
 #endif
 

@@ -755,12 +755,25 @@ __global__ void __launch_bounds__(kFusedMaxThreads) so3_fwd_fused(const FwdFused
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
   so3_fwd_fused_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
 }
-// name of an instantiation for the launch records, e.g. "so3_inv_fused<20>"
-#define S2C_LAUNCH_N(name, N, grid, block, smem, stream, params)                              \
-  ([&] {                                                                                      \
-    static const std::string kname = std::string(#name "<") + std::to_string(N) + ">";        \
-    return s2c::launch_impl<name<N>>(kname.c_str(), (long)(grid), (int)(block), (size_t)(smem), stream, params); \
-  }())
+// Launcher of a kernel family with a compile-time length, launch_<name><N>; the launch records carry the
+// instantiation's name, e.g. "so3_inv_fused<20>".  In the split build (build.py) only parts.cu defines
+// the launchers - and with them compiles the kernels -, lib.cu sees declarations.
+#if defined(S2C_SPLIT) && !defined(S2C_PART)
+#define S2C_LAUNCHER_N(name, P) \
+  template <int N>              \
+  int launch_##name(long grid, int block, size_t smem, stream_t st, const P& p);
+#else
+#define S2C_LAUNCHER_N(name, P)                                                           \
+  template <int N>                                                                        \
+  int launch_##name(long grid, int block, size_t smem, stream_t st, const P& p) {         \
+    static const std::string kname = std::string(#name "<") + std::to_string(N) + ">";    \
+    return s2c::launch_impl<name<N>>(kname.c_str(), grid, block, smem, st, p);            \
+  }
+#endif
+S2C_LAUNCHER_N(so3_inv_fused, InvFusedParams)
+S2C_LAUNCHER_N(so3_fwd_fused, FwdFusedParams)
+#define S2C_LAUNCH_N(name, N, grid, block, smem, stream, params) \
+  s2c::launch_##name<N>((long)(grid), (int)(block), (size_t)(smem), stream, params)
 #else
 #define S2C_LAUNCH_N(name, N, grid, block, smem, stream, params) \
   s2c::emu_launch<name##_impl<N>>(#name, (long)(grid), (int)(block), (size_t)(smem), params)

@@ -47,6 +47,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "backend.h"
 
 namespace s2c {
@@ -76,8 +78,8 @@ struct MmTcParams {
   int run;          // floats per outer contraction index: 2 fi (fwd), 2 fo (grad x), 2 nb (grad y)
   int kblk;         // floats per K block (multiple of 8, <= kTcKMax)
   int nblk;         // K blocks per run
-  int ksplit;       // CTAs sharing one output tile (each takes a slice of the outer contraction
-                    // index and adds its partial result atomically into the zeroed output); 1 = none
+  int kper;         // K blocks per CTA: a tile whose contraction has more is shared by several CTAs, each
+                    // adding its partial result atomically into the zeroed output (see tc_pick_kper)
   int* err;         // device flag, set to 1 on a wait time-out
   // plain products only (floats): element (row r, k) of a at r * a_rs + (k / 2) * a_ps + k % 2,
   // element (column c, k) of b likewise, element (r, c) of the result at r * c_rs + (c / 2) * c_ps + c % 2;
@@ -228,6 +230,19 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const float (&v)[16]) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// CTAs that share an output tile of degree l: each takes at most kper of its (2l + 1) * nblk K blocks.
+__host__ __device__ __forceinline__ int tc_splits(int l, int nblk, int kper) {
+  return ((2 * l + 1) * nblk + kper - 1) / kper;
+}
+
+// Vector reductions without a return value (one request per 8 / 16 bytes instead of one per float).
+__device__ __forceinline__ void tc_red2(float* p, float a, float b) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void tc_red4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
 // Staging slot e of a contiguous operand -> (row, 16-byte chunk of the K block): groups of 8 slots
 // cover 4 rows x 2 adjacent chunks, consecutive groups the chunk pairs of the same 4 rows (nchf,
 // the chunks per block, is even).
@@ -266,17 +281,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   int l = p.nl - 1;
   long t = blockIdx.x;
   for (;; --l) {
-    const int sl = p.ksplit < 2 * l + 1 ? p.ksplit : 2 * l + 1;
-    const long c = tc_tiles_for(OP, p.nb, p.fi, p.fo, l) * sl;
+    const long c = tc_tiles_for(OP, p.nb, p.fi, p.fo, l) * tc_splits(l, p.nblk, p.kper);
     if (t < c) break;
     t -= c;
   }
   const int L = 2 * l + 1;
-  // slice of the outer contraction index handled by this CTA
-  const int nsplit = p.ksplit < L ? p.ksplit : L;
+  // K blocks handled by this CTA: [it_lo, it_hi) of the L * nblk blocks (outer index, block of its run)
+  const int nsplit = tc_splits(l, p.nblk, p.kper);
   const int split = (int)(t % nsplit);
   t /= nsplit;
-  const int o_lo = (int)((long)split * L / nsplit), o_hi = (int)((long)(split + 1) * L / nsplit);
+  const int it_lo = (int)((long)split * L * p.nblk / nsplit), it_hi = (int)((long)(split + 1) * L * p.nblk / nsplit);
+  const int o_lo = it_lo / p.nblk, kb_lo = it_lo - o_lo * p.nblk;
   const TcGeom geo = tc_geom(OP, p.nb, p.fi, p.fo);
   const int RI = geo.RI, CW = geo.CW;
   const int M = L * RI, Np = L * CW;
@@ -284,7 +299,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   const int row0 = (int)(t / tiles_n) * kTcBM, col0 = (int)(t % tiles_n) * kTcBN;
   const long spec0 = (long)l * (4L * l * l - 1) / 3;
   const int fi2 = 2 * p.fi, fo2 = 2 * p.fo;
-  const int nit = (o_hi - o_lo) * p.nblk;                 // K blocks of this CTA
+  const int nit = it_hi - it_lo;                          // K blocks of this CTA
   // accumulator groups (one when the whole chain stays in the tensor core's accumulator)
   const int ngroups = FLUSH ? (nit + kTcFlushBlocks - 1) / kTcFlushBlocks : 1;
 
@@ -336,7 +351,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     constexpr int kStepsMax = kTcKMax / 8;
     const int steps_full = (p.kblk + 7) / 8;
     const int steps_tail = (p.run - (p.nblk - 1) * p.kblk + 7) / 8;
-    int kb = 0, s = 0, g = 0, ing = 0;           // block within its run, stage, group, block within its group
+    int kb = kb_lo, s = 0, g = 0, ing = 0;           // block within its run, stage, group, block within its group
     uint32_t full_par = 0;                        // parity of the `full` phase of the current round of stages
     for (int it = 0; it < nit && !*abort_flag; ++it) {
       if (FLUSH && ing == 0 && g >= 2)            // the collectors are done with this accumulator
@@ -485,8 +500,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
       return make_float4(u.x, u.y, w.x, w.y);
     };
     // the cursor of the loads runs two K blocks ahead of the one being staged
-    long cur_a = 0, cur_b = 0;
-    int cur_kb = 0;
+    long cur_a = kb_lo * a_stepk, cur_b = kb_lo * b_stepk;
+    int cur_kb = kb_lo;
     unsigned validA = 0, validB = 0;      // bit q: slot q has a source address at all
 #pragma unroll
     for (int q = 0; q < kSlots; ++q) {
@@ -619,9 +634,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
 #pragma unroll
       for (int c2 = 0; c2 < 16; ++c2) {
         const int gcol = col0 + cbase + 2 * c2;
-        if (gcol < Np)
-          *reinterpret_cast<float2*>(p.c + (long)r * p.c_rs + (long)(gcol >> 1) * p.c_ps) =
-              make_float2(v[2 * c2], v[2 * c2 + 1]);
+        if (gcol < Np) {
+          float* dst = p.c + (long)r * p.c_rs + (long)(gcol >> 1) * p.c_ps;
+          if (nsplit > 1) tc_red2(dst, v[2 * c2], v[2 * c2 + 1]);
+          else *reinterpret_cast<float2*>(dst) = make_float2(v[2 * c2], v[2 * c2 + 1]);
+        }
       }
     } else if (r < M) {
       if (VEC && nsplit == 1 && CW % 8 == 0 && reinterpret_cast<unsigned long long>(p.c) % 32 == 0) {
@@ -647,8 +664,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
             const int co = gcol / CW, rem = gcol - co * CW;
             float* dst = p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem;
             if (nsplit > 1) {
-#pragma unroll
-              for (int u = 0; u < 4; ++u) atomicAdd(dst + u, v[4 * c4 + u]);
+              tc_red4(dst, v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
             } else {
               *reinterpret_cast<float4*>(dst) =
                   make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
@@ -663,8 +679,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
             const int co = gcol / CW, rem = gcol - co * CW;
             float* dst = p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem;
             if (nsplit > 1) {
-              atomicAdd(dst, v[2 * c2]);
-              atomicAdd(dst + 1, v[2 * c2 + 1]);
+              tc_red2(dst, v[2 * c2], v[2 * c2 + 1]);
             } else {
               *reinterpret_cast<float2*>(dst) = make_float2(v[2 * c2], v[2 * c2 + 1]);
             }
@@ -686,6 +701,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   }
 }
 
+// One product: picks the instantiation (see FLUSH, VEC above).
+#if defined(S2C_SPLIT) && !defined(S2C_PART)
+template <int OP>
+int launch_so3_mm_tc(const char* name, long tiles, bool flush, bool vec, stream_t st, const MmTcParams& p);
+#else
+template <int OP>
+int launch_so3_mm_tc(const char* name, long tiles, bool flush, bool vec, stream_t st, const MmTcParams& p) {
+  if (flush)
+    return vec ? launch_impl<so3_mm_tc_kernel<OP, true, true>>(name, tiles, kTcThreads, kTcSmemBytes, st, p)
+               : launch_impl<so3_mm_tc_kernel<OP, true, false>>(name, tiles, kTcThreads, kTcSmemBytes, st, p);
+  return vec ? launch_impl<so3_mm_tc_kernel<OP, false, true>>(name, tiles, kTcThreads, kTcSmemBytes, st, p)
+             : launch_impl<so3_mm_tc_kernel<OP, false, false>>(name, tiles, kTcThreads, kTcSmemBytes, st, p);
+}
+#endif
+
 // 16-byte accesses need the run of the contraction index and the column width to be multiples of 4
 // floats: fwd and grad x: f_in and f_out even; grad y: batch and f_out even.  Other sizes take the
 // 8-byte variant.
@@ -694,11 +724,39 @@ inline bool so3_mm_tc_vec16(int op, int nb, int fi, int fo) {
   return (fi % 2 == 0) && (fo % 2 == 0);
 }
 
-inline long so3_mm_tc_tiles(int op, int nl, int nb, int fi, int fo, int ksplit = 1) {
+inline long so3_mm_tc_tiles(int op, int nl, int nb, int fi, int fo, int nblk, int kper) {
   long t = 0;
-  for (int l = 0; l < nl; ++l)
-    t += tc_tiles_for(op, nb, fi, fo, l) * (ksplit < 2 * l + 1 ? ksplit : 2 * l + 1);
+  for (int l = 0; l < nl; ++l) t += tc_tiles_for(op, nb, fi, fo, l) * tc_splits(l, nblk, kper);
   return t;
+}
+
+constexpr int kTcNoSplit = 1 << 30;
+
+// K blocks per CTA.  One CTA fits on an SM; a product with few output tiles and a long contraction (the
+// transposed kernel transform of a layer with few channels: one or two tiles of several hundred K
+// blocks; the gradients of small batches) leaves most of the 148 SMs idle for the length of the longest
+// tile.  Estimate of the makespan in K blocks: the longest CTA or the average load of an SM, where a
+// CTA costs kCta blocks on top of its own (set-up, pipeline fill, epilogue: about 6 us against 0.6 us a
+// block) and sharing costs another kShare (clearing the output, atomic adds).  The split is taken only
+// where the estimate drops by a tenth, so that large products keep one CTA per tile.
+inline int tc_pick_kper(int op, int nl, int nb, int fi, int fo, int nblk) {
+  constexpr double kCta = 8, kShare = 4;
+  auto estimate = [&](int kper) {
+    double load = 0, longest = 0;
+    for (int l = 0; l < nl; ++l) {
+      const int blocks = (2 * l + 1) * nblk, ns = tc_splits(l, nblk, kper);
+      load += (double)tc_tiles_for(op, nb, fi, fo, l) * (blocks + ns * kCta);
+      longest = std::max(longest, (double)((blocks + ns - 1) / ns));
+    }
+    return std::max(longest + kCta, load / 148) + (kper == kTcNoSplit ? 0 : kShare);
+  };
+  int best = kTcNoSplit;
+  double t = 0.9 * estimate(best);
+  for (int kper = 4; kper < (2 * nl - 1) * nblk; kper += (kper + 3) / 4) {
+    const double e = estimate(kper);
+    if (e < t) { t = e; best = kper; }
+  }
+  return best;
 }
 
 }  // namespace s2c

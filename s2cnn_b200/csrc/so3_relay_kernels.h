@@ -397,6 +397,7 @@ __global__ void __launch_bounds__(256, 3) so3_relay_fused(const RelayParams p) {
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
   so3_relay_fused_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
 }
+S2C_LAUNCHER_N(so3_relay_fused, RelayParams)
 #endif
 
 }  // namespace s2c

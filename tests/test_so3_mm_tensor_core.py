@@ -121,3 +121,26 @@ def test_kernel_transform_on_tensor_cores_matches_fp32_kernel_and_oracle(nf, ng,
         assert_close(ops.rft_backward(gd, Fd), want_b, "rft backward FP32 kernel")
     finally:
         _lib.cuda_lib().s2c_debug_force_general_path(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nl,nb,fi,fo", [(1, 1, 1, 1), (2, 1, 3, 2), (7, 5, 13, 9), (12, 2, 16, 16), (15, 4, 16, 24)])
+def test_products_shared_by_several_ctas(nl, nb, fi, fo):
+    """Few output tiles and a long contraction: the K blocks of a tile are split over CTAs (both gradients
+    and the transposed kernel transform), from a single block to hundreds, the last slice ragged."""
+    from s2cnn_b200 import _lib
+    from s2cnn_b200.ops import cuda_ops
+    ops = cuda_ops()
+    gen = torch.Generator().manual_seed(nl + fo)
+    x = torch.randn(n3(nl), nb, fi, 2, generator=gen)
+    y = torch.randn(n3(nl), fi, fo, 2, generator=gen)
+    gz = torch.randn(n3(nl), nb, fo, 2, generator=gen)
+    ref_gx, ref_gy = _grad_reference(x, y, gz, nl)
+    assert_close(ops.so3_mm_gradx(gz.cuda(), y.cuda(), nb, fi), ref_gx, "grad x")
+    assert_close(ops.so3_mm_grady(gz.cuda(), x.cuda(), fo), ref_gy, "grad y")
+    for ng in (6, 36):
+        F = torch.randn(ng, n3(nl), 2, generator=gen)
+        g = torch.randn(n3(nl), fi * fo, 2, generator=gen)
+        want = torch.einsum("sfc,asc->fa", g.double(), F.double()).float()
+        assert_close(ops.rft_backward(g.cuda(), F.cuda()), want, "rft backward")
+    assert _lib.cuda_lib().s2c_so3_mm_tc_status() == 0
