@@ -17,6 +17,7 @@
 #include "s2_fused_kernels.h"
 #include "so3_fused_kernels.h"
 #include "so3_relay_kernels.h"
+#include "so3_mid_kernels.h"
 #include "wigner_tiled.h"
 #include "wigner_rows.h"
 #include "cgemm_kernels.h"
@@ -103,6 +104,22 @@ static int plane_pipeline(long nbatch, int N, int K, void* ws, size_t ws_bytes, 
   return S2C_OK;
 }
 
+// 32 < N < 64: a plane kernel (so3_mid_kernels.h) and a tiled Wigner kernel per direction through
+// V[n][m][z][beta].  Signals per chunk: whole tiles of the Wigner kernel, as many as keep V in L2
+// (N = 60, K = 30: 0.85 MB per signal, 64 signals), within the workspace.
+static size_t so3_mid_v_per_z(int N, int K) { return (size_t)K * (2 * K - 1) * N * sizeof(float2); }
+static bool use_mid_kernels(int N) { return mid_supported(N) && g_force_general < 2; }
+static int mid_chunk(long nbatch, int N, int K, const void* ws, size_t ws_bytes, long* chunk) {
+  const size_t vz = so3_mid_v_per_z(N, K);
+  const long fit = ws ? (long)(ws_bytes / vz) : 0;
+  if (fit < 1)
+    return fail(S2C_ERR_WORKSPACE, "workspace smaller than one batch element (" + std::to_string(vz) +
+                                       " bytes needed)");
+  const long l2 = std::max(1L, (long)(((size_t)64 << 20) / vz) / kWigZT) * kWigZT;
+  *chunk = std::min(nbatch, std::min(fit, l2));
+  return S2C_OK;
+}
+
 static int check_b(int b_in, int b_out) {
   if (b_in < 1 || b_out < 1) return fail(S2C_ERR_BAD_ARG, "bandwidths must be >= 1");
   return S2C_OK;
@@ -159,18 +176,32 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
     };
     return plane_pipeline(nbatch, N, K, ws, ws_bytes, st, planes, wigner);
   }
+  const bool mid = use_mid_kernels(N);
   const size_t per_z = so3_ws_per_z(N, K);
   long chunk = (long)std::min<size_t>((size_t)nbatch, ws_bytes / per_z);
-  if (chunk < 1 || ws == nullptr)
+  if (mid) {
+    S2C_TRY(mid_chunk(nbatch, N, K, ws, ws_bytes, &chunk));
+  } else if (chunk < 1 || ws == nullptr) {
     return fail(S2C_ERR_WORKSPACE, "workspace smaller than one batch element (" +
                                        std::to_string(per_z) + " bytes needed)");
+  }
   const int G = fft_group(N, N), Gg = fft_group(N, N / 2);  // alpha passes, gamma passes
   const size_t fft_smem = fft_smem_bytes(N, G);
   for (long z0 = 0; z0 < nbatch; z0 += chunk) {
     const long zc = std::min(chunk, nbatch - z0);
     float2* u = (float2*)ws;
-    float2* v = u + (size_t)zc * K * N * N;
-    {
+    float2* v = mid ? u : u + (size_t)zc * K * N * N;
+    if (mid) {
+      MidParams g;
+      g.x = x + (size_t)z0 * N * N * N * in_stride; g.out = nullptr;
+      g.stride = in_stride; g.off = in_off;
+      g.v = v; g.tw = fft.tw; g.bias = nullptr; g.nfeat = 1; g.z0 = z0;
+      g.nbatch = (int)zc; g.K = K; g.inv_k = 1.f / (float)K;
+      int rc = S2C_OK;
+      S2C_DISPATCH_MID(N, rc = S2C_LAUNCH_N(so3_fwd_mid, kN, zc * ((kN + mid_nb(kN) - 1) / mid_nb(kN)),
+                                            kMidThreads, mid_smem_bytes(kN), st, g));
+      if (rc) return rc;
+    } else {
     FwdGammaParams g;
     g.x = x + (size_t)z0 * N * N * N * in_stride;
     g.in_stride = in_stride;
@@ -296,17 +327,21 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     };
     return plane_pipeline(nbatch, N, K, ws, ws_bytes, st, wigner, planes);
   }
+  const bool mid = use_mid_kernels(N);
   const size_t per_z = so3_ws_per_z(N, K);
   long chunk = (long)std::min<size_t>((size_t)nbatch, ws_bytes / per_z);
-  if (chunk < 1 || ws == nullptr)
+  if (mid) {
+    S2C_TRY(mid_chunk(nbatch, N, K, ws, ws_bytes, &chunk));
+  } else if (chunk < 1 || ws == nullptr) {
     return fail(S2C_ERR_WORKSPACE, "workspace smaller than one batch element (" +
                                        std::to_string(per_z) + " bytes needed)");
+  }
   const int G = fft_group(N, N), Gg = fft_group(N, N / 2);  // alpha passes, gamma passes
   const size_t fft_smem = fft_smem_bytes(N, G);
   for (long z0 = 0; z0 < nbatch; z0 += chunk) {
     const long zc = std::min(chunk, nbatch - z0);
     float2* t = (float2*)ws;                                   // [z][K][N][N]
-    float2* s = t + (size_t)zc * K * N * N;                    // [K][2K-1][z][N]
+    float2* s = mid ? t : t + (size_t)zc * K * N * N;          // [K][2K-1][z][N]
     InvWignerParams w;
     w.x = x + z0;
     w.x_zstride = nbatch;
@@ -324,6 +359,18 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     } else {
       const size_t wsm = align_up((size_t)K * N * sizeof(float), 16) + (size_t)K * w.ZT * sizeof(float2);
       S2C_TRY(S2C_LAUNCH(so3_inv_wigner, (long)pan.npairs * w.nzt, kThreads, wsm, st, w));
+    }
+    if (mid) {
+      MidParams g;
+      g.x = nullptr; g.out = out + (size_t)z0 * N * N * N * out_stride;
+      g.stride = out_stride; g.off = out_off;
+      g.v = s; g.tw = fft.tw; g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0;
+      g.nbatch = (int)zc; g.K = K; g.inv_k = 1.f / (float)K;
+      int rc = S2C_OK;
+      S2C_DISPATCH_MID(N, rc = S2C_LAUNCH_N(so3_inv_mid, kN, zc * ((kN + mid_nb(kN) - 1) / mid_nb(kN)),
+                                            kMidThreads, mid_smem_bytes(kN), st, g));
+      if (rc) return rc;
+      continue;
     }
     InvAlphaParams a;
     a.s = s;

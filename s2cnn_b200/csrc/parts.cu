@@ -11,6 +11,7 @@
 #include "so3_kernels.h"
 #include "so3_fused_kernels.h"
 #include "so3_relay_kernels.h"
+#include "so3_mid_kernels.h"
 #include "so3_mm_tc.h"
 
 namespace s2c {
@@ -19,6 +20,9 @@ namespace s2c {
   template int launch_so3_inv_fused<N>(long, int, size_t, stream_t, const InvFusedParams&);          \
   template int launch_so3_fwd_fused<N>(long, int, size_t, stream_t, const FwdFusedParams&);          \
   template int launch_so3_relay_fused<N>(long, int, size_t, stream_t, const RelayParams&);
+#define S2C_MID(N)                                                                  \
+  template int launch_so3_fwd_mid<N>(long, int, size_t, stream_t, const MidParams&); \
+  template int launch_so3_inv_mid<N>(long, int, size_t, stream_t, const MidParams&);
 #define S2C_TC_OP(OP) \
   template int launch_so3_mm_tc<OP>(const char*, long, bool, bool, stream_t, const MmTcParams&);
 
@@ -40,6 +44,12 @@ S2C_LENGTH(20) S2C_LENGTH(16) S2C_LENGTH(18)
 S2C_TC_OP(kTcFwd) S2C_TC_OP(kTcGradX)
 #elif S2C_PART == 8
 S2C_TC_OP(kTcGradY) S2C_TC_OP(kTcPlainCC) S2C_TC_OP(kTcPlainSC)
+#elif S2C_PART == 9
+S2C_MID(34) S2C_MID(38) S2C_MID(46) S2C_MID(58) S2C_MID(62)
+#elif S2C_PART == 10
+S2C_MID(36) S2C_MID(40) S2C_MID(42) S2C_MID(44) S2C_MID(48)
+#elif S2C_PART == 11
+S2C_MID(50) S2C_MID(52) S2C_MID(54) S2C_MID(56) S2C_MID(60)
 #endif
 
 }  // namespace s2c
