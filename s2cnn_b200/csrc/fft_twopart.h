@@ -39,6 +39,19 @@ S2C_HD constexpr int two_block_freq(int n, int r1, int b) {
   return f;
 }
 
+// ... and the block whose frequencies are f + r1 q (f < r1)
+S2C_HD constexpr int two_freq_block(int n, int r1, int f) {
+  int len = n, span = r1, b = 0;
+  while (span > 1) {
+    const int r = two_radix(len);
+    len /= r;
+    span /= r;
+    b += (f % r) * span;
+    f /= r;
+  }
+  return b;
+}
+
 // a * w^DIR with the roundings spelled out: which of the two products of a component is fused into the
 // addition is the compiler's choice in ctw() (and changes with constant operands), but it decides the last
 // bit, and a training step of a deep network amplifies last bits through its ReLUs and batch

@@ -14,10 +14,10 @@
 #include "fft_device.h"
 #include "so3_kernels.h"
 #include "so3_plane_kernels.h"
-#include "s2_fused_kernels.h"
 #include "so3_fused_kernels.h"
 #include "so3_relay_kernels.h"
 #include "so3_mid_kernels.h"
+#include "s2_kernels.h"
 #include "wigner_tiled.h"
 #include "wigner_rows.h"
 #include "cgemm_kernels.h"
@@ -229,7 +229,7 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
     w.ZT = (int)std::min<long>(32, zc);
     w.nzt = (int)((zc + w.ZT - 1) / w.ZT);
     w.mode = mode;
-    if (N % (4 * kWigHalves) == 0 && fwd_wigner_t_smem(N, b_out) <= (size_t)dev_smem_limit() - 1024) {
+    if (fwd_wigner_t_fits(N, b_out, kWigZT, dev_smem_limit())) {
       w.ZT = kWigZT;
       w.nzt = (int)((zc + kWigZT - 1) / kWigZT);
       S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)pan.npairs * w.nzt, kThreads,
@@ -351,7 +351,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     w.ZT = (int)std::min<long>(32, zc);
     w.nzt = (int)((zc + w.ZT - 1) / w.ZT);
     w.mode = mode;
-    if (N % 4 == 0 && inv_wigner_t_smem(N, K) <= (size_t)dev_smem_limit() - 1024) {
+    if (inv_wigner_t_smem(N, K) <= (size_t)dev_smem_limit() - 1024) {
       w.ZT = kWigZT;
       w.nzt = (int)((zc + kWigZT - 1) / kWigZT);
       S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)pan.npairs * w.nzt, kThreads,
@@ -780,22 +780,37 @@ int s2c_s2_fft(const float* x, int x_is_real, float* out, long nbatch, int b_in,
   stream_t st = as_stream(stream);
   const int N = 2 * b_in, K = b_out;
   FftDev fft;
-  PanelsDev pan;
   S2C_TRY(TableCache::get().fft(N, fft));
-  S2C_TRY(TableCache::get().panels(b_in, b_out, K, !for_grad, true, pan));
-  if (!g_force_general && x_is_real && N % 2 == 0 && s2_fwd_fused_smem(N) <= 96 * 1024) {
-    // real signal whose packed half plane fits in shared memory: one kernel, no scratch
+  // A real signal with few degrees: one kernel, no scratch (a block reads the whole table of K^2 N
+  // values for its signal; from K = 33 on the tiled contraction, which shares panels, is the faster one).
+  if (!g_force_general && x_is_real && K <= kS2FusedK && s2_length(N) && N < 128) {
     S2FwdFusedParams f;
     f.x = x; f.out = (float2*)out; f.out_zstride = nbatch;
-    f.pan = pan; f.fft = fft; f.N = N; f.K = K;
-    return S2C_LAUNCH(s2_fwd_fused, nbatch, kThreads, s2_fwd_fused_smem(N), st, f);
+    f.tw = fft.tw; f.K = K;
+    S2C_TRY(TableCache::get().s2_transposed(b_in, b_out, !for_grad, &f.wt));
+    return s2_dispatch<1, 64>(N, [&](auto nc) {
+      constexpr int kN = decltype(nc)::value;
+      return S2C_LAUNCH_N(s2_fwd_fused, kN, nbatch, 256, s2_fwd_fused_smem(kN, K), st, f);
+    });
   }
+  PanelsDev pan;
+  S2C_TRY(TableCache::get().panels(b_in, b_out, K, !for_grad, true, pan));
   const size_t per_z = s2_ws_per_z(N, K);
   long chunk = (long)std::min<size_t>((size_t)nbatch, ws_bytes / per_z);
   if (chunk < 1 || !ws) return fail(S2C_ERR_WORKSPACE, "s2c_s2_fft: workspace too small");
   const int G = fft_group(N, N), Gg = fft_group(N, N / 2);  // alpha passes, gamma passes
   for (long z0 = 0; z0 < nbatch; z0 += chunk) {
     const long zc = std::min(chunk, nbatch - z0);
+    if (!g_force_general && s2_length(N)) {
+      S2RowsParams r;
+      r.x = x + (size_t)z0 * N * N * (x_is_real ? 1 : 2); r.out = nullptr;
+      r.complex = !x_is_real; r.v = (float2*)ws; r.tw = fft.tw;
+      r.nbatch = (int)zc; r.K = K;
+      S2C_TRY((s2_dispatch<1, 64>(N, [&](auto nc) {
+        constexpr int kN = decltype(nc)::value;
+        return S2C_LAUNCH_N(s2_fwd_rows, kN, zc * s2_rows_groups(kN), 256, s2_fwd_rows_smem(kN), st, r);
+      })));
+    } else {
     FwdAlphaParams a;
     a.in = x + (size_t)z0 * N * N * (x_is_real ? 1 : 2);
     a.in_real = x_is_real ? 1 : 0;
@@ -804,6 +819,7 @@ int s2c_s2_fft(const float* x, int x_is_real, float* out, long nbatch, int b_in,
     a.nrows = zc * N;
     a.fft = fft;
     S2C_TRY(S2C_LAUNCH(so3_fwd_alpha, (a.nrows + G - 1) / G, kThreads, fft_smem_bytes(N, G), st, a));
+    }
     FwdWignerParams w;
     w.v = (const float2*)ws;
     w.out = (float2*)out + z0;
@@ -813,6 +829,13 @@ int s2c_s2_fft(const float* x, int x_is_real, float* out, long nbatch, int b_in,
     w.ZT = (int)std::min<long>(32, zc);
     w.nzt = (int)((zc + w.ZT - 1) / w.ZT);
     w.mode = kS2;
+    if (const int zt = wig_s2_zt(pan.npairs, zc); fwd_wigner_t_fits(N, b_out, zt, dev_smem_limit())) {
+      w.ZT = zt;
+      w.nzt = (int)((zc + zt - 1) / zt);
+      S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)pan.npairs * w.nzt, kThreads,
+                         fwd_wigner_t_smem(N, b_out, zt), st, w));
+      continue;
+    }
     const size_t wsm = align_up((size_t)b_out * (N + 1) * sizeof(float), 16) +
                        (size_t)w.ZT * (N + 1) * sizeof(float2);
     S2C_TRY(S2C_LAUNCH(so3_fwd_wigner, (long)pan.npairs * w.nzt, kThreads, wsm, st, w));
@@ -846,8 +869,26 @@ int s2c_s2_ifft(const float* x, float* out, int out_is_real, long nbatch, int b_
     w.ZT = (int)std::min<long>(32, zc);
     w.nzt = (int)((zc + w.ZT - 1) / w.ZT);
     w.mode = kS2;
-    const size_t wsm = align_up((size_t)K * N * sizeof(float), 16) + (size_t)K * w.ZT * sizeof(float2);
-    S2C_TRY(S2C_LAUNCH(so3_inv_wigner, (long)pan.npairs * w.nzt, kThreads, wsm, st, w));
+    if (const int zt = wig_s2_zt(pan.npairs, zc); inv_wigner_t_smem(N, K, zt) <= (size_t)dev_smem_limit() - 1024) {
+      w.ZT = zt;
+      w.nzt = (int)((zc + zt - 1) / zt);
+      S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)pan.npairs * w.nzt, kThreads,
+                         inv_wigner_t_smem(N, K, zt), st, w));
+    } else {
+      const size_t wsm = align_up((size_t)K * N * sizeof(float), 16) + (size_t)K * w.ZT * sizeof(float2);
+      S2C_TRY(S2C_LAUNCH(so3_inv_wigner, (long)pan.npairs * w.nzt, kThreads, wsm, st, w));
+    }
+    if (!g_force_general && s2_length(N)) {
+      S2RowsParams r;
+      r.x = nullptr; r.out = out + (size_t)z0 * N * N * (out_is_real ? 1 : 2);
+      r.complex = !out_is_real; r.v = (float2*)ws; r.tw = fft.tw;
+      r.nbatch = (int)zc; r.K = K;
+      S2C_TRY((s2_dispatch<1, 64>(N, [&](auto nc) {
+        constexpr int kN = decltype(nc)::value;
+        return S2C_LAUNCH_N(s2_inv_rows, kN, zc * s2_rows_groups(kN), 256, s2_inv_rows_smem(kN), st, r);
+      })));
+      continue;
+    }
     InvAlphaParams a;
     a.s = (const float2*)ws;
     a.out = out + (size_t)z0 * N * N * (out_is_real ? 1 : 2);

@@ -12,6 +12,7 @@
 #include "so3_fused_kernels.h"
 #include "so3_relay_kernels.h"
 #include "so3_mid_kernels.h"
+#include "s2_kernels.h"
 #include "so3_mm_tc.h"
 
 namespace s2c {
@@ -25,6 +26,11 @@ namespace s2c {
   template int launch_so3_inv_mid<N>(long, int, size_t, stream_t, const MidParams&);
 #define S2C_TC_OP(OP) \
   template int launch_so3_mm_tc<OP>(const char*, long, bool, bool, stream_t, const MmTcParams&);
+
+#define S2C_S2(N)                                                                          \
+  template int launch_s2_fwd_fused<N>(long, int, size_t, stream_t, const S2FwdFusedParams&); \
+  template int launch_s2_fwd_rows<N>(long, int, size_t, stream_t, const S2RowsParams&);      \
+  template int launch_s2_inv_rows<N>(long, int, size_t, stream_t, const S2RowsParams&);
 
 #if S2C_PART == 0
 S2C_LENGTH(32)
@@ -50,6 +56,18 @@ S2C_MID(34) S2C_MID(38) S2C_MID(46) S2C_MID(58) S2C_MID(62)
 S2C_MID(36) S2C_MID(40) S2C_MID(42) S2C_MID(44) S2C_MID(48)
 #elif S2C_PART == 11
 S2C_MID(50) S2C_MID(52) S2C_MID(54) S2C_MID(56) S2C_MID(60)
+#elif S2C_PART == 12
+S2C_S2(2) S2C_S2(4) S2C_S2(18) S2C_S2(20) S2C_S2(34) S2C_S2(36) S2C_S2(50) S2C_S2(52) S2C_S2(66)
+S2C_S2(68) S2C_S2(88) S2C_S2(90) S2C_S2(108) S2C_S2(110) S2C_S2(128)
+#elif S2C_PART == 13
+S2C_S2(6) S2C_S2(16) S2C_S2(22) S2C_S2(32) S2C_S2(38) S2C_S2(48) S2C_S2(54) S2C_S2(64) S2C_S2(70)
+S2C_S2(84) S2C_S2(92) S2C_S2(104) S2C_S2(112) S2C_S2(126)
+#elif S2C_PART == 14
+S2C_S2(8) S2C_S2(14) S2C_S2(24) S2C_S2(30) S2C_S2(40) S2C_S2(46) S2C_S2(56) S2C_S2(62) S2C_S2(72)
+S2C_S2(80) S2C_S2(96) S2C_S2(102) S2C_S2(114) S2C_S2(124)
+#elif S2C_PART == 15
+S2C_S2(10) S2C_S2(12) S2C_S2(26) S2C_S2(28) S2C_S2(42) S2C_S2(44) S2C_S2(58) S2C_S2(60) S2C_S2(76)
+S2C_S2(78) S2C_S2(98) S2C_S2(100) S2C_S2(116) S2C_S2(120)
 #endif
 
 }  // namespace s2c

@@ -421,6 +421,33 @@ class TableCache {
     return S2C_OK;
   }
 
+  // S2 panels transposed for the single-kernel analysis: [beta][l * l + l + m], so that threads that own
+  // neighbouring coefficients read neighbouring values.
+  int s2_transposed(int b_beta, int nl, bool weighted, const float** out) {
+    std::lock_guard<std::mutex> g(mu_);
+    auto key = std::make_tuple(dev_current(), b_beta, nl, (int)weighted);
+    auto it = s2t_.find(key);
+    if (it == s2t_.end()) {
+      std::vector<float> data;
+      std::vector<long long> off;
+      build_panels(b_beta, nl, nl, weighted, true, data, off);
+      const int nbeta = 2 * b_beta, kk = nl * nl;
+      std::vector<float> t((size_t)nbeta * kk);
+      for (int l = 0; l < nl; ++l)
+        for (int m = -l; m <= l; ++m) {
+          const float* row = data.data() + off[m + nl - 1] + (size_t)(l - std::abs(m)) * nbeta;
+          for (int j = 0; j < nbeta; ++j) t[(size_t)j * kk + l * l + l + m] = row[j];
+        }
+      void* d = dev_alloc(t.size() * sizeof(float));
+      if (!d) return fail(S2C_ERR_CUDA, "table allocation failed");
+      const int rc = dev_upload(d, t.data(), t.size() * sizeof(float));
+      if (rc) return rc;
+      it = s2t_.emplace(key, (const float*)d).first;
+    }
+    *out = it->second;
+    return S2C_OK;
+  }
+
   int quad_weights(int b, const float** out) {
     std::lock_guard<std::mutex> g(mu_);
     const int dev = dev_current();
@@ -453,6 +480,8 @@ class TableCache {
     for (auto& kv : quad_) dev_free((void*)kv.second);
     for (auto& kv : grouped_) dev_free((void*)kv.second.first);
     for (auto& kv : half_) { dev_free((void*)kv.second.first); dev_free((void*)kv.second.second); }
+    for (auto& kv : s2t_) dev_free((void*)kv.second);
+    s2t_.clear();
     half_.clear();
     grouped_.clear();
     fft_.clear();
@@ -465,6 +494,7 @@ class TableCache {
   std::map<std::pair<int, int>, FftDev> fft_;
   std::map<std::tuple<int, int, int, int, int, int>, PanelsDev> panels_;
   std::map<std::pair<int, int>, const float*> quad_;
+  std::map<std::tuple<int, int, int, int>, const float*> s2t_;
   std::map<std::tuple<int, int, int, int, int, int>, std::pair<const float*, int>> grouped_;
   std::map<std::tuple<int, int, int, int, int, int>, std::pair<const float*, const long long*>> half_;
 };

@@ -13,37 +13,47 @@
 
 namespace s2c {
 
-constexpr int kWigZT = 64;  // batch elements per block tile (even)
-constexpr int kWigHalves = 1;  // pieces of the beta range in the forward contraction
+constexpr int kWigZT = 64;  // batch elements per block tile (even): SO(3), and the most for S2
 
-inline size_t fwd_wigner_t_smem(int N, int nl) {
-  return (size_t)((nl + 3) / 4 * 4) * (N / kWigHalves + 4) * sizeof(float) +
-         (size_t)kWigZT * (N / kWigHalves + 2) * sizeof(float2);
+// Rows of N mod 4 = 2 betas are staged with two columns of zeros.
+S2C_HD constexpr int wig_np(int N) { return (N + 3) / 4 * 4; }
+inline size_t fwd_wigner_t_smem(int N, int nl, int zt = kWigZT) {
+  return (size_t)((nl + 3) / 4 * 4) * (wig_np(N) + 4) * sizeof(float) +
+         (size_t)zt * (wig_np(N) + 2) * sizeof(float2);
+}
+// the kernels take 4 x 2 (or 4 x 1) outputs per thread and tile, two tiles per thread
+inline bool fwd_wigner_t_fits(int N, int nl, int zt, int smem_limit) {
+  return (nl + 3) / 4 * ((zt + 1) / 2) <= 2 * kThreads && fwd_wigner_t_smem(N, nl, zt) <= (size_t)smem_limit - 1024;
+}
+// Batch elements per block for the S2 transforms: only 2K - 1 table panels exist, so small batches take
+// smaller tiles until about two blocks per SM are there.
+inline int wig_s2_zt(int npairs, long nbatch) {
+  int zt = kWigZT;
+  while (zt > 8 && npairs * ((nbatch + zt - 1) / zt) < 2 * 148) zt /= 2;
+  return zt;
 }
 
 // X[l][z] = sum_beta W[l][beta] V[z][beta]   (+ Hermitian mirror row)
 //
-// The beta range can be processed in kWigHalves pieces with the accumulators kept in registers
-// (less shared memory per block, more blocks per SM); one piece is the faster setting.  Panel rows
-// and batch rows are staged exactly as they lie in memory (16-byte copies, no transposition): the
-// beta loop runs four samples at a time, a thread reads W[l][beta..beta+3] for its four degrees
-// (the whole warp shares the address: broadcast) and V[z][beta..beta+3] for its two batch elements
-// z = tz and tz + ceil(zc/2) (row stride N + 2 complex numbers, so the 8 lanes of a 16-byte access phase
-// hit 8 different bank groups).
+// Panel rows and batch rows are staged exactly as they lie in memory (no transposition): the beta loop
+// runs four samples at a time, a thread reads W[l][beta..beta+3] for its four degrees (the whole warp
+// shares the address: broadcast) and V[z][beta..beta+3] for its two batch elements z = tz and
+// tz + ceil(zc/2) (row stride N + 2 complex numbers, so the 8 lanes of a 16-byte access phase hit 8
+// different bank groups).  S2 transforms (kS2) are the n = 0 column without mirror rows.
 S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
-  const int N = p.N, NH = N / kWigHalves;
+  const int N = p.N, NH = wig_np(N);
   const int pair = ctx.bid / p.nzt, zt = ctx.bid - pair * p.nzt;
   int m, n;
-  so3_pair_decode(pair, p.K, m, n);
+  if (p.mode == kS2) { m = pair - (p.K - 1); n = 0; } else so3_pair_decode(pair, p.K, m, n);
   const int am = m < 0 ? -m : m;
   const int lmin = am > n ? am : n;
   const int L = p.nl - lmin;
   if (L <= 0) return;
-  const int z0 = zt * kWigZT;
-  const int zc = (p.nbatch - z0) < kWigZT ? (p.nbatch - z0) : kWigZT;
+  const int z0 = zt * p.ZT;
+  const int zc = (p.nbatch - z0) < p.ZT ? (p.nbatch - z0) : p.ZT;
   const int LDW = NH + 4, LDV = NH + 2, ZH = (zc + 1) / 2;   // a thread's batch elements: tz, tz + ZH
   float* Ws = reinterpret_cast<float*>(smem);                                        // [nl up to 4][LDW]
-  float2* Vs = reinterpret_cast<float2*>(Ws + (size_t)((p.nl + 3) / 4 * 4) * LDW);    // [kWigZT][LDV]
+  float2* Vs = reinterpret_cast<float2*>(Ws + (size_t)((p.nl + 3) / 4 * 4) * LDW);    // [ZT][LDV]
   const int LT = (L + 3) / 4;
   const float* panel = p.pan.data + p.pan.off[pair];
   const int nm = 2 * p.K - 1, mi = m + p.K - 1;
@@ -58,9 +68,8 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) { ar[t][i][0] = ar[t][i][1] = ai[t][i][0] = ai[t][i][1] = 0.f; }
 
-  for (int half = 0; half < kWigHalves; ++half) {
-    if (half) ctx.sync();
-    {
+  {
+    if (N % 4 == 0) {
       const int n4 = NH / 4, total = LT * 4 * n4;                    // rows past L are zero
       for (int base = ctx.tid; base < total; base += 4 * ctx.nthr) {
         float4 v[4];
@@ -70,7 +79,7 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
           v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (idx < total && idx / n4 < L) {
             const int l = idx / n4, c4 = idx - l * n4;
-            v[u] = *reinterpret_cast<const float4*>(panel + (long)l * N + half * NH + 4 * c4);
+            v[u] = *reinterpret_cast<const float4*>(panel + (long)l * N + 4 * c4);
           }
         }
 #pragma unroll
@@ -81,6 +90,14 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
             *reinterpret_cast<float4*>(Ws + l * LDW + 4 * c4) = v[u];
           }
         }
+      }
+    } else {   // panel rows start on 8-byte boundaries only
+      const int n2 = NH / 2, total = LT * 4 * n2;
+      for (int idx = ctx.tid; idx < total; idx += ctx.nthr) {
+        const int l = idx / n2, c2 = idx - l * n2;
+        float2 v = make_float2(0.f, 0.f);
+        if (l < L && 2 * c2 < N) v = *reinterpret_cast<const float2*>(panel + (long)l * N + 2 * c2);
+        *reinterpret_cast<float2*>(Ws + l * LDW + 2 * c2) = v;
       }
     }
     {
@@ -93,7 +110,7 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
           v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (idx < total && idx / n2 < zc) {
             const int zz = idx / n2, c2 = idx - zz * n2;
-            v[u] = *reinterpret_cast<const float4*>(vsrc + (long)zz * N + half * NH + 2 * c2);
+            if (2 * c2 < N) v[u] = *reinterpret_cast<const float4*>(vsrc + (long)zz * N + 2 * c2);
           }
         }
 #pragma unroll
@@ -161,6 +178,10 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
   auto emit = [&](int li, int zz, float re, float im) {
     if (li >= L || zz >= zc) return;
     const int l = lmin + li;
+    if (p.mode == kS2) {
+      p.out[((long)l * l + l + m) * p.out_zstride + z0 + zz] = make_float2(re, im);
+      return;
+    }
     float2* o1 = p.out + so3_row(l, m, n) * p.out_zstride + z0 + zz;
     float2* o2 = p.out + so3_row(l, -m, -n) * p.out_zstride + z0 + zz;
     if (p.mode == kSo3Real) {
@@ -194,28 +215,28 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
   }
 }
 
-inline size_t inv_wigner_t_smem(int N, int K) {
-  return (size_t)K * N * sizeof(float) + (size_t)K * (kWigZT + 2) * sizeof(float2);
+inline size_t inv_wigner_t_smem(int N, int K, int zt = kWigZT) {
+  return (size_t)K * wig_np(N) * sizeof(float) + (size_t)K * (zt + 2) * sizeof(float2);
 }
 
 // S[z][beta] = sum_l W[l][beta] Xs[l][z],  Xs = symmetrised spectrum
 S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
-  const int N = p.N;
+  const int N = p.N, NP = wig_np(N);
   const int pair = ctx.bid / p.nzt, zt = ctx.bid - pair * p.nzt;
   int m, n;
-  so3_pair_decode(pair, p.K, m, n);
+  if (p.mode == kS2) { m = pair - (p.K - 1); n = 0; } else so3_pair_decode(pair, p.K, m, n);
   const int am = m < 0 ? -m : m;
   const int lmin = am > n ? am : n;
   const int L = p.pan.nl - lmin;
   if (L <= 0) return;
-  const int z0 = zt * kWigZT;
-  const int zc = (p.nbatch - z0) < kWigZT ? (p.nbatch - z0) : kWigZT;
-  const int ZP = kWigZT + 2;
-  float* Ws = reinterpret_cast<float*>(smem);                            // [L][N]
-  float2* Xs = reinterpret_cast<float2*>(Ws + (size_t)p.pan.nl * N);      // [L][ZP]
+  const int z0 = zt * p.ZT;
+  const int zc = (p.nbatch - z0) < p.ZT ? (p.nbatch - z0) : p.ZT;
+  const int ZP = p.ZT + 2;
+  float* Ws = reinterpret_cast<float*>(smem);                            // [L][NP]
+  float2* Xs = reinterpret_cast<float2*>(Ws + (size_t)p.pan.nl * NP);     // [L][ZP]
   const int Z2 = (zc + 1) / 2;
   const float* panel = p.pan.data + p.pan.off[pair];
-  {
+  if (N % 4 == 0) {
     const float4* src = reinterpret_cast<const float4*>(panel);
     float4* dst4 = reinterpret_cast<float4*>(Ws);
     const int total = L * N / 4;
@@ -228,12 +249,23 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
       for (int u = 0; u < 4; ++u)
         if (base + u * ctx.nthr < total) dst4[base + u * ctx.nthr] = v[u];
     }
+  } else {   // panel rows start on 8-byte boundaries only; two columns of padding
+    const int n2 = NP / 2;
+    for (int idx = ctx.tid; idx < L * n2; idx += ctx.nthr) {
+      const int li = idx / n2, c2 = idx - li * n2;
+      float2 v = make_float2(0.f, 0.f);
+      if (2 * c2 < N) v = *reinterpret_cast<const float2*>(panel + (long)li * N + 2 * c2);
+      *reinterpret_cast<float2*>(Ws + li * NP + 2 * c2) = v;
+    }
   }
   const float fudge = ((m - n) & 1) ? -1.f : 1.f;
   for (int it = ctx.tid; it < L * Z2 * 2; it += ctx.nthr) {
     const int li = it / (Z2 * 2), zz = it - li * (Z2 * 2);
     float2 v = make_float2(0.f, 0.f);
-    if (zz < zc) {
+    if (zz < zc && p.mode == kS2) {
+      const long l = lmin + li;
+      v = p.x[(l * l + l + m) * p.x_zstride + z0 + zz];
+    } else if (zz < zc) {
       const int l = lmin + li;
       float2 a = p.x[so3_row(l, m, n) * p.x_zstride + z0 + zz];
       float2 b = p.x[so3_row(l, -m, -n) * p.x_zstride + z0 + zz];
@@ -248,7 +280,7 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
   ctx.sync();
   const int nm = 2 * p.K - 1, mi = m + p.K - 1;
   float2* dst = p.s + (((long)n * nm + mi) * p.nbatch + z0) * N;
-  const int B4 = N / 4;
+  const int B4 = NP / 4;
   for (int tile = ctx.tid; tile < B4 * Z2; tile += ctx.nthr) {
     const int tz = tile / B4, tb = tile - tz * B4;  // consecutive threads -> consecutive beta
     float ar[2][4], ai[2][4];
@@ -259,7 +291,7 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
     const float* wp = Ws + 4 * tb;
     const float2* xp = Xs + 2 * tz;
     for (int li = 0; li < L; ++li) {
-      const float4 w4 = *reinterpret_cast<const float4*>(wp + li * N);
+      const float4 w4 = *reinterpret_cast<const float4*>(wp + li * NP);
       const float4 x4 = *reinterpret_cast<const float4*>(xp + li * ZP);  // (re0, im0, re1, im1)
       const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
@@ -276,7 +308,7 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
       if (zz >= zc) continue;
       float4* o = reinterpret_cast<float4*>(dst + (long)zz * N + 4 * tb);
       o[0] = make_float4(ar[j][0], ai[j][0], ar[j][1], ai[j][1]);
-      o[1] = make_float4(ar[j][2], ai[j][2], ar[j][3], ai[j][3]);
+      if (4 * tb + 2 < N) o[1] = make_float4(ar[j][2], ai[j][2], ar[j][3], ai[j][3]);
     }
   }
 }

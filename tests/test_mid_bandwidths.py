@@ -35,7 +35,10 @@ def test_mid_planes_match_three_passes(backend, b, b_spec, nb):
     finally:
         ops.lib.s2c_debug_force_general_path(0)
     for g, w in zip(got, want):
-        assert torch.equal(g, w) if backend == "cuda" else torch.allclose(g, w, rtol=1e-5, atol=1e-5)
+        if backend == "cuda":
+            assert torch.equal(g, w)
+        else:   # the host compiler rounds the generic FFT's products differently
+            assert_close(g, w, "planes vs passes")
 
 
 @pytest.mark.parametrize("backend", backends.BACKENDS)
