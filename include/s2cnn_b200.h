@@ -270,12 +270,15 @@ int s2c_project_on_sphere(const float* verts, int nv, const int* faces, int nf, 
  * an application has no reason to touch them.
  *   s2c_debug_force_general_path(level): 1 routes small bandwidths (2b <= 32) through the general
  *     kernels instead of the single-kernel path; 2 additionally replaces the plane kernels of
- *     2b = 64 / 128 (both row transforms of a (z, beta) plane in one kernel) by the three separate
- *     passes every other size uses; 0 restores the defaults.
+ *     32 < 2b <= 64 and 2b = 128 (both row transforms of a (z, beta) plane in one kernel) by the three
+ *     separate passes every other size uses; 0 restores the defaults.
  *   s2c_debug_plane_chunk(signals): signals per chunk of the large-bandwidth path (1 .. 8); 0
- *     restores the default (8, or what the workspace holds). */
+ *     restores the default (8, or what the workspace holds).
+ *   s2c_debug_cluster(mode): single-kernel path: 1 always the cluster kernels, 2 never (the kernels
+ *     whose blocks walk beta); 0 restores the choice by batch size. */
 void s2c_debug_force_general_path(int level);
 void s2c_debug_plane_chunk(int signals);
+void s2c_debug_cluster(int mode);
 
 #ifdef __cplusplus
 }

@@ -43,6 +43,7 @@ _SIGNATURES = {
     "s2c_so3_rfft_relu": (c_int, [_P, _P, c_long, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_rfft_sums": (c_int, [_P, _P, _P, c_long, c_int, c_int, c_int, _P]),
     "s2c_debug_force_general_path": (None, [c_int]),
+    "s2c_debug_cluster": (None, [c_int]),
     "s2c_debug_plane_chunk": (None, [c_int]),
     "s2c_so3_fft": (c_int, [_P, _P, c_long, c_int, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_rifft": (c_int, [_P, _P, c_long, c_int, c_int, c_int, _P, c_int, _P, c_size_t, _P]),

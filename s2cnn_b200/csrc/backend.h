@@ -235,6 +235,42 @@ __device__ __forceinline__ void st_global_256(float* p, const float8& v) {
                : "memory");
 }
 
+// ---- thread-block clusters: block rank, cluster barrier, access to the other blocks' shared memory ------
+struct ClCtx {
+  int tid, nthr, bid, rank;      // bid: cluster index, rank: block within the cluster
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+  __device__ __forceinline__ void sync_cluster() const {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  }
+};
+typedef unsigned cl_addr;        // shared::cluster address
+// where `local` (an address of this block's shared memory) lies in block `rank` of the cluster
+__device__ __forceinline__ cl_addr cl_map(const ClCtx&, const float2* local, int rank) {
+  cl_addr a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float2 cl_load(cl_addr base, int off) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(base + 8u * (unsigned)off) : "memory");
+  return v;
+}
+// two complex numbers at a 16-byte boundary (off even)
+__device__ __forceinline__ float4 cl_load4(cl_addr base, int off) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(base + 8u * (unsigned)off) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cl_store4(cl_addr base, int off, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(base + 8u * (unsigned)off), "f"(v.x), "f"(v.y),
+               "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void cl_store_float(cl_addr base, int off, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(base + 4u * (unsigned)off), "f"(v) : "memory");
+}
+
+
 __device__ __forceinline__ bool bulk_wait(const Ctx&, unsigned long long* bar, unsigned parity) {
   const unsigned addr = smem_u32(bar);
   for (int spin = 0; spin < (1 << 20); ++spin) {
@@ -267,6 +303,9 @@ struct float2 {
 };
 struct float4 {
   float x, y, z, w;
+};
+struct int2 {
+  int x, y;
 };
 struct int4 {
   int x, y, z, w;
@@ -426,6 +465,66 @@ inline float8 ld_global_256(const float* p) {
 inline void st_global_256(float* p, const float8& v) {
   *reinterpret_cast<float4*>(p) = v.lo;
   *reinterpret_cast<float4*>(p + 4) = v.hi;
+}
+// A cluster: the fibers of all its blocks run as one group (a block barrier is then a cluster barrier, which
+// is stronger), every block with shared memory of its own.
+struct EmuCluster {
+  unsigned char* smem = nullptr;
+  size_t stride = 0;
+};
+inline EmuCluster& emu_cluster() {
+  static thread_local EmuCluster c;
+  return c;
+}
+struct ClCtx {
+  int tid, nthr, bid, rank;
+  void sync() const {
+    EmuBlock* b = emu_cur();
+    if (b->nthr > 1) swapcontext(&b->th[rank * nthr + tid], &b->sched);
+  }
+  void sync_cluster() const { sync(); }
+};
+typedef unsigned char* cl_addr;
+inline cl_addr cl_map(const ClCtx& ctx, const float2* local, int rank) {
+  return (cl_addr)local + (long)(rank - ctx.rank) * (long)emu_cluster().stride;
+}
+inline float2 cl_load(cl_addr base, int off) { return reinterpret_cast<float2*>(base)[off]; }
+inline float4 cl_load4(cl_addr base, int off) { return *reinterpret_cast<float4*>(reinterpret_cast<float2*>(base) + off); }
+inline void cl_store4(cl_addr base, int off, float4 v) { *reinterpret_cast<float4*>(reinterpret_cast<float2*>(base) + off) = v; }
+inline void cl_store_float(cl_addr base, int off, float v) { reinterpret_cast<float*>(base)[off] = v; }
+
+template <class Impl, class P>
+struct EmuClusterLaunch {
+  const P* p;
+  int bid, nthr;
+  static void entry(int fiber, void* a) {
+    EmuClusterLaunch* self = (EmuClusterLaunch*)a;
+    ClCtx ctx{fiber % self->nthr, self->nthr, self->bid, fiber / self->nthr};
+    Impl::run(ctx, *self->p, emu_cluster().smem + ctx.rank * emu_cluster().stride);
+  }
+};
+template <class Impl, class P>
+inline int emu_launch_cluster(const char* kname, long nclusters, int c, int block, size_t smem, const P& p) {
+  if (nclusters <= 0) return S2C_OK;
+  if (smem > (size_t)dev_smem_limit())
+    return fail(S2C_ERR_UNSUPPORTED, std::string(kname) + ": shared memory over the limit");
+  const size_t stride = (smem + 63) / 64 * 64 + 64;   // a guard behind every block's shared memory
+  std::vector<unsigned char> sm(stride * c + 64, 0xA5);
+  emu_cluster().smem = sm.data() + ((64 - (uintptr_t)sm.data() % 64) % 64);
+  emu_cluster().stride = stride;
+  EmuClusterLaunch<Impl, P> L;
+  L.p = &p;
+  L.nthr = block;
+  for (long b = 0; b < nclusters; ++b) {
+    L.bid = (int)b;
+    emu_run_block(c * block, &EmuClusterLaunch<Impl, P>::entry, &L);
+    for (int r = 0; r < c; ++r)
+      for (size_t i = smem; i < stride; ++i)
+        if (emu_cluster().smem[r * stride + i] != 0xA5)
+          return fail(S2C_ERR_CUDA, std::string(kname) + ": write past the shared memory of a block");
+  }
+  ++g_launch_count;
+  return S2C_OK;
 }
 inline bool bulk_wait(const Ctx& ctx, unsigned long long*, unsigned) {
   ctx.sync();

@@ -16,6 +16,7 @@
 #include "so3_plane_kernels.h"
 #include "so3_fused_kernels.h"
 #include "so3_relay_kernels.h"
+#include "so3_cluster_kernels.h"
 #include "so3_mid_kernels.h"
 #include "s2_kernels.h"
 #include "wigner_tiled.h"
@@ -30,6 +31,7 @@ namespace s2c {
 thread_local long g_launch_count = 0;
 // test switches (process-wide, race-free; see the "test hooks" section of the header)
 static std::atomic<int> g_force_general{0};   // 1 = no single-kernel path, 2 = also no plane kernels
+static std::atomic<int> g_cluster{0};         // cluster kernels: 0 by batch size, 1 always, 2 never
 static std::atomic<int> g_plane_chunk{0};     // plane path: signals per chunk (0 = default)
 
 #define S2C_TRY(expr)            \
@@ -120,6 +122,20 @@ static int mid_chunk(long nbatch, int N, int K, const void* ws, size_t ws_bytes,
   return S2C_OK;
 }
 
+// Small bandwidths: whether the batch is small enough for the cluster kernels, by the number of groups of
+// kFusedZG batch elements (a walking block, or a cluster of cl_size(N) blocks, each).  A walking kernel takes
+// the same time for any batch up to one block per SM and resident block; the clusters' time grows from a third of
+// that with the batch, at b = 16 to the same at 55 (analysis) and 95 (synthesis) groups, b = 15 at 80 and 130,
+// b = 12 at 53 and 88, b = 10 at 600 and 500, b = 6 at 800 and 500.  The relay of N > 20 keeps several times the
+// shared memory of a synthesis per walking block (one block of 8 warps per SM) and is never the faster one.
+enum ClKind { kClAnalysis, kClSynthesis, kClRelay };
+static bool so3_prefers_cluster(ClKind kind, int N, long nbatch) {
+  if (const int forced = g_cluster.load()) return forced == 1;
+  const long groups = (nbatch + kFusedZG - 1) / kFusedZG;
+  if (N <= 20) return groups <= 500;
+  return kind == kClRelay || groups <= (kind == kClAnalysis ? 55 : 95);
+}
+
 static int check_b(int b_in, int b_out) {
   if (b_in < 1 || b_out < 1) return fail(S2C_ERR_BAD_ARG, "bandwidths must be >= 1");
   return S2C_OK;
@@ -138,6 +154,21 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
   S2C_TRY(TableCache::get().panels(b_in, b_out, K, weighted, false, pan));
   if (b_out > b_in && mode == kSo3Real)  // rows with |m| or |n| >= b_in stay zero (so3_fft.py:44-48)
     S2C_TRY(dev_memset_async(out, 0, (size_t)so3_nspec(b_out) * nbatch * sizeof(float2), st));
+  if (!g_force_general && N <= kFusedMaxN && b_out <= kFusedMaxDegrees &&
+      so3_prefers_cluster(kClAnalysis, N, nbatch)) {
+    ClFwdParams f;
+    f.x = x; f.in_stride = in_stride; f.in_off = in_off;
+    f.out = out; f.out_zstride = nbatch;
+    S2C_TRY(TableCache::get().cluster(b_in, b_out, K, weighted, f.tab));
+    f.nbatch = (int)nbatch; f.K = K;
+    f.mode = mode; f.relu = relu;
+    f.wide = in_stride == 1 && in_off == 0 && N % 4 == 0 && (uintptr_t)x % 32 == 0;
+    f.sums = sums;
+    int rc = S2C_OK;
+    S2C_DISPATCH_N(N, rc = S2C_LAUNCH_CL(so3_fwd_cl, kN, (nbatch + kFusedZG - 1) / kFusedZG,
+                                         cl_smem_bytes(N, K, 0), st, f));
+    return rc;
+  }
   if (!g_force_general && N <= kFusedMaxN &&
       fwd_fused_smem_bytes(N, pan.nrows) <= (size_t)dev_smem_limit() - 1024) {
     FwdFusedParams f;
@@ -269,6 +300,34 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
   PanelsDev pan;
   S2C_TRY(TableCache::get().fft(N, fft));
   S2C_TRY(TableCache::get().panels(b_out, K, K, weighted, false, pan));
+  if (!g_force_general && N <= kFusedMaxN && so3_prefers_cluster(kClSynthesis, N, nbatch)) {
+    ClInvParams f;
+    f.in.x = x; f.in.x_zstride = nbatch; f.in.mode = mode;
+    f.in.xs = f.in.ys = nullptr; f.in.s2_nb = f.in.s2_fin = f.in.s2_fout = 0;
+    f.out = out; f.out_stride = out_stride; f.out_off = out_off;
+    f.bias = bias; f.nfeat = nfeat > 0 ? nfeat : 1;
+    S2C_TRY(TableCache::get().cluster(b_out, K, K, weighted, f.tab));
+    f.nbatch = (int)nbatch; f.K = K;
+    f.iw = nullptr; f.isum = nullptr;
+    f.mask = mask;
+    if (mask && (out_stride != 1 || out_off != 0))
+      return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output only");
+    f.wide = out_stride == 1 && out_off == 0 && N % 4 == 0 && out && (uintptr_t)out % 32 == 0 &&
+             (uintptr_t)mask % 32 == 0;
+    if (integral) {
+      S2C_TRY(TableCache::get().quad_weights(b_out, &f.iw));
+      f.isum = integral;
+    }
+    if (prod) {
+      f.in.mode = kS2Product;
+      f.in.xs = prod->xs; f.in.ys = prod->ys;
+      f.in.s2_nb = prod->nb; f.in.s2_fin = prod->fin; f.in.s2_fout = prod->fout;
+    }
+    int rc = S2C_OK;
+    S2C_DISPATCH_N(N, rc = S2C_LAUNCH_CL(so3_inv_cl, kN, (nbatch + kFusedZG - 1) / kFusedZG,
+                                         cl_smem_bytes(N, K, f.tab.max_rows), st, f));
+    return rc;
+  }
   if (!g_force_general && N <= kFusedMaxN &&
       fused_smem_bytes(N, pan.nrows) <= (size_t)dev_smem_limit() - 1024) {
     InvFusedParams f;
@@ -615,6 +674,7 @@ int s2c_so3_rfft_sums(const float* x, float* out, float* sums, long nbatch, int 
 }
 
 void s2c_debug_force_general_path(int level) { g_force_general = level < 0 ? 0 : level; }
+void s2c_debug_cluster(int mode) { g_cluster = mode; }
 void s2c_debug_plane_chunk(int signals) { g_plane_chunk = signals < 0 ? 0 : signals; }
 
 int s2c_so3_fft(const float* x, float* out, long nbatch, int b_in, int b_out, int for_grad,
@@ -681,6 +741,21 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
   if (N > kFusedMaxN || b_next > b_mid || b_in > b_mid)
     return fail(S2C_ERR_UNSUPPORTED,
                 std::string(who) + ": needs 2 b <= 32, b_in <= b and b_next <= b");
+  if (so3_prefers_cluster(kClRelay, N, nz)) {
+    ClRelayParams f;
+    S2C_TRY(TableCache::get().cluster(b_mid, b_in, b_in, false, f.tin));
+    S2C_TRY(TableCache::get().cluster(b_mid, b_next, b_next, true, f.tout));
+    f.in.x = x; f.in.x_zstride = nz; f.in.mode = xs ? kS2Product : kSo3Real;
+    f.in.xs = xs; f.in.ys = ys;
+    f.in.s2_nb = s2_nb; f.in.s2_fin = s2_fin; f.in.s2_fout = nfeat;
+    f.bias = bias; f.nfeat = nfeat > 0 ? nfeat : 1;
+    f.out = (float2*)out; f.out_zstride = nz;
+    f.nbatch = (int)nz; f.Kin = b_in; f.Kout = b_next;
+    int rc = S2C_OK;
+    S2C_DISPATCH_N(N, rc = S2C_LAUNCH_CL(so3_relay_cl, kN, (nz + kFusedZG - 1) / kFusedZG,
+                                         cl_smem_bytes(N, std::max(b_in, b_next), f.tin.max_rows), st, f));
+    return rc;
+  }
   FftDev fft;
   RelayParams f;
   S2C_TRY(TableCache::get().fft(N, fft));
@@ -701,7 +776,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
   int rc = S2C_OK;
   const long grid = (nz + kFusedZG - 1) / kFusedZG;
   const size_t sm = relay_smem_bytes(N, b_in, f.pin.nrows, f.pout.nrows, f.BG);
-  S2C_DISPATCH_N(N, rc = S2C_LAUNCH_N(so3_relay_fused, kN, grid, 256, sm, st, f));
+  S2C_DISPATCH_N20(N, rc = S2C_LAUNCH_N(so3_relay_fused, kN, grid, 256, sm, st, f));
   return rc;
 }
 

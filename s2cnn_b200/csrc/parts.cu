@@ -11,6 +11,7 @@
 #include "so3_kernels.h"
 #include "so3_fused_kernels.h"
 #include "so3_relay_kernels.h"
+#include "so3_cluster_kernels.h"
 #include "so3_mid_kernels.h"
 #include "s2_kernels.h"
 #include "so3_mm_tc.h"
@@ -20,6 +21,10 @@ namespace s2c {
 #define S2C_LENGTH(N)                                                                                \
   template int launch_so3_inv_fused<N>(long, int, size_t, stream_t, const InvFusedParams&);          \
   template int launch_so3_fwd_fused<N>(long, int, size_t, stream_t, const FwdFusedParams&);          \
+  template int launch_so3_inv_cl<N>(long, int, size_t, stream_t, const ClInvParams&);                \
+  template int launch_so3_fwd_cl<N>(long, int, size_t, stream_t, const ClFwdParams&);                \
+  template int launch_so3_relay_cl<N>(long, int, size_t, stream_t, const ClRelayParams&);
+#define S2C_RELAY(N) \
   template int launch_so3_relay_fused<N>(long, int, size_t, stream_t, const RelayParams&);
 #define S2C_MID(N)                                                                  \
   template int launch_so3_fwd_mid<N>(long, int, size_t, stream_t, const MidParams&); \
@@ -37,15 +42,15 @@ S2C_LENGTH(32)
 #elif S2C_PART == 1
 S2C_LENGTH(30)
 #elif S2C_PART == 2
-S2C_LENGTH(28) S2C_LENGTH(2) S2C_LENGTH(4)
+S2C_LENGTH(28) S2C_LENGTH(2) S2C_RELAY(2) S2C_LENGTH(4) S2C_RELAY(4)
 #elif S2C_PART == 3
-S2C_LENGTH(26) S2C_LENGTH(6)
+S2C_LENGTH(26) S2C_LENGTH(6) S2C_RELAY(6)
 #elif S2C_PART == 4
-S2C_LENGTH(24) S2C_LENGTH(8) S2C_LENGTH(10)
+S2C_LENGTH(24) S2C_LENGTH(8) S2C_RELAY(8) S2C_LENGTH(10) S2C_RELAY(10)
 #elif S2C_PART == 5
-S2C_LENGTH(22) S2C_LENGTH(12) S2C_LENGTH(14)
+S2C_LENGTH(22) S2C_LENGTH(12) S2C_RELAY(12) S2C_LENGTH(14) S2C_RELAY(14)
 #elif S2C_PART == 6
-S2C_LENGTH(20) S2C_LENGTH(16) S2C_LENGTH(18)
+S2C_LENGTH(20) S2C_RELAY(20) S2C_LENGTH(16) S2C_RELAY(16) S2C_LENGTH(18) S2C_RELAY(18)
 #elif S2C_PART == 7
 S2C_TC_OP(kTcFwd) S2C_TC_OP(kTcGradX)
 #elif S2C_PART == 8

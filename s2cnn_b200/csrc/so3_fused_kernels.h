@@ -1,5 +1,5 @@
 // Fused SO(3) transforms for small bandwidths (N = 2b <= 32): one kernel per direction, no
-// scratch in global memory.  A block owns ZG consecutive batch elements (so that its accesses to
+// scratch in global memory (small batches: so3_cluster_kernels.h).  A block owns ZG consecutive batch elements (so that its accesses to
 // the [spectrum][batch] layout are whole 32-byte sectors) and walks the beta axis in groups; all
 // intermediates of a group live in shared memory, every 1-D FFT runs in the registers of one
 // thread (fft_reg.h).
@@ -779,25 +779,34 @@ S2C_LAUNCHER_N(so3_fwd_fused, FwdFusedParams)
   s2c::emu_launch<name##_impl<N>>(#name, (long)(grid), (int)(block), (size_t)(smem), params)
 #endif
 
-// run-time N -> compile-time N
+// run-time N -> compile-time N, up to 20 and up to 32
+#define S2C_CASES_20(CALL)                                                                   \
+    case 2: { constexpr int kN = 2; CALL; } break;                                       \
+    case 4: { constexpr int kN = 4; CALL; } break;                                       \
+    case 6: { constexpr int kN = 6; CALL; } break;                                       \
+    case 8: { constexpr int kN = 8; CALL; } break;                                       \
+    case 10: { constexpr int kN = 10; CALL; } break;                                     \
+    case 12: { constexpr int kN = 12; CALL; } break;                                     \
+    case 14: { constexpr int kN = 14; CALL; } break;                                     \
+    case 16: { constexpr int kN = 16; CALL; } break;                                     \
+    case 18: { constexpr int kN = 18; CALL; } break;                                     \
+    case 20: { constexpr int kN = 20; CALL; } break;                                     
+#define S2C_CASES_32(CALL)                                                                   \
+    case 22: { constexpr int kN = 22; CALL; } break;                                     \
+    case 24: { constexpr int kN = 24; CALL; } break;                                     \
+    case 26: { constexpr int kN = 26; CALL; } break;                                     \
+    case 28: { constexpr int kN = 28; CALL; } break;                                     \
+    case 30: { constexpr int kN = 30; CALL; } break;                                     \
+    case 32: { constexpr int kN = 32; CALL; } break;                                     
+#define S2C_DISPATCH_N20(N, CALL)                                                            \
+  switch (N) {                                                                               \
+    S2C_CASES_20(CALL)                                                                       \
+    default: rc = s2c::fail(s2c::S2C_ERR_UNSUPPORTED, "no fused kernel for this length");    \
+  }
 #define S2C_DISPATCH_N(N, CALL)                                                              \
   switch (N) {                                                                               \
-    case 2: { constexpr int kN = 2; CALL; } break;                                           \
-    case 4: { constexpr int kN = 4; CALL; } break;                                           \
-    case 6: { constexpr int kN = 6; CALL; } break;                                           \
-    case 8: { constexpr int kN = 8; CALL; } break;                                           \
-    case 10: { constexpr int kN = 10; CALL; } break;                                         \
-    case 12: { constexpr int kN = 12; CALL; } break;                                         \
-    case 14: { constexpr int kN = 14; CALL; } break;                                         \
-    case 16: { constexpr int kN = 16; CALL; } break;                                         \
-    case 18: { constexpr int kN = 18; CALL; } break;                                         \
-    case 20: { constexpr int kN = 20; CALL; } break;                                         \
-    case 22: { constexpr int kN = 22; CALL; } break;                                         \
-    case 24: { constexpr int kN = 24; CALL; } break;                                         \
-    case 26: { constexpr int kN = 26; CALL; } break;                                         \
-    case 28: { constexpr int kN = 28; CALL; } break;                                         \
-    case 30: { constexpr int kN = 30; CALL; } break;                                         \
-    case 32: { constexpr int kN = 32; CALL; } break;                                         \
+    S2C_CASES_20(CALL)                                                                       \
+    S2C_CASES_32(CALL)                                                                       \
     default: rc = s2c::fail(s2c::S2C_ERR_UNSUPPORTED, "no fused kernel for this length");    \
   }
 

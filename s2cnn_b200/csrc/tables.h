@@ -62,6 +62,7 @@ struct PanelsDev {
 constexpr int kFusedZG = 4;    // batch elements per block
 constexpr int kMaxBG = 8;      // upper bound of the betas per group
 constexpr int kFusedMaxN = 32;
+constexpr int kFusedMaxDegrees = 255;   // degrees are packed in 8 bits
 constexpr int kFusedMaxThreads = 512;
 // Betas per group: the largest divisor of N that keeps the per-group transform count
 // (ZG * BG * N/2 threads, one transform each) within one pass of a 256-thread block.
@@ -71,6 +72,30 @@ inline int fused_bg(int N) {
     if (N % d == 0 && d <= kMaxBG && kFusedZG * d * (N / 2) <= 256) best = d;
   return best;
 }
+
+// ---- clusters of so3_cluster_kernels.h ---------------------------------------------------------------------
+// Blocks per cluster, betas per block: about four betas (one FFT per thread and phase for 128 - 256 threads),
+// powers of two up to the portable 8.
+S2C_HD constexpr int cl_size(int N) { return N <= 6 ? 1 : N <= 10 ? 2 : N <= 20 ? 4 : 8; }
+S2C_HD constexpr int cl_betas(int N) { return (N + cl_size(N) - 1) / cl_size(N); }
+S2C_HD constexpr int cl_threads(int N) {
+  return kFusedZG * cl_betas(N) * (N / 2) < 128 ? 128 : (kFusedZG * cl_betas(N) * (N / 2) + 31) / 32 * 32;
+}
+// blocks per SM the register allocation leaves room for
+S2C_HD constexpr int cl_min_blocks(int N) { return N <= 10 ? 6 : N <= 22 ? 4 : N <= 30 ? 3 : 2; }
+
+// Work lists of the contractions for one (beta grid, nl, K), see so3_cluster_kernels.h: the pairs sorted by their
+// number of degrees, pair i belonging to block i mod C of a cluster.
+struct ClTables {
+  const float* w;        // Wigner panel rows [row][N]
+  const int4* pairs;     // [npairs] {first panel row, L, FFT row of m, n}
+  const int* lrow;       // [npairs] first row of the pair in its block's list of spectrum rows
+  const int2* rows;      // [C][max_rows] {l | (m + 128) << 8 | n << 16, place in the block's list}, by (l, n, m)
+  const int* nrows;      // [C]
+  const int4* tasks;     // [C][max_tasks] {panel row, degrees (1 or 2), FFT row of m, n | l << 8}
+  const int* ntasks;     // [C]
+  int npairs, max_rows, max_tasks;
+};
 
 S2C_HD int so3_npairs(int K) { return K + (K - 1) * (2 * K - 1); }
 S2C_HD int so3_pair_index(int m, int n, int K) {
@@ -386,6 +411,92 @@ class TableCache {
     return S2C_OK;
   }
 
+  // Work lists of the cluster kernels (the panels themselves are those of panels()).
+  int cluster(int b_beta, int nl, int K, bool weighted, ClTables& out) {
+    PanelsDev pan;
+    const int rc0 = panels(b_beta, nl, K, weighted, false, pan);
+    if (rc0) return rc0;
+    std::lock_guard<std::mutex> g(mu_);
+    auto key = std::make_tuple(dev_current(), b_beta, nl, K);
+    auto it = cluster_.find(key);
+    if (it == cluster_.end()) {
+      const int N = 2 * b_beta, C = cl_size(N);
+      struct Pair { int row, L, m, n; };
+      std::vector<Pair> pairs;
+      int row = 0;
+      for (int i = 0; i < so3_npairs(K); ++i) {
+        Pair p;
+        so3_pair_decode(i, K, p.m, p.n);
+        p.L = nl - std::max(std::abs(p.m), p.n);
+        p.row = row;
+        row += std::max(p.L, 0);
+        if (p.L > 0) pairs.push_back(p);
+      }
+      std::stable_sort(pairs.begin(), pairs.end(), [](const Pair& a, const Pair& b) { return a.L > b.L; });
+      std::vector<std::vector<int2>> rows(C);
+      std::vector<std::vector<int4>> tasks(C);
+      std::vector<int4> pv;
+      std::vector<int> lrow;
+      for (size_t i = 0; i < pairs.size(); ++i) {
+        const Pair& p = pairs[i];
+        const int r = (int)(i % C), fm = p.m < 0 ? p.m + N : p.m, l0 = std::max(std::abs(p.m), p.n);
+        pv.push_back(make_int4(p.row, p.L, fm, p.n));
+        lrow.push_back((int)rows[r].size());
+        for (int li = 0; li < p.L; ++li) {
+          int2 e;
+          e.x = (l0 + li) | ((p.m + 128) << 8) | (p.n << 16);
+          e.y = (int)rows[r].size();
+          rows[r].push_back(e);
+        }
+        for (int li = 0; li < p.L; li += 2)
+          tasks[r].push_back(make_int4(p.row + li, std::min(2, p.L - li), fm, p.n | ((l0 + li) << 8)));
+      }
+      ClTables t;
+      t.npairs = (int)pairs.size();
+      t.max_rows = t.max_tasks = 0;
+      std::vector<int> nrows, ntasks;
+      for (int r = 0; r < C; ++r) {
+        // neighbouring work items with the same (l, n): the same address of the second S2 spectrum when the
+        // product s2_mm is computed on the fly
+        auto key_of = [](const int2& e) { return ((e.x & 0xff) << 16) | (((e.x >> 16) & 0xff) << 8) | ((e.x >> 8) & 0xff); };
+        std::sort(rows[r].begin(), rows[r].end(), [&](const int2& a, const int2& b) { return key_of(a) < key_of(b); });
+        nrows.push_back((int)rows[r].size());
+        ntasks.push_back((int)tasks[r].size());
+        t.max_rows = std::max(t.max_rows, nrows.back());
+        t.max_tasks = std::max(t.max_tasks, ntasks.back());
+      }
+      std::vector<int2> rv((size_t)C * t.max_rows, int2());
+      std::vector<int4> tv((size_t)C * t.max_tasks, int4());
+      for (int r = 0; r < C; ++r) {
+        std::copy(rows[r].begin(), rows[r].end(), rv.begin() + (size_t)r * t.max_rows);
+        std::copy(tasks[r].begin(), tasks[r].end(), tv.begin() + (size_t)r * t.max_tasks);
+      }
+      // one allocation, 16-byte lists first
+      const size_t sizes[6] = {pv.size() * sizeof(int4), tv.size() * sizeof(int4), rv.size() * sizeof(int2),
+                               lrow.size() * sizeof(int), nrows.size() * sizeof(int), ntasks.size() * sizeof(int)};
+      const void* src[6] = {pv.data(), tv.data(), rv.data(), lrow.data(), nrows.data(), ntasks.data()};
+      size_t off[7] = {0};
+      for (int i = 0; i < 6; ++i) off[i + 1] = off[i] + sizes[i];
+      std::vector<unsigned char> all(off[6]);
+      for (int i = 0; i < 6; ++i) std::memcpy(all.data() + off[i], src[i], sizes[i]);
+      unsigned char* d = (unsigned char*)dev_alloc(all.size());
+      if (!d) return fail(S2C_ERR_CUDA, "table allocation failed");
+      const int rc = dev_upload(d, all.data(), all.size());
+      if (rc) return rc;
+      t.w = nullptr;
+      t.pairs = (const int4*)(d + off[0]);
+      t.tasks = (const int4*)(d + off[1]);
+      t.rows = (const int2*)(d + off[2]);
+      t.lrow = (const int*)(d + off[3]);
+      t.nrows = (const int*)(d + off[4]);
+      t.ntasks = (const int*)(d + off[5]);
+      it = cluster_.emplace(key, t).first;
+    }
+    out = it->second;
+    out.w = pan.data;
+    return S2C_OK;
+  }
+
   // First half of the beta range of every SO(3) panel (rows of nbeta / 2 floats), for kernels that
   // obtain the second half from d^l_{m,n}(pi - beta_j) = (-1)^(l+n) d^l_{-m,n}(beta_j) and the
   // symmetry of the SOFT grid and its quadrature weights under beta -> pi - beta.  `off` holds
@@ -479,6 +590,8 @@ class TableCache {
     }
     for (auto& kv : quad_) dev_free((void*)kv.second);
     for (auto& kv : grouped_) dev_free((void*)kv.second.first);
+    for (auto& kv : cluster_) dev_free((void*)kv.second.pairs);
+    cluster_.clear();
     for (auto& kv : half_) { dev_free((void*)kv.second.first); dev_free((void*)kv.second.second); }
     for (auto& kv : s2t_) dev_free((void*)kv.second);
     s2t_.clear();
@@ -496,6 +609,7 @@ class TableCache {
   std::map<std::pair<int, int>, const float*> quad_;
   std::map<std::tuple<int, int, int, int>, const float*> s2t_;
   std::map<std::tuple<int, int, int, int, int, int>, std::pair<const float*, int>> grouped_;
+  std::map<std::tuple<int, int, int, int>, ClTables> cluster_;
   std::map<std::tuple<int, int, int, int, int, int>, std::pair<const float*, const long long*>> half_;
 };
 
