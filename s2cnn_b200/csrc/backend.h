@@ -217,6 +217,16 @@ __device__ __forceinline__ void bulk_load_issue(void* dst, const void* src, unsi
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
+// two independent single-precision operations in one instruction, each rounded as the scalar one
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
 // 32-byte global accesses (one full sector per lane and instruction); p must be 32-byte aligned
 struct float8 {
   float4 lo, hi;
@@ -453,6 +463,7 @@ inline void bulk_barrier_init(unsigned long long*) {}
 inline void bulk_load_issue(void* dst, const void* src, unsigned bytes, unsigned long long*) {
   std::memcpy(dst, src, bytes);
 }
+inline float2 fma2(float2 a, float2 b, float2 c) { return make_float2(std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)); }
 struct float8 {
   float4 lo, hi;
 };

@@ -272,8 +272,7 @@ struct Cl {
         for (int bi = 0; bi < BC; ++bi)
 #pragma unroll
           for (int z = 0; z < ZG; ++z) {
-            s[bi][z].x = fmaf(wv[bi], xv[z].x, s[bi][z].x);
-            s[bi][z].y = fmaf(wv[bi], xv[z].y, s[bi][z].y);
+            s[bi][z] = fma2(make_float2(wv[bi], wv[bi]), xv[z], s[bi][z]);
           }
       }
       const cl_addr dst = cl_map(ctx, b.planes + pr.z * b.RS + pr.w * ZG, c);
@@ -426,10 +425,8 @@ struct Cl {
         for (int bi = 0; bi < BC; ++bi)
 #pragma unroll
           for (int z = 0; z < ZT; ++z) {
-            a0[z].x = fmaf(u0[bi], xv[bi][z].x, a0[z].x);
-            a0[z].y = fmaf(u0[bi], xv[bi][z].y, a0[z].y);
-            a1[z].x = fmaf(u1[bi], xv[bi][z].x, a1[z].x);
-            a1[z].y = fmaf(u1[bi], xv[bi][z].y, a1[z].y);
+            a0[z] = fma2(make_float2(u0[bi], u0[bi]), xv[bi][z], a0[z]);
+            a1[z] = fma2(make_float2(u1[bi], u1[bi]), xv[bi][z], a1[z]);
           }
       }
       emit<ZT>(out, zstride, b, zf, l, m, n, a0, mode);

@@ -278,8 +278,7 @@ struct so3_inv_fused_impl {
             for (int bi = 0; bi < 4; ++bi)
 #pragma unroll
               for (int z = 0; z < ZG; ++z) {
-                s[bi][z].x = fmaf(wv[bi], xv[z].x, s[bi][z].x);
-                s[bi][z].y = fmaf(wv[bi], xv[z].y, s[bi][z].y);
+                s[bi][z] = fma2(make_float2(wv[bi], wv[bi]), xv[z], s[bi][z]);
               }
           }
           float2* pl = planes + info.z * KP + info.w;
@@ -307,8 +306,7 @@ struct so3_inv_fused_impl {
 #pragma unroll
           for (int z = 0; z < ZG; ++z) {
             const float2 xv = xh_at(xrow + li, z);
-            acc[z].x = fmaf(wv, xv.x, acc[z].x);
-            acc[z].y = fmaf(wv, xv.y, acc[z].y);
+            acc[z] = fma2(make_float2(wv, wv), xv, acc[z]);
           }
         }
         float2* pl = planes + (size_t)bi * plane_sz + info.z * KP + info.w;
@@ -681,8 +679,7 @@ struct so3_fwd_fused_impl {
 #pragma unroll
             for (int z = 0; z < ZG; ++z) {
               const float2 xv = src[(size_t)(z * 4 + bi) * plane_sz];
-              a[z].x = fmaf(wv[bi], xv.x, a[z].x);
-              a[z].y = fmaf(wv[bi], xv.y, a[z].y);
+              a[z] = fma2(make_float2(wv[bi], wv[bi]), xv, a[z]);
             }
           acc4[r] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
           acc4[p.nrows + r] = make_float4(a[2].x, a[2].y, a[3].x, a[3].y);
@@ -706,8 +703,7 @@ struct so3_fwd_fused_impl {
 #pragma unroll
           for (int z = 0; z < ZG; ++z) {
             const float2 xv = src[(size_t)(z * p.BG + bi) * plane_sz];
-            a[z].x = fmaf(wv, xv.x, a[z].x);
-            a[z].y = fmaf(wv, xv.y, a[z].y);
+            a[z] = fma2(make_float2(wv, wv), xv, a[z]);
           }
         }
         acc4[r] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);

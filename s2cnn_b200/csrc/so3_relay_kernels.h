@@ -216,8 +216,7 @@ struct so3_relay_fused_impl {
             for (int bi = 0; bi < 4; ++bi)
 #pragma unroll
               for (int z = 0; z < ZG; ++z) {
-                s[bi][z].x = fmaf(wv[bi], xv[z].x, s[bi][z].x);
-                s[bi][z].y = fmaf(wv[bi], xv[z].y, s[bi][z].y);
+                s[bi][z] = fma2(make_float2(wv[bi], wv[bi]), xv[z], s[bi][z]);
               }
           }
           float2* pl = planes + info.z * KP + info.w;
@@ -245,8 +244,7 @@ struct so3_relay_fused_impl {
 #pragma unroll
           for (int z = 0; z < ZG; ++z) {
             const float2 xv = xh_at(xrow + li, z);
-            s[z].x = fmaf(wv, xv.x, s[z].x);
-            s[z].y = fmaf(wv, xv.y, s[z].y);
+            s[z] = fma2(make_float2(wv, wv), xv, s[z]);
           }
         }
         float2* pl = planes + (size_t)bi * plane_sz + info.z * KP + info.w;
@@ -366,8 +364,7 @@ struct so3_relay_fused_impl {
 #pragma unroll
           for (int z = 0; z < ZG; ++z) {
             const float2 xv = src[(size_t)(z * p.BG + bi) * plane_sz];
-            a[z].x = fmaf(wv, xv.x, a[z].x);
-            a[z].y = fmaf(wv, xv.y, a[z].y);
+            a[z] = fma2(make_float2(wv, wv), xv, a[z]);
           }
         }
         acc4[r] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);

@@ -332,20 +332,20 @@ struct so3_fwd_wigner_r_impl {
         const float sl = ((l + n) & 1) ? -1.f : 1.f;
 #pragma unroll
         for (int z = 0; z < kRowsZQ; ++z) {
-          float pr = 0.f, pi = 0.f, qr = 0.f, qi = 0.f;
+          float2 xp = make_float2(0.f, 0.f), xq = make_float2(0.f, 0.f);
 #pragma unroll
           for (int jj = 0; jj < JL; ++jj) {
             const float a = va[r][jj], b = vb[r][jj], sa = sl * a, sb = sl * b;
             // X_{+m} = sum A Vp_{+m} + s B Vq_{+m};   X_{-m} = sum B Vp_{-m} + s A Vq_{-m}
-            pr = fmaf(a, vp[0][z][jj].x, pr);  pi = fmaf(a, vp[0][z][jj].y, pi);
-            pr = fmaf(sb, vq[0][z][jj].x, pr); pi = fmaf(sb, vq[0][z][jj].y, pi);
-            qr = fmaf(b, vp[1][z][jj].x, qr);  qi = fmaf(b, vp[1][z][jj].y, qi);
-            qr = fmaf(sa, vq[1][z][jj].x, qr); qi = fmaf(sa, vq[1][z][jj].y, qi);
+            xp = fma2(make_float2(a, a), vp[0][z][jj], xp);
+            xp = fma2(make_float2(sb, sb), vq[0][z][jj], xp);
+            xq = fma2(make_float2(b, b), vp[1][z][jj], xq);
+            xq = fma2(make_float2(sa, sa), vq[1][z][jj], xq);
           }
-          val[r * 16 + 0 * 8 + z * 2 + 0] = pr;
-          val[r * 16 + 0 * 8 + z * 2 + 1] = pi;
-          val[r * 16 + 1 * 8 + z * 2 + 0] = qr;
-          val[r * 16 + 1 * 8 + z * 2 + 1] = qi;
+          val[r * 16 + 0 * 8 + z * 2 + 0] = xp.x;
+          val[r * 16 + 0 * 8 + z * 2 + 1] = xp.y;
+          val[r * 16 + 1 * 8 + z * 2 + 0] = xq.x;
+          val[r * 16 + 1 * 8 + z * 2 + 1] = xq.y;
         }
       }
       const float mine = rows_reduce32(ctx, val, lane, xch);   // value `lane` summed over the warp
@@ -477,10 +477,10 @@ struct so3_inv_wigner_r_impl {
           for (int jj = 0; jj < JL; ++jj) {
             const float sa = sl * a[jj], sb = sl * b[jj];
             // S_{+m}[j] += A X_{+m};  S_{+m}[N-1-j] += s B X_{+m};  S_{-m}[j] += B X_{-m};  S_{-m}[N-1-j] += s A X_{-m}
-            sp[0][z][jj].x = fmaf(a[jj], xp.x, sp[0][z][jj].x); sp[0][z][jj].y = fmaf(a[jj], xp.y, sp[0][z][jj].y);
-            sq[0][z][jj].x = fmaf(sb, xp.x, sq[0][z][jj].x);    sq[0][z][jj].y = fmaf(sb, xp.y, sq[0][z][jj].y);
-            sp[1][z][jj].x = fmaf(b[jj], xm.x, sp[1][z][jj].x); sp[1][z][jj].y = fmaf(b[jj], xm.y, sp[1][z][jj].y);
-            sq[1][z][jj].x = fmaf(sa, xm.x, sq[1][z][jj].x);    sq[1][z][jj].y = fmaf(sa, xm.y, sq[1][z][jj].y);
+            sp[0][z][jj] = fma2(make_float2(a[jj], a[jj]), xp, sp[0][z][jj]);
+            sq[0][z][jj] = fma2(make_float2(sb, sb), xp, sq[0][z][jj]);
+            sp[1][z][jj] = fma2(make_float2(b[jj], b[jj]), xm, sp[1][z][jj]);
+            sq[1][z][jj] = fma2(make_float2(sa, sa), xm, sq[1][z][jj]);
           }
         }
       }

@@ -62,11 +62,11 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
   // threads share the beta loop; at most two tiles per thread either way (LT <= 16, 256 threads)
   const bool narrow = LT * ZH < ctx.nthr;
   const int ntiles = narrow ? LT * zc : LT * ZH;
-  float ar[2][4][2], ai[2][4][2];
+  float2 acc[2][4][2];
 #pragma unroll
   for (int t = 0; t < 2; ++t)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { ar[t][i][0] = ar[t][i][1] = ai[t][i][0] = ai[t][i][1] = 0.f; }
+    for (int i = 0; i < 4; ++i) acc[t][i][0] = acc[t][i][1] = make_float2(0.f, 0.f);
 
   {
     if (N % 4 == 0) {
@@ -138,10 +138,10 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const float4 w4 = *reinterpret_cast<const float4*>(wp + i * LDW + bt);
-            ar[t][i][0] = fmaf(w4.x, va.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4.x, va.y, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4.y, va.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4.y, va.w, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4.z, vb.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4.z, vb.y, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4.w, vb.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4.w, vb.w, ai[t][i][0]);
+            acc[t][i][0] = fma2(make_float2(w4.x, w4.x), make_float2(va.x, va.y), acc[t][i][0]);
+            acc[t][i][0] = fma2(make_float2(w4.y, w4.y), make_float2(va.z, va.w), acc[t][i][0]);
+            acc[t][i][0] = fma2(make_float2(w4.z, w4.z), make_float2(vb.x, vb.y), acc[t][i][0]);
+            acc[t][i][0] = fma2(make_float2(w4.w, w4.w), make_float2(vb.z, vb.w), acc[t][i][0]);
           }
         }
       } else {
@@ -159,14 +159,14 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
           const float4 b1 = *reinterpret_cast<const float4*>(v1 + bt + 2);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            ar[t][i][0] = fmaf(w4[i].x, a0.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].x, a0.y, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4[i].y, a0.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].y, a0.w, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4[i].z, b0.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].z, b0.y, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4[i].w, b0.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].w, b0.w, ai[t][i][0]);
-            ar[t][i][1] = fmaf(w4[i].x, a1.x, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].x, a1.y, ai[t][i][1]);
-            ar[t][i][1] = fmaf(w4[i].y, a1.z, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].y, a1.w, ai[t][i][1]);
-            ar[t][i][1] = fmaf(w4[i].z, b1.x, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].z, b1.y, ai[t][i][1]);
-            ar[t][i][1] = fmaf(w4[i].w, b1.z, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].w, b1.w, ai[t][i][1]);
+            acc[t][i][0] = fma2(make_float2(w4[i].x, w4[i].x), make_float2(a0.x, a0.y), acc[t][i][0]);
+            acc[t][i][0] = fma2(make_float2(w4[i].y, w4[i].y), make_float2(a0.z, a0.w), acc[t][i][0]);
+            acc[t][i][0] = fma2(make_float2(w4[i].z, w4[i].z), make_float2(b0.x, b0.y), acc[t][i][0]);
+            acc[t][i][0] = fma2(make_float2(w4[i].w, w4[i].w), make_float2(b0.z, b0.w), acc[t][i][0]);
+            acc[t][i][1] = fma2(make_float2(w4[i].x, w4[i].x), make_float2(a1.x, a1.y), acc[t][i][1]);
+            acc[t][i][1] = fma2(make_float2(w4[i].y, w4[i].y), make_float2(a1.z, a1.w), acc[t][i][1]);
+            acc[t][i][1] = fma2(make_float2(w4[i].z, w4[i].z), make_float2(b1.x, b1.y), acc[t][i][1]);
+            acc[t][i][1] = fma2(make_float2(w4[i].w, w4[i].w), make_float2(b1.z, b1.w), acc[t][i][1]);
           }
         }
       }
@@ -175,7 +175,8 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
 
   const float fudge = ((m - n) & 1) ? -1.f : 1.f;
   const bool self = (m == 0 && n == 0);
-  auto emit = [&](int li, int zz, float re, float im) {
+  auto emit = [&](int li, int zz, float2 v) {
+    const float re = v.x, im = v.y;
     if (li >= L || zz >= zc) return;
     const int l = lmin + li;
     if (p.mode == kS2) {
@@ -203,13 +204,13 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
     if (narrow) {
       const int tl = tile / zc, zz = tile - tl * zc;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) emit(4 * tl + i, zz, ar[t][i][0], ai[t][i][0]);
+      for (int i = 0; i < 4; ++i) emit(4 * tl + i, zz, acc[t][i][0]);
     } else {
       const int tl = tile / ZH, tz = tile - tl * ZH;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        emit(4 * tl + i, tz, ar[t][i][0], ai[t][i][0]);
-        emit(4 * tl + i, tz + ZH, ar[t][i][1], ai[t][i][1]);
+        emit(4 * tl + i, tz, acc[t][i][0]);
+        emit(4 * tl + i, tz + ZH, acc[t][i][1]);
       }
     }
   }
@@ -283,11 +284,11 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
   const int B4 = NP / 4;
   for (int tile = ctx.tid; tile < B4 * Z2; tile += ctx.nthr) {
     const int tz = tile / B4, tb = tile - tz * B4;  // consecutive threads -> consecutive beta
-    float ar[2][4], ai[2][4];
+    float2 acc[2][4];
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) { ar[j][i] = 0.f; ai[j][i] = 0.f; }
+      for (int i = 0; i < 4; ++i) acc[j][i] = make_float2(0.f, 0.f);
     const float* wp = Ws + 4 * tb;
     const float2* xp = Xs + 2 * tz;
     for (int li = 0; li < L; ++li) {
@@ -296,10 +297,8 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
       const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        ar[0][i] = fmaf(w[i], x4.x, ar[0][i]);
-        ai[0][i] = fmaf(w[i], x4.y, ai[0][i]);
-        ar[1][i] = fmaf(w[i], x4.z, ar[1][i]);
-        ai[1][i] = fmaf(w[i], x4.w, ai[1][i]);
+        acc[0][i] = fma2(make_float2(w[i], w[i]), make_float2(x4.x, x4.y), acc[0][i]);
+        acc[1][i] = fma2(make_float2(w[i], w[i]), make_float2(x4.z, x4.w), acc[1][i]);
       }
     }
 #pragma unroll
@@ -307,8 +306,8 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
       const int zz = 2 * tz + j;
       if (zz >= zc) continue;
       float4* o = reinterpret_cast<float4*>(dst + (long)zz * N + 4 * tb);
-      o[0] = make_float4(ar[j][0], ai[j][0], ar[j][1], ai[j][1]);
-      if (4 * tb + 2 < N) o[1] = make_float4(ar[j][2], ai[j][2], ar[j][3], ai[j][3]);
+      o[0] = make_float4(acc[j][0].x, acc[j][0].y, acc[j][1].x, acc[j][1].y);
+      if (4 * tb + 2 < N) o[1] = make_float4(acc[j][2].x, acc[j][2].y, acc[j][3].x, acc[j][3].y);
     }
   }
 }
