@@ -24,9 +24,13 @@
 // Tiling: one CTA per (l, 128-row tile, 128-column tile); the K loop walks blocks of at most
 // kTcKMax floats (outer contraction index, slice of its run of floats).  The CTA is warp
 // specialised (17 warps):
-//   * 12 producer warps read the two operands from global memory (register prefetch one block
-//     ahead), split them into hi / lo TF32 parts and stage them in shared memory in the canonical
-//     K-major, no-swizzle UMMA layout (8 rows x 16 bytes core matrices), kTcStages stages deep; a
+//   * 12 producer warps in three groups of four; a group stages every third K block.  A thread owns one row of
+//     the row operand and half the K range of one complex column of the column operand: two pointers and
+//     constant offsets, no per-slot geometry.  The row operand goes, split into hi / lo TF32 parts, into
+//     TENSOR MEMORY (its thread is its TMEM lane; two stages of 64 columns), the column operand into shared
+//     memory in the canonical K-major, no-swizzle UMMA layout (8 rows x 16 bytes core matrices; the real
+//     columns of a tile are its rows 0 - 63, the imaginary ones 64 - 127: one load and one split serve both),
+//     kTcStages stages deep.  The next block's loads are issued before the barrier waits of the current one; a
 //     warp arrives on the stage's "full" mbarrier once its lanes have written their share;
 //   * one issuer warp waits for "full", issues the nine tcgen05.mma of the block (hi*hi, lo*hi,
 //     hi*lo for each k-step of 8) from one elected lane and commits them to the stage's "empty"
@@ -35,8 +39,12 @@
 //   * 4 collector warps (one per TMEM lane quarter) add each finished accumulator, with proper
 //     rounding, into a third tensor-memory region and hand the accumulator back ("accumulator
 //     free") - all of it while the tensor core fills the other one.
+// With both operands in shared memory a K block moved 48 KB of stores and 72 KB of MMA reads through a
+// 128-byte-per-clock pipe (960 clocks) and its producers, every warp taking part in every block, issued
+// about 1600 instructions: 1250 clocks per block measured, 480 us for 100 -> 100 channels at nl = 10, batch 32.
+// Now 24 KB of stores and 36 KB of reads remain, beside 600 - 750 clocks of MMA.
 // The epilogue (all 16 non-issuer warps) reads the last accumulator and the sum region with
-// tcgen05.ld (32 lanes x 32 columns per warp and instruction) and stores the result directly in
+// tcgen05.ld (32 lanes x 16 real and 16 imaginary columns per warp) and stores the result directly in
 // its interleaved layout.  Every mbarrier wait is bounded; on a time-out the waiting thread raises a
 // block-wide abort flag, every role leaves its loop, the kernel raises the error flag, frees its
 // TMEM columns and returns.
@@ -102,14 +110,14 @@ __host__ __device__ __forceinline__ TcGeom tc_geom(int op, int nb, int fi, int f
 
 constexpr int kTcBM = 128, kTcBN = 128;
 constexpr int kTcKMax = 24;                       // floats per K block
-constexpr int kTcStages = 4;
+constexpr int kTcStages = 6;                      // of the column operand (shared memory)
 constexpr int kTcLBO = kTcBM * 16 + 64;           // bytes between K-adjacent core matrices (padded)
 constexpr int kTcSBO = 128;                       // bytes between row-adjacent core matrices
 constexpr int kTcBufBytes = (kTcKMax / 4) * kTcLBO;   // one operand buffer (hi or lo)
-constexpr int kTcStageBytes = 4 * kTcBufBytes;        // A hi, A lo, B hi, B lo
+constexpr int kTcStageBytes = 2 * kTcBufBytes;        // B hi, B lo
 constexpr int kTcSmemBytes = kTcStages * kTcStageBytes + 256;   // + mbarriers, TMEM slot, abort flag
-constexpr int kTcProducerWarps = 12, kTcCollectorWarps = 4;
-constexpr int kTcProducers = 32 * kTcProducerWarps;
+constexpr int kTcGroups = 3, kTcGroupWarps = 4;     // producer groups (a group = one warp per TMEM lane quarter)
+constexpr int kTcProducerWarps = kTcGroups * kTcGroupWarps, kTcCollectorWarps = 4;
 constexpr int kTcFirstProducer = 32 * (1 + kTcCollectorWarps);  // thread index of the first producer
 constexpr int kTcThreads = 32 * (1 + kTcCollectorWarps + kTcProducerWarps);
 // K blocks accumulated by the tensor core before the partial sum is added, in FP32 with rounding,
@@ -119,9 +127,13 @@ constexpr int kTcFlushBlocks = 8;
 // longest chain (in MMAs) left to the tensor core's own accumulation without partial sums: its
 // truncation bias stays below about 1e-5 relative
 constexpr int kTcChainMax = 200;
-// tensor-memory columns: two alternating accumulators and the FP32 sum region (power of two)
+// tensor-memory columns: two alternating accumulators, the FP32 sum region and two stages of the row operand
+// (hi in columns 0 - 23, lo in 32 - 55 of each)
 constexpr int kTcTmemCols = 512;
 constexpr int kTcSumCol = 2 * kTcBN;
+constexpr int kTcACol = 3 * kTcBN, kTcAStages = 2, kTcAPitch = 64, kTcALo = 32;
+static_assert(kTcACol + kTcAStages * kTcAPitch == kTcTmemCols && kTcKMax <= kTcALo, "tensor memory");
+static_assert(kTcSmemBytes > 114 * 1024, "one CTA per SM: each allocates all of the tensor memory");
 
 __device__ __forceinline__ uint32_t tc_smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -165,14 +177,15 @@ __device__ __forceinline__ bool tc_mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
-__device__ __forceinline__ void tc_mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+// row operand in tensor memory, column operand in shared memory
+__device__ __forceinline__ void tc_mma_tf32(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
                                             uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
       :
-      : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -243,15 +256,17 @@ __device__ __forceinline__ void tc_red4(float* p, float a, float b, float c, flo
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// Staging slot e of a contiguous operand -> (row, 16-byte chunk of the K block): groups of 8 slots
-// cover 4 rows x 2 adjacent chunks, consecutive groups the chunk pairs of the same 4 rows (nchf,
-// the chunks per block, is even).
-__device__ __forceinline__ void tc_slot_contiguous(int e, int nchf, int& r, int& ch) {
-  const int g = e >> 3, u = e & 7, npair = nchf >> 1;
-  const int rq = g / npair, cp = g - rq * npair;
-  r = 4 * rq + (u >> 1);
-  ch = 2 * cp + (u & 1);
+// 8 columns of a lane's row (completes with tcgen05.wait::st)
+__device__ __forceinline__ void tc_st8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+               "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+               "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+               : "memory");
 }
+// v = hi + lo with hi carrying the 10 explicit TF32 mantissa bits (the tensor core ignores the
+// lower 13 bits of its inputs, so lo = v - hi needs no further rounding)
+__device__ __forceinline__ float tc_hi(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFFE000u); }
 
 __host__ __device__ __forceinline__ long tc_tiles_for(int op, int nb, int fi, int fo, int l) {
   const TcGeom g = tc_geom(op, nb, fi, fo);
@@ -306,7 +321,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   // ---- set-up: barriers, tensor memory ------------------------------------------------------
   if (tid == 0) {
     for (int i = 0; i < kTcStages; ++i) {
-      tc_mbar_init(&full[i], kTcProducerWarps);
+      tc_mbar_init(&full[i], kTcGroupWarps);
       tc_mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -343,8 +358,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     // instruction descriptor: D = F32, A = B = TF32, both K-major, N = 128, M = 128
     const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kTcBN >> 3) << 17) |
                            ((uint32_t)(kTcBM >> 4) << 24);
-    // The operand descriptors of every (stage, buffer, k-step) differ from the one of stage 0,
-    // A hi, k-step 0 only in the 14-bit start-address field (bytes >> 4), so they are obtained by
+    // The descriptors of every (stage, buffer, k-step) of the column operand differ from the one of stage 0,
+    // hi, k-step 0 only in the 14-bit start-address field (bytes >> 4), so they are obtained by
     // adding constants (the whole staging area is below 256 KB, the field cannot overflow).
     const uint64_t d0 = tc_smem_desc(tc_smem_u32(smem));
     constexpr uint64_t kDBuf = kTcBufBytes >> 4, kDStage = kTcStageBytes >> 4, kDStep = (2u * kTcLBO) >> 4;
@@ -360,16 +375,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (lane == 0) {
         const int ksteps = kb + 1 == p.nblk ? steps_tail : steps_full;
-        const uint64_t da = d0 + (uint64_t)s * kDStage;
+        const uint64_t db = d0 + (uint64_t)s * kDStage;
+        const uint32_t ta = tmem_base + kTcACol + (uint32_t)(it % kTcAStages) * kTcAPitch;
         const uint32_t acc = tmem_base + (FLUSH ? (uint32_t)((g & 1) * kTcBN) : 0u);
 #pragma unroll
         for (int ks = 0; ks < kStepsMax; ++ks) {
           if (ks < ksteps) {
-            const uint64_t dah = da + ks * kDStep, dal = dah + kDBuf;
-            const uint64_t dbh = dah + 2 * kDBuf, dbl = dah + 3 * kDBuf;
-            tc_mma_tf32(acc, dah, dbh, idesc, ((FLUSH ? ing == 0 : it == 0) && ks == 0) ? 0u : 1u);
-            tc_mma_tf32(acc, dal, dbh, idesc, 1u);
-            tc_mma_tf32(acc, dah, dbl, idesc, 1u);
+            const uint64_t dbh = db + ks * kDStep, dbl = dbh + kDBuf;
+            const uint32_t tah = ta + 8 * ks, tal = tah + kTcALo;
+            tc_mma_tf32(acc, tah, dbh, idesc, ((FLUSH ? ing == 0 : it == 0) && ks == 0) ? 0u : 1u);
+            tc_mma_tf32(acc, tal, dbh, idesc, 1u);
+            tc_mma_tf32(acc, tah, dbl, idesc, 1u);
           }
         }
         tc_commit(&empty[s]);     // arrives when these MMAs have read the stage
@@ -410,190 +426,144 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     }
   } else {
     // ================================ producers =================================================
-    const int pt = tid - kTcFirstProducer;
     // operand addressing (floats): offset of outer contraction index `o`, element `kf` of its run =
     //   contiguous:  o * ko + kf          strided:  o * ko + (kf / 2) * st + (kf % 2)
     constexpr bool plain = OP == kTcPlainCC || OP == kTcPlainSC;
     constexpr bool a_str = OP == kTcGradY || OP == kTcPlainSC, b_str = OP == kTcFwd || OP == kTcGradY;
-    long a_ko, b_ko, a_st = 0, b_st = 0;
+    long a_ko, b_ko, a_st = 2, b_st = 2;
     if (OP == kTcFwd)        { a_ko = (long)p.nb * fi2;      b_ko = (long)p.fi * fo2;      b_st = fo2; }
     else if (OP == kTcGradX) { a_ko = (long)p.nb * fo2;      b_ko = (long)L * p.fi * fo2; }
     else if (OP == kTcGradY) { a_ko = (long)L * p.nb * fi2;  b_ko = (long)L * p.nb * fo2;  a_st = fi2; b_st = fo2; }
     else                       { a_ko = 0; b_ko = 0; a_st = p.a_ps; b_st = p.b_ps; }   // one outer index
+    const int group = (warp - 1 - kTcCollectorWarps) / kTcGroupWarps;
+    const int t = tid - kTcFirstProducer - group * 32 * kTcGroupWarps;       // thread of the group
+    const int nprs = p.kblk / 2;                                 // complex numbers (pairs of floats) per full block
+    const int tail = (p.run - (p.nblk - 1) * p.kblk) / 2;        // pairs of a run's last block (VEC: even)
 
-    // Per-thread staging slots.  Everything that does not change along K is computed once per
-    // slot: the global address of its 16-byte chunk in K block 0 (null for a row, column or chunk
-    // outside the problem), its place in a stage buffer, whether it lies inside the shorter last
-    // block of a run, and for the column operand whether it builds an "imaginary" column.  The K
-    // loop then only adds one running offset per operand (advanced by a constant per block and by
-    // another per outer index - no division, no per-slot geometry).  A strided operand maps
-    // consecutive threads to consecutive rows of one chunk (neighbouring 8-byte loads; 32 lanes store
-    // 512 contiguous bytes).  A contiguous operand maps every 8 consecutive threads to 4 rows x 2
-    // adjacent chunks: each row's two chunks are one 32-byte sector of global memory, consecutive
-    // groups of 8 walk along the same rows, and with chunk columns 128 * 16 + 64 bytes apart the 8
-    // 16-byte stores of a quarter warp fall into 8 different bank groups.
-    constexpr int kSlots = kTcBM * (kTcKMax / 4) / kTcProducers;  // 2 for A and 2 for B
-    static_assert(kSlots * kTcProducers == kTcBM * (kTcKMax / 4), "slots per producer");
-    float4 ra0[kSlots], rb0[kSlots], ra1[kSlots], rb1[kSlots];   // two K blocks in flight
-    const int nchf = p.kblk / 4;                                 // chunks per full block
-    const int tail = p.run - (p.nblk - 1) * p.kblk;              // floats of a run's last block (even; VEC: multiple of 4)
-    const float* gA[kSlots];
-    const float* gB[kSlots];
-    int soA[kSlots], soB[kSlots];
-    unsigned tailA = 0, tailB = 0;        // bit q: slot q has data in the last block of a run ...
-    unsigned tailA2 = 0, tailB2 = 0;      // ... but only its first complex number (8-byte variant)
-    unsigned oddB = 0;                    // bit q: slot q stages an "imaginary" column
-    unsigned live = 0;                    // bit q: slot q is written at all (zeros if its pointer is null)
-#pragma unroll
-    for (int q = 0; q < kSlots; ++q) {
-      const int e = pt + kTcProducers * q;
-      if (e < kTcBM * nchf) live |= 1u << q;
-      {
-        int r, ch;
-        if (a_str) { r = e % kTcBM; ch = e / kTcBM; } else { tc_slot_contiguous(e, nchf, r, ch); }
-        const int gr = row0 + r;
-        const bool okA = r < kTcBM && ch < nchf && gr < M;
-        const int ro = gr / RI, ri = gr - ro * RI;
-        long base;
-        if (OP == kTcFwd)        base = ((spec0 + (long)ro * L) * p.nb + ri) * fi2;
-        else if (OP == kTcGradX) base = ((spec0 + (long)ro * L) * p.nb + ri) * fo2;
-        else if (OP == kTcGradY) base = (spec0 + ro) * p.nb * fi2 + 2 * ri;
-        else                       base = (long)gr * p.a_rs;
-        base += (long)o_lo * a_ko + (a_str ? (long)(2 * ch) * a_st : 4 * ch);
-        gA[q] = okA ? p.a + base : nullptr;
-        soA[q] = ch * kTcLBO + r * 16;
-        if (4 * ch < tail) tailA |= 1u << q;
-        if (tail - 4 * ch == 2) tailA2 |= 1u << q;
-      }
-      {
-        int rr, ch;
-        if (b_str) { rr = e % kTcBN; ch = e / kTcBN; } else { tc_slot_contiguous(e, nchf, rr, ch); }
-        const int gcol = col0 + rr;
-        const bool okB = rr < kTcBN && ch < nchf && gcol < Np;
-        const int co = gcol / CW, rem = gcol - co * CW;
-        const int in = rem >> 1;
-        if (rem & 1) oddB |= 1u << q;
-        long base;
-        if (OP == kTcFwd)        base = ((spec0 + (long)co * L) * p.fi * p.fo + in) * 2;
-        else if (OP == kTcGradX) base = ((spec0 + co) * p.fi + in) * fo2;
-        else if (OP == kTcGradY) base = (spec0 + co) * p.nb * fo2 + 2 * in;
-        else                       base = (long)gcol * p.b_rs;
-        base += (long)o_lo * b_ko + (b_str ? (long)(2 * ch) * b_st : 4 * ch);
-        gB[q] = okB ? p.b + base : nullptr;
-        soB[q] = ch * kTcLBO + rr * 16;
-        if (4 * ch < tail) tailB |= 1u << q;
-        if (tail - 4 * ch == 2) tailB2 |= 1u << q;
-      }
+    // row operand: this thread's row = its TMEM lane
+    const float* gA = nullptr;
+    {
+      const int gr = row0 + 32 * (warp & 3) + lane;
+      const int ro = gr / RI, ri = gr - ro * RI;
+      long base;
+      if (OP == kTcFwd)        base = ((spec0 + (long)ro * L) * p.nb + ri) * fi2;
+      else if (OP == kTcGradX) base = ((spec0 + (long)ro * L) * p.nb + ri) * fo2;
+      else if (OP == kTcGradY) base = (spec0 + ro) * p.nb * fi2 + 2 * ri;
+      else                       base = (long)gr * p.a_rs;
+      if (gr < M) gA = p.a + base;
     }
-    // offsets (floats) from K block 0 to the next block of a run / to block 0 of the next outer index
-    const long a_stepk = a_str ? (long)(p.kblk >> 1) * a_st : p.kblk;
-    const long b_stepk = b_str ? (long)(p.kblk >> 1) * b_st : p.kblk;
-    const long a_stepo = a_ko - (long)(p.nblk - 1) * a_stepk;
-    const long b_stepo = b_ko - (long)(p.nblk - 1) * b_stepk;
+    // column operand: complex column t % 64, pairs 6 (t / 64) .. + 5 of the block; plain products: column t, all
+    constexpr int kBPairs = plain ? kTcKMax / 2 : kTcKMax / 4;
+    const int bcol = plain ? t : (t & 63), bp0 = plain ? 0 : kBPairs * (t >> 6);
+    const float* gB = nullptr;
+    {
+      const int gcol = col0 + (plain ? bcol : 2 * bcol);
+      const int co = gcol / CW, in = (gcol - co * CW) >> 1;
+      long base;
+      if (OP == kTcFwd)        base = ((spec0 + (long)co * L) * p.fi * p.fo + in) * 2;
+      else if (OP == kTcGradX) base = ((spec0 + co) * p.fi + in) * fo2;
+      else if (OP == kTcGradY) base = (spec0 + co) * p.nb * fo2 + 2 * in;
+      else                       base = (long)gcol * p.b_rs;
+      if (gcol < Np) gB = p.b + base + (long)bp0 * b_st;
+    }
+    // offsets (floats) from one block of a run to the next
+    const long a_stepk = (long)(p.kblk >> 1) * a_st, b_stepk = (long)(p.kblk >> 1) * b_st;
 
-    // four consecutive K floats of one row: (re, im) of two complex numbers
-    auto load4 = [&](const float* src, bool strided, long st, bool only_first) {
-      if (VEC && !strided) return __ldg(reinterpret_cast<const float4*>(src));
-      const float2 u = __ldg(reinterpret_cast<const float2*>(src));
-      float2 w = make_float2(0.f, 0.f);
-      if (VEC || !only_first) w = __ldg(reinterpret_cast<const float2*>(src + (strided ? st : 2)));
-      return make_float4(u.x, u.y, w.x, w.y);
-    };
-    // the cursor of the loads runs two K blocks ahead of the one being staged
-    long cur_a = kb_lo * a_stepk, cur_b = kb_lo * b_stepk;
-    int cur_kb = kb_lo;
-    unsigned validA = 0, validB = 0;      // bit q: slot q has a source address at all
+    float2 ra[kTcKMax / 2], rb[kBPairs];                         // the block to be staged next
+    // `cnt` pairs, `step` floats apart (2: consecutive), zeros beyond; null: a row outside the problem
+    auto load_pairs = [&](auto& r, const float* src, bool strided, long step, int cnt) {
+      constexpr int n = sizeof(r) / sizeof(float2);
+      if (VEC && !strided) {                                     // cnt is even, 16-byte aligned
 #pragma unroll
-    for (int q = 0; q < kSlots; ++q) {
-      if (gA[q]) validA |= 1u << q;
-      if (gB[q]) validB |= 1u << q;
-    }
-    auto prefetch = [&](float4 (&ra)[kSlots], float4 (&rb)[kSlots]) {
-      const bool last = cur_kb + 1 == p.nblk;
-      if (!last) {
-        // a full block: every slot that has a source is loaded; the others hold the zeros they were
-        // given before the loop (or by the last block of the previous run)
-#pragma unroll
-        for (int q = 0; q < kSlots; ++q) {
-          if ((validA >> q) & 1u) ra[q] = load4(gA[q] + cur_a, a_str, a_st, false);
-          if ((validB >> q) & 1u) rb[q] = load4(gB[q] + cur_b, b_str, b_st, false);
+        for (int q = 0; q < n; q += 2) {
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (src && q < cnt) v = __ldg(reinterpret_cast<const float4*>(src + 2 * q));
+          r[q] = make_float2(v.x, v.y);
+          r[q + 1] = make_float2(v.z, v.w);
         }
-        ++cur_kb; cur_a += a_stepk; cur_b += b_stepk;
-        return;
-      }
+      } else {
 #pragma unroll
-      for (int q = 0; q < kSlots; ++q) {
-        ra[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (((validA & tailA) >> q) & 1u)
-          ra[q] = load4(gA[q] + cur_a, a_str, a_st, (tailA2 >> q) & 1u);
-        rb[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (((validB & tailB) >> q) & 1u)
-          rb[q] = load4(gB[q] + cur_b, b_str, b_st, (tailB2 >> q) & 1u);
+        for (int q = 0; q < n; ++q) {
+          r[q] = make_float2(0.f, 0.f);
+          if (src && q < cnt) r[q] = __ldg(reinterpret_cast<const float2*>(src + q * step));
+        }
       }
-      cur_kb = 0; cur_a += a_stepo; cur_b += b_stepo;
     };
-    // v = hi + lo with hi carrying the 10 explicit TF32 mantissa bits (the tensor core ignores the
-    // lower 13 bits of its inputs, so lo = v - hi needs no further rounding)
-    auto split_store = [&](unsigned char* hi_buf, unsigned char* lo_buf, int so, float4 v) {
-      float4 hi, lo;
-      hi.x = __uint_as_float(__float_as_uint(v.x) & 0xFFFFE000u);
-      hi.y = __uint_as_float(__float_as_uint(v.y) & 0xFFFFE000u);
-      hi.z = __uint_as_float(__float_as_uint(v.z) & 0xFFFFE000u);
-      hi.w = __uint_as_float(__float_as_uint(v.w) & 0xFFFFE000u);
-      lo.x = v.x - hi.x;
-      lo.y = v.y - hi.y;
-      lo.z = v.z - hi.z;
-      lo.w = v.w - hi.w;
-      *reinterpret_cast<float4*>(hi_buf + so) = hi;
-      *reinterpret_cast<float4*>(lo_buf + so) = lo;
+    int cur_o = o_lo, cur_kb = kb_lo + group;                    // the block loaded next
+    while (cur_kb >= p.nblk) { cur_kb -= p.nblk; ++cur_o; }
+    auto prefetch = [&]() {
+      const int cnt = cur_kb + 1 == p.nblk ? tail : nprs;
+      load_pairs(ra, gA ? gA + cur_o * a_ko + cur_kb * a_stepk : nullptr, a_str, a_st, cnt);
+      load_pairs(rb, gB ? gB + cur_o * b_ko + cur_kb * b_stepk : nullptr, b_str, b_st, cnt - bp0);
+      cur_kb += kTcGroups;
+      while (cur_kb >= p.nblk) { cur_kb -= p.nblk; ++cur_o; }
     };
-    // Real rows of the column operand, per complex number (a, b) of the run:
-    //   fwd, grad y (conjugated operand):  even column (a, b)    odd column (-b, a)
-    //   grad x (plain product):            even column (a, -b)   odd column ( b, a)
-    constexpr bool conj_b = OP != kTcGradX;
-    auto column_rows = [&](float4 v, bool odd) {
-      if (plain) return v;
-      if (conj_b) return odd ? make_float4(-v.y, v.x, -v.w, v.z) : v;
-      return odd ? make_float4(v.y, v.x, v.w, v.z) : make_float4(v.x, -v.y, v.z, -v.w);
+    // two adjacent pairs of one row: 16 bytes of the hi and of the lo buffer
+    auto store_split = [&](unsigned char* dst, float2 u, float2 w) {
+      const float4 hi = make_float4(tc_hi(u.x), tc_hi(u.y), tc_hi(w.x), tc_hi(w.y));
+      *reinterpret_cast<float4*>(dst) = hi;
+      *reinterpret_cast<float4*>(dst + kTcBufBytes) = make_float4(u.x - hi.x, u.y - hi.y, w.x - hi.z, w.y - hi.w);
     };
-
-    // stage K block `it` from the registers that hold it, then refill them with block it + 2
-    auto stage_block = [&](int it, float4 (&ra)[kSlots], float4 (&rb)[kSlots]) {
+    if (group < nit) prefetch();
+    // tcgen05.st is executed by whole warps: the exits of this loop are decided by votes
+    auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };
+    for (int it = group; it < nit; it += kTcGroups) {
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
       const int s = it % kTcStages;
-      unsigned char* stage = smem + (size_t)s * kTcStageBytes;
-      if (it >= kTcStages) {  // the MMAs that read this stage kTcStages blocks ago must have finished
-        if (!wait(&empty[s], (uint32_t)((it / kTcStages - 1) & 1))) return false;
+      if (it >= kTcStages) {   // the MMAs that read this stage kTcStages blocks ago must have finished
+        if (!warp_wait(&empty[s], (uint32_t)((it / kTcStages - 1) & 1))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
+      // ---- column operand.  Real rows per complex number (a, b) of the run:
+      //   fwd, grad y (conjugated operand):  real column (a, b)    imaginary column (-b, a)
+      //   grad x (plain product):            real column (a, -b)   imaginary column ( b, a)
+      unsigned char* stage = smem + (size_t)s * kTcStageBytes + bcol * 16 + (bp0 / 2) * kTcLBO;
 #pragma unroll
-      for (int q = 0; q < kSlots; ++q) {
-        if ((live >> q) & 1u) {
-          float4 va = ra[q];
-          if (OP == kTcPlainCC)   // (__fmul_rn: the product must not be contracted into the hi / lo split)
-            va = make_float4(__fmul_rn(va.x, p.a_scale), __fmul_rn(va.y, p.a_scale),
-                             __fmul_rn(va.z, p.a_scale), __fmul_rn(va.w, p.a_scale));
-          split_store(stage, stage + kTcBufBytes, soA[q], va);
-          split_store(stage + 2 * kTcBufBytes, stage + 3 * kTcBufBytes, soB[q],
-                      column_rows(rb[q], (oddB >> q) & 1u));
+      for (int q = 0; q < kBPairs; q += 2) {
+        if (bp0 + q >= nprs) break;
+        const float2 u = rb[q], w = rb[q + 1];
+        unsigned char* dst = stage + (q / 2) * kTcLBO;
+        if (plain) {
+          store_split(dst, u, w);
+        } else if (OP == kTcGradX) {
+          store_split(dst, make_float2(u.x, -u.y), make_float2(w.x, -w.y));
+          store_split(dst + 64 * 16, make_float2(u.y, u.x), make_float2(w.y, w.x));
+        } else {
+          store_split(dst, u, w);
+          store_split(dst + 64 * 16, make_float2(-u.y, u.x), make_float2(-w.y, w.x));
         }
       }
-      if (it + 2 < nit) prefetch(ra, rb);
-      // make the generic-proxy writes visible to the tensor core (async proxy), then hand over:
-      // one arrival per producer warp
+      // make the generic-proxy writes visible to the tensor core (async proxy)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      // ---- row operand, once the block two before has been read
+      if (it >= kTcAStages) {
+        const int e = it - kTcAStages;
+        if (!warp_wait(&empty[e % kTcStages], (uint32_t)((e / kTcStages) & 1))) break;
+      }
       __syncwarp();
-      if (lane == 0)
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem_u32(&full[s])) : "memory");
-      return true;
-    };
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t ta = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + kTcACol + (uint32_t)(it % kTcAStages) * kTcAPitch;
 #pragma unroll
-    for (int q = 0; q < kSlots; ++q)
-      ra0[q] = rb0[q] = ra1[q] = rb1[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    prefetch(ra0, rb0);
-    if (nit > 1) prefetch(ra1, rb1);
-    for (int it = 0; it < nit && !*abort_flag; it += 2) {
-      if (!stage_block(it, ra0, rb0)) break;
-      if (it + 1 < nit && !stage_block(it + 1, ra1, rb1)) break;
+      for (int ks = 0; ks < kTcKMax / 8; ++ks) {
+        if (4 * ks >= nprs) break;
+        float hi[8], lo[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float2 v = ra[4 * ks + i];
+          if (OP == kTcPlainCC)   // (__fmul_rn: the product must not be contracted into the hi / lo split)
+            v = make_float2(__fmul_rn(v.x, p.a_scale), __fmul_rn(v.y, p.a_scale));
+          hi[2 * i] = tc_hi(v.x); hi[2 * i + 1] = tc_hi(v.y);
+          lo[2 * i] = v.x - hi[2 * i]; lo[2 * i + 1] = v.y - hi[2 * i + 1];
+        }
+        tc_st8(ta + 8 * ks, hi);
+        tc_st8(ta + kTcALo + 8 * ks, lo);
+      }
+      if (it + kTcGroups < nit) prefetch();
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)   // hand over: one arrival per producer warp
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem_u32(&full[s])) : "memory");
     }
   }
 
@@ -623,10 +593,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     const uint32_t last_acc = FLUSH ? (uint32_t)(((ngroups - 1) & 1) * kTcBN) : 0u;
     const int cbase = kColsPerWarp * cg;
     float v[32];
-    tc_ld32(tmem_base + ((uint32_t)(32 * q) << 16) + last_acc + (uint32_t)cbase, v);
+    // 32 result columns of a lane's row; spectral products: real and imaginary columns from the two halves
+    auto load_columns = [&](uint32_t region, float (&o)[32]) {
+      const uint32_t base = tmem_base + ((uint32_t)(32 * q) << 16) + region;
+      if constexpr (OP == kTcPlainCC || OP == kTcPlainSC) {
+        tc_ld32(base + (uint32_t)cbase, o);
+      } else {
+        float re[16], im[16];
+        tc_ld16(base + (uint32_t)(cbase / 2), re);
+        tc_ld16(base + (uint32_t)(kTcBN / 2 + cbase / 2), im);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { o[2 * i] = re[i]; o[2 * i + 1] = im[i]; }
+      }
+    };
+    load_columns(last_acc, v);
     if (FLUSH && ngroups > 1) {
       float w[32];
-      tc_ld32(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(kTcSumCol + cbase), w);
+      load_columns((uint32_t)kTcSumCol, w);
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] += w[i];
     }
