@@ -278,7 +278,8 @@ struct so3_inv_fused_impl {
             for (int bi = 0; bi < 4; ++bi)
 #pragma unroll
               for (int z = 0; z < ZG; ++z) {
-                s[bi][z] = fma2(make_float2(wv[bi], wv[bi]), xv[z], s[bi][z]);
+                s[bi][z].x = fmaf(wv[bi], xv[z].x, s[bi][z].x);
+                s[bi][z].y = fmaf(wv[bi], xv[z].y, s[bi][z].y);
               }
           }
           float2* pl = planes + info.z * KP + info.w;
@@ -306,7 +307,8 @@ struct so3_inv_fused_impl {
 #pragma unroll
           for (int z = 0; z < ZG; ++z) {
             const float2 xv = xh_at(xrow + li, z);
-            acc[z] = fma2(make_float2(wv, wv), xv, acc[z]);
+            acc[z].x = fmaf(wv, xv.x, acc[z].x);
+            acc[z].y = fmaf(wv, xv.y, acc[z].y);
           }
         }
         float2* pl = planes + (size_t)bi * plane_sz + info.z * KP + info.w;

@@ -42,7 +42,8 @@
 // With both operands in shared memory a K block moved 48 KB of stores and 72 KB of MMA reads through a
 // 128-byte-per-clock pipe (960 clocks) and its producers, every warp taking part in every block, issued
 // about 1600 instructions: 1250 clocks per block measured, 480 us for 100 -> 100 channels at nl = 10, batch 32.
-// Now 24 KB of stores and 36 KB of reads remain, beside 600 - 750 clocks of MMA.
+// Now 24 KB of stores and 36 KB of reads remain; 820 clocks per block in a lone CTA, 960 on a full chip, where
+// nine 128 x 128 x 8 MMAs alone take 750.
 // The epilogue (all 16 non-issuer warps) reads the last accumulator and the sum region with
 // tcgen05.ld (32 lanes x 16 real and 16 imaginary columns per warp) and stores the result directly in
 // its interleaved layout.  Every mbarrier wait is bounded; on a time-out the waiting thread raises a
@@ -189,6 +190,14 @@ __device__ __forceinline__ void tc_mma_tf32(uint32_t tmem_d, uint32_t tmem_a, ui
       : "memory");
 }
 
+// One lane of a converged warp, elected in a way the compiler can follow: the code it guards then runs on
+// uniform registers.  With "lane == 0" every tcgen05.mma / commit first moved its operands there one by one,
+// about 70 clocks per instruction and 300 - 600 between K blocks (1280 -> 820 clocks per block of a lone CTA).
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    tc_smem_u32(bar))
@@ -290,7 +299,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   uint64_t* accfree = accdone + 2;                                   // [2] collectors -> issuer
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfree + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
   // ---- which tile ---------------------------------------------------------------------------
   int l = p.nl - 1;
@@ -342,7 +351,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   bool ok = true;
   // a wait that gives up tells every role to leave its loop
@@ -368,12 +377,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     const int steps_tail = (p.run - (p.nblk - 1) * p.kblk + 7) / 8;
     int kb = kb_lo, s = 0, g = 0, ing = 0;           // block within its run, stage, group, block within its group
     uint32_t full_par = 0;                        // parity of the `full` phase of the current round of stages
-    for (int it = 0; it < nit && !*abort_flag; ++it) {
+    for (int it = 0; it < nit; ++it) {
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
       if (FLUSH && ing == 0 && g >= 2)            // the collectors are done with this accumulator
-        if (!wait(&accfree[g & 1], (uint32_t)((g / 2 - 1) & 1))) break;
-      if (!wait(&full[s], full_par)) break;
+        if (!__all_sync(0xffffffffu, wait(&accfree[g & 1], (uint32_t)((g / 2 - 1) & 1)))) break;
+      if (!__all_sync(0xffffffffu, wait(&full[s], full_par))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (lane == 0) {
+      if (tc_elect()) {
         const int ksteps = kb + 1 == p.nblk ? steps_tail : steps_full;
         const uint64_t db = d0 + (uint64_t)s * kDStage;
         const uint32_t ta = tmem_base + kTcACol + (uint32_t)(it % kTcAStages) * kTcAPitch;
@@ -558,12 +568,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
         tc_st8(ta + 8 * ks, hi);
         tc_st8(ta + kTcALo + 8 * ks, lo);
       }
-      if (it + kTcGroups < nit) prefetch();
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0)   // hand over: one arrival per producer warp
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem_u32(&full[s])) : "memory");
+      if (it + kTcGroups < nit) prefetch();   // (after the hand-over: the loads take a few hundred clocks to issue)
     }
   }
 

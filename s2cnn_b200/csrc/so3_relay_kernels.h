@@ -216,7 +216,8 @@ struct so3_relay_fused_impl {
             for (int bi = 0; bi < 4; ++bi)
 #pragma unroll
               for (int z = 0; z < ZG; ++z) {
-                s[bi][z] = fma2(make_float2(wv[bi], wv[bi]), xv[z], s[bi][z]);
+                s[bi][z].x = fmaf(wv[bi], xv[z].x, s[bi][z].x);
+                s[bi][z].y = fmaf(wv[bi], xv[z].y, s[bi][z].y);
               }
           }
           float2* pl = planes + info.z * KP + info.w;
@@ -244,7 +245,8 @@ struct so3_relay_fused_impl {
 #pragma unroll
           for (int z = 0; z < ZG; ++z) {
             const float2 xv = xh_at(xrow + li, z);
-            s[z] = fma2(make_float2(wv, wv), xv, s[z]);
+            s[z].x = fmaf(wv, xv.x, s[z].x);
+            s[z].y = fmaf(wv, xv.y, s[z].y);
           }
         }
         float2* pl = planes + (size_t)bi * plane_sz + info.z * KP + info.w;
@@ -364,7 +366,8 @@ struct so3_relay_fused_impl {
 #pragma unroll
           for (int z = 0; z < ZG; ++z) {
             const float2 xv = src[(size_t)(z * p.BG + bi) * plane_sz];
-            a[z] = fma2(make_float2(wv, wv), xv, a[z]);
+            a[z].x = fmaf(wv, xv.x, a[z].x);
+            a[z].y = fmaf(wv, xv.y, a[z].y);
           }
         }
         acc4[r] = make_float4(a[0].x, a[0].y, a[1].x, a[1].y);
