@@ -22,6 +22,7 @@
 #include "wigner_tiled.h"
 #include "wigner_rows.h"
 #include "cgemm_kernels.h"
+#include "rotate_kernels.h"
 #include "s2_mm_thin.h"
 #include "so3_mm_tc.h"
 #include "misc_kernels.h"
@@ -1240,11 +1241,10 @@ int s2c_so3_rotate_spectrum(const float* U, const float* x, float* z, int b, lon
                             int adjoint, void* st) {
   if (!U || !x || !z || b < 1 || nbatch < 1 || nbatch > 0x7fffffffL / (2 * b))
     return fail(S2C_ERR_BAD_ARG, "s2c_so3_rotate_spectrum: bad argument");
-  CgemmParams p = rotation_params(b, nbatch, adjoint ? 1 : 0);
-  p.A = (const float2*)U;
-  p.B = (const float2*)x;
-  p.C = (float2*)z;
-  return S2C_LAUNCH(cgemm_grouped, cgemm_total_tiles(p), 256, cgemm_smem_bytes(), as_stream(st), p);
+  RotateParams p;
+  p.U = (const float2*)U; p.x = (const float2*)x; p.z = (float2*)z;
+  p.nl = b; p.adjoint = adjoint != 0; p.nbatch = nbatch;
+  return S2C_LAUNCH(so3_rotate_rows, rot_blocks(b, nbatch), kRotThreads, rot_smem_bytes(b), as_stream(st), p);
 }
 
 

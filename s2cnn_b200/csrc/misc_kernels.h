@@ -167,14 +167,27 @@ struct IntegrateBwdParams {
 };
 
 S2C_KERNEL(so3_integrate_bwd, IntegrateBwdParams) {
-  const int plane = p.N * p.N;
-  const long per = (long)p.N * plane;
-  for (long e = (long)ctx.bid * ctx.nthr + ctx.tid; e < p.total; e += (long)ctx.nblk * ctx.nthr) {
-    const long z = e / per;
-    const int beta = (int)((e - z * per) / plane);
-    float v = p.g[z] * p.w[beta];
-    if (p.relu && !(p.x[e] > 0.f)) v = 0.f;
-    p.gx[e] = v;
+  // a block writes whole (z, beta) planes, 16 bytes per thread ((2b)^2 is a multiple of 4): one index split per
+  // plane instead of two 64-bit divisions per sample (3200 signals at b = 5: 29 us)
+  const int plane4 = p.N * p.N / 4;
+  const long planes = p.total / ((long)plane4 * 4);
+  const int per = ctx.nthr / plane4 > 0 ? ctx.nthr / plane4 : 1;       // planes side by side in a block
+  const int sub = plane4 < ctx.nthr ? ctx.tid / plane4 : 0;
+  const int first = plane4 < ctx.nthr ? ctx.tid - sub * plane4 : ctx.tid, step = plane4 < ctx.nthr ? plane4 : ctx.nthr;
+  if (sub >= per) return;
+  for (long pl = (long)ctx.bid * per + sub; pl < planes; pl += (long)ctx.nblk * per) {
+    const long z = pl / p.N;
+    const float v = p.g[z] * p.w[pl - z * p.N];
+    float4* o = reinterpret_cast<float4*>(p.gx) + pl * plane4;
+    const float4* x = reinterpret_cast<const float4*>(p.x) + pl * plane4;
+    for (int e = first; e < plane4; e += step) {
+      float4 r = make_float4(v, v, v, v);
+      if (p.relu) {
+        const float4 a = x[e];
+        r = make_float4(a.x > 0.f ? v : 0.f, a.y > 0.f ? v : 0.f, a.z > 0.f ? v : 0.f, a.w > 0.f ? v : 0.f);
+      }
+      o[e] = r;
+    }
   }
 }
 

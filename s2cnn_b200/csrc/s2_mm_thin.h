@@ -117,21 +117,39 @@ S2C_KERNEL_BOUNDS(s2_mm_grady_thin, S2ThinParams, 1024, 1) {
   float2 acc[kThinFi];
 #pragma unroll
   for (int k = 0; k < kThinFi; ++k) acc[k] = make_float2(0.f, 0.f);
+  // the rows (m, i) in one run over the slices, four in flight: with a loop over m around one over i a batch
+  // smaller than the slices left most threads idle and every m waited for its own loads (f_out = 8, batch 32,
+  // b = 30: 168 us)
   if (sl < nsl) {
-    for (int m = 0; m < L; ++m) {
-      const float2* g = p.gz + (((long)so3_offset(l) + (long)m * L + n) * p.nb) * p.fo + j;
-      const float2* xr = p.other + ((long)(l * l + m) * p.nb) * p.fi;
-#pragma unroll 4
-      for (int i = sl; i < p.nb; i += nsl) {
-        const float2 gv = g[(long)i * p.fo];
+    const float2* g0 = p.gz + ((long)so3_offset(l) + n) * p.nb * p.fo + j;
+    const float2* x0 = p.other + (long)l * l * p.nb * p.fi;
+    const long gm = (long)L * p.nb * p.fo;                  // from m to m + 1
+    const int rows = L * p.nb, dm = nsl / p.nb, di = nsl - dm * p.nb;
+    int m = sl / p.nb, i = sl - m * p.nb;
+    for (int q = sl; q < rows; q += 4 * nsl) {
+      float2 gv[4];
+      int rq[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        rq[u] = q + u * nsl;
+        gv[u] = make_float2(0.f, 0.f);
+        if (rq[u] < rows) gv[u] = g0[m * gm + (long)i * p.fo];
+        m += dm;
+        i += di;
+        if (i >= p.nb) { i -= p.nb; ++m; }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (rq[u] >= rows) break;
+        const float2* xr = x0 + (long)rq[u] * p.fi;         // rows of x are contiguous in (m, i)
 #pragma unroll
         for (int k = 0; k < kThinFi; ++k) {
           if (k < p.fi) {
-            const float2 xv = xr[i * p.fi + k];   // conj(gv) * xv
-            acc[k].x = fmaf(gv.x, xv.x, acc[k].x);
-            acc[k].x = fmaf(gv.y, xv.y, acc[k].x);
-            acc[k].y = fmaf(gv.x, xv.y, acc[k].y);
-            acc[k].y = fmaf(-gv.y, xv.x, acc[k].y);
+            const float2 xv = xr[k];   // conj(gv) * xv
+            acc[k].x = fmaf(gv[u].x, xv.x, acc[k].x);
+            acc[k].x = fmaf(gv[u].y, xv.y, acc[k].x);
+            acc[k].y = fmaf(gv[u].x, xv.y, acc[k].y);
+            acc[k].y = fmaf(-gv[u].y, xv.x, acc[k].y);
           }
         }
       }

@@ -62,11 +62,11 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
   // threads share the beta loop; at most two tiles per thread either way (LT <= 16, 256 threads)
   const bool narrow = LT * ZH < ctx.nthr;
   const int ntiles = narrow ? LT * zc : LT * ZH;
-  float2 acc[2][4][2];
+  float ar[2][4][2], ai[2][4][2];
 #pragma unroll
   for (int t = 0; t < 2; ++t)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[t][i][0] = acc[t][i][1] = make_float2(0.f, 0.f);
+    for (int i = 0; i < 4; ++i) { ar[t][i][0] = ar[t][i][1] = ai[t][i][0] = ai[t][i][1] = 0.f; }
 
   {
     if (N % 4 == 0) {
@@ -138,10 +138,10 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const float4 w4 = *reinterpret_cast<const float4*>(wp + i * LDW + bt);
-            acc[t][i][0] = fma2(make_float2(w4.x, w4.x), make_float2(va.x, va.y), acc[t][i][0]);
-            acc[t][i][0] = fma2(make_float2(w4.y, w4.y), make_float2(va.z, va.w), acc[t][i][0]);
-            acc[t][i][0] = fma2(make_float2(w4.z, w4.z), make_float2(vb.x, vb.y), acc[t][i][0]);
-            acc[t][i][0] = fma2(make_float2(w4.w, w4.w), make_float2(vb.z, vb.w), acc[t][i][0]);
+            ar[t][i][0] = fmaf(w4.x, va.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4.x, va.y, ai[t][i][0]);
+            ar[t][i][0] = fmaf(w4.y, va.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4.y, va.w, ai[t][i][0]);
+            ar[t][i][0] = fmaf(w4.z, vb.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4.z, vb.y, ai[t][i][0]);
+            ar[t][i][0] = fmaf(w4.w, vb.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4.w, vb.w, ai[t][i][0]);
           }
         }
       } else {
@@ -159,14 +159,14 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
           const float4 b1 = *reinterpret_cast<const float4*>(v1 + bt + 2);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            acc[t][i][0] = fma2(make_float2(w4[i].x, w4[i].x), make_float2(a0.x, a0.y), acc[t][i][0]);
-            acc[t][i][0] = fma2(make_float2(w4[i].y, w4[i].y), make_float2(a0.z, a0.w), acc[t][i][0]);
-            acc[t][i][0] = fma2(make_float2(w4[i].z, w4[i].z), make_float2(b0.x, b0.y), acc[t][i][0]);
-            acc[t][i][0] = fma2(make_float2(w4[i].w, w4[i].w), make_float2(b0.z, b0.w), acc[t][i][0]);
-            acc[t][i][1] = fma2(make_float2(w4[i].x, w4[i].x), make_float2(a1.x, a1.y), acc[t][i][1]);
-            acc[t][i][1] = fma2(make_float2(w4[i].y, w4[i].y), make_float2(a1.z, a1.w), acc[t][i][1]);
-            acc[t][i][1] = fma2(make_float2(w4[i].z, w4[i].z), make_float2(b1.x, b1.y), acc[t][i][1]);
-            acc[t][i][1] = fma2(make_float2(w4[i].w, w4[i].w), make_float2(b1.z, b1.w), acc[t][i][1]);
+            ar[t][i][0] = fmaf(w4[i].x, a0.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].x, a0.y, ai[t][i][0]);
+            ar[t][i][0] = fmaf(w4[i].y, a0.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].y, a0.w, ai[t][i][0]);
+            ar[t][i][0] = fmaf(w4[i].z, b0.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].z, b0.y, ai[t][i][0]);
+            ar[t][i][0] = fmaf(w4[i].w, b0.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].w, b0.w, ai[t][i][0]);
+            ar[t][i][1] = fmaf(w4[i].x, a1.x, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].x, a1.y, ai[t][i][1]);
+            ar[t][i][1] = fmaf(w4[i].y, a1.z, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].y, a1.w, ai[t][i][1]);
+            ar[t][i][1] = fmaf(w4[i].z, b1.x, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].z, b1.y, ai[t][i][1]);
+            ar[t][i][1] = fmaf(w4[i].w, b1.z, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].w, b1.w, ai[t][i][1]);
           }
         }
       }
@@ -175,8 +175,7 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
 
   const float fudge = ((m - n) & 1) ? -1.f : 1.f;
   const bool self = (m == 0 && n == 0);
-  auto emit = [&](int li, int zz, float2 v) {
-    const float re = v.x, im = v.y;
+  auto emit = [&](int li, int zz, float re, float im) {
     if (li >= L || zz >= zc) return;
     const int l = lmin + li;
     if (p.mode == kS2) {
@@ -204,13 +203,13 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
     if (narrow) {
       const int tl = tile / zc, zz = tile - tl * zc;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) emit(4 * tl + i, zz, acc[t][i][0]);
+      for (int i = 0; i < 4; ++i) emit(4 * tl + i, zz, ar[t][i][0], ai[t][i][0]);
     } else {
       const int tl = tile / ZH, tz = tile - tl * ZH;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        emit(4 * tl + i, tz, acc[t][i][0]);
-        emit(4 * tl + i, tz + ZH, acc[t][i][1]);
+        emit(4 * tl + i, tz, ar[t][i][0], ai[t][i][0]);
+        emit(4 * tl + i, tz + ZH, ar[t][i][1], ai[t][i][1]);
       }
     }
   }
