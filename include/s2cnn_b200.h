@@ -88,8 +88,7 @@ int s2c_so3_rfft(const float* x, float* out, long nbatch, int b_in, int b_out, i
                  void* workspace, size_t workspace_bytes, void* stream);
 /* s2c_so3_rfft of max(x, 0): the ReLU that precedes an SO3Convolution in the reference's models
  * (e.g. examples/mnist/run.py:88-93) applied while the signal is read, so the activated tensor
- * never exists in memory.  Only for 2 b_in <= 32 (single-kernel path); other sizes return
- * "unsupported". */
+ * never exists in memory.  Only for 2 b_in < 64; other sizes return "unsupported". */
 int s2c_so3_rfft_relu(const float* x, float* out, long nbatch, int b_in, int b_out,
                       void* workspace, size_t workspace_bytes, void* stream);
 /* s2c_so3_rfft plus one by-product: sums [nbatch] = the plain sum of every signal over its (2b)^3
@@ -100,6 +99,9 @@ int s2c_so3_rfft_relu(const float* x, float* out, long nbatch, int b_in, int b_o
  * and write nothing. */
 int s2c_so3_rfft_sums(const float* x, float* out, float* sums, long nbatch, int b_in, int b_out,
                       int for_grad, void* stream);
+/* The same with a workspace (s2c_so3_fft_workspace), for 2 b_in < 64. */
+int s2c_so3_rfft_sums_ws(const float* x, float* out, float* sums, long nbatch, int b_in, int b_out,
+                         int for_grad, void* workspace, size_t workspace_bytes, void* stream);
 /* x [nbatch, 2b_in, 2b_in, 2b_in, 2] complex -> out [nspec(b_out), nbatch, 2].
  * Replaces so3_fft, s2cnn/soft/so3_fft.py:12-61. */
 int s2c_so3_fft(const float* x, float* out, long nbatch, int b_in, int b_out, int for_grad,
@@ -115,9 +117,11 @@ int s2c_so3_rifft(const float* x, float* out, long nbatch, int b_in, int b_out, 
 /* Backward of "so3_rfft(relu(a))" with respect to a, in one kernel:
  *   out = so3_rifft(x, for_grad = 1, b_out) where act > 0, else 0
  * x [nspec(b_in), nbatch, 2] = gradient of the spectrum, act [nbatch, 2b_out, 2b_out, 2b_out] = the
- * signal the forward pass read, out of the same shape.  Only for 2 b_out <= 32 (single-kernel path);
- * other sizes return "unsupported".  Replaces the backward of SO3_fft_real (s2cnn/soft/so3_fft.py:
+ * signal the forward pass read, out of the same shape.  Only for 2 b_out <= 32 (single-kernel path), with
+ * a workspace (_ws) for 2 b_out < 64; other sizes return "unsupported".  Replaces the backward of SO3_fft_real (s2cnn/soft/so3_fft.py:
  * 453-456: so3_ifft(for_grad=True), real part) followed by the backward of F.relu. */
+int s2c_so3_rifft_relu_grad_ws(const float* x, const float* act, float* out, long nbatch, int b_in,
+                               int b_out, void* workspace, size_t workspace_bytes, void* stream);
 int s2c_so3_rifft_relu_grad(const float* x, const float* act, float* out, long nbatch, int b_in,
                             int b_out, void* stream);
 /* so3_integrate(relu(so3_rifft(x) + bias)) without writing the signal: out [nbatch] - the tail

@@ -187,8 +187,8 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
                                         fused_threads(sm, (size_t)dev_smem_limit()), sm, st, f));
     return rc;
   }
-  if (relu) return fail(S2C_ERR_UNSUPPORTED, "fused ReLU input needs the small-bandwidth path");
-  if (sums) return fail(S2C_ERR_UNSUPPORTED, "per-signal sums need the small-bandwidth path");
+  if (relu && !use_mid_kernels(N)) return fail(S2C_ERR_UNSUPPORTED, "fused ReLU input needs 2 b < 64");
+  if (sums && (!use_mid_kernels(N) || !ws)) return fail(S2C_ERR_UNSUPPORTED, "per-signal sums need 2 b < 64");
   if (use_plane_kernels(N)) {
     HalfPanelsDev hp;
     hp.nbeta = N; hp.nl = b_out; hp.K = K; hp.npairs = pan.npairs;
@@ -228,11 +228,17 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
       g.x = x + (size_t)z0 * N * N * N * in_stride; g.out = nullptr;
       g.stride = in_stride; g.off = in_off;
       g.v = v; g.tw = fft.tw; g.bias = nullptr; g.nfeat = 1; g.z0 = z0;
+      g.relu = relu; g.mask = nullptr;
       g.nbatch = (int)zc; g.K = K; g.inv_k = 1.f / (float)K;
       int rc = S2C_OK;
       S2C_DISPATCH_MID(N, rc = S2C_LAUNCH_N(so3_fwd_mid, kN, zc * ((kN + mid_nb(kN) - 1) / mid_nb(kN)),
                                             kMidThreads, mid_smem_bytes(kN), st, g));
       if (rc) return rc;
+      if (sums) {
+        MidSumsParams q;
+        q.v = v + (size_t)(K - 1) * zc * N; q.sums = sums + z0; q.nbatch = (int)zc; q.N = N;
+        S2C_TRY(S2C_LAUNCH(so3_mid_sums, (zc + 31) / 32, 32, 0, st, q));
+      }
     } else {
     FwdGammaParams g;
     g.x = x + (size_t)z0 * N * N * N * in_stride;
@@ -365,7 +371,8 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
   }
   if (integral)
     return fail(S2C_ERR_UNSUPPORTED, "fused ReLU + integration needs the small-bandwidth path");
-  if (mask) return fail(S2C_ERR_UNSUPPORTED, "masked synthesis needs the small-bandwidth path");
+  if (mask && (!use_mid_kernels(N) || !ws || out_stride != 1 || out_off != 0))
+    return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output and 2 b < 64");
   if (use_plane_kernels(N)) {
     HalfPanelsDev hp;
     hp.nbeta = N; hp.nl = K; hp.K = K; hp.npairs = pan.npairs;
@@ -411,6 +418,11 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     w.ZT = (int)std::min<long>(32, zc);
     w.nzt = (int)((zc + w.ZT - 1) / w.ZT);
     w.mode = mode;
+    if (prod) {
+      w.xs = prod->xs; w.ys = prod->ys;
+      w.s2_nb = prod->nb; w.s2_fin = prod->fin; w.s2_fout = prod->fout;
+      w.z0 = z0;
+    }
     if (inv_wigner_t_smem(N, K) <= (size_t)dev_smem_limit() - 1024) {
       w.ZT = kWigZT;
       w.nzt = (int)((zc + kWigZT - 1) / kWigZT);
@@ -424,6 +436,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
       MidParams g;
       g.x = nullptr; g.out = out + (size_t)z0 * N * N * N * out_stride;
       g.stride = out_stride; g.off = out_off;
+      g.relu = 0; g.mask = mask ? mask + (size_t)z0 * N * N * N : nullptr;
       g.v = s; g.tw = fft.tw; g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0;
       g.nbatch = (int)zc; g.K = K; g.inv_k = 1.f / (float)K;
       int rc = S2C_OK;
@@ -665,6 +678,15 @@ int s2c_so3_rfft_relu(const float* x, float* out, long nbatch, int b_in, int b_o
                       as_stream(stream), true);
 }
 
+int s2c_so3_rfft_sums_ws(const float* x, float* out, float* sums, long nbatch, int b_in, int b_out,
+                         int for_grad, void* ws, size_t ws_bytes, void* stream) {
+  S2C_TRY(check_b(b_in, b_out));
+  if (!x || !out || !sums || nbatch < 1)
+    return fail(S2C_ERR_BAD_ARG, "s2c_so3_rfft_sums_ws: bad argument");
+  return so3_analysis(x, 1, 0, (float2*)out, nbatch, b_in, b_out, !for_grad, kSo3Real, ws, ws_bytes,
+                      as_stream(stream), false, sums);
+}
+
 int s2c_so3_rfft_sums(const float* x, float* out, float* sums, long nbatch, int b_in, int b_out,
                       int for_grad, void* stream) {
   S2C_TRY(check_b(b_in, b_out));
@@ -696,6 +718,15 @@ int s2c_so3_rifft(const float* x, float* out, long nbatch, int b_in, int b_out, 
   if (bias && nfeature < 1) return fail(S2C_ERR_BAD_ARG, "s2c_so3_rifft: nfeature must be >= 1 with a bias");
   return so3_synthesis((const float2*)x, out, 1, 0, nbatch, b_in, b_out, for_grad != 0, kSo3Real,
                        bias, nfeature, ws, ws_bytes, as_stream(stream));
+}
+
+int s2c_so3_rifft_relu_grad_ws(const float* x, const float* act, float* out, long nbatch, int b_in,
+                               int b_out, void* ws, size_t ws_bytes, void* stream) {
+  S2C_TRY(check_b(b_in, b_out));
+  if (!x || !act || !out || nbatch < 1)
+    return fail(S2C_ERR_BAD_ARG, "s2c_so3_rifft_relu_grad_ws: bad argument");
+  return so3_synthesis((const float2*)x, out, 1, 0, nbatch, b_in, b_out, true, kSo3Real, nullptr, 0,
+                       ws, ws_bytes, as_stream(stream), nullptr, nullptr, act);
 }
 
 int s2c_so3_rifft_relu_grad(const float* x, const float* act, float* out, long nbatch, int b_in,
@@ -802,6 +833,12 @@ int s2c_so3_rifft_relu_rfft(const float* x, float* out, long nbatch, int b_in, i
                       b_in, b_mid, b_next, bias, as_stream(stream), "s2c_so3_rifft_relu_rfft");
 }
 
+// 32 < 2 b < 64: the product is evaluated while the tiled Wigner kernel stages the spectrum (b = 30, 256 signals:
+// 74 MB less to write and read)
+static bool s2_product_in_wigner(int b) {
+  return use_mid_kernels(2 * b) && inv_wigner_t_smem(2 * b, b) <= (size_t)dev_smem_limit() - 1024;
+}
+
 size_t s2c_s2_conv_synthesis_workspace(int nbatch, int f_out, int b) {
   if (so3_synthesis_is_fused(b, b)) return 16;
   const size_t z_bytes = (size_t)so3_nspec(b) * nbatch * f_out * sizeof(float2);
@@ -823,6 +860,13 @@ int s2c_s2_conv_synthesis(const float* xs, const float* ys, float* out, int nbat
                          as_stream(stream), &pr);
   }
   // larger bandwidths: product into the head of the workspace, then the general synthesis
+  if (s2_product_in_wigner(b)) {
+    S2ProductArgs pr;
+    pr.xs = (const float2*)xs; pr.ys = (const float2*)ys;
+    pr.nb = nbatch; pr.fin = f_in; pr.fout = f_out;
+    return so3_synthesis(nullptr, out, 1, 0, nz, b, b, false, kSo3Real, bias, f_out, ws, ws_bytes,
+                         as_stream(stream), &pr);
+  }
   const size_t z_bytes = (size_t)so3_nspec(b) * nz * sizeof(float2);
   if (!ws || ws_bytes <= z_bytes)
     return fail(S2C_ERR_WORKSPACE, "s2c_s2_conv_synthesis: workspace too small");

@@ -296,6 +296,11 @@ struct InvWignerParams {
   float2* s;         // [n][mi][z][beta]
   PanelsDev pan;
   int nbatch, N, K, ZT, nzt, mode;
+  // so3_inv_wigner_t, optional: the spectrum is s2_mm(xs, ys), evaluated while it is staged; z0 = first signal
+  const float2* xs = nullptr;   // [l * m, s2_nb, s2_fin]
+  const float2* ys = nullptr;   // [l * m, s2_fin, s2_fout]
+  int s2_nb = 0, s2_fin = 0, s2_fout = 0;
+  long z0 = 0;
 };
 
 S2C_KERNEL(so3_inv_wigner, InvWignerParams) {

@@ -47,6 +47,8 @@ struct MidParams {
   int nfeat;
   long z0;
   int nbatch, K;
+  int relu;            // analysis: transform max(x, 0)
+  const float* mask;   // synthesis, optional (unit stride): samples where this signal is <= 0 are written as 0
   float inv_k;         // 1 / K (index split without an integer division)
 };
 
@@ -80,6 +82,10 @@ struct so3_fwd_mid_impl {
 #pragma unroll
         for (int k = 0; k < R1; ++k)
           v[k] = make_float2(p.x[(e0 + k * R2) * p.stride + p.off], p.x[(e0 + N + k * R2) * p.stride + p.off]);
+      }
+      if (p.relu) {
+#pragma unroll
+        for (int k = 0; k < R1; ++k) v[k] = make_float2(v[k].x > 0.f ? v[k].x : 0.f, v[k].y > 0.f ? v[k].y : 0.f);
       }
       two_head<N, -1>(v, j, tw);
       float2* a = A + pl * PSA + t * LD + j;
@@ -236,6 +242,13 @@ struct so3_inv_mid_impl {
         r0[2 * i] = u.x + add; r1[2 * i] = u.y + add;
         r0[2 * i + 1] = u.z + add; r1[2 * i + 1] = u.w + add;
       }
+      if (p.mask) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          if (!(p.mask[e0 + i] > 0.f)) r0[i] = 0.f;
+          if (!(p.mask[e0 + N + i] > 0.f)) r1[i] = 0.f;
+        }
+      }
       if (p.stride == 1) {
         if constexpr (W == 4) {
           *reinterpret_cast<float4*>(p.out + e0) = make_float4(r0[0], r0[1], r0[2], r0[3]);
@@ -254,6 +267,20 @@ struct so3_inv_mid_impl {
     }
   }
 };
+
+// by-product of the analysis: the plain sum of every signal, i.e. its (0, 0) bins summed over beta
+struct MidSumsParams {
+  const float2* v;     // V[n = 0][m = 0]: [z][beta]
+  float* sums;
+  int nbatch, N;
+};
+S2C_KERNEL(so3_mid_sums, MidSumsParams) {
+  const int z = ctx.bid * ctx.nthr + ctx.tid;
+  if (z >= p.nbatch) return;
+  float s = 0.f;
+  for (int b = 0; b < p.N; ++b) s += p.v[(long)z * p.N + b].x;
+  p.sums[z] = s;
+}
 
 #ifndef S2C_EMUL
 template <int N>

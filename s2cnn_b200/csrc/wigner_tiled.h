@@ -219,6 +219,21 @@ inline size_t inv_wigner_t_smem(int N, int K, int zt = kWigZT) {
   return (size_t)K * wig_np(N) * sizeof(float) + (size_t)K * (zt + 2) * sizeof(float2);
 }
 
+// one entry of s2_mm(xs, ys), multiply-adds in the order of cgemm_grouped
+S2C_D float2 wig_s2_product(const InvWignerParams& p, int l, int m, int n, int i, int j) {
+  const float2* xr = p.xs + ((long)(l * l + l + m) * p.s2_nb + i) * p.s2_fin;
+  const float2* yr = p.ys + (long)(l * l + l + n) * p.s2_fin * p.s2_fout + j;
+  float re = 0.f, im = 0.f;
+  for (int k = 0; k < p.s2_fin; ++k) {
+    const float2 a = xr[k], b = yr[(long)k * p.s2_fout];
+    re = fmaf(a.x, b.x, re);
+    re = fmaf(a.y, b.y, re);
+    im = fmaf(a.x, -b.y, im);
+    im = fmaf(a.y, b.x, im);
+  }
+  return make_float2(re, im);
+}
+
 // S[z][beta] = sum_l W[l][beta] Xs[l][z],  Xs = symmetrised spectrum
 S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
   const int N = p.N, NP = wig_np(N);
@@ -265,6 +280,11 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
     if (zz < zc && p.mode == kS2) {
       const long l = lmin + li;
       v = p.x[(l * l + l + m) * p.x_zstride + z0 + zz];
+    } else if (zz < zc && p.xs) {
+      const int l = lmin + li;
+      const int z = (int)(p.z0 + z0 + zz), i = z / p.s2_fout, j = z - i * p.s2_fout;
+      const float2 a = wig_s2_product(p, l, m, n, i, j), b = wig_s2_product(p, l, -m, -n, i, j);
+      v = make_float2(0.5f * (a.x + fudge * b.x), 0.5f * (a.y - fudge * b.y));
     } else if (zz < zc) {
       const int l = lmin + li;
       float2 a = p.x[so3_row(l, m, n) * p.x_zstride + z0 + zz];

@@ -18,7 +18,7 @@ model is left as traced.  The result computes the same function.
     relu -> so3_integrate                  so3_relu_integrate(x)
 
 A chain is only rewritten when the intermediate tensor has no other consumer and the sizes are
-ones the fused kernels take (2 b <= 32, non-increasing bandwidth); otherwise it stays as it is.
+ones the fused kernels take (2 b <= 32, non-increasing bandwidth; a ReLU on load 2 b < 64); otherwise it stays as it is.
 """
 import sys
 from operator import getitem as _getitem
@@ -179,7 +179,7 @@ def fuse(model):
                 dst.args = (src,)
                 dst.kwargs = dict(dst.kwargs, input_spectrum=True)
                 graph.erase_node(node)
-            elif 2 * consumer.b_in <= 32:
+            elif 2 * consumer.b_in < 64:
                 dst.args = (src,)
                 dst.kwargs = dict(dst.kwargs, relu_input=True)
                 graph.erase_node(node)

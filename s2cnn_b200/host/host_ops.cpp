@@ -68,7 +68,7 @@ long s2_bandwidth(long nspec) {
 // ---- one build of the library ---------------------------------------------------------------------
 #define S2C_API(X)                                                                                 \
   X(last_error) X(is_cuda_build) X(tables_computed) X(so3_fft_workspace) X(so3_rfft)               \
-  X(so3_rfft_relu) X(so3_rfft_sums) X(so3_fft) X(so3_rifft) X(so3_rifft_relu_grad)                 \
+  X(so3_rfft_relu) X(so3_rfft_sums) X(so3_rfft_sums_ws) X(so3_rifft_relu_grad_ws) X(so3_fft) X(so3_rifft) X(so3_rifft_relu_grad)                 \
   X(so3_rifft_relu_integrate) X(s2_conv_relu_so3_rfft) X(so3_rifft_relu_rfft)                      \
   X(s2_conv_synthesis_workspace) X(s2_conv_synthesis) X(so3_ifft) X(s2_fft_workspace) X(s2_fft)    \
   X(s2_ifft) X(so3_mm) X(so3_mm_gradx) X(so3_mm_grady) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
@@ -217,18 +217,21 @@ struct Ops {
     const Tensor x = x_.contiguous();
     const auto lead = x.sizes().slice(0, x.dim() - 3);
     const long nb = lead_numel(lead);
-    if (2 * b_in <= 32) {
+    if (2 * b_in < 64) {
       Tensor out = empty_like_shape(x, spectrum_shape(so3_nspec(b_out), lead));
       Tensor sums = empty_like_shape(x, lead);
       Ctx c(*this, x);
-      const int rc = call_rc("s2c_so3_rfft_sums", so3_rfft_sums_, cptr(x), ptr(out), ptr(sums), nb, (int)b_in,
-                             (int)b_out, (int)for_grad, c.stream);
+      Tensor ws;
+      if (2 * b_in > 32) ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
+      const int rc = call_rc("s2c_so3_rfft_sums_ws", so3_rfft_sums_ws_, cptr(x), ptr(out), ptr(sums), nb, (int)b_in,
+                             (int)b_out, (int)for_grad, ws.defined() ? ws.mutable_data_ptr() : nullptr,
+                             ws.defined() ? (size_t)ws.numel() : (size_t)0, c.stream);
       if (rc == 0) {
         log_new_tables("so3_rfft", b_in, b_out);
         return {out, sums};
       }
-      if (rc != 4)   // 4: outside the single-kernel path, nothing written
-        raise_s2c("s2c_so3_rfft_sums failed (status " + std::to_string(rc) + "): " + last_error_());
+      if (rc != 4)   // 4: no such kernel for this size, nothing written
+        raise_s2c("s2c_so3_rfft_sums_ws failed (status " + std::to_string(rc) + "): " + last_error_());
     }
     return {so3_rfft(x, for_grad, b_out, false), x.sum({-3, -2, -1})};
   }
@@ -275,6 +278,12 @@ struct Ops {
     check(x.size(-1) == 2 && x.sizes().slice(1, x.dim() - 2) == lead, "so3_rifft_relu_grad: shapes differ");
     Tensor out = at::empty_like(act);
     Ctx c(*this, x);
+    if (2 * b_out > 32) {
+      const long nb = lead_numel(lead);
+      const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
+      S2C_CALL(so3_rifft_relu_grad_ws, cptr(x), cptr(act), ptr(out), nb, (int)b_in, (int)b_out, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+      return out;
+    }
     S2C_CALL(so3_rifft_relu_grad, cptr(x), cptr(act), ptr(out), lead_numel(lead), (int)b_in, (int)b_out, c.stream);
     return out;
   }

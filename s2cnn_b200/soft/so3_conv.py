@@ -67,7 +67,7 @@ class SO3Convolution(Module):
             assert x.size(2) == 2 * self.b_in
             assert x.size(3) == 2 * self.b_in
             assert x.size(4) == 2 * self.b_in
-            if relu_input and 2 * self.b_in <= 32:
+            if relu_input and 2 * self.b_in < 64:
                 x = SO3_fft_real_relu.apply(x, self.b_out)
             else:
                 if relu_input:

@@ -58,7 +58,7 @@ class SO3_fft_real_relu:
     """``SO3_fft_real`` of ``relu(x)`` with the activation applied while the signal is read (the
     ReLU between two convolutions of the reference's models, e.g. examples/mnist/run.py:88-93,
     folded into the consumer); its backward writes 0 where x <= 0 inside the synthesis kernel, without
-    a separate pass over the gradient signal.  Needs 2 b_in <= 32."""
+    a separate pass over the gradient signal.  Needs 2 b_in < 64."""
 
     @staticmethod
     def apply(x, b_out=None):
