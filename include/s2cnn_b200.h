@@ -139,6 +139,16 @@ int s2c_so3_rifft_relu_integrate(const float* x, float* out, long nbatch, int b_
  * and the head of the next SO3Convolution.forward (s2cnn/soft/so3_conv.py:50). */
 int s2c_s2_conv_relu_so3_rfft(const float* xs, const float* ys, float* out, int nbatch, int f_in,
                               int f_out, int b, int b_next, const float* bias, void* stream);
+/* Scratch for the _ws variants of the two fused calls, which hand large batches (2b >= 10) to kernels that
+ * work through a workspace; without one (or with too little) the calls above are what runs. */
+size_t s2c_so3_relay_workspace(long nbatch, int b_in, int b_mid, int b_next);
+int s2c_s2_conv_relu_so3_rfft_ws(const float* xs, const float* ys, float* out, int nbatch, int f_in,
+                                 int f_out, int b, int b_next, const float* bias, void* workspace,
+                                 size_t workspace_bytes, void* stream);
+int s2c_so3_rifft_relu_rfft_ws(const float* x, float* out, long nbatch, int b_in, int b_mid, int b_next,
+                               const float* bias, int nfeature, void* workspace,
+                               size_t workspace_bytes, void* stream);
+
 /* The same relay between two SO3Convolutions:
  *   out = so3_rfft(relu(so3_rifft(x, b_out = b_mid) + bias), b_out = b_next)
  * x [nspec(b_in), nbatch, 2], out [nspec(b_next), nbatch, 2]; bias [nfeature] or NULL as in
@@ -278,8 +288,8 @@ int s2c_project_on_sphere(const float* verts, int nv, const int* faces, int nf, 
  *     separate passes every other size uses; 0 restores the defaults.
  *   s2c_debug_plane_chunk(signals): signals per chunk of the large-bandwidth path (1 .. 8); 0
  *     restores the default (8, or what the workspace holds).
- *   s2c_debug_cluster(mode): single-kernel path: 1 always the cluster kernels, 2 never (the kernels
- *     whose blocks walk beta); 0 restores the choice by batch size. */
+ *   s2c_debug_cluster(mode): 2b <= 32: 1 the cluster kernels, 2 the kernels whose blocks walk beta, 3 the
+ *     plane kernels (where they exist and a workspace is given); 0 restores the choice by batch size. */
 void s2c_debug_force_general_path(int level);
 void s2c_debug_plane_chunk(int signals);
 void s2c_debug_cluster(int mode);

@@ -43,6 +43,9 @@ _SIGNATURES = {
     "s2c_so3_rfft_relu": (c_int, [_P, _P, c_long, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_rfft_sums_ws": (c_int, [_P, _P, _P, c_long, c_int, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_rifft_relu_grad_ws": (c_int, [_P, _P, _P, c_long, c_int, c_int, _P, c_size_t, _P]),
+    "s2c_so3_relay_workspace": (c_size_t, [c_long, c_int, c_int, c_int]),
+    "s2c_s2_conv_relu_so3_rfft_ws": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, c_size_t, _P]),
+    "s2c_so3_rifft_relu_rfft_ws": (c_int, [_P, _P, c_long, c_int, c_int, c_int, _P, c_int, _P, c_size_t, _P]),
     "s2c_so3_rfft_sums": (c_int, [_P, _P, _P, c_long, c_int, c_int, c_int, _P]),
     "s2c_debug_force_general_path": (None, [c_int]),
     "s2c_debug_cluster": (None, [c_int]),

@@ -16,7 +16,7 @@ from concurrent.futures import ThreadPoolExecutor
 PKG = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(PKG, "csrc", "lib.cu")
 PARTS_SRC = os.path.join(PKG, "csrc", "parts.cu")
-N_PARTS = 16
+N_PARTS = 18
 LIB_DIR = os.path.join(PKG, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libs2cnn_b200.so")
 

@@ -19,6 +19,7 @@
 #include "so3_cluster_kernels.h"
 #include "so3_mid_kernels.h"
 #include "s2_kernels.h"
+#include "so3_small_kernels.h"
 #include "wigner_tiled.h"
 #include "wigner_rows.h"
 #include "cgemm_kernels.h"
@@ -32,7 +33,7 @@ namespace s2c {
 thread_local long g_launch_count = 0;
 // test switches (process-wide, race-free; see the "test hooks" section of the header)
 static std::atomic<int> g_force_general{0};   // 1 = no single-kernel path, 2 = also no plane kernels
-static std::atomic<int> g_cluster{0};         // cluster kernels: 0 by batch size, 1 always, 2 never
+static std::atomic<int> g_cluster{0};         // 2b <= 32: 0 by batch size, 1 cluster, 2 walking, 3 plane kernels
 static std::atomic<int> g_plane_chunk{0};     // plane path: signals per chunk (0 = default)
 
 #define S2C_TRY(expr)            \
@@ -137,6 +138,19 @@ static bool so3_prefers_cluster(ClKind kind, int N, long nbatch) {
   return kind == kClRelay || groups <= (kind == kClAnalysis ? 55 : 95);
 }
 
+// Large batches at 10 <= 2 b <= 32: plane kernels (so3_small_kernels.h) and the tiled Wigner kernels, through a
+// workspace that holds at least one tile of signals.
+static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, const void* ws, size_t ws_bytes) {
+  const int forced = g_cluster.load();
+  if (g_force_general || !small_supported(N) || !ws || forced == 1 || forced == 2) return false;
+  if (ws_bytes < so3_mid_v_per_z(N, K) * (size_t)std::min<long>(kWigZT, nbatch) ||
+      !fwd_wigner_t_fits(N, nl, kWigZT, dev_smem_limit()))
+    return false;
+  if (forced == 3) return true;
+  (void)kind;
+  return (nbatch + kFusedZG - 1) / kFusedZG > 160;
+}
+
 static int check_b(int b_in, int b_out) {
   if (b_in < 1 || b_out < 1) return fail(S2C_ERR_BAD_ARG, "bandwidths must be >= 1");
   return S2C_OK;
@@ -155,7 +169,8 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
   S2C_TRY(TableCache::get().panels(b_in, b_out, K, weighted, false, pan));
   if (b_out > b_in && mode == kSo3Real)  // rows with |m| or |n| >= b_in stay zero (so3_fft.py:44-48)
     S2C_TRY(dev_memset_async(out, 0, (size_t)so3_nspec(b_out) * nbatch * sizeof(float2), st));
-  if (!g_force_general && N <= kFusedMaxN && b_out <= kFusedMaxDegrees &&
+  const bool small = so3_prefers_planes(kClAnalysis, N, K, b_out, nbatch, ws, ws_bytes);
+  if (!small && !g_force_general && N <= kFusedMaxN && b_out <= kFusedMaxDegrees &&
       so3_prefers_cluster(kClAnalysis, N, nbatch)) {
     ClFwdParams f;
     f.x = x; f.in_stride = in_stride; f.in_off = in_off;
@@ -170,7 +185,7 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
                                          cl_smem_bytes(N, K, 0), st, f));
     return rc;
   }
-  if (!g_force_general && N <= kFusedMaxN &&
+  if (!small && !g_force_general && N <= kFusedMaxN &&
       fwd_fused_smem_bytes(N, pan.nrows) <= (size_t)dev_smem_limit() - 1024) {
     FwdFusedParams f;
     f.x = x; f.in_stride = in_stride; f.in_off = in_off;
@@ -187,8 +202,8 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
                                         fused_threads(sm, (size_t)dev_smem_limit()), sm, st, f));
     return rc;
   }
-  if (relu && !use_mid_kernels(N)) return fail(S2C_ERR_UNSUPPORTED, "fused ReLU input needs 2 b < 64");
-  if (sums && (!use_mid_kernels(N) || !ws)) return fail(S2C_ERR_UNSUPPORTED, "per-signal sums need 2 b < 64");
+  if (relu && !small && !use_mid_kernels(N)) return fail(S2C_ERR_UNSUPPORTED, "fused ReLU input needs 2 b < 64");
+  if (sums && !small && (!use_mid_kernels(N) || !ws)) return fail(S2C_ERR_UNSUPPORTED, "per-signal sums need 2 b < 64");
   if (use_plane_kernels(N)) {
     HalfPanelsDev hp;
     hp.nbeta = N; hp.nl = b_out; hp.K = K; hp.npairs = pan.npairs;
@@ -208,7 +223,7 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
     };
     return plane_pipeline(nbatch, N, K, ws, ws_bytes, st, planes, wigner);
   }
-  const bool mid = use_mid_kernels(N);
+  const bool mid = small || use_mid_kernels(N);
   const size_t per_z = so3_ws_per_z(N, K);
   long chunk = (long)std::min<size_t>((size_t)nbatch, ws_bytes / per_z);
   if (mid) {
@@ -223,7 +238,17 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
     const long zc = std::min(chunk, nbatch - z0);
     float2* u = (float2*)ws;
     float2* v = mid ? u : u + (size_t)zc * K * N * N;
-    if (mid) {
+    if (small) {
+      SmallParams g;
+      g.x = x + (size_t)z0 * N * N * N * in_stride; g.out = nullptr;
+      g.stride = in_stride; g.off = in_off;
+      g.v = v; g.v2 = nullptr; g.bias = nullptr; g.nfeat = 1; g.z0 = z0; g.mask = nullptr; g.relu = relu;
+      g.wide = in_stride == 1 && N % 4 == 0 && (uintptr_t)x % 32 == 0;
+      g.nplanes = zc * N; g.K = K; g.K2 = 0;
+      int rc = S2C_OK;
+      S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_fwd_small, kN, st, g));
+      if (rc) return rc;
+    } else if (mid) {
       MidParams g;
       g.x = x + (size_t)z0 * N * N * N * in_stride; g.out = nullptr;
       g.stride = in_stride; g.off = in_off;
@@ -234,11 +259,6 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
       S2C_DISPATCH_MID(N, rc = S2C_LAUNCH_N(so3_fwd_mid, kN, zc * ((kN + mid_nb(kN) - 1) / mid_nb(kN)),
                                             kMidThreads, mid_smem_bytes(kN), st, g));
       if (rc) return rc;
-      if (sums) {
-        MidSumsParams q;
-        q.v = v + (size_t)(K - 1) * zc * N; q.sums = sums + z0; q.nbatch = (int)zc; q.N = N;
-        S2C_TRY(S2C_LAUNCH(so3_mid_sums, (zc + 31) / 32, 32, 0, st, q));
-      }
     } else {
     FwdGammaParams g;
     g.x = x + (size_t)z0 * N * N * N * in_stride;
@@ -257,6 +277,11 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
     a.nrows = zc * K * N;
     a.fft = fft;
     S2C_TRY(S2C_LAUNCH(so3_fwd_alpha, (a.nrows + G - 1) / G, kThreads, fft_smem, st, a));
+    }
+    if (sums) {
+      MidSumsParams q;
+      q.v = v + (size_t)(K - 1) * zc * N; q.sums = sums + z0; q.nbatch = (int)zc; q.N = N;
+      S2C_TRY(S2C_LAUNCH(so3_mid_sums, (zc + 31) / 32, 32, 0, st, q));
     }
     FwdWignerParams w;
     w.v = v;
@@ -307,7 +332,9 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
   PanelsDev pan;
   S2C_TRY(TableCache::get().fft(N, fft));
   S2C_TRY(TableCache::get().panels(b_out, K, K, weighted, false, pan));
-  if (!g_force_general && N <= kFusedMaxN && so3_prefers_cluster(kClSynthesis, N, nbatch)) {
+  const bool small = !integral && so3_prefers_planes(kClSynthesis, N, K, K, nbatch, ws, ws_bytes) &&
+                     (!mask || (out_stride == 1 && out_off == 0));
+  if (!small && !g_force_general && N <= kFusedMaxN && so3_prefers_cluster(kClSynthesis, N, nbatch)) {
     ClInvParams f;
     f.in.x = x; f.in.x_zstride = nbatch; f.in.mode = mode;
     f.in.xs = f.in.ys = nullptr; f.in.s2_nb = f.in.s2_fin = f.in.s2_fout = 0;
@@ -335,7 +362,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
                                          cl_smem_bytes(N, K, f.tab.max_rows), st, f));
     return rc;
   }
-  if (!g_force_general && N <= kFusedMaxN &&
+  if (!small && !g_force_general && N <= kFusedMaxN &&
       fused_smem_bytes(N, pan.nrows) <= (size_t)dev_smem_limit() - 1024) {
     InvFusedParams f;
     f.x = x; f.x_zstride = nbatch;
@@ -371,7 +398,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
   }
   if (integral)
     return fail(S2C_ERR_UNSUPPORTED, "fused ReLU + integration needs the small-bandwidth path");
-  if (mask && (!use_mid_kernels(N) || !ws || out_stride != 1 || out_off != 0))
+  if (mask && !small && (!use_mid_kernels(N) || !ws || out_stride != 1 || out_off != 0))
     return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output and 2 b < 64");
   if (use_plane_kernels(N)) {
     HalfPanelsDev hp;
@@ -394,7 +421,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     };
     return plane_pipeline(nbatch, N, K, ws, ws_bytes, st, wigner, planes);
   }
-  const bool mid = use_mid_kernels(N);
+  const bool mid = small || use_mid_kernels(N);
   const size_t per_z = so3_ws_per_z(N, K);
   long chunk = (long)std::min<size_t>((size_t)nbatch, ws_bytes / per_z);
   if (mid) {
@@ -431,6 +458,19 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     } else {
       const size_t wsm = align_up((size_t)K * N * sizeof(float), 16) + (size_t)K * w.ZT * sizeof(float2);
       S2C_TRY(S2C_LAUNCH(so3_inv_wigner, (long)pan.npairs * w.nzt, kThreads, wsm, st, w));
+    }
+    if (small) {
+      SmallParams g;
+      g.x = nullptr; g.out = out + (size_t)z0 * N * N * N * out_stride;
+      g.stride = out_stride; g.off = out_off;
+      g.v = s; g.v2 = nullptr; g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0; g.relu = 0;
+      g.mask = mask ? mask + (size_t)z0 * N * N * N : nullptr;
+      g.wide = out_stride == 1 && N % 4 == 0 && (uintptr_t)out % 32 == 0 && (uintptr_t)mask % 32 == 0;
+      g.nplanes = zc * N; g.K = K; g.K2 = 0;
+      int rc = S2C_OK;
+      S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_inv_small, kN, st, g));
+      if (rc) return rc;
+      continue;
     }
     if (mid) {
       MidParams g;
@@ -768,11 +808,42 @@ static int relay_bg(int N, int Kin, int nrows_in, int nrows_out) {
 // product of xs and ys when xs is set), + bias, ReLU, analysis to bandwidth b_next
 static int relay_launch(const float2* x, const float2* xs, const float2* ys, int s2_nb, int s2_fin,
                         float* out, long nz, int nfeat, int b_in, int b_mid, int b_next,
-                        const float* bias, stream_t st, const char* who) {
+                        const float* bias, void* ws, size_t ws_bytes, stream_t st, const char* who) {
   const int N = 2 * b_mid;
   if (N > kFusedMaxN || b_next > b_mid || b_in > b_mid)
     return fail(S2C_ERR_UNSUPPORTED,
                 std::string(who) + ": needs 2 b <= 32, b_in <= b and b_next <= b");
+  const size_t v1 = so3_mid_v_per_z(N, b_in), v2 = so3_mid_v_per_z(N, b_next);
+  if (so3_prefers_planes(kClRelay, N, b_in, b_next, nz, ws, ws_bytes) &&
+      ws_bytes >= (v1 + v2) * (size_t)std::min<long>(kWigZT, nz)) {
+    PanelsDev pin, pout;
+    S2C_TRY(TableCache::get().panels(b_mid, b_in, b_in, false, false, pin));
+    S2C_TRY(TableCache::get().panels(b_mid, b_next, b_next, true, false, pout));
+    const long l2 = std::max(1L, (long)(((size_t)64 << 20) / (v1 + v2)) / kWigZT) * kWigZT;
+    const long chunk = std::min(nz, std::min(l2, (long)(ws_bytes / (v1 + v2))));
+    for (long z0 = 0; z0 < nz; z0 += chunk) {
+      const long zc = std::min(chunk, nz - z0);
+      float2* v = (float2*)ws;
+      float2* vo = v + (size_t)zc * (v1 / sizeof(float2));
+      InvWignerParams w;
+      w.x = xs ? nullptr : x + z0; w.x_zstride = nz; w.s = v; w.pan = pin;
+      w.nbatch = (int)zc; w.N = N; w.K = b_in; w.ZT = kWigZT; w.nzt = (int)((zc + kWigZT - 1) / kWigZT); w.mode = kSo3Real;
+      w.xs = xs; w.ys = ys; w.s2_nb = s2_nb; w.s2_fin = s2_fin; w.s2_fout = nfeat; w.z0 = z0;
+      S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)pin.npairs * w.nzt, kThreads, inv_wigner_t_smem(N, b_in), st, w));
+      SmallParams g;
+      g.x = nullptr; g.out = nullptr; g.stride = 1; g.off = 0; g.v = v; g.v2 = vo;
+      g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0; g.mask = nullptr; g.relu = 1; g.wide = 0;
+      g.nplanes = zc * N; g.K = b_in; g.K2 = b_next;
+      int rc = S2C_OK;
+      S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_relay_small, kN, st, g));
+      if (rc) return rc;
+      FwdWignerParams f;
+      f.v = vo; f.out = (float2*)out + z0; f.out_zstride = nz; f.pan = pout;
+      f.nbatch = (int)zc; f.N = N; f.K = b_next; f.nl = b_next; f.ZT = kWigZT; f.nzt = w.nzt; f.mode = kSo3Real;
+      S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)pout.npairs * f.nzt, kThreads, fwd_wigner_t_smem(N, b_next), st, f));
+    }
+    return S2C_OK;
+  }
   if (so3_prefers_cluster(kClRelay, N, nz)) {
     ClRelayParams f;
     S2C_TRY(TableCache::get().cluster(b_mid, b_in, b_in, false, f.tin));
@@ -812,25 +883,43 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
   return rc;
 }
 
-int s2c_s2_conv_relu_so3_rfft(const float* xs, const float* ys, float* out, int nbatch, int f_in,
-                              int f_out, int b, int b_next, const float* bias, void* stream) {
+size_t s2c_so3_relay_workspace(long nbatch, int b_in, int b_mid, int b_next) {
+  if (!small_supported(2 * b_mid) || b_in < 1 || b_next < 1) return 16;
+  const size_t v = so3_mid_v_per_z(2 * b_mid, b_in) + so3_mid_v_per_z(2 * b_mid, b_next);
+  const long l2 = std::max(1L, (long)(((size_t)64 << 20) / v) / kWigZT) * kWigZT;
+  return v * (size_t)std::min(l2, std::max(1L, nbatch));
+}
+
+int s2c_s2_conv_relu_so3_rfft_ws(const float* xs, const float* ys, float* out, int nbatch, int f_in,
+                                 int f_out, int b, int b_next, const float* bias, void* ws,
+                                 size_t ws_bytes, void* stream) {
   S2C_TRY(check_b(b, b_next));
   if (!xs || !ys || !out || nbatch < 1 || f_in < 1 || f_out < 1)
     return fail(S2C_ERR_BAD_ARG, "s2c_s2_conv_relu_so3_rfft: bad argument");
   return relay_launch(nullptr, (const float2*)xs, (const float2*)ys, nbatch, f_in, out,
-                      (long)nbatch * f_out, f_out, b, b, b_next, bias, as_stream(stream),
+                      (long)nbatch * f_out, f_out, b, b, b_next, bias, ws, ws_bytes, as_stream(stream),
                       "s2c_s2_conv_relu_so3_rfft");
 }
 
-int s2c_so3_rifft_relu_rfft(const float* x, float* out, long nbatch, int b_in, int b_mid, int b_next,
-                            const float* bias, int nfeature, void* stream) {
+int s2c_s2_conv_relu_so3_rfft(const float* xs, const float* ys, float* out, int nbatch, int f_in,
+                              int f_out, int b, int b_next, const float* bias, void* stream) {
+  return s2c_s2_conv_relu_so3_rfft_ws(xs, ys, out, nbatch, f_in, f_out, b, b_next, bias, nullptr, 0, stream);
+}
+
+int s2c_so3_rifft_relu_rfft_ws(const float* x, float* out, long nbatch, int b_in, int b_mid, int b_next,
+                               const float* bias, int nfeature, void* ws, size_t ws_bytes, void* stream) {
   S2C_TRY(check_b(b_in, b_mid));
   S2C_TRY(check_b(b_mid, b_next));
   if (!x || !out || nbatch < 1) return fail(S2C_ERR_BAD_ARG, "s2c_so3_rifft_relu_rfft: bad argument");
   if (bias && nfeature < 1)
     return fail(S2C_ERR_BAD_ARG, "s2c_so3_rifft_relu_rfft: nfeature must be >= 1 with a bias");
   return relay_launch((const float2*)x, nullptr, nullptr, 0, 0, out, nbatch, bias ? nfeature : 0,
-                      b_in, b_mid, b_next, bias, as_stream(stream), "s2c_so3_rifft_relu_rfft");
+                      b_in, b_mid, b_next, bias, ws, ws_bytes, as_stream(stream), "s2c_so3_rifft_relu_rfft");
+}
+
+int s2c_so3_rifft_relu_rfft(const float* x, float* out, long nbatch, int b_in, int b_mid, int b_next,
+                            const float* bias, int nfeature, void* stream) {
+  return s2c_so3_rifft_relu_rfft_ws(x, out, nbatch, b_in, b_mid, b_next, bias, nfeature, nullptr, 0, stream);
 }
 
 // 32 < 2 b < 64: the product is evaluated while the tiled Wigner kernel stages the spectrum (b = 30, 256 signals:
@@ -840,7 +929,8 @@ static bool s2_product_in_wigner(int b) {
 }
 
 size_t s2c_s2_conv_synthesis_workspace(int nbatch, int f_out, int b) {
-  if (so3_synthesis_is_fused(b, b)) return 16;
+  if (so3_synthesis_is_fused(b, b))
+    return small_supported(2 * b) ? s2c_so3_fft_workspace((long)nbatch * f_out, b, b) : 16;
   const size_t z_bytes = (size_t)so3_nspec(b) * nbatch * f_out * sizeof(float2);
   return z_bytes + s2c_so3_fft_workspace((long)nbatch * f_out, b, b);
 }

@@ -14,6 +14,7 @@
 #include "so3_cluster_kernels.h"
 #include "so3_mid_kernels.h"
 #include "s2_kernels.h"
+#include "so3_small_kernels.h"
 #include "so3_mm_tc.h"
 
 namespace s2c {
@@ -29,6 +30,10 @@ namespace s2c {
 #define S2C_MID(N)                                                                  \
   template int launch_so3_fwd_mid<N>(long, int, size_t, stream_t, const MidParams&); \
   template int launch_so3_inv_mid<N>(long, int, size_t, stream_t, const MidParams&);
+#define S2C_SMALL(N)                                                                     \
+  template int launch_so3_fwd_small<N>(long, int, size_t, stream_t, const SmallParams&);   \
+  template int launch_so3_inv_small<N>(long, int, size_t, stream_t, const SmallParams&);   \
+  template int launch_so3_relay_small<N>(long, int, size_t, stream_t, const SmallParams&);
 #define S2C_TC_OP(OP) \
   template int launch_so3_mm_tc<OP>(const char*, long, bool, bool, stream_t, const MmTcParams&);
 
@@ -73,6 +78,10 @@ S2C_S2(80) S2C_S2(96) S2C_S2(102) S2C_S2(114) S2C_S2(124)
 #elif S2C_PART == 15
 S2C_S2(10) S2C_S2(12) S2C_S2(26) S2C_S2(28) S2C_S2(42) S2C_S2(44) S2C_S2(58) S2C_S2(60) S2C_S2(76)
 S2C_S2(78) S2C_S2(98) S2C_S2(100) S2C_S2(116) S2C_S2(120)
+#elif S2C_PART == 16
+S2C_SMALL(32) S2C_SMALL(30) S2C_SMALL(24) S2C_SMALL(16) S2C_SMALL(14) S2C_SMALL(10)
+#elif S2C_PART == 17
+S2C_SMALL(28) S2C_SMALL(26) S2C_SMALL(22) S2C_SMALL(20) S2C_SMALL(18) S2C_SMALL(12)
 #endif
 
 }  // namespace s2c

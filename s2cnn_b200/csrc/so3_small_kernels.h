@@ -1,0 +1,334 @@
+// Plane kernels of the SO(3) transform for small bandwidths (10 <= N = 2b <= 32) and LARGE batches: both row
+// transforms of P neighbouring (z, beta) planes in one block, every 1-D FFT in the registers of one thread
+// (fft_reg.h), between the signal and the [n][m][z][beta] array of the tiled Wigner kernels (wigner_tiled.h).
+//
+// The single-kernel transforms (so3_fused_kernels.h) keep the spectrum of four batch elements, the Wigner slice and
+// the planes of a beta group in one block: at b = 16 that is 210 KB, one block of 16 warps per SM whose eight beta
+// groups pass four block barriers each (0.34 instructions per clock and scheduler, 4 of 12 stall cycles at
+// barriers).  For a large batch the Wigner contraction is better off on its own - a tile shares each table row
+// among 64 signals - and what is left needs one barrier and 35 KB: several blocks per SM overlap their loads,
+// transforms and stores.  The array between the two stays in L2 (chunks of at most 64 MB).
+//
+//   so3_fwd_small    two real rows per thread (optional ReLU on load) -> n -> columns alpha -> m -> V
+//   so3_inv_small    V -> columns m -> alpha -> two rows per thread n -> gamma (+ bias, mask) -> store
+//   so3_relay_small  the synthesis, + bias, ReLU, forward row transform in the same registers, then the rest of
+//                    the analysis: the signal between two layers never exists in memory
+//
+// The planes of a block are consecutive in (z, beta), so that V is moved in runs of 8 P bytes.  Same FFTs, same
+// sums in the same order as the single-kernel transforms: the results are the same bit for bit.
+#pragma once
+
+#include "backend.h"
+#include "fft_reg.h"
+#include "so3_fused_kernels.h"
+#include "so3_kernels.h"
+
+namespace s2c {
+
+S2C_HD constexpr bool small_supported(int N) { return N >= 10 && N <= 32 && N % 2 == 0; }
+S2C_HD constexpr int small_planes(int N) { return 256 / N / 4 * 4 < 8 ? 8 : 256 / N / 4 * 4; }
+S2C_HD constexpr int small_threads(int N) { return (small_planes(N) * (N / 2) + 31) / 32 * 32; }
+S2C_HD constexpr int small_kp(int N) { return N / 2 | 1; }                 // odd row stride (complex)
+// plane stride: the lanes of a column phase run over the planes, then over n
+S2C_HD constexpr int small_ps(int N) {
+  int ps = N * small_kp(N);
+  while (ps % 16 != (small_planes(N) < 12 ? 2 : 1)) ++ps;
+  return ps;
+}
+inline size_t small_smem_bytes(int N) { return (size_t)small_planes(N) * small_ps(N) * sizeof(float2); }
+
+struct SmallParams {
+  const float* x;      // analysis: real signal, element e at x[e * stride + off]
+  float* out;          // synthesis: the same
+  long stride, off;
+  float2* v;           // [n < K][m + K - 1][z][beta]: analysis output, synthesis / relay input
+  float2* v2;          // relay output, bandwidth K2
+  const float* bias;   // optional [nfeat]; feature of signal z is (z0 + z) % nfeat
+  int nfeat;
+  long z0;
+  const float* mask;   // synthesis, optional (unit stride): samples where this signal is <= 0 are written as 0
+  int relu, wide;      // wide: 32-byte accesses to x / out / mask
+  long nplanes;        // signals * N
+  int K, K2;
+};
+
+template <int N>
+struct Small {
+  static constexpr int P = small_planes(N), H = N / 2, KP = small_kp(N), PS = small_ps(N);
+
+  // columns of the K kept frequencies n: thread = (plane, n)
+  static S2C_D void columns_inv(const Ctx& ctx, const SmallParams& p, long q0, float2* planes) {
+    const int pl = ctx.tid % P, n = ctx.tid / P, K = p.K;
+    if (n >= K || q0 + pl >= p.nplanes) return;
+    const float2* s = p.v + ((long)n * (2 * K - 1) + K - 1) * p.nplanes + q0 + pl;      // frequency m = 0
+    float2 v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int m = i < H ? i : i - N;
+      v[i] = make_float2(0.f, 0.f);
+      if (m < K && m > -K) {
+        if (n == 0 && m < 0) {                               // only m >= 0 is stored: Hermitian
+          const float2 c = s[-m * p.nplanes];
+          v[i] = make_float2(c.x, -c.y);
+        } else {
+          v[i] = s[m * p.nplanes];
+        }
+      }
+    }
+    fft_reg<N, +1>(v, nullptr);
+    float2* col = planes + pl * PS + n;
+    static_for<0, N>([&](auto ic) {
+      constexpr int a = decltype(ic)::value;
+      col[a * KP] = v[fft_reg_pos<N>(a)];
+    });
+  }
+  static S2C_D void columns_fwd(const Ctx& ctx, const SmallParams& p, long q0, const float2* planes, float2* out, int K) {
+    const int pl = ctx.tid % P, n = ctx.tid / P;
+    if (n >= K || q0 + pl >= p.nplanes) return;
+    const float2* col = planes + pl * PS + n;
+    float2 v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = col[i * KP];
+    fft_reg<N, -1>(v, nullptr);
+    float2* o = out + ((long)n * (2 * K - 1) + K - 1) * p.nplanes + q0 + pl;
+    static_for<0, N>([&](auto ic) {
+      constexpr int f = decltype(ic)::value;
+      constexpr int m = f < H ? f : f - N;
+      if (m < K && m > (n == 0 ? -1 : -K)) o[m * p.nplanes] = v[fft_reg_pos<N>(f)];
+    });
+  }
+
+  // rows alpha = ap, ap + N/2 of a plane: one complex transform for two real rows
+  static S2C_D void pack_rows(const float2* r1, int K, float2 (&v)[N]) {
+    const float2* r2 = r1 + H * KP;
+    {
+      const float2 t1 = r1[0], t2 = r2[0];
+      v[0] = make_float2(t1.x, t2.x);  // T[alpha][0] is real for a Hermitian spectrum
+    }
+    v[H] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int n = 1; n < H; ++n) {
+      if (n < K) {
+        const float2 t1 = r1[n], t2 = r2[n];
+        v[n] = make_float2(t1.x - t2.y, t1.y + t2.x);      // T1 + i T2
+        v[N - n] = make_float2(t1.x + t2.y, t2.x - t1.y);  // conj(T1) + i conj(T2)
+      } else {
+        v[n] = make_float2(0.f, 0.f);
+        v[N - n] = make_float2(0.f, 0.f);
+      }
+    }
+  }
+  static S2C_D void split_rows(float2* r1, int K, const float2 (&v)[N]) {
+    float2* r2 = r1 + H * KP;
+    static_for<0, H>([&](auto ic) {
+      constexpr int n = decltype(ic)::value;
+      constexpr int pn = fft_reg_pos<N>(n), pq = fft_reg_pos<N>(n == 0 ? 0 : N - n);
+      if (n < K) {
+        const float2 zk = v[pn], zq = v[pq];
+        r1[n] = make_float2(0.5f * (zk.x + zq.x), 0.5f * (zk.y - zq.y));
+        r2[n] = make_float2(0.5f * (zk.y + zq.y), -0.5f * (zk.x - zq.x));
+      }
+    });
+  }
+
+  // the samples of two rows in pieces of 8, 4 (32- and 16-byte accesses; rows of N % 8 == 4 floats start on a sector
+  // boundary only every other row) or 2 floats: f(first, count)
+  template <class F>
+  static S2C_D void pieces(bool wide, int ap, F&& f) {
+    using I2 = std::integral_constant<int, 2>;
+    using I4 = std::integral_constant<int, 4>;
+    using I8 = std::integral_constant<int, 8>;
+    if constexpr (N % 8 == 0) {
+      if (wide) { static_for<0, N / 8>([&](auto ic) { f(std::integral_constant<int, 8 * decltype(ic)::value>{}, I8{}); }); return; }
+    } else if constexpr (N % 4 == 0) {
+      if (wide && (ap & 1)) {
+        f(std::integral_constant<int, 0>{}, I4{});
+        static_for<0, N / 8>([&](auto ic) { f(std::integral_constant<int, 4 + 8 * decltype(ic)::value>{}, I8{}); });
+        return;
+      }
+      if (wide) {
+        static_for<0, N / 8>([&](auto ic) { f(std::integral_constant<int, 8 * decltype(ic)::value>{}, I8{}); });
+        f(std::integral_constant<int, N - 4>{}, I4{});
+        return;
+      }
+    }
+    if constexpr (N % 4 == 0) static_for<0, N / 4>([&](auto ic) { f(std::integral_constant<int, 4 * decltype(ic)::value>{}, I4{}); });
+    else static_for<0, N / 2>([&](auto ic) { f(std::integral_constant<int, 2 * decltype(ic)::value>{}, I2{}); });
+  }
+  template <int C>
+  static S2C_D void ld(const float* p, float (&v)[C]) {
+    if constexpr (C == 8) {
+      const float8 a = ld_global_256(p);
+      v[0] = a.lo.x; v[1] = a.lo.y; v[2] = a.lo.z; v[3] = a.lo.w;
+      v[4] = a.hi.x; v[5] = a.hi.y; v[6] = a.hi.z; v[7] = a.hi.w;
+    } else if constexpr (C == 4) {
+      const float4 a = *reinterpret_cast<const float4*>(p);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    } else {
+      const float2 a = *reinterpret_cast<const float2*>(p);
+      v[0] = a.x; v[1] = a.y;
+    }
+  }
+  template <int C>
+  static S2C_D void st(float* p, const float (&v)[C]) {
+    if constexpr (C == 8) {
+      float8 a;
+      a.lo = make_float4(v[0], v[1], v[2], v[3]);
+      a.hi = make_float4(v[4], v[5], v[6], v[7]);
+      st_global_256(p, a);
+    } else if constexpr (C == 4) {
+      *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+      *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    }
+  }
+};
+
+template <int N>
+struct so3_fwd_small_impl {
+  static S2C_D void run(const Ctx& ctx, const SmallParams& p, unsigned char* smem) {
+    using S = Small<N>;
+    constexpr int H = N / 2;
+    float2* planes = reinterpret_cast<float2*>(smem);
+    const long q0 = (long)ctx.bid * S::P;
+    const int ap = ctx.tid % H, pl = ctx.tid / H;
+    if (pl < S::P && q0 + pl < p.nplanes) {
+      const long row1 = ((q0 + pl) * N + ap) * (long)N, row2 = row1 + (long)H * N;
+      float2 v[N];
+      if (p.stride == 1) {
+        S::pieces(p.wide, ap, [&](auto gc, auto cc) {
+          constexpr int g = decltype(gc)::value, C = decltype(cc)::value;
+          float a[C], b[C];
+          S::ld(p.x + row1 + g, a);
+          S::ld(p.x + row2 + g, b);
+#pragma unroll
+          for (int i = 0; i < C; ++i) v[g + i] = make_float2(a[i], b[i]);
+        });
+      } else {
+#pragma unroll
+        for (int g = 0; g < N; ++g)
+          v[g] = make_float2(p.x[(row1 + g) * p.stride + p.off], p.x[(row2 + g) * p.stride + p.off]);
+      }
+      if (p.relu) {
+#pragma unroll
+        for (int g = 0; g < N; ++g) v[g] = make_float2(v[g].x > 0.f ? v[g].x : 0.f, v[g].y > 0.f ? v[g].y : 0.f);
+      }
+      fft_reg<N, -1>(v, nullptr);
+      S::split_rows(planes + pl * S::PS + ap * S::KP, p.K, v);
+    }
+    ctx.sync();
+    S::columns_fwd(ctx, p, q0, planes, p.v, p.K);
+  }
+};
+
+template <int N>
+struct so3_inv_small_impl {
+  static S2C_D void run(const Ctx& ctx, const SmallParams& p, unsigned char* smem) {
+    using S = Small<N>;
+    constexpr int H = N / 2;
+    float2* planes = reinterpret_cast<float2*>(smem);
+    const long q0 = (long)ctx.bid * S::P;
+    S::columns_inv(ctx, p, q0, planes);
+    ctx.sync();
+    const int ap = ctx.tid % H, pl = ctx.tid / H;
+    if (pl >= S::P || q0 + pl >= p.nplanes) return;
+    float2 v[N];
+    S::pack_rows(planes + pl * S::PS + ap * S::KP, p.K, v);
+    fft_reg<N, +1>(v, nullptr);
+    float add = 0.f;
+    if (p.bias) add = p.bias[(p.z0 + (q0 + pl) / N) % p.nfeat];
+    const long row1 = ((q0 + pl) * N + ap) * (long)N, row2 = row1 + (long)H * N;
+    if (p.stride == 1) {
+      S::pieces(p.wide, ap, [&](auto gc, auto cc) {
+        constexpr int g = decltype(gc)::value, C = decltype(cc)::value;
+        float a[C], b[C];
+        static_for<0, C>([&](auto ic) {
+          constexpr int i = decltype(ic)::value;
+          constexpr int pos = fft_reg_pos<N>(g + i);
+          a[i] = v[pos].x + add;
+          b[i] = v[pos].y + add;
+        });
+        if (p.mask) {
+          float k1[C], k2[C];
+          S::ld(p.mask + row1 + g, k1);
+          S::ld(p.mask + row2 + g, k2);
+#pragma unroll
+          for (int i = 0; i < C; ++i) {
+            a[i] = k1[i] > 0.f ? a[i] : 0.f;
+            b[i] = k2[i] > 0.f ? b[i] : 0.f;
+          }
+        }
+        S::st(p.out + row1 + g, a);
+        S::st(p.out + row2 + g, b);
+      });
+    } else {
+      static_for<0, N>([&](auto ic) {
+        constexpr int g = decltype(ic)::value;
+        constexpr int pg = fft_reg_pos<N>(g);
+        p.out[(row1 + g) * p.stride + p.off] = v[pg].x + add;
+        p.out[(row2 + g) * p.stride + p.off] = v[pg].y + add;
+      });
+    }
+  }
+};
+
+template <int N>
+struct so3_relay_small_impl {
+  static S2C_D void run(const Ctx& ctx, const SmallParams& p, unsigned char* smem) {
+    using S = Small<N>;
+    constexpr int H = N / 2;
+    float2* planes = reinterpret_cast<float2*>(smem);
+    const long q0 = (long)ctx.bid * S::P;
+    S::columns_inv(ctx, p, q0, planes);
+    ctx.sync();
+    const int ap = ctx.tid % H, pl = ctx.tid / H;
+    if (pl < S::P && q0 + pl < p.nplanes) {
+      float2* r1 = planes + pl * S::PS + ap * S::KP;
+      float2 v[N];
+      S::pack_rows(r1, p.K, v);
+      fft_reg<N, +1>(v, nullptr);
+      float add = 0.f;
+      if (p.bias) add = p.bias[(p.z0 + (q0 + pl) / N) % p.nfeat];
+      float2 u[N];
+      static_for<0, N>([&](auto gc) {
+        constexpr int g = decltype(gc)::value;
+        constexpr int pg = fft_reg_pos<N>(g);
+        const float a1 = v[pg].x + add, a2 = v[pg].y + add;   // samples gamma = g of both rows
+        u[g] = make_float2(a1 > 0.f ? a1 : 0.f, a2 > 0.f ? a2 : 0.f);
+      });
+      fft_reg<N, -1>(u, nullptr);
+      S::split_rows(r1, p.K2, u);      // in place: a thread owns its two rows
+    }
+    ctx.sync();
+    S::columns_fwd(ctx, p, q0, planes, p.v2, p.K2);
+  }
+};
+
+#ifndef S2C_EMUL
+#define S2C_SMALL_KERNEL(name)                                                                   \
+  template <int N>                                                                               \
+  __global__ void __launch_bounds__(small_threads(N)) name(const SmallParams p) {                \
+    extern __shared__ float4 s2c_dyn_smem[];                                                     \
+    Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};                 \
+    name##_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));                 \
+  }                                                                                              \
+  S2C_LAUNCHER_N(name, SmallParams)
+S2C_SMALL_KERNEL(so3_fwd_small)
+S2C_SMALL_KERNEL(so3_inv_small)
+S2C_SMALL_KERNEL(so3_relay_small)
+#endif
+#define S2C_LAUNCH_SMALL(name, N, stream, params)                                                \
+  S2C_LAUNCH_N(name, N, ((params).nplanes + small_planes(N) - 1) / small_planes(N), small_threads(N), small_smem_bytes(N), stream, params)
+#define S2C_DISPATCH_SMALL(N, CALL)                                                              \
+  switch (N) {                                                                                   \
+    case 10: { constexpr int kN = 10; CALL; } break;                                             \
+    case 12: { constexpr int kN = 12; CALL; } break;                                             \
+    case 14: { constexpr int kN = 14; CALL; } break;                                             \
+    case 16: { constexpr int kN = 16; CALL; } break;                                             \
+    case 18: { constexpr int kN = 18; CALL; } break;                                             \
+    case 20: { constexpr int kN = 20; CALL; } break;                                             \
+    S2C_CASES_32(CALL)                                                                           \
+    default: rc = s2c::fail(s2c::S2C_ERR_UNSUPPORTED, "no plane kernel for this length");        \
+  }
+
+}  // namespace s2c

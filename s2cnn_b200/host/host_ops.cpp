@@ -68,8 +68,8 @@ long s2_bandwidth(long nspec) {
 // ---- one build of the library ---------------------------------------------------------------------
 #define S2C_API(X)                                                                                 \
   X(last_error) X(is_cuda_build) X(tables_computed) X(so3_fft_workspace) X(so3_rfft)               \
-  X(so3_rfft_relu) X(so3_rfft_sums) X(so3_rfft_sums_ws) X(so3_rifft_relu_grad_ws) X(so3_fft) X(so3_rifft) X(so3_rifft_relu_grad)                 \
-  X(so3_rifft_relu_integrate) X(s2_conv_relu_so3_rfft) X(so3_rifft_relu_rfft)                      \
+  X(so3_rfft_relu) X(so3_rfft_sums_ws) X(so3_relay_workspace) X(s2_conv_relu_so3_rfft_ws) X(so3_rifft_relu_rfft_ws) X(so3_rifft_relu_grad_ws) X(so3_fft) X(so3_rifft)                 \
+  X(so3_rifft_relu_integrate)                      \
   X(s2_conv_synthesis_workspace) X(s2_conv_synthesis) X(so3_ifft) X(s2_fft_workspace) X(s2_fft)    \
   X(s2_ifft) X(so3_mm) X(so3_mm_gradx) X(so3_mm_grady) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
   X(s2_mm_grady) X(rft_forward) X(rft_forward_t) X(rft_forward_scaled) X(rft_backward) X(so3_integrate)                  \
@@ -221,11 +221,9 @@ struct Ops {
       Tensor out = empty_like_shape(x, spectrum_shape(so3_nspec(b_out), lead));
       Tensor sums = empty_like_shape(x, lead);
       Ctx c(*this, x);
-      Tensor ws;
-      if (2 * b_in > 32) ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
+      const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
       const int rc = call_rc("s2c_so3_rfft_sums_ws", so3_rfft_sums_ws_, cptr(x), ptr(out), ptr(sums), nb, (int)b_in,
-                             (int)b_out, (int)for_grad, ws.defined() ? ws.mutable_data_ptr() : nullptr,
-                             ws.defined() ? (size_t)ws.numel() : (size_t)0, c.stream);
+                             (int)b_out, (int)for_grad, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
       if (rc == 0) {
         log_new_tables("so3_rfft", b_in, b_out);
         return {out, sums};
@@ -278,13 +276,9 @@ struct Ops {
     check(x.size(-1) == 2 && x.sizes().slice(1, x.dim() - 2) == lead, "so3_rifft_relu_grad: shapes differ");
     Tensor out = at::empty_like(act);
     Ctx c(*this, x);
-    if (2 * b_out > 32) {
-      const long nb = lead_numel(lead);
-      const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
-      S2C_CALL(so3_rifft_relu_grad_ws, cptr(x), cptr(act), ptr(out), nb, (int)b_in, (int)b_out, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
-      return out;
-    }
-    S2C_CALL(so3_rifft_relu_grad, cptr(x), cptr(act), ptr(out), lead_numel(lead), (int)b_in, (int)b_out, c.stream);
+    const long nb = lead_numel(lead);
+    const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
+    S2C_CALL(so3_rifft_relu_grad_ws, cptr(x), cptr(act), ptr(out), nb, (int)b_in, (int)b_out, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
     return out;
   }
 
@@ -323,7 +317,8 @@ struct Ops {
     check(!bp || nfeat == d.fo, "s2_conv_relu_so3_rfft: one bias per output feature");
     Tensor out = empty_like_shape(xs, {so3_nspec(b_next), d.nb, d.fo, 2});
     Ctx c(*this, xs);
-    S2C_CALL(s2_conv_relu_so3_rfft, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, (int)b_next, bp, c.stream);
+    const Tensor ws = workspace(so3_relay_workspace_(d.nb * d.fo, (int)d.b, (int)d.b, (int)b_next), xs);
+    S2C_CALL(s2_conv_relu_so3_rfft_ws, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, (int)b_next, bp, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
     return out;
   }
 
@@ -340,7 +335,9 @@ struct Ops {
     check(!bp || (!lead.empty() && lead.back() == nfeat), "so3_rifft_relu_rfft: one bias per feature");
     Tensor out = empty_like_shape(x, spectrum_shape(so3_nspec(b_next), lead));
     Ctx c(*this, x);
-    S2C_CALL(so3_rifft_relu_rfft, cptr(x), ptr(out), lead_numel(lead), (int)b_in, (int)b_mid, (int)b_next, bp, nfeat, c.stream);
+    const long nb = lead_numel(lead);
+    const Tensor ws = workspace(so3_relay_workspace_(nb, (int)b_in, (int)b_mid, (int)b_next), x);
+    S2C_CALL(so3_rifft_relu_rfft_ws, cptr(x), ptr(out), nb, (int)b_in, (int)b_mid, (int)b_next, bp, nfeat, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
     return out;
   }
 

@@ -1,4 +1,4 @@
-"""The cluster kernels of 2b <= 32 against the kernels whose blocks walk beta: same sums in the same order, so
+"""The cluster kernels and the plane kernels of 2b <= 32 against the kernels whose blocks walk beta: same sums in the same order, so
 equal to the last bit on the GPU.  One block per cluster, two, four and eight, betas that do not divide evenly
 (2b = 12, 18, 22, 26, 30: a short last block; 28: an empty one), batches that end inside a group of four, more degrees
 than the grid holds, a fused product with a feature count that is no multiple of four, masks, sums, the integral."""
@@ -14,7 +14,7 @@ n3 = O.so3_nspec
 
 @pytest.mark.parametrize("backend", backends.BACKENDS)
 @pytest.mark.parametrize("b,b_spec,nb", [(1, 1, 1), (3, 3, 5), (5, 2, 4), (6, 8, 3), (9, 9, 2), (10, 6, 9), (11, 11, 4),
-                                         (13, 4, 1), (14, 14, 8), (15, 9, 6), (16, 16, 4)])
+                                         (7, 7, 70), (12, 5, 3), (13, 4, 1), (14, 14, 8), (15, 9, 6), (16, 16, 4)])
 def test_cluster_kernels_match_walking_kernels(backend, b, b_spec, nb):
     ops, dev = backends.get(backend)
     gen = torch.Generator().manual_seed(31 * b + b_spec)
@@ -39,14 +39,15 @@ def test_cluster_kernels_match_walking_kernels(backend, b, b_spec, nb):
         return out
 
     res = []
-    for mode in (1, 2):
+    for mode in (2, 1, 3):
         ops.lib.s2c_debug_cluster(mode)
         try:
             res.append(all_ops())
         finally:
             ops.lib.s2c_debug_cluster(0)
     for k in res[0]:
-        if k in ("sums", "integral") or backend != "cuda":    # summed over threads in another order
-            assert_close(res[0][k], res[1][k], k)
-        else:
-            assert torch.equal(res[0][k], res[1][k]), k
+        for other, mode in zip(res[1:], (1, 3)):
+            if k in ("sums", "integral") or backend != "cuda":    # summed over threads in another order
+                assert_close(other[k], res[0][k], "%s, mode %d" % (k, mode))
+            else:
+                assert torch.equal(other[k], res[0][k]), (k, mode)
