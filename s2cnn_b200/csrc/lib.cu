@@ -20,6 +20,7 @@
 #include "so3_mid_kernels.h"
 #include "s2_kernels.h"
 #include "so3_small_kernels.h"
+#include "wigner_columns.h"
 #include "wigner_tiled.h"
 #include "wigner_rows.h"
 #include "cgemm_kernels.h"
@@ -144,11 +145,22 @@ static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, c
   const int forced = g_cluster.load();
   if (g_force_general || !small_supported(N) || !ws || forced == 1 || forced == 2) return false;
   if (ws_bytes < so3_mid_v_per_z(N, K) * (size_t)std::min<long>(kWigZT, nbatch) ||
-      !fwd_wigner_t_fits(N, nl, kWigZT, dev_smem_limit()))
+      nl > kColMaxDegrees)
     return false;
   if (forced == 3) return true;
   (void)kind;
   return (nbatch + kFusedZG - 1) / kFusedZG > 160;
+}
+
+static int launch_fwd_wigner_col(FwdWignerParams w, stream_t st) {
+  w.ZT = std::min(kColZT, (w.nbatch + 31) / 32 * 32);
+  w.nzt = (w.nbatch + w.ZT - 1) / w.ZT;
+  return S2C_LAUNCH(so3_fwd_wigner_col, (long)w.pan.npairs * w.nzt, w.ZT, wigner_col_smem(w.N, w.nl), st, w);
+}
+static int launch_inv_wigner_col(InvWignerParams w, stream_t st) {
+  w.ZT = std::min(kColZT, (w.nbatch + 31) / 32 * 32);
+  w.nzt = (w.nbatch + w.ZT - 1) / w.ZT;
+  return S2C_LAUNCH(so3_inv_wigner_col, (long)w.pan.npairs * w.nzt, w.ZT, wigner_col_smem(w.N, w.pan.nl), st, w);
 }
 
 static int check_b(int b_in, int b_out) {
@@ -244,7 +256,7 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
       g.stride = in_stride; g.off = in_off;
       g.v = v; g.v2 = nullptr; g.bias = nullptr; g.nfeat = 1; g.z0 = z0; g.mask = nullptr; g.relu = relu;
       g.wide = in_stride == 1 && N % 4 == 0 && (uintptr_t)x % 32 == 0;
-      g.nplanes = zc * N; g.K = K; g.K2 = 0;
+      g.nplanes = zc * N; g.nz = (int)zc; g.K = K; g.K2 = 0;
       int rc = S2C_OK;
       S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_fwd_small, kN, st, g));
       if (rc) return rc;
@@ -281,6 +293,7 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
     if (sums) {
       MidSumsParams q;
       q.v = v + (size_t)(K - 1) * zc * N; q.sums = sums + z0; q.nbatch = (int)zc; q.N = N;
+      q.zs = small ? 1 : N; q.bs = small ? (int)zc : 1;
       S2C_TRY(S2C_LAUNCH(so3_mid_sums, (zc + 31) / 32, 32, 0, st, q));
     }
     FwdWignerParams w;
@@ -292,6 +305,10 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
     w.ZT = (int)std::min<long>(32, zc);
     w.nzt = (int)((zc + w.ZT - 1) / w.ZT);
     w.mode = mode;
+    if (small) {
+      S2C_TRY(launch_fwd_wigner_col(w, st));
+      continue;
+    }
     if (fwd_wigner_t_fits(N, b_out, kWigZT, dev_smem_limit())) {
       w.ZT = kWigZT;
       w.nzt = (int)((zc + kWigZT - 1) / kWigZT);
@@ -450,7 +467,9 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
       w.s2_nb = prod->nb; w.s2_fin = prod->fin; w.s2_fout = prod->fout;
       w.z0 = z0;
     }
-    if (inv_wigner_t_smem(N, K) <= (size_t)dev_smem_limit() - 1024) {
+    if (small) {
+      S2C_TRY(launch_inv_wigner_col(w, st));
+    } else if (inv_wigner_t_smem(N, K) <= (size_t)dev_smem_limit() - 1024) {
       w.ZT = kWigZT;
       w.nzt = (int)((zc + kWigZT - 1) / kWigZT);
       S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)pan.npairs * w.nzt, kThreads,
@@ -466,7 +485,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
       g.v = s; g.v2 = nullptr; g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0; g.relu = 0;
       g.mask = mask ? mask + (size_t)z0 * N * N * N : nullptr;
       g.wide = out_stride == 1 && N % 4 == 0 && (uintptr_t)out % 32 == 0 && (uintptr_t)mask % 32 == 0;
-      g.nplanes = zc * N; g.K = K; g.K2 = 0;
+      g.nplanes = zc * N; g.nz = (int)zc; g.K = K; g.K2 = 0;
       int rc = S2C_OK;
       S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_inv_small, kN, st, g));
       if (rc) return rc;
@@ -827,20 +846,20 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
       float2* vo = v + (size_t)zc * (v1 / sizeof(float2));
       InvWignerParams w;
       w.x = xs ? nullptr : x + z0; w.x_zstride = nz; w.s = v; w.pan = pin;
-      w.nbatch = (int)zc; w.N = N; w.K = b_in; w.ZT = kWigZT; w.nzt = (int)((zc + kWigZT - 1) / kWigZT); w.mode = kSo3Real;
+      w.nbatch = (int)zc; w.N = N; w.K = b_in; w.mode = kSo3Real;
       w.xs = xs; w.ys = ys; w.s2_nb = s2_nb; w.s2_fin = s2_fin; w.s2_fout = nfeat; w.z0 = z0;
-      S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)pin.npairs * w.nzt, kThreads, inv_wigner_t_smem(N, b_in), st, w));
+      S2C_TRY(launch_inv_wigner_col(w, st));
       SmallParams g;
       g.x = nullptr; g.out = nullptr; g.stride = 1; g.off = 0; g.v = v; g.v2 = vo;
       g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0; g.mask = nullptr; g.relu = 1; g.wide = 0;
-      g.nplanes = zc * N; g.K = b_in; g.K2 = b_next;
+      g.nplanes = zc * N; g.nz = (int)zc; g.K = b_in; g.K2 = b_next;
       int rc = S2C_OK;
       S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_relay_small, kN, st, g));
       if (rc) return rc;
       FwdWignerParams f;
       f.v = vo; f.out = (float2*)out + z0; f.out_zstride = nz; f.pan = pout;
-      f.nbatch = (int)zc; f.N = N; f.K = b_next; f.nl = b_next; f.ZT = kWigZT; f.nzt = w.nzt; f.mode = kSo3Real;
-      S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)pout.npairs * f.nzt, kThreads, fwd_wigner_t_smem(N, b_next), st, f));
+      f.nbatch = (int)zc; f.N = N; f.K = b_next; f.nl = b_next; f.mode = kSo3Real;
+      S2C_TRY(launch_fwd_wigner_col(f, st));
     }
     return S2C_OK;
   }

@@ -270,15 +270,15 @@ struct so3_inv_mid_impl {
 
 // by-product of the analysis: the plain sum of every signal, i.e. its (0, 0) bins summed over beta
 struct MidSumsParams {
-  const float2* v;     // V[n = 0][m = 0]: [z][beta]
+  const float2* v;     // V[n = 0][m = 0], element (z, beta) at v[z * zs + beta * bs]
   float* sums;
-  int nbatch, N;
+  int nbatch, N, zs, bs;
 };
 S2C_KERNEL(so3_mid_sums, MidSumsParams) {
   const int z = ctx.bid * ctx.nthr + ctx.tid;
   if (z >= p.nbatch) return;
   float s = 0.f;
-  for (int b = 0; b < p.N; ++b) s += p.v[(long)z * p.N + b].x;
+  for (int b = 0; b < p.N; ++b) s += p.v[(long)z * p.zs + (long)b * p.bs].x;
   p.sums[z] = s;
 }
 

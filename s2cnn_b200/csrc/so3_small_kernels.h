@@ -1,12 +1,12 @@
 // Plane kernels of the SO(3) transform for small bandwidths (10 <= N = 2b <= 32) and LARGE batches: both row
 // transforms of P neighbouring (z, beta) planes in one block, every 1-D FFT in the registers of one thread
-// (fft_reg.h), between the signal and the [n][m][z][beta] array of the tiled Wigner kernels (wigner_tiled.h).
+// (fft_reg.h), between the signal and the V[n][m][beta][z] array of wigner_columns.h.
 //
 // The single-kernel transforms (so3_fused_kernels.h) keep the spectrum of four batch elements, the Wigner slice and
 // the planes of a beta group in one block: at b = 16 that is 210 KB, one block of 16 warps per SM whose eight beta
 // groups pass four block barriers each (0.34 instructions per clock and scheduler, 4 of 12 stall cycles at
-// barriers).  For a large batch the Wigner contraction is better off on its own - a tile shares each table row
-// among 64 signals - and what is left needs one barrier and 35 KB: several blocks per SM overlap their loads,
+// barriers).  For a large batch the Wigner contraction is better off on its own - a block shares each table row
+// among 128 signals - and what is left needs one barrier and 35 KB: several blocks per SM overlap their loads,
 // transforms and stores.  The array between the two stays in L2 (chunks of at most 64 MB).
 //
 //   so3_fwd_small    two real rows per thread (optional ReLU on load) -> n -> columns alpha -> m -> V
@@ -14,7 +14,7 @@
 //   so3_relay_small  the synthesis, + bias, ReLU, forward row transform in the same registers, then the rest of
 //                    the analysis: the signal between two layers never exists in memory
 //
-// The planes of a block are consecutive in (z, beta), so that V is moved in runs of 8 P bytes.  Same FFTs, same
+// The planes of a block are consecutive in (beta, z), so that V is moved in runs of 8 P bytes.  Same FFTs, same
 // sums in the same order as the single-kernel transforms: the results are the same bit for bit.
 #pragma once
 
@@ -41,14 +41,15 @@ struct SmallParams {
   const float* x;      // analysis: real signal, element e at x[e * stride + off]
   float* out;          // synthesis: the same
   long stride, off;
-  float2* v;           // [n < K][m + K - 1][z][beta]: analysis output, synthesis / relay input
+  float2* v;           // [n < K][m + K - 1][beta][z]: analysis output, synthesis / relay input
   float2* v2;          // relay output, bandwidth K2
   const float* bias;   // optional [nfeat]; feature of signal z is (z0 + z) % nfeat
   int nfeat;
   long z0;
   const float* mask;   // synthesis, optional (unit stride): samples where this signal is <= 0 are written as 0
   int relu, wide;      // wide: 32-byte accesses to x / out / mask
-  long nplanes;        // signals * N
+  long nplanes;        // signals * N, plane q is (beta = q / nz, z = q % nz)
+  int nz;              // signals
   int K, K2;
 };
 
@@ -193,7 +194,8 @@ struct so3_fwd_small_impl {
     const long q0 = (long)ctx.bid * S::P;
     const int ap = ctx.tid % H, pl = ctx.tid / H;
     if (pl < S::P && q0 + pl < p.nplanes) {
-      const long row1 = ((q0 + pl) * N + ap) * (long)N, row2 = row1 + (long)H * N;
+      const int beta = (int)((q0 + pl) / p.nz), z = (int)(q0 + pl - (long)beta * p.nz);
+      const long row1 = (((long)z * N + beta) * N + ap) * (long)N, row2 = row1 + (long)H * N;
       float2 v[N];
       if (p.stride == 1) {
         S::pieces(p.wide, ap, [&](auto gc, auto cc) {
@@ -235,9 +237,10 @@ struct so3_inv_small_impl {
     float2 v[N];
     S::pack_rows(planes + pl * S::PS + ap * S::KP, p.K, v);
     fft_reg<N, +1>(v, nullptr);
+    const int beta = (int)((q0 + pl) / p.nz), z = (int)(q0 + pl - (long)beta * p.nz);
     float add = 0.f;
-    if (p.bias) add = p.bias[(p.z0 + (q0 + pl) / N) % p.nfeat];
-    const long row1 = ((q0 + pl) * N + ap) * (long)N, row2 = row1 + (long)H * N;
+    if (p.bias) add = p.bias[(p.z0 + z) % p.nfeat];
+    const long row1 = (((long)z * N + beta) * N + ap) * (long)N, row2 = row1 + (long)H * N;
     if (p.stride == 1) {
       S::pieces(p.wide, ap, [&](auto gc, auto cc) {
         constexpr int g = decltype(gc)::value, C = decltype(cc)::value;
@@ -288,7 +291,7 @@ struct so3_relay_small_impl {
       S::pack_rows(r1, p.K, v);
       fft_reg<N, +1>(v, nullptr);
       float add = 0.f;
-      if (p.bias) add = p.bias[(p.z0 + (q0 + pl) / N) % p.nfeat];
+      if (p.bias) add = p.bias[(p.z0 + (q0 + pl) % p.nz) % p.nfeat];
       float2 u[N];
       static_for<0, N>([&](auto gc) {
         constexpr int g = decltype(gc)::value;

@@ -1,0 +1,172 @@
+// Wigner-d contractions for 2b <= 32 and large batches: one batch element per thread.
+//
+// Same inputs, outputs and sums (same order) as wigner_tiled.h, between spectrum rows and V[n][m][beta][z] - the
+// batch innermost on both sides, so that every access of a warp is one run of 256 bytes and nothing but the table
+// goes through shared memory.  At b = 16 a frequency pair has 5 degrees on average: the tiles of 4 x 2 outputs
+// there share too little (512 signals: 44 us analysis, of which the copies into shared memory and the padded
+// tiles are most), while a thread that owns all degrees of one batch element reads each sample of V once and
+// each table entry as a broadcast of 16 bytes.  Bound by the L2 traffic of V.
+#pragma once
+
+#include "backend.h"
+#include "so3_kernels.h"
+#include "wigner_tiled.h"
+
+namespace s2c {
+
+constexpr int kColZT = 128;          // batch elements (threads) per block
+constexpr int kColMaxDegrees = 16;   // degrees a thread keeps in registers
+
+S2C_HD constexpr int col_nb(int N) { return (N + 7) / 8 * 8; }
+inline size_t wigner_col_smem(int N, int nl) { return (size_t)col_nb(N) * ((nl + 3) / 4 * 4) * sizeof(float); }
+
+// X[l][z] = sum_beta W[l][beta] V[beta][z]   (+ Hermitian mirror row); table as [beta][l], zero-padded
+S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
+  const int N = p.N;
+  const int pair = ctx.bid / p.nzt, zt = ctx.bid - pair * p.nzt;
+  int m, n;
+  so3_pair_decode(pair, p.K, m, n);
+  const int am = m < 0 ? -m : m;
+  const int lmin = am > n ? am : n;
+  const int L = p.nl - lmin;
+  if (L <= 0) return;
+  const int LT = (L + 3) / 4;
+  float* Ws = reinterpret_cast<float*>(smem);   // [beta][4 LT]
+  const float* panel = p.pan.data + p.pan.off[pair];
+  for (int i = ctx.tid; i < 4 * LT * N; i += ctx.nthr) {
+    const int l = i / N, bt = i - l * N;
+    Ws[bt * 4 * LT + l] = l < L ? panel[i] : 0.f;
+  }
+  ctx.sync();
+  const int z = zt * p.ZT + ctx.tid;
+  if (z >= p.nbatch) return;
+  const int nm = 2 * p.K - 1, mi = m + p.K - 1;
+  const float2* v = p.v + ((long)n * nm + mi) * N * p.nbatch + z;
+  const float fudge = ((m - n) & 1) ? -1.f : 1.f;
+  const bool self = (m == 0 && n == 0);
+  auto degrees = [&](auto tiles) {
+    constexpr int T = decltype(tiles)::value;
+    float2 re[2 * T], im[2 * T];                // two degrees each
+#pragma unroll
+    for (int i = 0; i < 2 * T; ++i) re[i] = im[i] = make_float2(0.f, 0.f);
+    for (int b0 = 0; b0 < N; b0 += 8) {
+      float2 c[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (b0 + u < N) c[u] = v[(long)(b0 + u) * p.nbatch];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (b0 + u < N) {
+          const float2 cr = make_float2(c[u].x, c[u].x), ci = make_float2(c[u].y, c[u].y);
+          const float4* w = reinterpret_cast<const float4*>(Ws + (b0 + u) * 4 * T);
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
+            const float4 w4 = w[t];
+            const float2 lo = make_float2(w4.x, w4.y), hi = make_float2(w4.z, w4.w);
+            re[2 * t] = fma2(lo, cr, re[2 * t]);
+            im[2 * t] = fma2(lo, ci, im[2 * t]);
+            re[2 * t + 1] = fma2(hi, cr, re[2 * t + 1]);
+            im[2 * t + 1] = fma2(hi, ci, im[2 * t + 1]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int li = 0; li < 4 * T; ++li) {
+      if (li >= L) continue;
+      const float x = li & 1 ? re[li / 2].y : re[li / 2].x, y = li & 1 ? im[li / 2].y : im[li / 2].x;
+      float2* o1 = p.out + so3_row(lmin + li, m, n) * p.out_zstride + z;
+      float2* o2 = p.out + so3_row(lmin + li, -m, -n) * p.out_zstride + z;
+      if (p.mode == kSo3Real) {
+        *o1 = make_float2(x, y);
+        if (!self) *o2 = make_float2(fudge * x, -fudge * y);
+      } else {  // += i * (x + i y); mirror += i * fudge * conj
+        float2 q = *o1;
+        *o1 = make_float2(q.x - y, q.y + x);
+        if (!self) {
+          q = *o2;
+          *o2 = make_float2(q.x + fudge * y, q.y + fudge * x);
+        }
+      }
+    }
+  };
+  if (LT == 1) degrees(std::integral_constant<int, 1>{});
+  else if (LT == 2) degrees(std::integral_constant<int, 2>{});
+  else if (LT == 3) degrees(std::integral_constant<int, 3>{});
+  else degrees(std::integral_constant<int, 4>{});
+}
+
+// S[beta][z] = sum_l W[l][beta] Xs[l][z],  Xs = symmetrised spectrum (or S2 product); table as [l][beta]
+S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) {
+  const int N = p.N, NP = col_nb(N);
+  const int pair = ctx.bid / p.nzt, zt = ctx.bid - pair * p.nzt;
+  int m, n;
+  so3_pair_decode(pair, p.K, m, n);
+  const int am = m < 0 ? -m : m;
+  const int lmin = am > n ? am : n;
+  const int L = p.pan.nl - lmin;
+  if (L <= 0) return;
+  const int LT = (L + 3) / 4;
+  float* Ws = reinterpret_cast<float*>(smem);   // [4 LT][NP]
+  const float* panel = p.pan.data + p.pan.off[pair];
+  for (int i = ctx.tid; i < 4 * LT * NP; i += ctx.nthr) {
+    const int l = i / NP, bt = i - l * NP;
+    Ws[i] = l < L && bt < N ? panel[l * N + bt] : 0.f;
+  }
+  ctx.sync();
+  const int z = zt * p.ZT + ctx.tid;
+  if (z >= p.nbatch) return;
+  const float fudge = ((m - n) & 1) ? -1.f : 1.f;
+  const int nm = 2 * p.K - 1, mi = m + p.K - 1;
+  float2* s = p.s + ((long)n * nm + mi) * N * p.nbatch + z;
+  auto degrees = [&](auto tiles) {
+    constexpr int T = decltype(tiles)::value;
+    float2 x[4 * T];
+#pragma unroll
+    for (int li = 0; li < 4 * T; ++li) {
+      x[li] = make_float2(0.f, 0.f);
+      if (li >= L) continue;
+      const int l = lmin + li;
+      float2 a, b;
+      if (p.xs) {
+        const int i = (int)((p.z0 + z) / p.s2_fout), j = (int)(p.z0 + z - (long)i * p.s2_fout);
+        a = wig_s2_product(p, l, m, n, i, j);
+        b = wig_s2_product(p, l, -m, -n, i, j);
+      } else {
+        a = p.x[so3_row(l, m, n) * p.x_zstride + z];
+        b = p.x[so3_row(l, -m, -n) * p.x_zstride + z];
+        if (p.mode == kSo3RotI) {  // multiply the spectrum by -i
+          a = make_float2(a.y, -a.x);
+          b = make_float2(b.y, -b.x);
+        }
+      }
+      x[li] = make_float2(0.5f * (a.x + fudge * b.x), 0.5f * (a.y - fudge * b.y));
+    }
+    for (int b0 = 0; b0 < N; b0 += 4) {
+      float2 r0 = make_float2(0.f, 0.f), r1 = r0, i0 = r0, i1 = r0;   // two betas each
+#pragma unroll
+      for (int li = 0; li < 4 * T; ++li) {
+        const float4 w4 = *reinterpret_cast<const float4*>(Ws + li * NP + b0);
+        const float2 lo = make_float2(w4.x, w4.y), hi = make_float2(w4.z, w4.w);
+        const float2 xr = make_float2(x[li].x, x[li].x), xi = make_float2(x[li].y, x[li].y);
+        r0 = fma2(lo, xr, r0);
+        i0 = fma2(lo, xi, i0);
+        r1 = fma2(hi, xr, r1);
+        i1 = fma2(hi, xi, i1);
+      }
+      float2* o = s + (long)b0 * p.nbatch;
+      o[0] = make_float2(r0.x, i0.x);
+      o[p.nbatch] = make_float2(r0.y, i0.y);
+      if (b0 + 2 < N) {
+        o[2L * p.nbatch] = make_float2(r1.x, i1.x);
+        o[3L * p.nbatch] = make_float2(r1.y, i1.y);
+      }
+    }
+  };
+  if (LT == 1) degrees(std::integral_constant<int, 1>{});
+  else if (LT == 2) degrees(std::integral_constant<int, 2>{});
+  else if (LT == 3) degrees(std::integral_constant<int, 3>{});
+  else degrees(std::integral_constant<int, 4>{});
+}
+
+}  // namespace s2c
