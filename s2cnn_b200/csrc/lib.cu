@@ -160,6 +160,8 @@ static int launch_fwd_wigner_col(FwdWignerParams w, stream_t st) {
 static int launch_inv_wigner_col(InvWignerParams w, stream_t st) {
   w.ZT = std::min(kColZT, (w.nbatch + 31) / 32 * 32);
   w.nzt = (w.nbatch + w.ZT - 1) / w.ZT;
+  if (w.xs)
+    return S2C_LAUNCH(so3_inv_wigner_col_s2, (long)w.pan.npairs * w.nzt, w.ZT, wigner_col_smem(w.N, w.pan.nl), st, w);
   return S2C_LAUNCH(so3_inv_wigner_col, (long)w.pan.npairs * w.nzt, w.ZT, wigner_col_smem(w.N, w.pan.nl), st, w);
 }
 
@@ -255,7 +257,6 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
       g.x = x + (size_t)z0 * N * N * N * in_stride; g.out = nullptr;
       g.stride = in_stride; g.off = in_off;
       g.v = v; g.v2 = nullptr; g.bias = nullptr; g.nfeat = 1; g.z0 = z0; g.mask = nullptr; g.relu = relu;
-      g.wide = in_stride == 1 && N % 4 == 0 && (uintptr_t)x % 32 == 0;
       g.nplanes = zc * N; g.nz = (int)zc; g.K = K; g.K2 = 0;
       int rc = S2C_OK;
       S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_fwd_small, kN, st, g));
@@ -484,7 +485,6 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
       g.stride = out_stride; g.off = out_off;
       g.v = s; g.v2 = nullptr; g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0; g.relu = 0;
       g.mask = mask ? mask + (size_t)z0 * N * N * N : nullptr;
-      g.wide = out_stride == 1 && N % 4 == 0 && (uintptr_t)out % 32 == 0 && (uintptr_t)mask % 32 == 0;
       g.nplanes = zc * N; g.nz = (int)zc; g.K = K; g.K2 = 0;
       int rc = S2C_OK;
       S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_inv_small, kN, st, g));
@@ -851,7 +851,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
       S2C_TRY(launch_inv_wigner_col(w, st));
       SmallParams g;
       g.x = nullptr; g.out = nullptr; g.stride = 1; g.off = 0; g.v = v; g.v2 = vo;
-      g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0; g.mask = nullptr; g.relu = 1; g.wide = 0;
+      g.bias = bias; g.nfeat = nfeat > 0 ? nfeat : 1; g.z0 = z0; g.mask = nullptr; g.relu = 1;
       g.nplanes = zc * N; g.nz = (int)zc; g.K = b_in; g.K2 = b_next;
       int rc = S2C_OK;
       S2C_DISPATCH_SMALL(N, rc = S2C_LAUNCH_SMALL(so3_relay_small, kN, st, g));

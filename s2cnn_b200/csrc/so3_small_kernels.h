@@ -47,11 +47,22 @@ struct SmallParams {
   int nfeat;
   long z0;
   const float* mask;   // synthesis, optional (unit stride): samples where this signal is <= 0 are written as 0
-  int relu, wide;      // wide: 32-byte accesses to x / out / mask
+  int relu;
   long nplanes;        // signals * N, plane q is (beta = q / nz, z = q % nz)
   int nz;              // signals
   int K, K2;
 };
+
+// 8 bytes from global to shared memory, not through registers
+#ifndef S2C_EMUL
+S2C_D void small_copy(float2* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+S2C_D void small_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+#else
+S2C_D void small_copy(float2* dst, const float* src) { *dst = *reinterpret_cast<const float2*>(src); }
+S2C_D void small_copy_wait() {}
+#endif
 
 template <int N>
 struct Small {
@@ -67,14 +78,11 @@ struct Small {
     for (int i = 0; i < N; ++i) {
       const int m = i < H ? i : i - N;
       v[i] = make_float2(0.f, 0.f);
-      if (m < K && m > -K) {
-        if (n == 0 && m < 0) {                               // only m >= 0 is stored: Hermitian
-          const float2 c = s[-m * p.nplanes];
-          v[i] = make_float2(c.x, -c.y);
-        } else {
-          v[i] = s[m * p.nplanes];
-        }
-      }
+      if (m < K && m > -K) v[i] = s[(m < 0 && n == 0 ? -m : m) * p.nplanes];
+    }
+    if (n == 0) {                                            // only m >= 0 is stored: Hermitian
+#pragma unroll
+      for (int i = H; i < N; ++i) v[i].y = -v[i].y;
     }
     fft_reg<N, +1>(v, nullptr);
     float2* col = planes + pl * PS + n;
@@ -132,56 +140,19 @@ struct Small {
     });
   }
 
-  // the samples of two rows in pieces of 8, 4 (32- and 16-byte accesses; rows of N % 8 == 4 floats start on a sector
-  // boundary only every other row) or 2 floats: f(first, count)
+  // Planes of a real signal go through the rows' own places in shared memory (row stride KP complex >= N floats), so
+  // that the lanes of a warp touch neighbouring samples in memory: a row per thread would take 32 cache lines per
+  // access (b = 15: 81 % of the L1 rate).  f(place in shared memory, offset in the signal) for every two samples; a
+  // thread keeps its plane and gamma and steps over alpha, so that all addresses are constants apart.
   template <class F>
-  static S2C_D void pieces(bool wide, int ap, F&& f) {
-    using I2 = std::integral_constant<int, 2>;
-    using I4 = std::integral_constant<int, 4>;
-    using I8 = std::integral_constant<int, 8>;
-    if constexpr (N % 8 == 0) {
-      if (wide) { static_for<0, N / 8>([&](auto ic) { f(std::integral_constant<int, 8 * decltype(ic)::value>{}, I8{}); }); return; }
-    } else if constexpr (N % 4 == 0) {
-      if (wide && (ap & 1)) {
-        f(std::integral_constant<int, 0>{}, I4{});
-        static_for<0, N / 8>([&](auto ic) { f(std::integral_constant<int, 4 + 8 * decltype(ic)::value>{}, I8{}); });
-        return;
-      }
-      if (wide) {
-        static_for<0, N / 8>([&](auto ic) { f(std::integral_constant<int, 8 * decltype(ic)::value>{}, I8{}); });
-        f(std::integral_constant<int, N - 4>{}, I4{});
-        return;
-      }
-    }
-    if constexpr (N % 4 == 0) static_for<0, N / 4>([&](auto ic) { f(std::integral_constant<int, 4 * decltype(ic)::value>{}, I4{}); });
-    else static_for<0, N / 2>([&](auto ic) { f(std::integral_constant<int, 2 * decltype(ic)::value>{}, I2{}); });
-  }
-  template <int C>
-  static S2C_D void ld(const float* p, float (&v)[C]) {
-    if constexpr (C == 8) {
-      const float8 a = ld_global_256(p);
-      v[0] = a.lo.x; v[1] = a.lo.y; v[2] = a.lo.z; v[3] = a.lo.w;
-      v[4] = a.hi.x; v[5] = a.hi.y; v[6] = a.hi.z; v[7] = a.hi.w;
-    } else if constexpr (C == 4) {
-      const float4 a = *reinterpret_cast<const float4*>(p);
-      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    } else {
-      const float2 a = *reinterpret_cast<const float2*>(p);
-      v[0] = a.x; v[1] = a.y;
-    }
-  }
-  template <int C>
-  static S2C_D void st(float* p, const float (&v)[C]) {
-    if constexpr (C == 8) {
-      float8 a;
-      a.lo = make_float4(v[0], v[1], v[2], v[3]);
-      a.hi = make_float4(v[4], v[5], v[6], v[7]);
-      st_global_256(p, a);
-    } else if constexpr (C == 4) {
-      *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-      *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-    }
+  static S2C_D void samples(const Ctx& ctx, const SmallParams& p, long q0, float2* planes, F&& f) {
+    const int c = ctx.tid % H, pl = ctx.tid / H;
+    if (pl >= P || q0 + pl >= p.nplanes) return;
+    const int beta = (int)((q0 + pl) / p.nz), z = (int)(q0 + pl - (long)beta * p.nz);
+    const long base = ((long)z * N + beta) * (N * N) + 2 * c;
+    float2* place = planes + pl * PS + c;
+#pragma unroll
+    for (int a = 0; a < N; ++a) f(place + a * KP, base + a * N);
   }
 };
 
@@ -192,21 +163,25 @@ struct so3_fwd_small_impl {
     constexpr int H = N / 2;
     float2* planes = reinterpret_cast<float2*>(smem);
     const long q0 = (long)ctx.bid * S::P;
+    if (p.stride == 1) {
+      S::samples(ctx, p, q0, planes, [&](float2* place, long at) { small_copy(place, p.x + at); });
+      small_copy_wait();
+      ctx.sync();
+    }
     const int ap = ctx.tid % H, pl = ctx.tid / H;
     if (pl < S::P && q0 + pl < p.nplanes) {
-      const int beta = (int)((q0 + pl) / p.nz), z = (int)(q0 + pl - (long)beta * p.nz);
-      const long row1 = (((long)z * N + beta) * N + ap) * (long)N, row2 = row1 + (long)H * N;
+      float2* r1 = planes + pl * S::PS + ap * S::KP;
       float2 v[N];
       if (p.stride == 1) {
-        S::pieces(p.wide, ap, [&](auto gc, auto cc) {
-          constexpr int g = decltype(gc)::value, C = decltype(cc)::value;
-          float a[C], b[C];
-          S::ld(p.x + row1 + g, a);
-          S::ld(p.x + row2 + g, b);
 #pragma unroll
-          for (int i = 0; i < C; ++i) v[g + i] = make_float2(a[i], b[i]);
-        });
+        for (int c = 0; c < H; ++c) {
+          const float2 a = r1[c], b = r1[H * S::KP + c];
+          v[2 * c] = make_float2(a.x, b.x);
+          v[2 * c + 1] = make_float2(a.y, b.y);
+        }
       } else {
+        const int beta = (int)((q0 + pl) / p.nz), z = (int)(q0 + pl - (long)beta * p.nz);
+        const long row1 = (((long)z * N + beta) * N + ap) * (long)N, row2 = row1 + (long)H * N;
 #pragma unroll
         for (int g = 0; g < N; ++g)
           v[g] = make_float2(p.x[(row1 + g) * p.stride + p.off], p.x[(row2 + g) * p.stride + p.off]);
@@ -216,7 +191,7 @@ struct so3_fwd_small_impl {
         for (int g = 0; g < N; ++g) v[g] = make_float2(v[g].x > 0.f ? v[g].x : 0.f, v[g].y > 0.f ? v[g].y : 0.f);
       }
       fft_reg<N, -1>(v, nullptr);
-      S::split_rows(planes + pl * S::PS + ap * S::KP, p.K, v);
+      S::split_rows(r1, p.K, v);        // in place: a thread owns its two rows
     }
     ctx.sync();
     S::columns_fwd(ctx, p, q0, planes, p.v, p.K);
@@ -233,45 +208,40 @@ struct so3_inv_small_impl {
     S::columns_inv(ctx, p, q0, planes);
     ctx.sync();
     const int ap = ctx.tid % H, pl = ctx.tid / H;
-    if (pl >= S::P || q0 + pl >= p.nplanes) return;
-    float2 v[N];
-    S::pack_rows(planes + pl * S::PS + ap * S::KP, p.K, v);
-    fft_reg<N, +1>(v, nullptr);
-    const int beta = (int)((q0 + pl) / p.nz), z = (int)(q0 + pl - (long)beta * p.nz);
-    float add = 0.f;
-    if (p.bias) add = p.bias[(p.z0 + z) % p.nfeat];
-    const long row1 = (((long)z * N + beta) * N + ap) * (long)N, row2 = row1 + (long)H * N;
-    if (p.stride == 1) {
-      S::pieces(p.wide, ap, [&](auto gc, auto cc) {
-        constexpr int g = decltype(gc)::value, C = decltype(cc)::value;
-        float a[C], b[C];
-        static_for<0, C>([&](auto ic) {
-          constexpr int i = decltype(ic)::value;
-          constexpr int pos = fft_reg_pos<N>(g + i);
-          a[i] = v[pos].x + add;
-          b[i] = v[pos].y + add;
+    if (pl < S::P && q0 + pl < p.nplanes) {
+      float2* r1 = planes + pl * S::PS + ap * S::KP;
+      float2 v[N];
+      S::pack_rows(r1, p.K, v);
+      fft_reg<N, +1>(v, nullptr);
+      const int beta = (int)((q0 + pl) / p.nz), z = (int)(q0 + pl - (long)beta * p.nz);
+      float add = 0.f;
+      if (p.bias) add = p.bias[(p.z0 + z) % p.nfeat];
+      if (p.stride == 1) {
+        static_for<0, H>([&](auto ic) {
+          constexpr int c = decltype(ic)::value, pa = fft_reg_pos<N>(2 * c), pb = fft_reg_pos<N>(2 * c + 1);
+          r1[c] = make_float2(v[pa].x + add, v[pb].x + add);
+          r1[H * S::KP + c] = make_float2(v[pa].y + add, v[pb].y + add);
         });
-        if (p.mask) {
-          float k1[C], k2[C];
-          S::ld(p.mask + row1 + g, k1);
-          S::ld(p.mask + row2 + g, k2);
-#pragma unroll
-          for (int i = 0; i < C; ++i) {
-            a[i] = k1[i] > 0.f ? a[i] : 0.f;
-            b[i] = k2[i] > 0.f ? b[i] : 0.f;
-          }
-        }
-        S::st(p.out + row1 + g, a);
-        S::st(p.out + row2 + g, b);
-      });
-    } else {
-      static_for<0, N>([&](auto ic) {
-        constexpr int g = decltype(ic)::value;
-        constexpr int pg = fft_reg_pos<N>(g);
-        p.out[(row1 + g) * p.stride + p.off] = v[pg].x + add;
-        p.out[(row2 + g) * p.stride + p.off] = v[pg].y + add;
-      });
+      } else {
+        const long row1 = (((long)z * N + beta) * N + ap) * (long)N, row2 = row1 + (long)H * N;
+        static_for<0, N>([&](auto ic) {
+          constexpr int g = decltype(ic)::value;
+          constexpr int pg = fft_reg_pos<N>(g);
+          p.out[(row1 + g) * p.stride + p.off] = v[pg].x + add;
+          p.out[(row2 + g) * p.stride + p.off] = v[pg].y + add;
+        });
+      }
     }
+    if (p.stride != 1) return;
+    ctx.sync();
+    S::samples(ctx, p, q0, planes, [&](float2* place, long at) {
+      float2 a = *place;
+      if (p.mask) {
+        const float2 k = *reinterpret_cast<const float2*>(p.mask + at);
+        a = make_float2(k.x > 0.f ? a.x : 0.f, k.y > 0.f ? a.y : 0.f);
+      }
+      *reinterpret_cast<float2*>(p.out + at) = a;
+    });
   }
 };
 

@@ -20,6 +20,14 @@ constexpr int kColMaxDegrees = 16;   // degrees a thread keeps in registers
 S2C_HD constexpr int col_nb(int N) { return (N + 7) / 8 * 8; }
 inline size_t wigner_col_smem(int N, int nl) { return (size_t)col_nb(N) * ((nl + 3) / 4 * 4) * sizeof(float); }
 
+// spectrum rows of successive degrees, in 32-bit arithmetic: row (l, m, n) is (l, 0, 0) + m (2l + 1) + n
+struct ColRows {
+  int l, centre;
+  S2C_D explicit ColRows(int l0) : l(l0), centre((int)so3_row(l0, 0, 0)) {}
+  S2C_D long at(int m, int n) const { return centre + m * (2 * l + 1) + n; }
+  S2C_D void next() { centre += 4 * l * (l + 2) + 5; ++l; }
+};
+
 // X[l][z] = sum_beta W[l][beta] V[beta][z]   (+ Hermitian mirror row); table as [beta][l], zero-padded
 S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
   const int N = p.N;
@@ -49,11 +57,14 @@ S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
     float2 re[2 * T], im[2 * T];                // two degrees each
 #pragma unroll
     for (int i = 0; i < 2 * T; ++i) re[i] = im[i] = make_float2(0.f, 0.f);
+    const float2* vb = v;
     for (int b0 = 0; b0 < N; b0 += 8) {
       float2 c[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (b0 + u < N) c[u] = v[(long)(b0 + u) * p.nbatch];
+      for (int u = 0; u < 8; ++u) {
+        if (b0 + u < N) c[u] = *vb;
+        vb += p.nbatch;
+      }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         if (b0 + u < N) {
@@ -71,12 +82,14 @@ S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
         }
       }
     }
+    ColRows row(lmin);
 #pragma unroll
     for (int li = 0; li < 4 * T; ++li) {
       if (li >= L) continue;
       const float x = li & 1 ? re[li / 2].y : re[li / 2].x, y = li & 1 ? im[li / 2].y : im[li / 2].x;
-      float2* o1 = p.out + so3_row(lmin + li, m, n) * p.out_zstride + z;
-      float2* o2 = p.out + so3_row(lmin + li, -m, -n) * p.out_zstride + z;
+      float2* o1 = p.out + row.at(m, n) * p.out_zstride + z;
+      float2* o2 = p.out + row.at(-m, -n) * p.out_zstride + z;
+      row.next();
       if (p.mode == kSo3Real) {
         *o1 = make_float2(x, y);
         if (!self) *o2 = make_float2(fudge * x, -fudge * y);
@@ -97,7 +110,8 @@ S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
 }
 
 // S[beta][z] = sum_l W[l][beta] Xs[l][z],  Xs = symmetrised spectrum (or S2 product); table as [l][beta]
-S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) {
+template <bool kProduct>
+S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned char* smem) {
   const int N = p.N, NP = col_nb(N);
   const int pair = ctx.bid / p.nzt, zt = ctx.bid - pair * p.nzt;
   int m, n;
@@ -122,19 +136,21 @@ S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) {
   auto degrees = [&](auto tiles) {
     constexpr int T = decltype(tiles)::value;
     float2 x[4 * T];
+    ColRows row(lmin);
 #pragma unroll
     for (int li = 0; li < 4 * T; ++li) {
       x[li] = make_float2(0.f, 0.f);
       if (li >= L) continue;
-      const int l = lmin + li;
       float2 a, b;
-      if (p.xs) {
+      if constexpr (kProduct) {
+        const int l = lmin + li;
         const int i = (int)((p.z0 + z) / p.s2_fout), j = (int)(p.z0 + z - (long)i * p.s2_fout);
         a = wig_s2_product(p, l, m, n, i, j);
         b = wig_s2_product(p, l, -m, -n, i, j);
       } else {
-        a = p.x[so3_row(l, m, n) * p.x_zstride + z];
-        b = p.x[so3_row(l, -m, -n) * p.x_zstride + z];
+        a = p.x[row.at(m, n) * p.x_zstride + z];
+        b = p.x[row.at(-m, -n) * p.x_zstride + z];
+        row.next();
         if (p.mode == kSo3RotI) {  // multiply the spectrum by -i
           a = make_float2(a.y, -a.x);
           b = make_float2(b.y, -b.x);
@@ -142,7 +158,8 @@ S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) {
       }
       x[li] = make_float2(0.5f * (a.x + fudge * b.x), 0.5f * (a.y - fudge * b.y));
     }
-    for (int b0 = 0; b0 < N; b0 += 4) {
+    float2* o = s;
+    for (int b0 = 0; b0 < N; b0 += 4, o += 4L * p.nbatch) {
       float2 r0 = make_float2(0.f, 0.f), r1 = r0, i0 = r0, i1 = r0;   // two betas each
 #pragma unroll
       for (int li = 0; li < 4 * T; ++li) {
@@ -154,7 +171,6 @@ S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) {
         r1 = fma2(hi, xr, r1);
         i1 = fma2(hi, xi, i1);
       }
-      float2* o = s + (long)b0 * p.nbatch;
       o[0] = make_float2(r0.x, i0.x);
       o[p.nbatch] = make_float2(r0.y, i0.y);
       if (b0 + 2 < N) {
@@ -168,5 +184,7 @@ S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) {
   else if (LT == 3) degrees(std::integral_constant<int, 3>{});
   else degrees(std::integral_constant<int, 4>{});
 }
+S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) { inv_wigner_col<false>(ctx, p, smem); }
+S2C_KERNEL_BOUNDS(so3_inv_wigner_col_s2, InvWignerParams, kColZT, 6) { inv_wigner_col<true>(ctx, p, smem); }
 
 }  // namespace s2c
