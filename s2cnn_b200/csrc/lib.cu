@@ -110,8 +110,17 @@ static int plane_pipeline(long nbatch, int N, int K, void* ws, size_t ws_bytes, 
 }
 
 // 32 < N < 64: a plane kernel (so3_mid_kernels.h) and a tiled Wigner kernel per direction through
-// V[n][m][z][beta].  Signals per chunk: whole tiles of the Wigner kernel, as many as keep V in L2
-// (N = 60, K = 30: 0.85 MB per signal, 64 signals), within the workspace.
+// V[n][m][z][beta].  Signals per chunk: whole tiles of the Wigner kernel, within the workspace.
+// A chunk's V may be larger than L2: fewer, longer launches weigh more than re-reading part of it (2560 signals at
+// b = 15, synthesis: 237 us in chunks of 64 MB, 227 of 96, 218 of 128 and 192; 512 signals at b = 30: 816 us in chunks
+// of 64 MB, 780 of 128, 757 of 192).  The chunks of a batch are equal, so that the last one is not a fraction.
+constexpr size_t kChunkBytes = (size_t)192 << 20;
+static long chunk_signals(long nbatch, size_t per_z) {
+  const long most = std::max(1L, (long)(kChunkBytes / per_z) / kWigZT) * kWigZT;
+  const long parts = (nbatch + most - 1) / most;
+  const long even = ((nbatch + parts - 1) / parts + kWigZT - 1) / kWigZT * kWigZT;
+  return std::min(nbatch, even);
+}
 static size_t so3_mid_v_per_z(int N, int K) { return (size_t)K * (2 * K - 1) * N * sizeof(float2); }
 static bool use_mid_kernels(int N) { return mid_supported(N) && g_force_general < 2; }
 static int mid_chunk(long nbatch, int N, int K, const void* ws, size_t ws_bytes, long* chunk) {
@@ -120,8 +129,7 @@ static int mid_chunk(long nbatch, int N, int K, const void* ws, size_t ws_bytes,
   if (fit < 1)
     return fail(S2C_ERR_WORKSPACE, "workspace smaller than one batch element (" + std::to_string(vz) +
                                        " bytes needed)");
-  const long l2 = std::max(1L, (long)(((size_t)64 << 20) / vz) / kWigZT) * kWigZT;
-  *chunk = std::min(nbatch, std::min(fit, l2));
+  *chunk = std::min(fit, chunk_signals(nbatch, vz));
   return S2C_OK;
 }
 
@@ -139,17 +147,21 @@ static bool so3_prefers_cluster(ClKind kind, int N, long nbatch) {
   return kind == kClRelay || groups <= (kind == kClAnalysis ? 55 : 95);
 }
 
-// Large batches at 10 <= 2 b <= 32: plane kernels (so3_small_kernels.h) and the tiled Wigner kernels, through a
-// workspace that holds at least one tile of signals.
+// Large batches at 18 <= 2 b <= 32: plane kernels (so3_small_kernels.h) and one signal per thread in the Wigner step
+// (wigner_columns.h), through a workspace that holds at least one tile of signals.  The lines are where they get
+// faster than the cluster kernels, and they stay faster than the walking kernels up to 5120 signals (b = 16: 570 ->
+// 438 us analysis, 598 -> 486 synthesis; b = 15: 712 -> 384, 783 -> 424; b = 12: 190 -> 185; b = 10: 113 -> 112,
+// 138 -> 124).  A spectrum of few degrees (K <= N / 3) leaves a cluster less to do per block: later lines.  At
+// 2 b <= 16 a whole spectrum fits beside the planes three blocks to an SM and the walking kernels are the faster ones.
 static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, const void* ws, size_t ws_bytes) {
   const int forced = g_cluster.load();
   if (g_force_general || !small_supported(N) || !ws || forced == 1 || forced == 2) return false;
-  if (ws_bytes < so3_mid_v_per_z(N, K) * (size_t)std::min<long>(kWigZT, nbatch) ||
-      nl > kColMaxDegrees)
-    return false;
+  if (ws_bytes < so3_mid_v_per_z(N, K) * (size_t)std::min<long>(kWigZT, nbatch) || nl > kColMaxDegrees) return false;
   if (forced == 3) return true;
-  (void)kind;
-  return (nbatch + kFusedZG - 1) / kFusedZG > 160;
+  const bool full = 3 * K > N, relay = kind == kClRelay;
+  if (N >= 26) return nbatch >= (full ? (relay ? 32 : 48) : 256);
+  if (N == 24) return nbatch >= (full ? 64 : relay ? 512 : 256);
+  return nbatch >= (N == 22 ? 256 : 600);
 }
 
 static int launch_fwd_wigner_col(FwdWignerParams w, stream_t st) {
@@ -838,8 +850,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
     PanelsDev pin, pout;
     S2C_TRY(TableCache::get().panels(b_mid, b_in, b_in, false, false, pin));
     S2C_TRY(TableCache::get().panels(b_mid, b_next, b_next, true, false, pout));
-    const long l2 = std::max(1L, (long)(((size_t)64 << 20) / (v1 + v2)) / kWigZT) * kWigZT;
-    const long chunk = std::min(nz, std::min(l2, (long)(ws_bytes / (v1 + v2))));
+    const long chunk = std::min(chunk_signals(nz, v1 + v2), (long)(ws_bytes / (v1 + v2)));
     for (long z0 = 0; z0 < nz; z0 += chunk) {
       const long zc = std::min(chunk, nz - z0);
       float2* v = (float2*)ws;
@@ -905,8 +916,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
 size_t s2c_so3_relay_workspace(long nbatch, int b_in, int b_mid, int b_next) {
   if (!small_supported(2 * b_mid) || b_in < 1 || b_next < 1) return 16;
   const size_t v = so3_mid_v_per_z(2 * b_mid, b_in) + so3_mid_v_per_z(2 * b_mid, b_next);
-  const long l2 = std::max(1L, (long)(((size_t)64 << 20) / v) / kWigZT) * kWigZT;
-  return v * (size_t)std::min(l2, std::max(1L, nbatch));
+  return v * (size_t)chunk_signals(std::max(1L, nbatch), v);
 }
 
 int s2c_s2_conv_relu_so3_rfft_ws(const float* xs, const float* ys, float* out, int nbatch, int f_in,

@@ -79,9 +79,9 @@ S2C_S2(80) S2C_S2(96) S2C_S2(102) S2C_S2(114) S2C_S2(124)
 S2C_S2(10) S2C_S2(12) S2C_S2(26) S2C_S2(28) S2C_S2(42) S2C_S2(44) S2C_S2(58) S2C_S2(60) S2C_S2(76)
 S2C_S2(78) S2C_S2(98) S2C_S2(100) S2C_S2(116) S2C_S2(120)
 #elif S2C_PART == 16
-S2C_SMALL(32) S2C_SMALL(30) S2C_SMALL(24) S2C_SMALL(16) S2C_SMALL(14) S2C_SMALL(10)
+S2C_SMALL(32) S2C_SMALL(30) S2C_SMALL(24) S2C_SMALL(18)
 #elif S2C_PART == 17
-S2C_SMALL(28) S2C_SMALL(26) S2C_SMALL(22) S2C_SMALL(20) S2C_SMALL(18) S2C_SMALL(12)
+S2C_SMALL(28) S2C_SMALL(26) S2C_SMALL(22) S2C_SMALL(20)
 #endif
 
 }  // namespace s2c

@@ -1,4 +1,4 @@
-// Plane kernels of the SO(3) transform for small bandwidths (10 <= N = 2b <= 32) and LARGE batches: both row
+// Plane kernels of the SO(3) transform for small bandwidths (18 <= N = 2b <= 32) and LARGE batches: both row
 // transforms of P neighbouring (z, beta) planes in one block, every 1-D FFT in the registers of one thread
 // (fft_reg.h), between the signal and the V[n][m][beta][z] array of wigner_columns.h.
 //
@@ -7,7 +7,8 @@
 // groups pass four block barriers each (0.34 instructions per clock and scheduler, 4 of 12 stall cycles at
 // barriers).  For a large batch the Wigner contraction is better off on its own - a block shares each table row
 // among 128 signals - and what is left needs one barrier and 35 KB: several blocks per SM overlap their loads,
-// transforms and stores.  The array between the two stays in L2 (chunks of at most 64 MB).
+// transforms and stores.  2560 signals at b = 15: analysis 398 -> 198 us, synthesis 437 -> 218 (floor, the signal
+// once: 44 us); half of it is this file's kernels (latency: 20 warps per SM, L1 at 65 %), half the Wigner step.
 //
 //   so3_fwd_small    two real rows per thread (optional ReLU on load) -> n -> columns alpha -> m -> V
 //   so3_inv_small    V -> columns m -> alpha -> two rows per thread n -> gamma (+ bias, mask) -> store
@@ -25,7 +26,7 @@
 
 namespace s2c {
 
-S2C_HD constexpr bool small_supported(int N) { return N >= 10 && N <= 32 && N % 2 == 0; }
+S2C_HD constexpr bool small_supported(int N) { return N >= 18 && N <= 32 && N % 2 == 0; }
 S2C_HD constexpr int small_planes(int N) { return 256 / N / 4 * 4 < 8 ? 8 : 256 / N / 4 * 4; }
 S2C_HD constexpr int small_threads(int N) { return (small_planes(N) * (N / 2) + 31) / 32 * 32; }
 S2C_HD constexpr int small_kp(int N) { return N / 2 | 1; }                 // odd row stride (complex)
@@ -277,10 +278,12 @@ struct so3_relay_small_impl {
   }
 };
 
+// Six blocks of 128 threads per SM (85 registers); N = 32 needs a few more and is faster with five (2560 signals:
+// 259 against 294 us) - the spills of 80 registers cost more than the sixth block gives.
 #ifndef S2C_EMUL
 #define S2C_SMALL_KERNEL(name)                                                                   \
   template <int N>                                                                               \
-  __global__ void __launch_bounds__(small_threads(N)) name(const SmallParams p) {                \
+  __global__ void __launch_bounds__(small_threads(N), N == 32 ? 5 : 768 / small_threads(N)) name(const SmallParams p) {                \
     extern __shared__ float4 s2c_dyn_smem[];                                                     \
     Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};                 \
     name##_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));                 \
@@ -294,10 +297,6 @@ S2C_SMALL_KERNEL(so3_relay_small)
   S2C_LAUNCH_N(name, N, ((params).nplanes + small_planes(N) - 1) / small_planes(N), small_threads(N), small_smem_bytes(N), stream, params)
 #define S2C_DISPATCH_SMALL(N, CALL)                                                              \
   switch (N) {                                                                                   \
-    case 10: { constexpr int kN = 10; CALL; } break;                                             \
-    case 12: { constexpr int kN = 12; CALL; } break;                                             \
-    case 14: { constexpr int kN = 14; CALL; } break;                                             \
-    case 16: { constexpr int kN = 16; CALL; } break;                                             \
     case 18: { constexpr int kN = 18; CALL; } break;                                             \
     case 20: { constexpr int kN = 20; CALL; } break;                                             \
     S2C_CASES_32(CALL)                                                                           \

@@ -5,7 +5,8 @@
 // goes through shared memory.  At b = 16 a frequency pair has 5 degrees on average: the tiles of 4 x 2 outputs
 // there share too little (512 signals: 44 us analysis, of which the copies into shared memory and the padded
 // tiles are most), while a thread that owns all degrees of one batch element reads each sample of V once and
-// each table entry as a broadcast of 16 bytes.  Bound by the L2 traffic of V.
+// each table entry as a broadcast of 16 bytes.  512 signals at b = 16: 23 us, bound by the
+// latency of V's loads (24 warps per SM), not by their rate.
 #pragma once
 
 #include "backend.h"
@@ -39,6 +40,19 @@ S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
   const int L = p.nl - lmin;
   if (L <= 0) return;
   const int LT = (L + 3) / 4;
+  // eight samples of V at a time, in flight while the table is staged or the eight before them are used
+  const int nm = 2 * p.K - 1, mi = m + p.K - 1;
+  const int z = zt * p.ZT + ctx.tid;
+  const float2* vb = p.v + ((long)n * nm + mi) * N * p.nbatch + z;
+  float2 next[8];
+  auto fetch = [&](int b0) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (b0 + u < N && z < p.nbatch) next[u] = *vb;
+      vb += p.nbatch;
+    }
+  };
+  fetch(0);
   float* Ws = reinterpret_cast<float*>(smem);   // [beta][4 LT]
   const float* panel = p.pan.data + p.pan.off[pair];
   for (int i = ctx.tid; i < 4 * LT * N; i += ctx.nthr) {
@@ -46,10 +60,7 @@ S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
     Ws[bt * 4 * LT + l] = l < L ? panel[i] : 0.f;
   }
   ctx.sync();
-  const int z = zt * p.ZT + ctx.tid;
   if (z >= p.nbatch) return;
-  const int nm = 2 * p.K - 1, mi = m + p.K - 1;
-  const float2* v = p.v + ((long)n * nm + mi) * N * p.nbatch + z;
   const float fudge = ((m - n) & 1) ? -1.f : 1.f;
   const bool self = (m == 0 && n == 0);
   auto degrees = [&](auto tiles) {
@@ -57,14 +68,11 @@ S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
     float2 re[2 * T], im[2 * T];                // two degrees each
 #pragma unroll
     for (int i = 0; i < 2 * T; ++i) re[i] = im[i] = make_float2(0.f, 0.f);
-    const float2* vb = v;
     for (int b0 = 0; b0 < N; b0 += 8) {
       float2 c[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (b0 + u < N) c[u] = *vb;
-        vb += p.nbatch;
-      }
+      for (int u = 0; u < 8; ++u) c[u] = next[u];
+      fetch(b0 + 8);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         if (b0 + u < N) {
@@ -123,13 +131,7 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
   const int LT = (L + 3) / 4;
   float* Ws = reinterpret_cast<float*>(smem);   // [4 LT][NP]
   const float* panel = p.pan.data + p.pan.off[pair];
-  for (int i = ctx.tid; i < 4 * LT * NP; i += ctx.nthr) {
-    const int l = i / NP, bt = i - l * NP;
-    Ws[i] = l < L && bt < N ? panel[l * N + bt] : 0.f;
-  }
-  ctx.sync();
   const int z = zt * p.ZT + ctx.tid;
-  if (z >= p.nbatch) return;
   const float fudge = ((m - n) & 1) ? -1.f : 1.f;
   const int nm = 2 * p.K - 1, mi = m + p.K - 1;
   float2* s = p.s + ((long)n * nm + mi) * N * p.nbatch + z;
@@ -140,7 +142,7 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
 #pragma unroll
     for (int li = 0; li < 4 * T; ++li) {
       x[li] = make_float2(0.f, 0.f);
-      if (li >= L) continue;
+      if (li >= L || z >= p.nbatch) continue;
       float2 a, b;
       if constexpr (kProduct) {
         const int l = lmin + li;
@@ -158,6 +160,12 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
       }
       x[li] = make_float2(0.5f * (a.x + fudge * b.x), 0.5f * (a.y - fudge * b.y));
     }
+    for (int i = ctx.tid; i < 4 * T * NP; i += ctx.nthr) {
+      const int l = i / NP, bt = i - l * NP;
+      Ws[i] = l < L && bt < N ? panel[l * N + bt] : 0.f;
+    }
+    ctx.sync();
+    if (z >= p.nbatch) return;
     float2* o = s;
     for (int b0 = 0; b0 < N; b0 += 4, o += 4L * p.nbatch) {
       float2 r0 = make_float2(0.f, 0.f), r1 = r0, i0 = r0, i1 = r0;   // two betas each
