@@ -153,12 +153,18 @@ static bool so3_prefers_cluster(ClKind kind, int N, long nbatch) {
 // 438 us analysis, 598 -> 486 synthesis; b = 15: 712 -> 384, 783 -> 424; b = 12: 190 -> 185; b = 10: 113 -> 112,
 // 138 -> 124).  A spectrum of few degrees (K <= N / 3) leaves a cluster less to do per block: later lines.  At
 // 2 b <= 16 a whole spectrum fits beside the planes three blocks to an SM and the walking kernels are the faster ones.
-static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, const void* ws, size_t ws_bytes) {
+// With an S2 product as input the Wigner step loads the product's factors for each degree of each signal, up to twice
+// what the single-kernel transforms load: worth it for the chained layers at 22 <= 2 b <= 30 (b = 15, six features,
+// 1280 signals: 448 -> 300 us; b = 10, 5120 signals: 155 -> 182, kept off) and for the lengths whose walking
+// blocks take betas in twos (263 -> 200 us; b = 16: 195 -> 226, kept off).
+static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, const void* ws, size_t ws_bytes,
+                               bool product = false) {
   const int forced = g_cluster.load();
   if (g_force_general || !small_supported(N) || !ws || forced == 1 || forced == 2) return false;
   if (ws_bytes < so3_mid_v_per_z(N, K) * (size_t)std::min<long>(kWigZT, nbatch) || nl > kColMaxDegrees) return false;
   if (forced == 3) return true;
   const bool full = 3 * K > N, relay = kind == kClRelay;
+  if (product) return N < 32 && N >= 22 && (relay ? nbatch >= 256 : N % 4 == 2 && nbatch >= 400);
   if (N >= 26) return nbatch >= (full ? (relay ? 32 : 48) : 256);
   if (N == 24) return nbatch >= (full ? 64 : relay ? 512 : 256);
   return nbatch >= (N == 22 ? 256 : 600);
@@ -362,7 +368,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
   PanelsDev pan;
   S2C_TRY(TableCache::get().fft(N, fft));
   S2C_TRY(TableCache::get().panels(b_out, K, K, weighted, false, pan));
-  const bool small = !integral && so3_prefers_planes(kClSynthesis, N, K, K, nbatch, ws, ws_bytes) &&
+  const bool small = !integral && so3_prefers_planes(kClSynthesis, N, K, K, nbatch, ws, ws_bytes, prod != nullptr) &&
                      (!mask || (out_stride == 1 && out_off == 0));
   if (!small && !g_force_general && N <= kFusedMaxN && so3_prefers_cluster(kClSynthesis, N, nbatch)) {
     ClInvParams f;
@@ -845,7 +851,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
     return fail(S2C_ERR_UNSUPPORTED,
                 std::string(who) + ": needs 2 b <= 32, b_in <= b and b_next <= b");
   const size_t v1 = so3_mid_v_per_z(N, b_in), v2 = so3_mid_v_per_z(N, b_next);
-  if (so3_prefers_planes(kClRelay, N, b_in, b_next, nz, ws, ws_bytes) &&
+  if (so3_prefers_planes(kClRelay, N, b_in, b_next, nz, ws, ws_bytes, xs != nullptr) &&
       ws_bytes >= (v1 + v2) * (size_t)std::min<long>(kWigZT, nz)) {
     PanelsDev pin, pout;
     S2C_TRY(TableCache::get().panels(b_mid, b_in, b_in, false, false, pin));

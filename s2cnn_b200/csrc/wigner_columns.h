@@ -11,7 +11,6 @@
 
 #include "backend.h"
 #include "so3_kernels.h"
-#include "wigner_tiled.h"
 
 namespace s2c {
 
@@ -138,27 +137,61 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
   auto degrees = [&](auto tiles) {
     constexpr int T = decltype(tiles)::value;
     float2 x[4 * T];
-    ColRows row(lmin);
+    if constexpr (kProduct) {
+      // the loads of all degrees are in flight together (one product after the other was 100 us of 290, b = 10, 5120
+      // signals); multiply-adds in the order of the single-kernel transforms
+      float2 a[4 * T], b[4 * T];
 #pragma unroll
-    for (int li = 0; li < 4 * T; ++li) {
-      x[li] = make_float2(0.f, 0.f);
-      if (li >= L || z >= p.nbatch) continue;
-      float2 a, b;
-      if constexpr (kProduct) {
-        const int l = lmin + li;
+      for (int li = 0; li < 4 * T; ++li) a[li] = b[li] = make_float2(0.f, 0.f);
+      if (z < p.nbatch) {
         const int i = (int)((p.z0 + z) / p.s2_fout), j = (int)(p.z0 + z - (long)i * p.s2_fout);
-        a = wig_s2_product(p, l, m, n, i, j);
-        b = wig_s2_product(p, l, -m, -n, i, j);
-      } else {
-        a = p.x[row.at(m, n) * p.x_zstride + z];
-        b = p.x[row.at(-m, -n) * p.x_zstride + z];
+        const long xs = (long)p.s2_nb * p.s2_fin, ys = (long)p.s2_fin * p.s2_fout;
+        const float2* x0 = p.xs + (long)(lmin * lmin + lmin) * xs + (long)i * p.s2_fin;   // row (lmin, 0)
+        const float2* y0 = p.ys + (long)(lmin * lmin + lmin) * ys + j;
+        for (int k = 0; k < p.s2_fin; ++k) {
+          const float2 *xr = x0 + k, *yr = y0 + (long)k * p.s2_fout;
+          float2 u[4 * T], v[4 * T], u2[4 * T], v2[4 * T];
+#pragma unroll
+          for (int li = 0; li < 4 * T; ++li) {
+            if (li < L) {
+              u[li] = xr[m * xs]; u2[li] = xr[-m * xs];
+              v[li] = yr[n * ys]; v2[li] = yr[-n * ys];
+            }
+            xr += 2L * (lmin + li + 1) * xs;
+            yr += 2L * (lmin + li + 1) * ys;
+          }
+          auto mul = [](float2 q, float2 r, float2& acc) {
+            acc.x = fmaf(q.x, r.x, acc.x);
+            acc.x = fmaf(q.y, r.y, acc.x);
+            acc.y = fmaf(q.y, r.x, acc.y);
+            acc.y = fmaf(-q.x, r.y, acc.y);
+          };
+#pragma unroll
+          for (int li = 0; li < 4 * T; ++li) {
+            if (li >= L) continue;
+            mul(u[li], v[li], a[li]);
+            mul(u2[li], v2[li], b[li]);
+          }
+        }
+      }
+#pragma unroll
+      for (int li = 0; li < 4 * T; ++li)
+        x[li] = make_float2(0.5f * (a[li].x + fudge * b[li].x), 0.5f * (a[li].y - fudge * b[li].y));
+    } else {
+      ColRows row(lmin);
+#pragma unroll
+      for (int li = 0; li < 4 * T; ++li) {
+        x[li] = make_float2(0.f, 0.f);
+        if (li >= L || z >= p.nbatch) continue;
+        float2 a = p.x[row.at(m, n) * p.x_zstride + z];
+        float2 b = p.x[row.at(-m, -n) * p.x_zstride + z];
         row.next();
         if (p.mode == kSo3RotI) {  // multiply the spectrum by -i
           a = make_float2(a.y, -a.x);
           b = make_float2(b.y, -b.x);
         }
+        x[li] = make_float2(0.5f * (a.x + fudge * b.x), 0.5f * (a.y - fudge * b.y));
       }
-      x[li] = make_float2(0.5f * (a.x + fudge * b.x), 0.5f * (a.y - fudge * b.y));
     }
     for (int i = ctx.tid; i < 4 * T * NP; i += ctx.nthr) {
       const int l = i / NP, bt = i - l * NP;
@@ -193,6 +226,6 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
   else degrees(std::integral_constant<int, 4>{});
 }
 S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) { inv_wigner_col<false>(ctx, p, smem); }
-S2C_KERNEL_BOUNDS(so3_inv_wigner_col_s2, InvWignerParams, kColZT, 6) { inv_wigner_col<true>(ctx, p, smem); }
+S2C_KERNEL_BOUNDS(so3_inv_wigner_col_s2, InvWignerParams, kColZT, 4) { inv_wigner_col<true>(ctx, p, smem); }
 
 }  // namespace s2c

@@ -219,8 +219,7 @@ inline size_t inv_wigner_t_smem(int N, int K, int zt = kWigZT) {
   return (size_t)K * wig_np(N) * sizeof(float) + (size_t)K * (zt + 2) * sizeof(float2);
 }
 
-// one entry of s2_mm(xs, ys), multiply-adds in the order of the single-kernel transforms (2b <= 32) or of
-// cgemm_grouped
+// one entry of s2_mm(xs, ys), multiply-adds in the order of cgemm_grouped
 S2C_D float2 wig_s2_product(const InvWignerParams& p, int l, int m, int n, int i, int j) {
   const float2* xr = p.xs + ((long)(l * l + l + m) * p.s2_nb + i) * p.s2_fin;
   const float2* yr = p.ys + (long)(l * l + l + n) * p.s2_fin * p.s2_fout + j;
@@ -229,13 +228,8 @@ S2C_D float2 wig_s2_product(const InvWignerParams& p, int l, int m, int n, int i
     const float2 a = xr[k], b = yr[(long)k * p.s2_fout];
     re = fmaf(a.x, b.x, re);
     re = fmaf(a.y, b.y, re);
-    if (p.N <= kFusedMaxN) {
-      im = fmaf(a.y, b.x, im);
-      im = fmaf(-a.x, b.y, im);
-    } else {
-      im = fmaf(a.x, -b.y, im);
-      im = fmaf(a.y, b.x, im);
-    }
+    im = fmaf(a.x, -b.y, im);
+    im = fmaf(a.y, b.x, im);
   }
   return make_float2(re, im);
 }
