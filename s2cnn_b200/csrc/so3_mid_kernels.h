@@ -55,6 +55,15 @@ struct MidParams {
 // it -> it / K, exact for the few thousand items of a block
 S2C_D int mid_div(int it, float inv_k) { return (int)(((float)it + 0.5f) * inv_k); }
 
+S2C_D void mid_ld(const float* p, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+S2C_D void mid_ld(const float* p, float (&v)[2]) {
+  const float2 a = *reinterpret_cast<const float2*>(p);
+  v[0] = a.x; v[1] = a.y;
+}
+
 template <int N>
 struct so3_fwd_mid_impl {
   static S2C_D void run(const Ctx& ctx, const MidParams& p, unsigned char* smem) {
@@ -231,37 +240,57 @@ struct so3_inv_mid_impl {
     if (p.bias) add = p.bias[(p.z0 + z) % p.nfeat];
     const long e00 = ((z * N + beta0) * N) * (long)N;
     constexpr int W = N % 4 == 0 ? 4 : 2, PR = N / W;        // samples per store, stores per row
-    for (int it = ctx.tid; it < bc * H * PR; it += ctx.nthr) {
-      const int c = it % PR, row = it / PR, pl = row / H, t = row - pl * H;
-      const float4* src = reinterpret_cast<const float4*>(B + pl * PSB + t * LD + c * W);
-      const long e0 = e00 + (long)row * 2 * N + c * W;
-      float r0[W], r1[W];
-#pragma unroll
-      for (int i = 0; i < W / 2; ++i) {
-        const float4 u = src[i];
-        r0[2 * i] = u.x + add; r1[2 * i] = u.y + add;
-        r0[2 * i + 1] = u.z + add; r1[2 * i + 1] = u.w + add;
-      }
+    // the mask's loads of four steps are in flight together, ahead of the stores the compiler keeps them
+    // behind (256 signals at b = 30: 409 us, 390 without a mask)
+    constexpr int U = 4;
+    const int total = bc * H * PR;
+    for (int base = ctx.tid; base < total; base += U * ctx.nthr) {
+      float k0[U][W], k1[U][W];
       if (p.mask) {
 #pragma unroll
-        for (int i = 0; i < W; ++i) {
-          if (!(p.mask[e0 + i] > 0.f)) r0[i] = 0.f;
-          if (!(p.mask[e0 + N + i] > 0.f)) r1[i] = 0.f;
+        for (int u = 0; u < U; ++u) {
+          const int it = base + u * ctx.nthr;
+          if (it >= total) break;
+          const float* k = p.mask + e00 + (long)(it / PR) * 2 * N + it % PR * W;
+          mid_ld(k, k0[u]);
+          mid_ld(k + N, k1[u]);
         }
       }
-      if (p.stride == 1) {
-        if constexpr (W == 4) {
-          *reinterpret_cast<float4*>(p.out + e0) = make_float4(r0[0], r0[1], r0[2], r0[3]);
-          *reinterpret_cast<float4*>(p.out + e0 + N) = make_float4(r1[0], r1[1], r1[2], r1[3]);
-        } else {
-          *reinterpret_cast<float2*>(p.out + e0) = make_float2(r0[0], r0[1]);
-          *reinterpret_cast<float2*>(p.out + e0 + N) = make_float2(r1[0], r1[1]);
-        }
-      } else {
 #pragma unroll
-        for (int i = 0; i < W; ++i) {
-          p.out[(e0 + i) * p.stride + p.off] = r0[i];
-          p.out[(e0 + N + i) * p.stride + p.off] = r1[i];
+      for (int u = 0; u < U; ++u) {
+        const int it = base + u * ctx.nthr;
+        if (it >= total) break;
+        const int c = it % PR, row = it / PR, pl = row / H, t = row - pl * H;
+        const float4* src = reinterpret_cast<const float4*>(B + pl * PSB + t * LD + c * W);
+        const long e0 = e00 + (long)row * 2 * N + c * W;
+        float r0[W], r1[W];
+#pragma unroll
+        for (int i = 0; i < W / 2; ++i) {
+          const float4 v = src[i];
+          r0[2 * i] = v.x + add; r1[2 * i] = v.y + add;
+          r0[2 * i + 1] = v.z + add; r1[2 * i + 1] = v.w + add;
+        }
+        if (p.mask) {
+#pragma unroll
+          for (int i = 0; i < W; ++i) {
+            if (!(k0[u][i] > 0.f)) r0[i] = 0.f;
+            if (!(k1[u][i] > 0.f)) r1[i] = 0.f;
+          }
+        }
+        if (p.stride == 1) {
+          if constexpr (W == 4) {
+            *reinterpret_cast<float4*>(p.out + e0) = make_float4(r0[0], r0[1], r0[2], r0[3]);
+            *reinterpret_cast<float4*>(p.out + e0 + N) = make_float4(r1[0], r1[1], r1[2], r1[3]);
+          } else {
+            *reinterpret_cast<float2*>(p.out + e0) = make_float2(r0[0], r0[1]);
+            *reinterpret_cast<float2*>(p.out + e0 + N) = make_float2(r1[0], r1[1]);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < W; ++i) {
+            p.out[(e0 + i) * p.stride + p.off] = r0[i];
+            p.out[(e0 + N + i) * p.stride + p.off] = r1[i];
+          }
         }
       }
     }

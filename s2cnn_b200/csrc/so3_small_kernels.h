@@ -143,9 +143,9 @@ struct Small {
 
   // Planes of a real signal go through the rows' own places in shared memory (row stride KP complex >= N floats), so
   // that the lanes of a warp touch neighbouring samples in memory: a row per thread would take 32 cache lines per
-  // access (b = 15: 81 % of the L1 rate).  f(place in shared memory, offset in the signal) for every two samples; a
+  // access (b = 15: 81 % of the L1 rate).  f(alpha, place in shared memory, offset in the signal) for every two samples; a
   // thread keeps its plane and gamma and steps over alpha, so that all addresses are constants apart.
-  template <class F>
+  template <int A0 = 0, int A1 = N, class F>
   static S2C_D void samples(const Ctx& ctx, const SmallParams& p, long q0, float2* planes, F&& f) {
     const int c = ctx.tid % H, pl = ctx.tid / H;
     if (pl >= P || q0 + pl >= p.nplanes) return;
@@ -153,7 +153,7 @@ struct Small {
     const long base = ((long)z * N + beta) * (N * N) + 2 * c;
     float2* place = planes + pl * PS + c;
 #pragma unroll
-    for (int a = 0; a < N; ++a) f(place + a * KP, base + a * N);
+    for (int a = A0; a < A1; ++a) f(a, place + a * KP, base + a * N);
   }
 };
 
@@ -165,7 +165,7 @@ struct so3_fwd_small_impl {
     float2* planes = reinterpret_cast<float2*>(smem);
     const long q0 = (long)ctx.bid * S::P;
     if (p.stride == 1) {
-      S::samples(ctx, p, q0, planes, [&](float2* place, long at) { small_copy(place, p.x + at); });
+      S::samples(ctx, p, q0, planes, [&](int, float2* place, long at) { small_copy(place, p.x + at); });
       small_copy_wait();
       ctx.sync();
     }
@@ -235,13 +235,23 @@ struct so3_inv_small_impl {
     }
     if (p.stride != 1) return;
     ctx.sync();
-    S::samples(ctx, p, q0, planes, [&](float2* place, long at) {
-      float2 a = *place;
-      if (p.mask) {
-        const float2 k = *reinterpret_cast<const float2*>(p.mask + at);
-        a = make_float2(k.x > 0.f ? a.x : 0.f, k.y > 0.f ? a.y : 0.f);
-      }
-      *reinterpret_cast<float2*>(p.out + at) = a;
+    if (!p.mask) {
+      S::samples(ctx, p, q0, planes, [&](int, float2* place, long at) { *reinterpret_cast<float2*>(p.out + at) = *place; });
+      return;
+    }
+    // the mask's loads of a quarter of the rows are in flight together: the compiler keeps a load behind the stores
+    // before it (one by one: 434 us for 3200 signals at b = 16, 839 MB; so: 190)
+    constexpr int G = (N + 3) / 4;
+    static_for<0, 4>([&](auto gc) {
+      constexpr int A0 = decltype(gc)::value * G, A1 = A0 + G < N ? A0 + G : N;
+      float2 keep[G];
+      S::template samples<A0, A1>(ctx, p, q0, planes, [&](int a, float2*, long at) {
+        keep[a - A0] = *reinterpret_cast<const float2*>(p.mask + at);
+      });
+      S::template samples<A0, A1>(ctx, p, q0, planes, [&](int a, float2* place, long at) {
+        const float2 k = keep[a - A0], v = *place;
+        *reinterpret_cast<float2*>(p.out + at) = make_float2(k.x > 0.f ? v.x : 0.f, k.y > 0.f ? v.y : 0.f);
+      });
     });
   }
 };
