@@ -1,7 +1,7 @@
 """The cluster kernels and the plane kernels of 2b <= 32 against the kernels whose blocks walk beta: same sums in the same order, so
 equal to the last bit on the GPU.  One block per cluster, two, four and eight, betas that do not divide evenly
 (2b = 12, 18, 22, 26, 30: a short last block; 28: an empty one), batches that end inside a group of four, more degrees
-than the grid holds, a fused product with a feature count that is no multiple of four, masks, sums, the integral."""
+than the grid holds, a fused product with a feature count that is no multiple of four, masks, sums, the integral, a tile of 128 signals and a rest."""
 import pytest
 import torch
 
@@ -14,7 +14,7 @@ n3 = O.so3_nspec
 
 @pytest.mark.parametrize("backend", backends.BACKENDS)
 @pytest.mark.parametrize("b,b_spec,nb", [(1, 1, 1), (3, 3, 5), (5, 2, 4), (6, 8, 3), (9, 9, 2), (10, 6, 9), (11, 11, 4),
-                                         (7, 7, 70), (12, 5, 3), (13, 4, 1), (14, 14, 8), (15, 9, 6), (16, 16, 4)])
+                                         (9, 4, 131), (12, 5, 3), (13, 4, 1), (14, 14, 8), (15, 9, 6), (16, 16, 4)])
 def test_cluster_kernels_match_walking_kernels(backend, b, b_spec, nb):
     ops, dev = backends.get(backend)
     gen = torch.Generator().manual_seed(31 * b + b_spec)
