@@ -153,10 +153,10 @@ static bool so3_prefers_cluster(ClKind kind, int N, long nbatch) {
 // 438 us analysis, 598 -> 486 synthesis; b = 15: 712 -> 384, 783 -> 424; b = 12: 190 -> 185; b = 10: 113 -> 112,
 // 138 -> 124).  A spectrum of few degrees (K <= N / 3) leaves a cluster less to do per block: later lines.  At
 // 2 b <= 16 a whole spectrum fits beside the planes three blocks to an SM and the walking kernels are the faster ones.
-// With an S2 product as input the Wigner step loads the product's factors for each degree of each signal, up to twice
-// what the single-kernel transforms load: worth it for the chained layers at 22 <= 2 b <= 30 (b = 15, six features,
-// 1280 signals: 448 -> 300 us; b = 10, 5120 signals: 155 -> 182, kept off) and for the lengths whose walking
-// blocks take betas in twos (263 -> 200 us; b = 16: 195 -> 226, kept off).
+// With an S2 product as input (six features; one in brackets) the chained layers gain at every length (b = 15, 1280 signals
+// 446 -> 214 us, b = 16 270 -> 198, b = 10, 5120 signals 215 -> 180 [154 -> 139]), the synthesis up to 1500 signals where
+// walking blocks take four betas at a time (b = 16: 193 -> 164 us, at 3200 signals 382 -> 428 [338 -> 302]; b = 12:
+// 77 -> 74, 136 -> 173) and everywhere else (b = 15, 3200 signals: 542 -> 361, b = 10, 5120: 161 -> 157 [134 -> 118]).
 static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, const void* ws, size_t ws_bytes,
                                bool product = false) {
   const int forced = g_cluster.load();
@@ -164,7 +164,7 @@ static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, c
   if (ws_bytes < so3_mid_v_per_z(N, K) * (size_t)std::min<long>(kWigZT, nbatch) || nl > kColMaxDegrees) return false;
   if (forced == 3) return true;
   const bool full = 3 * K > N, relay = kind == kClRelay;
-  if (product) return N < 32 && N >= 22 && (relay ? nbatch >= 256 : N % 4 == 2 && nbatch >= 400);
+  if (product) return nbatch >= (N >= 22 ? 256 : 600) && (relay || N < 24 || N % 4 != 0 || nbatch <= 1500);
   if (N >= 26) return nbatch >= (full ? (relay ? 32 : 48) : 256);
   if (N == 24) return nbatch >= (full ? 64 : relay ? 512 : 256);
   return nbatch >= (N == 22 ? 256 : 600);

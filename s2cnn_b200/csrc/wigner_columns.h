@@ -138,45 +138,53 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
     constexpr int T = decltype(tiles)::value;
     float2 x[4 * T];
     if constexpr (kProduct) {
-      // the loads of all degrees are in flight together (one product after the other was 100 us of 290, b = 10, 5120
-      // signals); multiply-adds in the order of the single-kernel transforms
-      float2 a[4 * T], b[4 * T];
+      // the loads of four degrees are in flight together (one product after the other: 101 us at b = 10, 5120
+      // signals; all degrees at once do not fit the registers); multiply-adds in the order of the single-kernel transforms
+      const unsigned zz = (unsigned)(p.z0 + z), i = zz / (unsigned)p.s2_fout, j = zz - i * (unsigned)p.s2_fout;
+      const long xs = (long)p.s2_nb * p.s2_fin, ys = (long)p.s2_fin * p.s2_fout;
+      const float2* x0 = p.xs + (long)(lmin * lmin + lmin) * xs + (long)i * p.s2_fin;   // row (l, 0), l = lmin
+      const float2* y0 = p.ys + (long)(lmin * lmin + lmin) * ys + j;
+      int l = lmin;
+      static_for<0, T>([&](auto tc) {
+        constexpr int t = decltype(tc)::value;
+        float2 a[4], b[4];
 #pragma unroll
-      for (int li = 0; li < 4 * T; ++li) a[li] = b[li] = make_float2(0.f, 0.f);
-      if (z < p.nbatch) {
-        const int i = (int)((p.z0 + z) / p.s2_fout), j = (int)(p.z0 + z - (long)i * p.s2_fout);
-        const long xs = (long)p.s2_nb * p.s2_fin, ys = (long)p.s2_fin * p.s2_fout;
-        const float2* x0 = p.xs + (long)(lmin * lmin + lmin) * xs + (long)i * p.s2_fin;   // row (lmin, 0)
-        const float2* y0 = p.ys + (long)(lmin * lmin + lmin) * ys + j;
-        for (int k = 0; k < p.s2_fin; ++k) {
-          const float2 *xr = x0 + k, *yr = y0 + (long)k * p.s2_fout;
-          float2 u[4 * T], v[4 * T], u2[4 * T], v2[4 * T];
+        for (int q = 0; q < 4; ++q) a[q] = b[q] = make_float2(0.f, 0.f);
+        if (z < p.nbatch) {
+          for (int k = 0; k < p.s2_fin; ++k) {
+            const float2 *xr = x0 + k, *yr = y0 + (long)k * p.s2_fout;
+            float2 u[4], v[4], u2[4], v2[4];
 #pragma unroll
-          for (int li = 0; li < 4 * T; ++li) {
-            if (li < L) {
-              u[li] = xr[m * xs]; u2[li] = xr[-m * xs];
-              v[li] = yr[n * ys]; v2[li] = yr[-n * ys];
+            for (int q = 0; q < 4; ++q) {
+              if (4 * t + q < L) {
+                u[q] = xr[m * xs]; u2[q] = xr[-m * xs];
+                v[q] = yr[n * ys]; v2[q] = yr[-n * ys];
+              }
+              xr += 2L * (l + q + 1) * xs;
+              yr += 2L * (l + q + 1) * ys;
             }
-            xr += 2L * (lmin + li + 1) * xs;
-            yr += 2L * (lmin + li + 1) * ys;
-          }
-          auto mul = [](float2 q, float2 r, float2& acc) {
-            acc.x = fmaf(q.x, r.x, acc.x);
-            acc.x = fmaf(q.y, r.y, acc.x);
-            acc.y = fmaf(q.y, r.x, acc.y);
-            acc.y = fmaf(-q.x, r.y, acc.y);
-          };
+            auto mul = [](float2 c, float2 d, float2& acc) {
+              acc.x = fmaf(c.x, d.x, acc.x);
+              acc.x = fmaf(c.y, d.y, acc.x);
+              acc.y = fmaf(c.y, d.x, acc.y);
+              acc.y = fmaf(-c.x, d.y, acc.y);
+            };
 #pragma unroll
-          for (int li = 0; li < 4 * T; ++li) {
-            if (li >= L) continue;
-            mul(u[li], v[li], a[li]);
-            mul(u2[li], v2[li], b[li]);
+            for (int q = 0; q < 4; ++q) {
+              if (4 * t + q >= L) continue;
+              mul(u[q], v[q], a[q]);
+              mul(u2[q], v2[q], b[q]);
+            }
           }
         }
-      }
 #pragma unroll
-      for (int li = 0; li < 4 * T; ++li)
-        x[li] = make_float2(0.5f * (a[li].x + fudge * b[li].x), 0.5f * (a[li].y - fudge * b[li].y));
+        for (int q = 0; q < 4; ++q)
+          x[4 * t + q] = make_float2(0.5f * (a[q].x + fudge * b[q].x), 0.5f * (a[q].y - fudge * b[q].y));
+        // rows (l, 0) -> (l + 4, 0): l (l + 1) grows by 8 l + 20
+        x0 += (8L * l + 20) * xs;
+        y0 += (8L * l + 20) * ys;
+        l += 4;
+      });
     } else {
       ColRows row(lmin);
 #pragma unroll
@@ -226,6 +234,6 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
   else degrees(std::integral_constant<int, 4>{});
 }
 S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) { inv_wigner_col<false>(ctx, p, smem); }
-S2C_KERNEL_BOUNDS(so3_inv_wigner_col_s2, InvWignerParams, kColZT, 4) { inv_wigner_col<true>(ctx, p, smem); }
+S2C_KERNEL_BOUNDS(so3_inv_wigner_col_s2, InvWignerParams, kColZT, 6) { inv_wigner_col<true>(ctx, p, smem); }
 
 }  // namespace s2c
