@@ -161,6 +161,10 @@ def kernel_bytes(B):
     out["rft_forward"] = (f0 * f1 * 24 * 4 + b1 * b1 * f0 * f1 * c) + (f1 * f2 * 192 * 4 + n3(b2) * f1 * f2 * c)
     out["so3_relay_fused<%d>" % (2 * b1)] = (b1 * b1 * (B * f0 + f0 * f1) * c + 2 * sig1 +
                                                n3(b2) * B * f1 * c)
+    # the same boundary when the batch takes the plane kernels
+    out["so3_inv_wigner_col_s2"] = b1 * b1 * (B * f0 + f0 * f1) * c
+    out["so3_relay_small<%d>" % (2 * b1)] = 2 * sig1
+    out["so3_fwd_wigner_col"] = n3(b2) * B * f1 * c
     sig2 = B * f2 * (2 * b2) ** 3 * 4
     out["so3_inv_fused<%d>" % (2 * b2)] = n3(b2) * B * f2 * c + 2 * sig2 + B * f2 * 4
     out["so3_mm_tc_kernel"] = n3(b2) * (B * f1 + f1 * f2 + B * f2) * c
