@@ -227,6 +227,12 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
   return d;
 }
+// max(v, 0) with NaN passed on, as torch's relu does (fmaxf and "v > 0 ? v : 0" turn NaN into 0)
+__device__ __forceinline__ float relu(float v) {
+  float r;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(v));
+  return r;
+}
 // 32-byte global accesses (one full sector per lane and instruction); p must be 32-byte aligned
 struct float8 {
   float4 lo, hi;
@@ -464,6 +470,7 @@ inline void bulk_load_issue(void* dst, const void* src, unsigned bytes, unsigned
   std::memcpy(dst, src, bytes);
 }
 inline float2 fma2(float2 a, float2 b, float2 c) { return make_float2(std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)); }
+inline float relu(float v) { return v <= 0.f ? 0.f : v; }
 struct float8 {
   float4 lo, hi;
 };
@@ -547,3 +554,8 @@ inline bool bulk_wait(const Ctx& ctx, unsigned long long*, unsigned) {
   s2c::emu_launch<name##_impl>(#name, (long)(grid), (int)(block), (size_t)(smem), params)
 
 #endif  // S2C_EMUL
+
+namespace s2c {
+// gradient of relu: v where the activation is positive or NaN, 0 elsewhere (torch's rule)
+S2C_HD float relu_grad(float act, float v) { return act <= 0.f ? 0.f : v; }
+}  // namespace s2c

@@ -139,10 +139,10 @@ S2C_KERNEL(so3_integrate_fwd, IntegrateParams) {
     for (int e = lane; e < total4; e += 32) {
       float4 v = src[e];
       if (p.relu) {
-        v.x = v.x > 0.f ? v.x : 0.f;
-        v.y = v.y > 0.f ? v.y : 0.f;
-        v.z = v.z > 0.f ? v.z : 0.f;
-        v.w = v.w > 0.f ? v.w : 0.f;
+        v.x = relu(v.x);
+        v.y = relu(v.y);
+        v.z = relu(v.z);
+        v.w = relu(v.w);
       }
       acc = fmaf(p.w[e / plane4], (v.x + v.y) + (v.z + v.w), acc);
     }
@@ -184,7 +184,7 @@ S2C_KERNEL(so3_integrate_bwd, IntegrateBwdParams) {
       float4 r = make_float4(v, v, v, v);
       if (p.relu) {
         const float4 a = x[e];
-        r = make_float4(a.x > 0.f ? v : 0.f, a.y > 0.f ? v : 0.f, a.z > 0.f ? v : 0.f, a.w > 0.f ? v : 0.f);
+        r = make_float4(relu_grad(a.x, v), relu_grad(a.y, v), relu_grad(a.z, v), relu_grad(a.w, v));
       }
       o[e] = r;
     }

@@ -374,7 +374,7 @@ struct so3_inv_fused_impl {
 #pragma unroll
           for (int g = 0; g < N; ++g) {
             const float a1 = v[g].x + add, a2 = v[g].y + add;
-            rs += (a1 > 0.f ? a1 : 0.f) + (a2 > 0.f ? a2 : 0.f);
+            rs += relu(a1) + relu(a2);
           }
           ipart = fmaf(p.iw[bg0 + bi], rs, ipart);
         } else
@@ -388,8 +388,8 @@ struct so3_inv_fused_impl {
             // boundary only every other row (the planes themselves do, 4 N^2 bytes apart): even
             // rows end, odd rows begin with a 16-byte piece.
             auto keep = [](float4 val, float4 k) {
-              return make_float4(k.x > 0.f ? val.x : 0.f, k.y > 0.f ? val.y : 0.f,
-                                 k.z > 0.f ? val.z : 0.f, k.w > 0.f ? val.w : 0.f);
+              return make_float4(relu_grad(k.x, val.x), relu_grad(k.y, val.y),
+                                 relu_grad(k.z, val.z), relu_grad(k.w, val.w));
             };
             auto quad = [&](auto gc, float4& o1, float4& o2) {
               constexpr int g = decltype(gc)::value;
@@ -443,10 +443,10 @@ struct so3_inv_fused_impl {
                 if (p.mask) {
                   const float4 k1 = *reinterpret_cast<const float4*>(p.mask + row1 + g);
                   const float4 k2 = *reinterpret_cast<const float4*>(p.mask + row2 + g);
-                  o1 = make_float4(k1.x > 0.f ? o1.x : 0.f, k1.y > 0.f ? o1.y : 0.f,
-                                   k1.z > 0.f ? o1.z : 0.f, k1.w > 0.f ? o1.w : 0.f);
-                  o2 = make_float4(k2.x > 0.f ? o2.x : 0.f, k2.y > 0.f ? o2.y : 0.f,
-                                   k2.z > 0.f ? o2.z : 0.f, k2.w > 0.f ? o2.w : 0.f);
+                  o1 = make_float4(relu_grad(k1.x, o1.x), relu_grad(k1.y, o1.y),
+                                   relu_grad(k1.z, o1.z), relu_grad(k1.w, o1.w));
+                  o2 = make_float4(relu_grad(k2.x, o2.x), relu_grad(k2.y, o2.y),
+                                   relu_grad(k2.z, o2.z), relu_grad(k2.w, o2.w));
                 }
                 *reinterpret_cast<float4*>(p.out + row1 + g) = o1;
                 *reinterpret_cast<float4*>(p.out + row2 + g) = o2;
@@ -456,8 +456,8 @@ struct so3_inv_fused_impl {
                 if (p.mask) {
                   const float2 k1 = *reinterpret_cast<const float2*>(p.mask + row1 + g);
                   const float2 k2 = *reinterpret_cast<const float2*>(p.mask + row2 + g);
-                  o1 = make_float2(k1.x > 0.f ? o1.x : 0.f, k1.y > 0.f ? o1.y : 0.f);
-                  o2 = make_float2(k2.x > 0.f ? o2.x : 0.f, k2.y > 0.f ? o2.y : 0.f);
+                  o1 = make_float2(relu_grad(k1.x, o1.x), relu_grad(k1.y, o1.y));
+                  o2 = make_float2(relu_grad(k2.x, o2.x), relu_grad(k2.y, o2.y));
                 }
                 *reinterpret_cast<float2*>(p.out + row1 + g) = o1;
                 *reinterpret_cast<float2*>(p.out + row2 + g) = o2;
@@ -604,8 +604,8 @@ struct so3_fwd_fused_impl {
           if (p.relu) {
 #pragma unroll
             for (int g = 0; g < N; ++g) {
-              v[g].x = v[g].x > 0.f ? v[g].x : 0.f;
-              v[g].y = v[g].y > 0.f ? v[g].y : 0.f;
+              v[g].x = relu(v[g].x);
+              v[g].y = relu(v[g].y);
             }
           }
         } else {

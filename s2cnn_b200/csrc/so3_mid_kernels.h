@@ -94,7 +94,7 @@ struct so3_fwd_mid_impl {
       }
       if (p.relu) {
 #pragma unroll
-        for (int k = 0; k < R1; ++k) v[k] = make_float2(v[k].x > 0.f ? v[k].x : 0.f, v[k].y > 0.f ? v[k].y : 0.f);
+        for (int k = 0; k < R1; ++k) v[k] = make_float2(relu(v[k].x), relu(v[k].y));
       }
       two_head<N, -1>(v, j, tw);
       float2* a = A + pl * PSA + t * LD + j;
@@ -273,8 +273,8 @@ struct so3_inv_mid_impl {
         if (p.mask) {
 #pragma unroll
           for (int i = 0; i < W; ++i) {
-            if (!(k0[u][i] > 0.f)) r0[i] = 0.f;
-            if (!(k1[u][i] > 0.f)) r1[i] = 0.f;
+            r0[i] = relu_grad(k0[u][i], r0[i]);
+            r1[i] = relu_grad(k1[u][i], r1[i]);
           }
         }
         if (p.stride == 1) {

@@ -316,7 +316,7 @@ struct so3_relay_fused_impl {
             constexpr int g = decltype(gc)::value;
             constexpr int pg = fft_reg_pos<N>(g);
             const float a1 = v[pg].x + add, a2 = v[pg].y + add;   // samples gamma = g of both rows
-            u[g] = make_float2(a1 > 0.f ? a1 : 0.f, a2 > 0.f ? a2 : 0.f);
+            u[g] = make_float2(relu(a1), relu(a2));
           });
           if (z >= zc) {
 #pragma unroll

@@ -189,7 +189,7 @@ struct so3_fwd_small_impl {
       }
       if (p.relu) {
 #pragma unroll
-        for (int g = 0; g < N; ++g) v[g] = make_float2(v[g].x > 0.f ? v[g].x : 0.f, v[g].y > 0.f ? v[g].y : 0.f);
+        for (int g = 0; g < N; ++g) v[g] = make_float2(relu(v[g].x), relu(v[g].y));
       }
       fft_reg<N, -1>(v, nullptr);
       S::split_rows(r1, p.K, v);        // in place: a thread owns its two rows
@@ -250,7 +250,7 @@ struct so3_inv_small_impl {
       });
       S::template samples<A0, A1>(ctx, p, q0, planes, [&](int a, float2* place, long at) {
         const float2 k = keep[a - A0], v = *place;
-        *reinterpret_cast<float2*>(p.out + at) = make_float2(k.x > 0.f ? v.x : 0.f, k.y > 0.f ? v.y : 0.f);
+        *reinterpret_cast<float2*>(p.out + at) = make_float2(relu_grad(k.x, v.x), relu_grad(k.y, v.y));
       });
     });
   }
@@ -278,7 +278,7 @@ struct so3_relay_small_impl {
         constexpr int g = decltype(gc)::value;
         constexpr int pg = fft_reg_pos<N>(g);
         const float a1 = v[pg].x + add, a2 = v[pg].y + add;   // samples gamma = g of both rows
-        u[g] = make_float2(a1 > 0.f ? a1 : 0.f, a2 > 0.f ? a2 : 0.f);
+        u[g] = make_float2(relu(a1), relu(a2));
       });
       fft_reg<N, -1>(u, nullptr);
       S::split_rows(r1, p.K2, u);      // in place: a thread owns its two rows
