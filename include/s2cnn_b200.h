@@ -215,6 +215,16 @@ int s2c_so3_mm_gradx(const float* gz, const float* y, float* gx, int nl, int nba
 /* gy = d/dy: replaces _cuda_SO3_mm.backward (grad-y instantiation), s2cnn/so3_mm.py:115-120. */
 int s2c_so3_mm_grady(const float* gz, const float* x, float* gy, int nl, int nbatch, int f_in,
                      int f_out, void* stream);
+/* The gradients are reproducible: equal inputs give equal results, bit for bit.  A gradient with few output
+ * tiles and a long contraction shares a tile between several thread blocks (of one cluster), which add their
+ * partial sums in a fixed order.  The _ws variants can share one tile between several clusters as well (the
+ * query says how much workspace that takes; it may be 0); without it the values differ by rounding only. */
+size_t s2c_so3_mm_gradx_workspace(int nl, int nbatch, int f_in, int f_out);
+size_t s2c_so3_mm_grady_workspace(int nl, int nbatch, int f_in, int f_out);
+int s2c_so3_mm_gradx_ws(const float* gz, const float* y, float* gx, int nl, int nbatch, int f_in,
+                        int f_out, void* workspace, size_t workspace_bytes, void* stream);
+int s2c_so3_mm_grady_ws(const float* gz, const float* x, float* gy, int nl, int nbatch, int f_in,
+                        int f_out, void* workspace, size_t workspace_bytes, void* stream);
 /* z[l,m,n,i,j] = sum_k x[l,m,i,k] conj(y[l,n,k,j]);  x [nl^2, nbatch, f_in, 2],
  * y [nl^2, f_in, f_out, 2], z [nspec(nl), nbatch, f_out, 2].
  * Replaces s2_mm / _cuda_s2_mm, s2cnn/s2_mm.py:10-28,104-137 (+ kernel s2mm.cu :140-198). */
@@ -247,6 +257,11 @@ int s2c_rft_forward_scaled(const float* x, const float* F, const float* Ft, floa
  * tensor cores when n_grid is even). */
 int s2c_rft_backward(const float* g, const float* F, float* gx, int nf, int n_grid, int nspec,
                      void* stream);
+/* scale times the same - the gradient of s2c_rft_forward_scaled - with a workspace as s2c_so3_mm_gradx_ws takes
+ * it (few channels, a long spectrum).  Reproducible like those. */
+size_t s2c_rft_backward_workspace(int nf, int n_grid, int nspec);
+int s2c_rft_backward_scaled(const float* g, const float* F, float* gx, int nf, int n_grid, int nspec,
+                            float scale, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- integration ---------------------------------------------------------------------------- */
 /* out[z] = sum_beta w_beta sum_{alpha,gamma} x[z, beta, alpha, gamma]; x [n, 2b, 2b, 2b].

@@ -68,6 +68,10 @@ _SIGNATURES = {
     "s2c_so3_mm_tc_status": (c_int, []),
     "s2c_so3_mm_gradx": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_so3_mm_grady": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
+    "s2c_so3_mm_gradx_workspace": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "s2c_so3_mm_grady_workspace": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "s2c_so3_mm_gradx_ws": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
+    "s2c_so3_mm_grady_ws": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
     "s2c_s2_mm": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_s2_mm_gradx": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_s2_mm_grady": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
@@ -75,6 +79,8 @@ _SIGNATURES = {
     "s2c_rft_forward_t": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P]),
     "s2c_rft_forward_scaled": (c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_float, _P]),
     "s2c_rft_backward": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P]),
+    "s2c_rft_backward_workspace": (c_size_t, [c_int, c_int, c_int]),
+    "s2c_rft_backward_scaled": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_float, _P, c_size_t, _P]),
     "s2c_so3_integrate": (c_int, [_P, _P, c_long, c_int, c_int, _P]),
     "s2c_so3_integrate_backward": (c_int, [_P, _P, _P, c_long, c_int, c_int, _P]),
     "s2c_so3_rotation_matrices": (c_int, [c_int, c_double, c_double, c_double, _P]),

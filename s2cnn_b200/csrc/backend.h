@@ -157,7 +157,7 @@ inline std::vector<TimingRec>& timing_recs() {   // guarded by timing_mutex()
 // is remembered per kernel: the attribute is set when a launch needs more than any launch before it
 // (cudaFuncSetAttribute on every launch was a tenth of the host time of a small call).
 template <auto kernel, class P>
-inline int launch_impl(const char* kname, long grid, int block, size_t smem, stream_t stream, const P& p) {
+inline int launch_impl(const char* kname, long grid, int block, size_t smem, stream_t stream, const P& p, int cluster = 1) {
   if (grid <= 0) return S2C_OK;
   if (grid > 2147483647L) return fail(S2C_ERR_UNSUPPORTED, std::string(kname) + ": grid too large");
   if (smem > 48 * 1024) {
@@ -180,7 +180,22 @@ inline int launch_impl(const char* kname, long grid, int block, size_t smem, str
     cudaEventCreate(&rec.b);
     cudaEventRecord(rec.a, stream);
   }
-  kernel<<<(unsigned)grid, block, smem, stream>>>(p);
+  if (cluster > 1) {   // clusters of a size chosen at run time (at most 8, a divisor of the grid)
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, p);   // (an error is reported below)
+  } else {
+    kernel<<<(unsigned)grid, block, smem, stream>>>(p);
+  }
   if (timed) {
     cudaEventRecord(rec.b, stream);
     std::lock_guard<std::mutex> lock(timing_mutex());

@@ -1167,59 +1167,86 @@ static int tc_err_flag(int** out) {
 #endif
 
 #ifndef S2C_EMUL
+// blocks of the contraction: `run` floats per outer index
+static void tc_blocks(MmTcParams& p) {
+  if (p.run <= kTcKMax) { p.kblk = (p.run + 7) / 8 * 8; p.nblk = 1; }
+  else { p.kblk = kTcKMax; p.nblk = (p.run + kTcKMax - 1) / kTcKMax; }
+}
+// whether the longest of the ns CTAs of a tile of `blocks` K blocks issues more MMAs than one accumulator may take
+static bool tc_flush(const MmTcParams& p, long blocks, int ns) {
+  if (ns == 1) return 3 * (blocks / p.nblk) * ((p.run + 7) / 8) > kTcChainMax;
+  return 3 * ((blocks + ns - 1) / ns) * (p.kblk / 8) > kTcChainMax;
+}
+static int tc_run(int op, int nb, int fi, int fo) { return 2 * (op == kTcFwd ? fi : op == kTcGradX ? fo : nb); }
+// CTAs per tile; several clusters to a tile only with the workspace they meet in
+static int tc_share(MmTcParams& p, int op, long tiles, void* ws, size_t ws_bytes, stream_t st) {
+  TcShare s = tc_pick_share(op, p.nl, p.nb, p.fi, p.fo, p.nblk, true);
+  if (s.groups > 1 && (!ws || (uintptr_t)ws % 16 != 0 || ws_bytes < tc_share_bytes(tiles, s.groups)))
+    s = tc_pick_share(op, p.nl, p.nb, p.fi, p.fo, p.nblk, false);
+  p.csize = s.csize; p.groups = s.groups;
+  if (s.groups == 1) return S2C_OK;
+  p.count = (int*)ws;
+  p.part = (float*)((unsigned char*)ws + tc_count_bytes(tiles));
+  return cuda_check(cudaMemsetAsync(ws, 0, tc_count_bytes(tiles), st), "counters of the shared tiles");
+}
+static size_t tc_share_workspace(int op, int nl, int nb, int fi, int fo, int run) {
+  if (g_force_general) return 0;
+  MmTcParams p;
+  p.run = run;
+  tc_blocks(p);
+  return tc_share_bytes(so3_mm_tc_tiles(op, nl, nb, fi, fo), tc_pick_share(op, nl, nb, fi, fo, p.nblk, true).groups);
+}
 // so3_mm or one of its gradients on the tensor cores; `handled` tells whether the shape qualified.
 static int so3_mm_tc_launch(int op, const float* a, const float* b, float* c, int nl, int nb, int fi,
-                            int fo, stream_t st, bool* handled) {
+                            int fo, void* ws, size_t ws_bytes, stream_t st, bool* handled) {
   *handled = !g_force_general;
   if (!*handled) return S2C_OK;
   MmTcParams p;
   p.a = a; p.b = b; p.c = c;
   p.nl = nl; p.nb = nb; p.fi = fi; p.fo = fo;
-  p.run = 2 * (op == kTcFwd ? fi : op == kTcGradX ? fo : nb);
-  if (p.run <= kTcKMax) { p.kblk = (p.run + 7) / 8 * 8; p.nblk = 1; }
-  else { p.kblk = kTcKMax; p.nblk = (p.run + kTcKMax - 1) / kTcKMax; }
+  p.run = tc_run(op, nb, fi, fo);
+  tc_blocks(p);
   S2C_TRY(tc_err_flag(&p.err));
+  const long tiles = so3_mm_tc_tiles(op, nl, nb, fi, fo);
+  p.csize = p.groups = 1;
+  p.part = nullptr; p.count = nullptr;
   // The forward product always runs one CTA per tile: its rounding is then the same whatever the batch.
-  p.kper = op == kTcFwd ? kTcNoSplit : tc_pick_kper(op, nl, nb, fi, fo, p.nblk);
-  if (p.kper != kTcNoSplit) {
-    const size_t out_bytes = (size_t)so3_nspec(nl) * (op == kTcGradX ? (size_t)nb * fi : (size_t)fi * fo) * sizeof(float2);
-    S2C_TRY(cuda_check(cudaMemsetAsync(c, 0, out_bytes, st), "so3_mm split-K output clear"));
-  }
-  const long tiles = so3_mm_tc_tiles(op, nl, nb, fi, fo, p.nblk, p.kper);
-  // MMAs of the longest CTA
-  const long chain_mmas = 3 * (p.kper == kTcNoSplit ? (2L * nl - 1) * ((p.run + 7) / 8) : (long)p.kper * (p.kblk / 8));
-  const bool flush = chain_mmas > kTcChainMax;
+  if (op != kTcFwd) S2C_TRY(tc_share(p, op, tiles, ws, ws_bytes, st));
+  const int ns = p.csize * p.groups;
+  const long ctas = tiles * ns;
+  const bool flush = tc_flush(p, (2L * nl - 1) * p.nblk, ns);
   const bool vec = so3_mm_tc_vec16(op, nb, fi, fo);
-  if (op == kTcFwd) return launch_so3_mm_tc<kTcFwd>("so3_mm_tc_kernel", tiles, flush, vec, st, p);
-  if (op == kTcGradX) return launch_so3_mm_tc<kTcGradX>("so3_mm_tc_gradx", tiles, flush, vec, st, p);
-  return launch_so3_mm_tc<kTcGradY>("so3_mm_tc_grady", tiles, flush, vec, st, p);
+  if (op == kTcFwd) return launch_so3_mm_tc<kTcFwd>("so3_mm_tc_kernel", ctas, flush, vec, st, p);
+  if (op == kTcGradX) return launch_so3_mm_tc<kTcGradX>("so3_mm_tc_gradx", ctas, flush, vec, st, p);
+  return launch_so3_mm_tc<kTcGradY>("so3_mm_tc_grady", ctas, flush, vec, st, p);
 }
 
 // A plain real product C[r][c] = sum_k A[r][k] B[c][k] (M rows, N columns, K terms; N and K even)
 // on the tensor-core pipeline: the kernel-grid -> spectrum transforms and their transposes.
 static int plain_tc_launch(bool a_strided, const float* a, const float* b, float* c, long M, long N,
                            long K, long a_rs, long a_ps, long b_rs, long b_ps, long c_rs, long c_ps,
-                           float a_scale, stream_t st) {
+                           float scale, void* ws, size_t ws_bytes, stream_t st) {
   MmTcParams p;
   p.a = a; p.b = b; p.c = c;
   p.nl = 1; p.nb = (int)M; p.fi = (int)(K / 2); p.fo = (int)(N / 2);
   p.run = (int)K;
-  if (p.run <= kTcKMax) { p.kblk = (p.run + 7) / 8 * 8; p.nblk = 1; }
-  else { p.kblk = kTcKMax; p.nblk = (p.run + kTcKMax - 1) / kTcKMax; }
+  tc_blocks(p);
   p.a_rs = a_rs; p.a_ps = a_ps; p.b_rs = b_rs; p.b_ps = b_ps; p.c_rs = c_rs; p.c_ps = c_ps;
-  p.a_scale = a_scale;
+  p.scale = scale;
   S2C_TRY(tc_err_flag(&p.err));
   // (one degree, l = 0, with M rows and N columns in the spectral geometry; the forward transform has a
   // short contraction and is not split)
-  p.kper = a_strided ? tc_pick_kper(kTcPlainSC, 1, (int)M, p.fi, p.fo, p.nblk) : kTcNoSplit;
-  if (p.kper != kTcNoSplit)
-    S2C_TRY(cuda_check(cudaMemsetAsync(c, 0, (size_t)M * N * sizeof(float), st), "rft split-K output clear"));
-  const long tiles = so3_mm_tc_tiles(kTcPlainSC, 1, (int)M, p.fi, p.fo, p.nblk, p.kper);
-  const bool flush = 3 * (p.kper == kTcNoSplit ? (K + 7) / 8 : (long)p.kper * (p.kblk / 8)) > kTcChainMax;
+  const long tiles = so3_mm_tc_tiles(kTcPlainSC, 1, (int)M, p.fi, p.fo);
+  p.csize = p.groups = 1;
+  p.part = nullptr; p.count = nullptr;
+  if (a_strided) S2C_TRY(tc_share(p, kTcPlainSC, tiles, ws, ws_bytes, st));
+  const int ns = p.csize * p.groups;
+  const long ctas = tiles * ns;
+  const bool flush = tc_flush(p, p.nblk, ns);
   // 16-byte loads need K a multiple of 4 and 16-byte aligned rows of every contiguous operand
   const bool vec = K % 4 == 0 && b_rs % 4 == 0 && (a_strided || a_rs % 4 == 0);
-  if (a_strided) return launch_so3_mm_tc<kTcPlainSC>("rft_tc_backward", tiles, flush, vec, st, p);
-  return launch_so3_mm_tc<kTcPlainCC>("rft_tc_forward", tiles, flush, vec, st, p);
+  if (a_strided) return launch_so3_mm_tc<kTcPlainSC>("rft_tc_backward", ctas, flush, vec, st, p);
+  return launch_so3_mm_tc<kTcPlainCC>("rft_tc_forward", ctas, flush, vec, st, p);
 }
 #endif
 
@@ -1228,7 +1255,7 @@ int s2c_so3_mm(const float* x, const float* y, float* z, int nl, int nb, int fi,
   if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
 #ifndef S2C_EMUL
   bool handled = false;
-  S2C_TRY(so3_mm_tc_launch(kTcFwd, x, y, z, nl, nb, fi, fo, as_stream(st), &handled));
+  S2C_TRY(so3_mm_tc_launch(kTcFwd, x, y, z, nl, nb, fi, fo, nullptr, 0, as_stream(st), &handled));
   if (handled) return S2C_OK;
 #endif
   return mm_dispatch(true, kMmFwd, x, y, z, nl, nb, fi, fo, as_stream(st));
@@ -1246,27 +1273,47 @@ int s2c_so3_mm_tc_status(void) {
   return 0;
 #endif
 }
-int s2c_so3_mm_gradx(const float* gz, const float* y, float* gx, int nl, int nb, int fi, int fo,
-                     void* st) {
+size_t s2c_so3_mm_gradx_workspace(int nl, int nb, int fi, int fo) {
+#ifndef S2C_EMUL
+  if (nl >= 1 && nb >= 1 && fi >= 1 && fo >= 1)
+    return tc_share_workspace(kTcGradX, nl, nb, fi, fo, tc_run(kTcGradX, nb, fi, fo));
+#endif
+  return 0;
+}
+int s2c_so3_mm_gradx_ws(const float* gz, const float* y, float* gx, int nl, int nb, int fi, int fo, void* ws,
+                        size_t ws_bytes, void* st) {
   if (!gz || !y || !gx) return fail(S2C_ERR_BAD_ARG, "s2c_so3_mm_gradx: null pointer");
   if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
 #ifndef S2C_EMUL
   bool handled = false;
-  S2C_TRY(so3_mm_tc_launch(kTcGradX, gz, y, gx, nl, nb, fi, fo, as_stream(st), &handled));
+  S2C_TRY(so3_mm_tc_launch(kTcGradX, gz, y, gx, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
   if (handled) return S2C_OK;
 #endif
   return mm_dispatch(true, kMmGradX, gz, y, gx, nl, nb, fi, fo, as_stream(st));
 }
-int s2c_so3_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo,
-                     void* st) {
+int s2c_so3_mm_gradx(const float* gz, const float* y, float* gx, int nl, int nb, int fi, int fo, void* st) {
+  return s2c_so3_mm_gradx_ws(gz, y, gx, nl, nb, fi, fo, nullptr, 0, st);
+}
+size_t s2c_so3_mm_grady_workspace(int nl, int nb, int fi, int fo) {
+#ifndef S2C_EMUL
+  if (nl >= 1 && nb >= 1 && fi >= 1 && fo >= 1)
+    return tc_share_workspace(kTcGradY, nl, nb, fi, fo, tc_run(kTcGradY, nb, fi, fo));
+#endif
+  return 0;
+}
+int s2c_so3_mm_grady_ws(const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo, void* ws,
+                        size_t ws_bytes, void* st) {
   if (!gz || !x || !gy) return fail(S2C_ERR_BAD_ARG, "s2c_so3_mm_grady: null pointer");
   if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
 #ifndef S2C_EMUL
   bool handled = false;
-  S2C_TRY(so3_mm_tc_launch(kTcGradY, x, gz, gy, nl, nb, fi, fo, as_stream(st), &handled));
+  S2C_TRY(so3_mm_tc_launch(kTcGradY, x, gz, gy, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
   if (handled) return S2C_OK;
 #endif
   return mm_dispatch(true, kMmGradY, x, gz, gy, nl, nb, fi, fo, as_stream(st));
+}
+int s2c_so3_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo, void* st) {
+  return s2c_so3_mm_grady_ws(gz, x, gy, nl, nb, fi, fo, nullptr, 0, st);
 }
 int s2c_s2_mm(const float* x, const float* y, float* z, int nl, int nb, int fi, int fo, void* st) {
   if (!x || !y || !z) return fail(S2C_ERR_BAD_ARG, "s2c_s2_mm: null pointer");
@@ -1306,7 +1353,7 @@ static int rft_forward_any(const float* x, const float* F, const float* Ft, floa
 #ifndef S2C_EMUL
   if (Ft && ng % 2 == 0)
     // C[f][(s, c)] = sum_a (scale x[f][a]) Ft[(s, c)][a], written to out[s][f][c]
-    return plain_tc_launch(false, x, Ft, out, nf, 2L * ns, ng, ng, 2, ng, 2, 2, 2L * nf, scale, st);
+    return plain_tc_launch(false, x, Ft, out, nf, 2L * ns, ng, ng, 2, ng, 2, 2, 2L * nf, scale, nullptr, 0, st);
 #endif
   if (!F) return fail(S2C_ERR_UNSUPPORTED, "rft with the transposed matrix: needs the CUDA build and an even n_grid");
   RftFwdParams p;
@@ -1337,23 +1384,34 @@ int s2c_rft_forward_scaled(const float* x, const float* F, const float* Ft, floa
   return rft_forward_any(x, F, Ft, out, nf, ng, ns, scale, as_stream(st));
 }
 
-int s2c_rft_backward(const float* g, const float* F, float* gx, int nf, int ng, int ns, void* st) {
+size_t s2c_rft_backward_workspace(int nf, int ng, int ns) {
+#ifndef S2C_EMUL
+  if (nf >= 1 && ng >= 1 && ns >= 1 && ng % 2 == 0) return tc_share_workspace(kTcPlainSC, 1, nf, ns, ng / 2, 2 * ns);
+#endif
+  return 0;
+}
+int s2c_rft_backward_scaled(const float* g, const float* F, float* gx, int nf, int ng, int ns, float scale, void* ws,
+                            size_t ws_bytes, void* st) {
   if (!g || !F || !gx || nf < 1 || ng < 1 || ns < 1)
     return fail(S2C_ERR_BAD_ARG, "s2c_rft_backward: bad argument");
 #ifndef S2C_EMUL
   if (!g_force_general && ng % 2 == 0) {
-    // gx[f][a] = sum_{(s, c)} g[s][f][c] F[a][(s, c)]: the row operand holds k = (s, c) as pairs
+    // gx[f][a] = scale sum_{(s, c)} g[s][f][c] F[a][(s, c)]: the row operand holds k = (s, c) as pairs
     // 2 nf floats apart
-    return plain_tc_launch(true, g, F, gx, nf, ng, 2L * ns, 2, 2L * nf, 2L * ns, 2, ng, 2, 1.f, as_stream(st));
+    return plain_tc_launch(true, g, F, gx, nf, ng, 2L * ns, 2, 2L * nf, 2L * ns, 2, ng, 2, scale, ws, ws_bytes,
+                           as_stream(st));
   }
 #endif
   RftBwdParams p;
   p.g = (const float2*)g; p.F = (const float2*)F; p.gx = gx;
-  p.nf = nf; p.ng = ng; p.ns = ns;
+  p.nf = nf; p.ng = ng; p.ns = ns; p.scale = scale;
   p.tiles_f = (nf + kRftTF - 1) / kRftTF;
   const long tiles_a = (ng + kRftTA - 1) / kRftTA;
   const size_t sm = kRftTS * kRftTF * 8 + kRftTA * (kRftTS + 1) * 8;
   return S2C_LAUNCH(rft_backward, p.tiles_f * tiles_a, 256, sm, as_stream(st), p);
+}
+int s2c_rft_backward(const float* g, const float* F, float* gx, int nf, int ng, int ns, void* st) {
+  return s2c_rft_backward_scaled(g, F, gx, nf, ng, ns, 1.f, nullptr, 0, st);
 }
 
 // ---- integration ---------------------------------------------------------------------------------

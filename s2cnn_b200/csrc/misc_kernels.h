@@ -62,13 +62,14 @@ S2C_KERNEL(rft_forward, RftFwdParams) {
   }
 }
 
-// ---- rft backward: gx[f][a] = sum_s  g[s][f] . F[a][s]   (real dot of complex pairs) ---------
+// ---- rft backward: gx[f][a] = scale sum_s  g[s][f] . F[a][s]   (real dot of complex pairs) ----
 struct RftBwdParams {
   const float2* g;   // [ns][nf]
   const float2* F;   // [ng][ns]
   float* gx;         // [nf][ng]
   int nf, ng, ns;
   int tiles_f;
+  float scale;
 };
 
 S2C_KERNEL(rft_backward, RftBwdParams) {
@@ -108,7 +109,7 @@ S2C_KERNEL(rft_backward, RftBwdParams) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int a = a0 + ag + 8 * q;
-      if (a < p.ng) p.gx[(long)(f0 + fi) * p.ng + a] = acc[q];
+      if (a < p.ng) p.gx[(long)(f0 + fi) * p.ng + a] = acc[q] * p.scale;
     }
   }
 }

@@ -59,6 +59,7 @@
 #include <algorithm>
 
 #include "backend.h"
+#include "so3_kernels.h"   // align_up
 
 namespace s2c {
 
@@ -87,14 +88,17 @@ struct MmTcParams {
   int run;          // floats per outer contraction index: 2 fi (fwd), 2 fo (grad x), 2 nb (grad y)
   int kblk;         // floats per K block (multiple of 8, <= kTcKMax)
   int nblk;         // K blocks per run
-  int kper;         // K blocks per CTA: a tile whose contraction has more is shared by several CTAs, each
-                    // adding its partial result atomically into the zeroed output (see tc_pick_kper)
+  int csize, groups;   // a tile's contraction is shared by csize * groups CTAs: `groups` clusters of csize, whose
+                    // partial results are added in the order of their K blocks (see tc_pick_share)
+  float* part;      // groups > 1: the clusters' sums (kTcTileFloats each, in grid order) and, zero at the launch,
+  int* count;       // eight arrival counters per tile
   int* err;         // device flag, set to 1 on a wait time-out
   // plain products only (floats): element (row r, k) of a at r * a_rs + (k / 2) * a_ps + k % 2,
   // element (column c, k) of b likewise, element (r, c) of the result at r * c_rs + (c / 2) * c_ps + c % 2;
   // nb = rows, fi = K / 2, fo = columns / 2, nl = 1
   long a_rs, a_ps, b_rs, b_ps, c_rs, c_ps;
-  float a_scale;    // kTcPlainCC: the row operand is multiplied by this (and rounded) while it is staged
+  float scale;      // kTcPlainCC: the row operand is multiplied by this (and rounded) while it is staged;
+                    // kTcPlainSC: the result is
 };
 
 // row / column geometry of one degree
@@ -252,17 +256,28 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const float (&v)[16]) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// CTAs that share an output tile of degree l: each takes at most kper of its (2l + 1) * nblk K blocks.
-__host__ __device__ __forceinline__ int tc_splits(int l, int nblk, int kper) {
-  return ((2 * l + 1) * nblk + kper - 1) / kper;
+// CTAs that share a tile form a cluster: each puts its partial result into its own shared memory, and rank r adds
+// all of them, in rank order, for its share of the tile's columns.  The result does not depend on which CTA
+// finishes when.  (Atomic adds into a cleared output took about the same time, but in the order of arrival:
+// gradients then differ from run to run.)  A contraction too long for one cluster is shared by several; the ranks
+// of a tile's last cluster to arrive add the clusters' sums, again in a fixed order.
+constexpr int kTcTileFloats = kTcBM * kTcBN;
+constexpr int kTcMaxCluster = 8;
+static_assert(kTcTileFloats * 4 <= kTcStages * kTcStageBytes, "a partial tile lies in the operand stages");
+__device__ __forceinline__ void tc_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
-
-// Vector reductions without a return value (one request per 8 / 16 bytes instead of one per float).
-__device__ __forceinline__ void tc_red2(float* p, float a, float b) {
-  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(a), "f"(b) : "memory");
-}
-__device__ __forceinline__ void tc_red4(float* p, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+// Arrival at a counter after this CTA's values have been written; true in the CTA that arrives last of n, whose
+// reads then see the others' values.  Called by all threads of the CTA; nobody waits for another CTA.
+__device__ __forceinline__ bool tc_last_of(int* counter, int n, int* flag) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) *flag = atomicAdd(counter, 1) == n - 1;
+  __syncthreads();
+  const bool last = *flag != 0;
+  __threadfence();
+  __syncthreads();       // the flag may be written again
+  return last;
 }
 
 // 8 columns of a lane's row (completes with tcgen05.wait::st)
@@ -299,19 +314,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   uint64_t* accfree = accdone + 2;                                   // [2] collectors -> issuer
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfree + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* last_flag = reinterpret_cast<int*>(tmem_slot + 2);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
   // ---- which tile ---------------------------------------------------------------------------
+  const int nsplit = p.csize * p.groups;
   int l = p.nl - 1;
   long t = blockIdx.x;
   for (;; --l) {
-    const long c = tc_tiles_for(OP, p.nb, p.fi, p.fo, l) * tc_splits(l, p.nblk, p.kper);
+    const long c = tc_tiles_for(OP, p.nb, p.fi, p.fo, l) * nsplit;
     if (t < c) break;
     t -= c;
   }
   const int L = 2 * l + 1;
   // K blocks handled by this CTA: [it_lo, it_hi) of the L * nblk blocks (outer index, block of its run)
-  const int nsplit = tc_splits(l, p.nblk, p.kper);
   const int split = (int)(t % nsplit);
   t /= nsplit;
   const int it_lo = (int)((long)split * L * p.nblk / nsplit), it_hi = (int)((long)(split + 1) * L * p.nblk / nsplit);
@@ -323,7 +339,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   const int row0 = (int)(t / tiles_n) * kTcBM, col0 = (int)(t % tiles_n) * kTcBN;
   const long spec0 = (long)l * (4L * l * l - 1) / 3;
   const int fi2 = 2 * p.fi, fo2 = 2 * p.fo;
-  const int nit = it_hi - it_lo;                          // K blocks of this CTA
+  const int nit = it_hi - it_lo;                          // K blocks of this CTA (a shared tile: possibly none)
   // accumulator groups (one when the whole chain stays in the tensor core's accumulator)
   const int ngroups = FLUSH ? (nit + kTcFlushBlocks - 1) / kTcFlushBlocks : 1;
 
@@ -575,7 +591,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
         for (int i = 0; i < 4; ++i) {
           float2 v = ra[4 * ks + i];
           if (OP == kTcPlainCC)   // (__fmul_rn: the product must not be contracted into the hi / lo split)
-            v = make_float2(__fmul_rn(v.x, p.a_scale), __fmul_rn(v.y, p.a_scale));
+            v = make_float2(__fmul_rn(v.x, p.scale), __fmul_rn(v.y, p.scale));
           hi[2 * i] = tc_hi(v.x); hi[2 * i + 1] = tc_hi(v.y);
           lo[2 * i] = v.x - hi[2 * i]; lo[2 * i + 1] = v.y - hi[2 * i + 1];
         }
@@ -595,7 +611,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   // (waited for by the collectors, which have followed every earlier phase of these barriers; the
   // block barrier below passes the fact on to the other warps)
   __syncwarp();
-  if (warp >= 1 && warp <= kTcCollectorWarps && !*abort_flag) {
+  if (nit > 0 && warp >= 1 && warp <= kTcCollectorWarps && !*abort_flag) {
     const int glast = ngroups - 1;
     wait(&accdone[glast & 1], (uint32_t)((glast / 2) & 1));
   }
@@ -604,19 +620,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   // ---- epilogue: TMEM -> registers -> z -----------------------------------------------------
-  if (ok && warp != 0) {
-    // warp w may only touch TMEM lanes 32 (w % 4) .. +31; the four warps sharing a lane quarter
-    // split the 128 accumulator columns between them
-    constexpr int kColsPerWarp = kTcBN / 4;
-    static_assert(kColsPerWarp == 32, "one tcgen05.ld of 32 columns per warp");
-    const int q = warp & 3, cg = (warp - 1) >> 2;
-    const int r = row0 + 32 * q + lane;
-    const int ro = r / RI, ri = r - ro * RI;
-    // c[((spec0 + ro * sro + co * sco) * RI + ri) * CW + rem]
-    const int sro = OP == kTcGradY ? 1 : L, sco = OP == kTcGradY ? L : 1;
+  // warp w may only touch TMEM lanes 32 (w % 4) .. +31; the four warps sharing a lane quarter
+  // split the 128 accumulator columns between them
+  constexpr int kColsPerWarp = kTcBN / 4;
+  static_assert(kColsPerWarp == 32, "one tcgen05.ld of 32 columns per warp");
+  const int q = warp & 3, cg = (warp - 1) >> 2;
+  const int r = row0 + 32 * q + lane;
+  const int cbase = kColsPerWarp * cg;
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = 0.f;
+  if (ok && warp != 0 && nit > 0) {
     const uint32_t last_acc = FLUSH ? (uint32_t)(((ngroups - 1) & 1) * kTcBN) : 0u;
-    const int cbase = kColsPerWarp * cg;
-    float v[32];
     // 32 result columns of a lane's row; spectral products: real and imaginary columns from the two halves
     auto load_columns = [&](uint32_t region, float (&o)[32]) {
       const uint32_t base = tmem_base + ((uint32_t)(32 * q) << 16) + region;
@@ -637,66 +652,98 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] += w[i];
     }
-    if (r < M && (OP == kTcPlainCC || OP == kTcPlainSC)) {
+  }
+  const int ro = r / RI, ri = r - ro * RI;
+  // c[((spec0 + ro * sro + co * sco) * RI + ri) * CW + rem]
+  const int sro = OP == kTcGradY ? 1 : L, sco = OP == kTcGradY ? L : 1;
+  // two columns (one complex number: never straddles an outer column index), four with VEC
+  auto store2 = [&](int gcol, float a, float b) {
+    if (gcol >= Np) return;
+    if constexpr (OP == kTcPlainCC || OP == kTcPlainSC) {
+      if (OP == kTcPlainSC) { a *= p.scale; b *= p.scale; }
+      *reinterpret_cast<float2*>(p.c + (long)r * p.c_rs + (long)(gcol >> 1) * p.c_ps) = make_float2(a, b);
+    } else {
+      const int co = gcol / CW, rem = gcol - co * CW;
+      *reinterpret_cast<float2*>(p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem) = make_float2(a, b);
+    }
+  };
+  auto store4 = [&](int gcol, float4 o) {
+    if constexpr (VEC && OP != kTcPlainCC && OP != kTcPlainSC) {
+      if (gcol >= Np) return;     // CW is a multiple of 4, so a group of 4 is all in or all out
+      const int co = gcol / CW, rem = gcol - co * CW;
+      *reinterpret_cast<float4*>(p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem) = o;
+    } else {
+      store2(gcol, o.x, o.y);
+      store2(gcol + 2, o.z, o.w);
+    }
+  };
+  constexpr bool kShares = OP == kTcGradX || OP == kTcGradY || OP == kTcPlainSC;
+  if (kShares && nsplit > 1) {
+    // ---- a shared tile.  16-byte chunk c4 of a thread's 32 columns lies at [c4][warp][lane]; rank r of the cluster
+    // takes the chunks 8 r / csize .. of every thread.  (All threads of all CTAs pass the barriers, also after a
+    // time-out: what is then added is undefined, and the flag below says so.)
+    const int rank = (int)blockIdx.x % p.csize, lo = 8 * rank / p.csize, hi = 8 * (rank + 1) / p.csize;
+    const int at = (warp - 1) * 32 + lane;
+    float4* const tile = reinterpret_cast<float4*>(smem);
+    if (warp != 0) {
 #pragma unroll
-      for (int c2 = 0; c2 < 16; ++c2) {
-        const int gcol = col0 + cbase + 2 * c2;
-        if (gcol < Np) {
-          float* dst = p.c + (long)r * p.c_rs + (long)(gcol >> 1) * p.c_ps;
-          if (nsplit > 1) tc_red2(dst, v[2 * c2], v[2 * c2 + 1]);
-          else *reinterpret_cast<float2*>(dst) = make_float2(v[2 * c2], v[2 * c2 + 1]);
-        }
-      }
-    } else if (r < M) {
-      if (VEC && nsplit == 1 && CW % 8 == 0 && reinterpret_cast<unsigned long long>(p.c) % 32 == 0) {
-        // a lane owns a row: 32-byte stores write whole sectors (16-byte ones would send every
-        // sector to L2 in two halves); CW % 8 == 0 keeps a group of 8 inside one outer column index
+      for (int c4 = 0; c4 < 8; ++c4) tile[c4 * 512 + at] = make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
+    }
+    tc_cluster_sync();
+    const int cl0 = ((int)blockIdx.x - split) / p.csize;         // first cluster of the tile
+    float4* const part = reinterpret_cast<float4*>(p.part);
+    const bool mine = warp != 0 && r < M;
+    if (mine) {
+      for (int c4 = lo; c4 < hi; ++c4) {
+        if (col0 + cbase + 4 * c4 >= Np) break;
+        float4 t[kTcMaxCluster], sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int c8 = 0; c8 < 4; ++c8) {
-          const int gcol = col0 + cbase + 8 * c8;
-          if (gcol < Np) {
-            const int co = gcol / CW, rem = gcol - co * CW;
-            float* dst = p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem;
-            float8 o;
-            o.lo = make_float4(v[8 * c8], v[8 * c8 + 1], v[8 * c8 + 2], v[8 * c8 + 3]);
-            o.hi = make_float4(v[8 * c8 + 4], v[8 * c8 + 5], v[8 * c8 + 6], v[8 * c8 + 7]);
-            st_global_256(dst, o);
-          }
-        }
-      } else if constexpr (VEC) {
+        for (int k = 0; k < kTcMaxCluster; ++k)
+          if (k < p.csize) t[k] = cl_load4(cl_map(ClCtx(), reinterpret_cast<const float2*>(tile), k), 2 * (c4 * 512 + at));
 #pragma unroll
-        for (int c4 = 0; c4 < 8; ++c4) {
-          const int gcol = col0 + cbase + 4 * c4;
-          if (gcol < Np) {  // CW is a multiple of 4, so a group of 4 is all in or all out
-            const int co = gcol / CW, rem = gcol - co * CW;
-            float* dst = p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem;
-            if (nsplit > 1) {
-              tc_red4(dst, v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
-            } else {
-              *reinterpret_cast<float4*>(dst) =
-                  make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]);
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int c2 = 0; c2 < 16; ++c2) {
-          const int gcol = col0 + cbase + 2 * c2;
-          if (gcol < Np) {  // one complex number: never straddles an outer column index
-            const int co = gcol / CW, rem = gcol - co * CW;
-            float* dst = p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem;
-            if (nsplit > 1) {
-              tc_red2(dst, v[2 * c2], v[2 * c2 + 1]);
-            } else {
-              *reinterpret_cast<float2*>(dst) = make_float2(v[2 * c2], v[2 * c2 + 1]);
-            }
-          }
-        }
+        for (int k = 0; k < kTcMaxCluster; ++k)
+          if (k < p.csize) { sum.x += t[k].x; sum.y += t[k].y; sum.z += t[k].z; sum.w += t[k].w; }
+        if (p.groups == 1) store4(col0 + cbase + 4 * c4, sum);
+        else __stcg(part + (size_t)(blockIdx.x / p.csize) * (kTcTileFloats / 4) + c4 * 512 + at, sum);
       }
     }
-  } else if (!ok && tid == 0) {
-    atomicExch(p.err, 1);
+    if (p.groups > 1 && tc_last_of(&p.count[(cl0 / p.groups) * kTcMaxCluster + rank], p.groups, last_flag) && mine) {
+      for (int c4 = lo; c4 < hi; ++c4) {
+        if (col0 + cbase + 4 * c4 >= Np) break;
+        const float4* src = part + (size_t)cl0 * (kTcTileFloats / 4) + c4 * 512 + at;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int g = 0; g < p.groups; ++g) {
+          const float4 t = __ldcg(src + (size_t)g * (kTcTileFloats / 4));
+          sum.x += t.x; sum.y += t.y; sum.z += t.z; sum.w += t.w;
+        }
+        store4(col0 + cbase + 4 * c4, sum);
+      }
+    }
+    tc_cluster_sync();     // the others have read this CTA's part
+  } else if (ok && warp != 0 && r < M) {
+    if (VEC && OP != kTcPlainCC && OP != kTcPlainSC && CW % 8 == 0 && reinterpret_cast<unsigned long long>(p.c) % 32 == 0) {
+      // a lane owns a row: 32-byte stores write whole sectors (16-byte ones would send every
+      // sector to L2 in two halves); CW % 8 == 0 keeps a group of 8 inside one outer column index
+#pragma unroll
+      for (int c8 = 0; c8 < 4; ++c8) {
+        const int gcol = col0 + cbase + 8 * c8;
+        if (gcol < Np) {
+          const int co = gcol / CW, rem = gcol - co * CW;
+          float* dst = p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem;
+          float8 o;
+          o.lo = make_float4(v[8 * c8], v[8 * c8 + 1], v[8 * c8 + 2], v[8 * c8 + 3]);
+          o.hi = make_float4(v[8 * c8 + 4], v[8 * c8 + 5], v[8 * c8 + 6], v[8 * c8 + 7]);
+          st_global_256(dst, o);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int c4 = 0; c4 < 8; ++c4)
+        store4(col0 + cbase + 4 * c4, make_float4(v[4 * c4], v[4 * c4 + 1], v[4 * c4 + 2], v[4 * c4 + 3]));
+    }
   }
+  if (!ok && tid == 0) atomicExch(p.err, 1);
 
   // ---- release tensor memory ------------------------------------------------------------------
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -711,15 +758,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
 // One product: picks the instantiation (see FLUSH, VEC above).
 #if defined(S2C_SPLIT) && !defined(S2C_PART)
 template <int OP>
-int launch_so3_mm_tc(const char* name, long tiles, bool flush, bool vec, stream_t st, const MmTcParams& p);
+int launch_so3_mm_tc(const char* name, long ctas, bool flush, bool vec, stream_t st, const MmTcParams& p);
 #else
 template <int OP>
-int launch_so3_mm_tc(const char* name, long tiles, bool flush, bool vec, stream_t st, const MmTcParams& p) {
+int launch_so3_mm_tc(const char* name, long ctas, bool flush, bool vec, stream_t st, const MmTcParams& p) {
   if (flush)
-    return vec ? launch_impl<so3_mm_tc_kernel<OP, true, true>>(name, tiles, kTcThreads, kTcSmemBytes, st, p)
-               : launch_impl<so3_mm_tc_kernel<OP, true, false>>(name, tiles, kTcThreads, kTcSmemBytes, st, p);
-  return vec ? launch_impl<so3_mm_tc_kernel<OP, false, true>>(name, tiles, kTcThreads, kTcSmemBytes, st, p)
-             : launch_impl<so3_mm_tc_kernel<OP, false, false>>(name, tiles, kTcThreads, kTcSmemBytes, st, p);
+    return vec ? launch_impl<so3_mm_tc_kernel<OP, true, true>>(name, ctas, kTcThreads, kTcSmemBytes, st, p, p.csize)
+               : launch_impl<so3_mm_tc_kernel<OP, true, false>>(name, ctas, kTcThreads, kTcSmemBytes, st, p, p.csize);
+  return vec ? launch_impl<so3_mm_tc_kernel<OP, false, true>>(name, ctas, kTcThreads, kTcSmemBytes, st, p, p.csize)
+             : launch_impl<so3_mm_tc_kernel<OP, false, false>>(name, ctas, kTcThreads, kTcSmemBytes, st, p, p.csize);
 }
 #endif
 
@@ -731,38 +778,49 @@ inline bool so3_mm_tc_vec16(int op, int nb, int fi, int fo) {
   return (fi % 2 == 0) && (fo % 2 == 0);
 }
 
-inline long so3_mm_tc_tiles(int op, int nl, int nb, int fi, int fo, int nblk, int kper) {
+inline long so3_mm_tc_tiles(int op, int nl, int nb, int fi, int fo) {
   long t = 0;
-  for (int l = 0; l < nl; ++l) t += tc_tiles_for(op, nb, fi, fo, l) * tc_splits(l, nblk, kper);
+  for (int l = 0; l < nl; ++l) t += tc_tiles_for(op, nb, fi, fo, l);
   return t;
 }
+inline size_t tc_count_bytes(long tiles) { return align_up((size_t)tiles * kTcMaxCluster * sizeof(int), 256); }
+inline size_t tc_share_bytes(long tiles, int groups) {
+  return groups > 1 ? tc_count_bytes(tiles) + (size_t)tiles * groups * kTcTileFloats * sizeof(float) : 0;
+}
 
-constexpr int kTcNoSplit = 1 << 30;
-
-// K blocks per CTA.  One CTA fits on an SM; a product with few output tiles and a long contraction (the
+struct TcShare {
+  int csize = 1, groups = 1;
+};
+// CTAs per tile.  One CTA fits on an SM; a product with few output tiles and a long contraction (the
 // transposed kernel transform of a layer with few channels: one or two tiles of several hundred K
 // blocks; the gradients of small batches) leaves most of the 148 SMs idle for the length of the longest
-// tile.  Estimate of the makespan in K blocks: the longest CTA or the average load of an SM, where a
-// CTA costs kCta blocks on top of its own (set-up, pipeline fill, epilogue: about 6 us against 0.6 us a
-// block) and sharing costs another kShare (clearing the output, atomic adds).  The split is taken only
-// where the estimate drops by a tenth, so that large products keep one CTA per tile.
-inline int tc_pick_kper(int op, int nl, int nb, int fi, int fo, int nblk) {
-  constexpr double kCta = 8, kShare = 4;
-  auto estimate = [&](int kper) {
-    double load = 0, longest = 0;
-    for (int l = 0; l < nl; ++l) {
-      const int blocks = (2 * l + 1) * nblk, ns = tc_splits(l, nblk, kper);
-      load += (double)tc_tiles_for(op, nb, fi, fo, l) * (blocks + ns * kCta);
-      longest = std::max(longest, (double)((blocks + ns - 1) / ns));
+// tile.  Estimate of the makespan in K blocks: where all clusters are resident at once the longest one, else at
+// least their average load and a last, short one (the grid starts with the highest degrees).  A CTA costs kCta
+// blocks on top of its own (set-up, pipeline fill, epilogue: about 6 us against 0.6 us a block), sharing within a
+// cluster another kShare and between clusters another kGather.  kSlots: clusters resident on the chip, by size
+// (cudaOccupancyMaxActiveClusters).  The split is taken only where the estimate drops by a tenth, so that large
+// products keep one CTA per tile.
+inline TcShare tc_pick_share(int op, int nl, int nb, int fi, int fo, int nblk, bool several_clusters) {
+  constexpr double kCta = 8, kShare = 4, kGather = 6;
+  constexpr int kSlots[kTcMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+  const long tiles = so3_mm_tc_tiles(op, nl, nb, fi, fo);
+  auto estimate = [&](int c, int groups) {
+    const int ns = c * groups;
+    double load = 0, shortest = 0, longest = 0;
+    for (int l = nl - 1; l >= 0; --l) {
+      const int blocks = (2 * l + 1) * nblk;
+      shortest = (blocks + ns - 1) / ns + kCta + (ns > 1 ? kShare : 0) + (groups > 1 ? kGather : 0);
+      longest = std::max(longest, shortest);
+      load += (double)tc_tiles_for(op, nb, fi, fo, l) * groups * shortest;
     }
-    return std::max(longest + kCta, load / 148) + (kper == kTcNoSplit ? 0 : kShare);
+    return tiles * groups <= kSlots[c] ? longest : std::max(longest, load / kSlots[c] + shortest);
   };
-  int best = kTcNoSplit;
-  double t = 0.9 * estimate(best);
-  for (int kper = 4; kper < (2 * nl - 1) * nblk; kper += (kper + 3) / 4) {
-    const double e = estimate(kper);
-    if (e < t) { t = e; best = kper; }
-  }
+  TcShare best;
+  double t = 0.9 * estimate(1, 1);
+  for (int c = 2; c <= kTcMaxCluster; ++c)
+    if (const double e = estimate(c, 1); e < t) { t = e; best.csize = c; }
+  for (int g = 2; several_clusters && tiles * g <= kSlots[kTcMaxCluster]; ++g)
+    if (const double e = estimate(kTcMaxCluster, g); e < t) { t = e; best.csize = kTcMaxCluster; best.groups = g; }
   return best;
 }
 

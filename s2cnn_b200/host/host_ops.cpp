@@ -71,8 +71,8 @@ long s2_bandwidth(long nspec) {
   X(so3_rfft_relu) X(so3_rfft_sums_ws) X(so3_relay_workspace) X(s2_conv_relu_so3_rfft_ws) X(so3_rifft_relu_rfft_ws) X(so3_rifft_relu_grad_ws) X(so3_fft) X(so3_rifft)                 \
   X(so3_rifft_relu_integrate)                      \
   X(s2_conv_synthesis_workspace) X(s2_conv_synthesis) X(so3_ifft) X(s2_fft_workspace) X(s2_fft)    \
-  X(s2_ifft) X(so3_mm) X(so3_mm_gradx) X(so3_mm_grady) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
-  X(s2_mm_grady) X(rft_forward) X(rft_forward_t) X(rft_forward_scaled) X(rft_backward) X(so3_integrate)                  \
+  X(s2_ifft) X(so3_mm) X(so3_mm_gradx_ws) X(so3_mm_gradx_workspace) X(so3_mm_grady_ws) X(so3_mm_grady_workspace) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
+  X(s2_mm_grady) X(rft_forward) X(rft_forward_t) X(rft_forward_scaled) X(rft_backward_scaled) X(rft_backward_workspace) X(so3_integrate)                  \
   X(so3_integrate_backward) X(so3_rotate_spectrum) X(project_on_sphere)
 
 struct Ops {
@@ -417,6 +417,21 @@ struct Ops {
     if (check_tc) check_tensor_core_status();
     return out;
   }
+  // a gradient product: the parts of tiles shared by several thread blocks lie in a workspace
+  template <class F, class W>
+  Tensor mm_grad(const char* name, F fn, W workspace_bytes, const Tensor& a_, const Tensor& b_, at::IntArrayRef shape, long nl, long nb, long fi, long fo) {
+    prep(a_);
+    prep(b_);
+    const Tensor a = a_.contiguous(), b = b_.contiguous();
+    Tensor out = empty_like_shape(a, shape);
+    Ctx c(*this, a);
+    const size_t bytes = workspace_bytes((int)nl, (int)nb, (int)fi, (int)fo);
+    Tensor ws;
+    if (bytes) ws = workspace(bytes, a);
+    call(name, fn, cptr(a), cptr(b), ptr(out), (int)nl, (int)nb, (int)fi, (int)fo, bytes ? ws.mutable_data_ptr() : nullptr, bytes, c.stream);
+    if (check_tc) check_tensor_core_status();
+    return out;
+  }
   // Waits for the device and raises if a tensor-core product has given up on one of its bounded
   // barrier waits since the library was loaded (its output is then undefined).
   void check_tensor_core_status() const {
@@ -433,11 +448,11 @@ struct Ops {
   }
   Tensor so3_mm_gradx(const Tensor& gz, const Tensor& y, int64_t nb, int64_t fi) {
     const long nl = so3_bandwidth(y.size(0)), fo = y.size(2);
-    return mm("s2c_so3_mm_gradx", so3_mm_gradx_, gz, y, {so3_nspec(nl), nb, fi, 2}, nl, nb, fi, fo);
+    return mm_grad("s2c_so3_mm_gradx", so3_mm_gradx_ws_, so3_mm_gradx_workspace_, gz, y, {so3_nspec(nl), nb, fi, 2}, nl, nb, fi, fo);
   }
   Tensor so3_mm_grady(const Tensor& gz, const Tensor& x, int64_t fo) {
     const long nl = so3_bandwidth(x.size(0)), nb = x.size(1), fi = x.size(2);
-    return mm("s2c_so3_mm_grady", so3_mm_grady_, gz, x, {so3_nspec(nl), fi, fo, 2}, nl, nb, fi, fo);
+    return mm_grad("s2c_so3_mm_grady", so3_mm_grady_ws_, so3_mm_grady_workspace_, gz, x, {so3_nspec(nl), fi, fo, 2}, nl, nb, fi, fo);
   }
   Tensor s2_mm(const Tensor& x, const Tensor& y) {
     const S2Product d = s2_product_dims(x, y);
@@ -494,8 +509,8 @@ struct Ops {
     S2C_CALL(rft_forward_scaled, cptr(x), cptr(F_), Ft ? cptr(*Ft) : nullptr, ptr(out), (int)lead_numel(lead), (int)ng, (int)ns, (float)scale, c.stream);
     return out;
   }
-  // g [nspec, nf, 2], F [n_grid, nspec, 2] -> [nf, n_grid]
-  Tensor rft_backward(const Tensor& g_, const Tensor& F_) {
+  // scale * F^T g: g [nspec, nf, 2], F [n_grid, nspec, 2] -> [nf, n_grid]
+  Tensor rft_backward(const Tensor& g_, const Tensor& F_, double scale) {
     prep(g_);
     prep(F_);
     const long ns = g_.size(0), nf = g_.size(1), ng = F_.size(0);
@@ -503,7 +518,10 @@ struct Ops {
     const Tensor g = g_.contiguous(), F = F_.contiguous();
     Tensor out = empty_like_shape(g, {nf, ng});
     Ctx c(*this, g);
-    S2C_CALL(rft_backward, cptr(g), cptr(F), ptr(out), (int)nf, (int)ng, (int)ns, c.stream);
+    const size_t bytes = rft_backward_workspace_((int)nf, (int)ng, (int)ns);
+    Tensor ws;
+    if (bytes) ws = workspace(bytes, g);
+    S2C_CALL(rft_backward_scaled, cptr(g), cptr(F), ptr(out), (int)nf, (int)ng, (int)ns, (float)scale, bytes ? ws.mutable_data_ptr() : nullptr, bytes, c.stream);
     return out;
   }
 
@@ -707,7 +725,7 @@ struct Rft : torch::autograd::Function<Rft> {
   static tensor_list backward(AutogradContext* ctx, tensor_list g) {
     const auto saved = ctx->get_saved_variables();
     const Tensor& F = saved[0];
-    const Tensor gx = ops_of(ctx)->rft_backward(g[0].contiguous().view({F.size(1), -1, 2}), F);
+    const Tensor gx = ops_of(ctx)->rft_backward(g[0].contiguous().view({F.size(1), -1, 2}), F, 1.0);
     return {Variable(), gx.view(ctx->saved_data["shape"].toIntVector()), Variable(), Variable(), Variable(), Variable()};
   }
 };
@@ -782,7 +800,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("s2_mm_grady", &Ops::s2_mm_grady, "gz"_a, "x"_a, "fo"_a, nogil)
       .def("rft_forward", &Ops::rft_forward, "x"_a, "F"_a, nogil)
       .def("rft_forward_t", &Ops::rft_forward_t, "x"_a, "Ft"_a, nogil)
-      .def("rft_backward", &Ops::rft_backward, "g"_a, "F"_a, nogil)
+      .def("rft_backward", &Ops::rft_backward, "g"_a, "F"_a, "scale"_a = 1.0, nogil)
       .def("so3_integrate", &Ops::so3_integrate, "x"_a, "relu"_a = false, nogil)
       .def("so3_integrate_backward", &Ops::so3_integrate_backward, "g"_a, "b"_a, "x"_a = none, "relu"_a = false, nogil)
       .def("so3_rotate_spectrum", &Ops::so3_rotate_spectrum, "U"_a, "x"_a, "b"_a, "adjoint"_a = false, nogil)
