@@ -171,5 +171,7 @@ def host_module():
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
         mod.set_error_type(S2cError)
+        from .ops import _traced
+        mod.set_traced(_traced)
         _host_module = mod
     return _host_module

@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
 #include <cmath>
@@ -39,6 +40,14 @@ using torch::autograd::Variable;
 // Set as Python exceptions and carried as python_error, so that the type survives the autograd
 // engine (which rethrows the exception of a backward pass in the thread that called it).
 PyObject* g_s2c_error = nullptr;   // s2cnn_b200._lib.S2cError
+PyObject* g_traced = nullptr;      // s2cnn_b200.ops._traced
+// Whether torch.jit.trace is recording this thread's calls, other than within an op that it records as one node.
+thread_local int g_inside_traced_op = 0;
+bool tracing() { return torch::jit::tracer::isTracing() && g_inside_traced_op == 0; }
+struct InsideTracedOp {   // a Python context manager
+  void enter() { ++g_inside_traced_op; }
+  void exit(pybind11::args) { --g_inside_traced_op; }
+};
 
 [[noreturn]] void raise(PyObject* type, const std::string& msg) {
   pybind11::gil_scoped_acquire gil;
@@ -98,7 +107,14 @@ struct Ops {
   }
 
   // -- helpers --------------------------------------------------------------------------------------
+  // These ops write through raw pointers, which neither a tracer (it would record the allocation of the
+  // result and nothing that fills it) nor forward-mode differentiation sees: refused here.  The
+  // differentiable ops are recorded by a tracer as one node each, see S2C_TRACED.
   void prep(const Tensor& t) const {
+    if (tracing())
+      raise(PyExc_RuntimeError, "s2cnn_b200: torch.jit.trace cannot record this op (the differentiable layers and transforms can be traced)");
+    if (t._fw_grad(0).defined())
+      raise(PyExc_NotImplementedError, "s2cnn_b200 ops do not implement forward-mode automatic differentiation (no jvp)");
     if (t.scalar_type() != at::kFloat)
       raise(PyExc_TypeError, std::string("s2cnn_b200 kernels are float32 only, got ") + c10::toString(t.scalar_type()));
     if (t.is_cuda() != is_cuda)
@@ -759,6 +775,17 @@ struct RotateSpectrum : torch::autograd::Function<RotateSpectrum> {
   }
 };
 
+// Under torch.jit.trace an op runs as a Python autograd function (ops._traced), which the tracer records as one
+// node that calls the op again.
+template <class... A>
+Tensor traced(Ops& o, const char* name, const A&... args) {
+  pybind11::gil_scoped_acquire gil;
+  const pybind11::handle fn(g_traced);
+  return fn(pybind11::cast(&o, pybind11::return_value_policy::reference), name, args...).template cast<Tensor>();
+}
+#define S2C_TRACED(name, ...) \
+  if (tracing()) return traced(o, name, __VA_ARGS__)
+
 int64_t id(Ops& o) { return reinterpret_cast<int64_t>(&o); }
 int64_t b_arg(const std::optional<int64_t>& b) { return b ? *b : 0; }
 
@@ -773,6 +800,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       e.restore();
     }
   });
+  pybind11::class_<InsideTracedOp>(m, "InsideTracedOp")
+      .def(pybind11::init<>())
+      .def("__enter__", &InsideTracedOp::enter)
+      .def("__exit__", &InsideTracedOp::exit);
+  m.def("set_traced", [](py::object f) { g_traced = f.release().ptr(); });
   m.def("set_error_type", [](py::object t) { g_s2c_error = t.release().ptr(); });
   using namespace py::literals;
   const auto nogil = py::call_guard<py::gil_scoped_release>();
@@ -807,36 +839,47 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("project_on_sphere", &Ops::project_on_sphere, "verts"_a, "faces"_a, "grid"_a, nogil)
       // -- the same ops with their autograd rules
       .def("ag_s2_fft_real", [](Ops& o, const Tensor& x, std::optional<int64_t> b) {
+            S2C_TRACED("ag_s2_fft_real", x, b);
             return wants_grad(x) ? S2FftReal::apply(id(o), x, b_arg(b)) : o.s2_fft(x, false, b, true);
           }, "x"_a, "b_out"_a = none, nogil)
       .def("ag_s2_ifft_real", [](Ops& o, const Tensor& x, std::optional<int64_t> b) {
+            S2C_TRACED("ag_s2_ifft_real", x, b);
             return wants_grad(x) ? S2IfftReal::apply(id(o), x, b_arg(b)) : o.s2_ifft(x, false, b, true);
           }, "x"_a, "b_out"_a = none, nogil)
       .def("ag_so3_fft_real", [](Ops& o, const Tensor& x, std::optional<int64_t> b, bool relu) {
+            S2C_TRACED("ag_so3_fft_real", x, b, relu);
             return wants_grad(x) ? So3FftReal::apply(id(o), x, b_arg(b), relu) : o.so3_rfft(x, false, b, relu);
           }, "x"_a, "b_out"_a = none, "relu"_a = false, nogil)
       .def("ag_so3_ifft_real", [](Ops& o, const Tensor& x, std::optional<int64_t> b) {
+            S2C_TRACED("ag_so3_ifft_real", x, b);
             return wants_grad(x) ? So3IfftReal::apply(id(o), x, b_arg(b)) : o.so3_rifft(x, false, b, std::nullopt);
           }, "x"_a, "b_out"_a = none, nogil)
       .def("ag_so3_ifft_real_bias", [](Ops& o, const Tensor& x, const Tensor& bias) {
+            S2C_TRACED("ag_so3_ifft_real_bias", x, bias);
             return wants_grad(x, bias) ? So3IfftRealBias::apply(id(o), x, bias) : o.so3_rifft(x, false, std::nullopt, bias);
           }, "x"_a, "bias"_a, nogil)
       .def("ag_s2_product_synthesis", [](Ops& o, const Tensor& x, const Tensor& y, const Tensor& bias) {
+            S2C_TRACED("ag_s2_product_synthesis", x, y, bias);
             return wants_grad(x, y, bias) ? S2ProductSynthesis::apply(id(o), x, y, bias) : o.s2_conv_synthesis(x, y, bias);
           }, "x"_a, "y"_a, "bias"_a, nogil)
       .def("ag_so3_mm", [](Ops& o, const Tensor& x, const Tensor& y) {
+            S2C_TRACED("ag_so3_mm", x, y);
             return wants_grad(x, y) ? SpectralMm<true>::apply(id(o), x, y) : o.so3_mm(x, y);
           }, "x"_a, "y"_a, nogil)
       .def("ag_s2_mm", [](Ops& o, const Tensor& x, const Tensor& y) {
+            S2C_TRACED("ag_s2_mm", x, y);
             return wants_grad(x, y) ? SpectralMm<false>::apply(id(o), x, y) : o.s2_mm(x, y);
           }, "x"_a, "y"_a, nogil)
       .def("ag_rft", [](Ops& o, const Tensor& x, const Tensor& F, const OptTensor& Ft, double scale, const OptTensor& Fg) {
+            S2C_TRACED("ag_rft", x, F, Ft, scale, Fg);
             return wants_grad(x) ? Rft::apply(id(o), x, F, Ft, scale, Fg ? *Fg : F) : o.rft_forward_scaled(x, F, Ft, scale);
           }, "x"_a, "F"_a, "Ft"_a = none, "scale"_a = 1.0, "Fg"_a = none, nogil)
       .def("ag_so3_integrate", [](Ops& o, const Tensor& x, bool relu) {
+            S2C_TRACED("ag_so3_integrate", x, relu);
             return wants_grad(x) ? So3Integrate::apply(id(o), x, relu) : o.so3_integrate(x, relu);
           }, "x"_a, "relu"_a = false, nogil)
       .def("ag_rotate_spectrum", [](Ops& o, const Tensor& x, const Tensor& U, int64_t b) {
+            S2C_TRACED("ag_rotate_spectrum", x, U, b);
             return wants_grad(x) ? RotateSpectrum::apply(id(o), x, U, b) : o.so3_rotate_spectrum(U, x, b, false);
           }, "x"_a, "U"_a, "b"_a, nogil);
 }

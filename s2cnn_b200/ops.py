@@ -14,6 +14,8 @@ reference's autograd rules.
 import logging
 import os
 
+import torch
+
 from . import _lib
 
 
@@ -36,6 +38,32 @@ def _log_new_tables(what, n):
 
 def _flag(name):
     return os.environ.get(name, "0") not in ("", "0")
+
+
+class _Traced(torch.autograd.Function):
+    """One differentiable op inside ``torch.jit.trace``, recorded as a single Python call.  Its backward
+    runs the op again and differentiates that with the op's own rule."""
+
+    @staticmethod
+    def forward(ctx, op, *args):
+        ctx.op, ctx.others = op, [None if isinstance(a, torch.Tensor) else a for a in args]
+        ctx.save_for_backward(*[a if isinstance(a, torch.Tensor) else None for a in args])
+        with _lib.host_module().InsideTracedOp():
+            return op(*args)
+
+    @staticmethod
+    def backward(ctx, grad):
+        args = [o if t is None else t.detach().requires_grad_(need) for t, o, need in
+                zip(ctx.saved_tensors, ctx.others, ctx.needs_input_grad[1:])]
+        with torch.enable_grad():
+            out = ctx.op(*args)
+        wanted = [a for a, need in zip(args, ctx.needs_input_grad[1:]) if need]
+        grads = iter(torch.autograd.grad(out, wanted, grad, allow_unused=True))
+        return (None,) + tuple(next(grads) if need else None for need in ctx.needs_input_grad[1:])
+
+
+def _traced(native, name, *args):
+    return _Traced.apply(getattr(native, name), *args)
 
 
 class Ops:
