@@ -170,6 +170,12 @@ static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, c
   return nbatch >= (N == 22 ? 256 : 600);
 }
 
+// 2b >= 66 with 2b mod 4 = 2: the tiled Wigner kernels stage these panels in small pieces and keep few threads busy on
+// few signals; below these lines (signals x 2b) the untiled ones are the faster ones.  Analysis, tiled / untiled: 1
+// signal b = 45 71 / 53 us, 8 signals b = 39 149 / 139, 32 signals b = 33 259 / 255, b = 39 385 / 386, b = 45
+// 358 / 372; synthesis: 1 signal b = 45 55 / 47, 8 signals b = 33 92 / 88, 16 signals b = 33 146 / 146, b = 45 184 / 189.
+static bool few_for_tiles(int N, long zc, long line) { return N > 64 && N % 4 == 2 && zc * N <= line; }
+
 static int launch_fwd_wigner_col(FwdWignerParams w, stream_t st) {
   w.ZT = std::min(kColZT, (w.nbatch + 31) / 32 * 32);
   w.nzt = (w.nbatch + w.ZT - 1) / w.ZT;
@@ -328,7 +334,7 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
       S2C_TRY(launch_fwd_wigner_col(w, st));
       continue;
     }
-    if (fwd_wigner_t_fits(N, b_out, kWigZT, dev_smem_limit())) {
+    if (!few_for_tiles(N, zc, 2240) && fwd_wigner_t_fits(N, b_out, kWigZT, dev_smem_limit())) {
       w.ZT = kWigZT;
       w.nzt = (int)((zc + kWigZT - 1) / kWigZT);
       S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)pan.npairs * w.nzt, kThreads,
@@ -488,7 +494,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     }
     if (small) {
       S2C_TRY(launch_inv_wigner_col(w, st));
-    } else if (inv_wigner_t_smem(N, K) <= (size_t)dev_smem_limit() - 1024) {
+    } else if (!few_for_tiles(N, zc, 800) && inv_wigner_t_smem(N, K) <= (size_t)dev_smem_limit() - 1024) {
       w.ZT = kWigZT;
       w.nzt = (int)((zc + kWigZT - 1) / kWigZT);
       S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)pan.npairs * w.nzt, kThreads,

@@ -337,10 +337,16 @@ struct so3_fwd_wigner_r_impl {
           for (int jj = 0; jj < JL; ++jj) {
             const float a = va[r][jj], b = vb[r][jj], sa = sl * a, sb = sl * b;
             // X_{+m} = sum A Vp_{+m} + s B Vq_{+m};   X_{-m} = sum B Vp_{-m} + s A Vq_{-m}
-            xp = fma2(make_float2(a, a), vp[0][z][jj], xp);
-            xp = fma2(make_float2(sb, sb), vq[0][z][jj], xp);
-            xq = fma2(make_float2(b, b), vp[1][z][jj], xq);
-            xq = fma2(make_float2(sa, sa), vq[1][z][jj], xq);
+            // (packed multiply-adds for two betas per lane only: with one, 64 signals at b = 32, 29 degrees, took
+            // 163 us packed and 148 scalar)
+            auto mul_add = [](float w, float2 v, float2 acc) {
+              if constexpr (JL == 1) return make_float2(fmaf(w, v.x, acc.x), fmaf(w, v.y, acc.y));
+              else return fma2(make_float2(w, w), v, acc);
+            };
+            xp = mul_add(a, vp[0][z][jj], xp);
+            xp = mul_add(sb, vq[0][z][jj], xp);
+            xq = mul_add(b, vp[1][z][jj], xq);
+            xq = mul_add(sa, vq[1][z][jj], xq);
           }
           val[r * 16 + 0 * 8 + z * 2 + 0] = xp.x;
           val[r * 16 + 0 * 8 + z * 2 + 1] = xp.y;
