@@ -81,6 +81,11 @@ int s2c_so3_ft_matrix(int b, const double* grid, int n_grid, float* F);
  * holds at least one batch element works (the batch is processed in chunks). */
 size_t s2c_so3_fft_workspace(long nbatch, int b_in, int b_out);
 size_t s2c_so3_fft_workspace_min(int b_in, int b_out);
+/* What one call uses in full: b_in, b_out as in its own arguments, 0 where the kernels that such a batch takes
+ * need no scratch (NULL may then be passed).  Analysis: s2c_so3_rfft, _rfft_relu, _rfft_sums_ws, _fft;
+ * synthesis: s2c_so3_rifft, _rifft_relu_grad_ws, _ifft. */
+size_t s2c_so3_analysis_workspace(long nbatch, int b_in, int b_out);
+size_t s2c_so3_synthesis_workspace(long nbatch, int b_in, int b_out);
 
 /* x [nbatch, 2b_in, 2b_in, 2b_in] real -> out [nspec(b_out), nbatch, 2].
  * Replaces so3_rfft, s2cnn/soft/so3_fft.py:64-112 (+ kernel so3fft.cu :246-350, REAL_IN). */
@@ -99,7 +104,7 @@ int s2c_so3_rfft_relu(const float* x, float* out, long nbatch, int b_in, int b_o
  * and write nothing. */
 int s2c_so3_rfft_sums(const float* x, float* out, float* sums, long nbatch, int b_in, int b_out,
                       int for_grad, void* stream);
-/* The same with a workspace (s2c_so3_fft_workspace), for 2 b_in < 64. */
+/* The same with a workspace (s2c_so3_analysis_workspace), for 2 b_in < 64. */
 int s2c_so3_rfft_sums_ws(const float* x, float* out, float* sums, long nbatch, int b_in, int b_out,
                          int for_grad, void* workspace, size_t workspace_bytes, void* stream);
 /* x [nbatch, 2b_in, 2b_in, 2b_in, 2] complex -> out [nspec(b_out), nbatch, 2].
@@ -139,9 +144,11 @@ int s2c_so3_rifft_relu_integrate(const float* x, float* out, long nbatch, int b_
  * and the head of the next SO3Convolution.forward (s2cnn/soft/so3_conv.py:50). */
 int s2c_s2_conv_relu_so3_rfft(const float* xs, const float* ys, float* out, int nbatch, int f_in,
                               int f_out, int b, int b_next, const float* bias, void* stream);
-/* Scratch for the _ws variants of the two fused calls, which hand large batches (2b >= 10) to kernels that
- * work through a workspace; without one (or with too little) the calls above are what runs. */
+/* Scratch for the _ws variants of the two fused calls, which hand large batches at 18 <= 2b <= 32 to kernels
+ * that work through a workspace; 0 where the call takes other kernels.  Without one (or with too little) the
+ * calls above are what runs. */
 size_t s2c_so3_relay_workspace(long nbatch, int b_in, int b_mid, int b_next);
+size_t s2c_s2_conv_relu_so3_rfft_workspace(int nbatch, int f_out, int b, int b_next);
 int s2c_s2_conv_relu_so3_rfft_ws(const float* xs, const float* ys, float* out, int nbatch, int f_in,
                                  int f_out, int b, int b_next, const float* bias, void* workspace,
                                  size_t workspace_bytes, void* stream);

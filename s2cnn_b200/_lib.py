@@ -38,12 +38,15 @@ _SIGNATURES = {
     "s2c_s2_ft_matrix": (c_int, [c_int, _P, c_int, _P]),
     "s2c_so3_ft_matrix": (c_int, [c_int, _P, c_int, _P]),
     "s2c_so3_fft_workspace": (c_size_t, [c_long, c_int, c_int]),
+    "s2c_so3_analysis_workspace": (c_size_t, [c_long, c_int, c_int]),
+    "s2c_so3_synthesis_workspace": (c_size_t, [c_long, c_int, c_int]),
     "s2c_so3_fft_workspace_min": (c_size_t, [c_int, c_int]),
     "s2c_so3_rfft": (c_int, [_P, _P, c_long, c_int, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_rfft_relu": (c_int, [_P, _P, c_long, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_rfft_sums_ws": (c_int, [_P, _P, _P, c_long, c_int, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_rifft_relu_grad_ws": (c_int, [_P, _P, _P, c_long, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_relay_workspace": (c_size_t, [c_long, c_int, c_int, c_int]),
+    "s2c_s2_conv_relu_so3_rfft_workspace": (c_size_t, [c_int, c_int, c_int, c_int]),
     "s2c_s2_conv_relu_so3_rfft_ws": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, c_size_t, _P]),
     "s2c_so3_rifft_relu_rfft_ws": (c_int, [_P, _P, c_long, c_int, c_int, c_int, _P, c_int, _P, c_size_t, _P]),
     "s2c_so3_rfft_sums": (c_int, [_P, _P, _P, c_long, c_int, c_int, c_int, _P]),

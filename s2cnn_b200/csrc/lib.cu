@@ -176,6 +176,53 @@ static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, c
 // 358 / 372; synthesis: 1 signal b = 45 55 / 47, 8 signals b = 33 92 / 88, 16 signals b = 33 146 / 146, b = 45 184 / 189.
 static bool few_for_tiles(int N, long zc, long line) { return N > 64 && N % 4 == 2 && zc * N <= line; }
 
+// Which kernels a transform takes: one rule for the dispatcher and for the workspace queries.
+//   cluster, walking: one kernel, no workspace          planes: so3_small_kernels.h, 18 <= 2b <= 32
+//   mid: so3_mid_kernels.h, 32 < 2b < 64                rows: 2b = 64, 128            passes: any other size
+enum So3Route { kCluster, kWalking, kPlanes, kMid, kRows, kPasses };
+// rows (m, n, l) of the table panels: degrees below nl, |m|, |n| < K, one of each mirror pair
+static int panel_rows(int nl, int K) {
+  const long all = so3_nspec(K) + (long)(nl - K) * (2 * K - 1) * (2 * K - 1);
+  return (int)((all - nl) / 2 + nl);
+}
+static bool has_smem(size_t bytes) { return bytes <= (size_t)dev_smem_limit() - 1024; }
+static So3Route big_route(int N) { return use_plane_kernels(N) ? kRows : use_mid_kernels(N) ? kMid : kPasses; }
+static So3Route analysis_route(int N, int K, int nl, long nbatch, const void* ws, size_t ws_bytes) {
+  if (so3_prefers_planes(kClAnalysis, N, K, nl, nbatch, ws, ws_bytes)) return kPlanes;
+  if (!g_force_general && N <= kFusedMaxN) {
+    if (nl <= kFusedMaxDegrees && so3_prefers_cluster(kClAnalysis, N, nbatch)) return kCluster;
+    if (has_smem(fwd_fused_smem_bytes(N, panel_rows(nl, K)))) return kWalking;
+  }
+  return big_route(N);
+}
+// `one_kernel`: a synthesis that writes no signal (its integral)
+static So3Route synthesis_route(int N, int K, long nbatch, const void* ws, size_t ws_bytes, bool product = false,
+                                bool one_kernel = false) {
+  if (!one_kernel && so3_prefers_planes(kClSynthesis, N, K, K, nbatch, ws, ws_bytes, product)) return kPlanes;
+  if (!g_force_general && N <= kFusedMaxN) {
+    if (so3_prefers_cluster(kClSynthesis, N, nbatch)) return kCluster;
+    if (has_smem(fused_smem_bytes(N, panel_rows(K, K)))) return kWalking;
+  }
+  return big_route(N);
+}
+static bool relay_takes_planes(int N, int Kin, int Kout, long nbatch, const void* ws, size_t ws_bytes, bool product) {
+  return so3_prefers_planes(kClRelay, N, Kin, Kout, nbatch, ws, ws_bytes, product) &&
+         ws_bytes >= (so3_mid_v_per_z(N, Kin) + so3_mid_v_per_z(N, Kout)) * (size_t)std::min<long>(kWigZT, nbatch);
+}
+// a workspace that no route finds too small, for the queries
+static const void* const kAnyWorkspace = (const void*)16;
+constexpr size_t kAnySize = ~(size_t)0 / 2;
+// scratch that a route uses up in full (every transform also works with less, in shorter chunks)
+static size_t route_workspace(So3Route r, int N, int K, long nbatch) {
+  if (r == kPlanes || r == kMid) return so3_mid_v_per_z(N, K) * (size_t)chunk_signals(nbatch, so3_mid_v_per_z(N, K));
+  if (r == kRows) return so3_v_per_z(N, K) * (size_t)std::min<long>(kRowsZC, nbatch);
+  if (r == kPasses) {
+    const size_t per_z = so3_ws_per_z(N, K);
+    return per_z * (size_t)std::min((long)std::max<size_t>(32, ((size_t)256 << 20) / per_z), nbatch);
+  }
+  return 0;
+}
+
 static int launch_fwd_wigner_col(FwdWignerParams w, stream_t st) {
   w.ZT = std::min(kColZT, (w.nbatch + 31) / 32 * 32);
   w.nzt = (w.nbatch + w.ZT - 1) / w.ZT;
@@ -207,9 +254,9 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
   S2C_TRY(TableCache::get().panels(b_in, b_out, K, weighted, false, pan));
   if (b_out > b_in && mode == kSo3Real)  // rows with |m| or |n| >= b_in stay zero (so3_fft.py:44-48)
     S2C_TRY(dev_memset_async(out, 0, (size_t)so3_nspec(b_out) * nbatch * sizeof(float2), st));
-  const bool small = so3_prefers_planes(kClAnalysis, N, K, b_out, nbatch, ws, ws_bytes);
-  if (!small && !g_force_general && N <= kFusedMaxN && b_out <= kFusedMaxDegrees &&
-      so3_prefers_cluster(kClAnalysis, N, nbatch)) {
+  const So3Route route = analysis_route(N, K, b_out, nbatch, ws, ws_bytes);
+  const bool small = route == kPlanes, mid = small || route == kMid;
+  if (route == kCluster) {
     ClFwdParams f;
     f.x = x; f.in_stride = in_stride; f.in_off = in_off;
     f.out = out; f.out_zstride = nbatch;
@@ -223,8 +270,7 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
                                          cl_smem_bytes(N, K, 0), st, f));
     return rc;
   }
-  if (!small && !g_force_general && N <= kFusedMaxN &&
-      fwd_fused_smem_bytes(N, pan.nrows) <= (size_t)dev_smem_limit() - 1024) {
+  if (route == kWalking) {
     FwdFusedParams f;
     f.x = x; f.in_stride = in_stride; f.in_off = in_off;
     f.out = out; f.out_zstride = nbatch;
@@ -240,9 +286,9 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
                                         fused_threads(sm, (size_t)dev_smem_limit()), sm, st, f));
     return rc;
   }
-  if (relu && !small && !use_mid_kernels(N)) return fail(S2C_ERR_UNSUPPORTED, "fused ReLU input needs 2 b < 64");
-  if (sums && !small && (!use_mid_kernels(N) || !ws)) return fail(S2C_ERR_UNSUPPORTED, "per-signal sums need 2 b < 64");
-  if (use_plane_kernels(N)) {
+  if (relu && !mid) return fail(S2C_ERR_UNSUPPORTED, "fused ReLU input needs 2 b < 64");
+  if (sums && (!mid || !ws)) return fail(S2C_ERR_UNSUPPORTED, "per-signal sums need 2 b < 64");
+  if (route == kRows) {
     HalfPanelsDev hp;
     hp.nbeta = N; hp.nl = b_out; hp.K = K; hp.npairs = pan.npairs;
     S2C_TRY(TableCache::get().half_panels(b_in, b_out, K, weighted, &hp.data, &hp.off));
@@ -261,7 +307,6 @@ static int so3_analysis(const float* x, long in_stride, long in_off, float2* out
     };
     return plane_pipeline(nbatch, N, K, ws, ws_bytes, st, planes, wigner);
   }
-  const bool mid = small || use_mid_kernels(N);
   const size_t per_z = so3_ws_per_z(N, K);
   long chunk = (long)std::min<size_t>((size_t)nbatch, ws_bytes / per_z);
   if (mid) {
@@ -360,8 +405,7 @@ struct S2ProductArgs {
 static bool so3_synthesis_is_fused(int b_in, int b_out) {
   const int N = 2 * b_out, K = std::min(b_in, b_out);
   if (g_force_general || N > kFusedMaxN) return false;
-  const int nrows = (so3_nspec(K) - K) / 2 + K;  // half-plane rows: the (0,0) pair is its own mirror
-  return fused_smem_bytes(N, nrows) <= (size_t)dev_smem_limit() - 1024;
+  return has_smem(fused_smem_bytes(N, panel_rows(K, K)));
 }
 
 static int so3_synthesis(const float2* x, float* out, long out_stride, long out_off, long nbatch,
@@ -374,9 +418,11 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
   PanelsDev pan;
   S2C_TRY(TableCache::get().fft(N, fft));
   S2C_TRY(TableCache::get().panels(b_out, K, K, weighted, false, pan));
-  const bool small = !integral && so3_prefers_planes(kClSynthesis, N, K, K, nbatch, ws, ws_bytes, prod != nullptr) &&
-                     (!mask || (out_stride == 1 && out_off == 0));
-  if (!small && !g_force_general && N <= kFusedMaxN && so3_prefers_cluster(kClSynthesis, N, nbatch)) {
+  const So3Route route = synthesis_route(N, K, nbatch, ws, ws_bytes, prod != nullptr, integral != nullptr);
+  const bool small = route == kPlanes, mid = small || route == kMid;
+  if (mask && (out_stride != 1 || out_off != 0))
+    return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output only");
+  if (route == kCluster) {
     ClInvParams f;
     f.in.x = x; f.in.x_zstride = nbatch; f.in.mode = mode;
     f.in.xs = f.in.ys = nullptr; f.in.s2_nb = f.in.s2_fin = f.in.s2_fout = 0;
@@ -386,8 +432,6 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     f.nbatch = (int)nbatch; f.K = K;
     f.iw = nullptr; f.isum = nullptr;
     f.mask = mask;
-    if (mask && (out_stride != 1 || out_off != 0))
-      return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output only");
     f.wide = out_stride == 1 && out_off == 0 && N % 4 == 0 && out && (uintptr_t)out % 32 == 0 &&
              (uintptr_t)mask % 32 == 0;
     if (integral) {
@@ -404,8 +448,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
                                          cl_smem_bytes(N, K, f.tab.max_rows), st, f));
     return rc;
   }
-  if (!small && !g_force_general && N <= kFusedMaxN &&
-      fused_smem_bytes(N, pan.nrows) <= (size_t)dev_smem_limit() - 1024) {
+  if (route == kWalking) {
     InvFusedParams f;
     f.x = x; f.x_zstride = nbatch;
     f.out = out; f.out_stride = out_stride; f.out_off = out_off;
@@ -416,8 +459,6 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     f.xs = nullptr; f.ys = nullptr; f.s2_nb = f.s2_fin = f.s2_fout = 0;
     f.iw = nullptr; f.isum = nullptr;
     f.mask = mask;
-    if (mask && (out_stride != 1 || out_off != 0))
-      return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output only");
     f.wide = out_stride == 1 && out_off == 0 && N % 4 == 0 && out && (uintptr_t)out % 32 == 0 &&
              (uintptr_t)mask % 32 == 0;
     if (integral) {
@@ -440,9 +481,8 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
   }
   if (integral)
     return fail(S2C_ERR_UNSUPPORTED, "fused ReLU + integration needs the small-bandwidth path");
-  if (mask && !small && (!use_mid_kernels(N) || !ws || out_stride != 1 || out_off != 0))
-    return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output and 2 b < 64");
-  if (use_plane_kernels(N)) {
+  if (mask && (!mid || !ws)) return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output and 2 b < 64");
+  if (route == kRows) {
     HalfPanelsDev hp;
     hp.nbeta = N; hp.nl = K; hp.K = K; hp.npairs = pan.npairs;
     S2C_TRY(TableCache::get().half_panels(b_out, K, K, weighted, &hp.data, &hp.off));
@@ -463,7 +503,6 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     };
     return plane_pipeline(nbatch, N, K, ws, ws_bytes, st, wigner, planes);
   }
-  const bool mid = small || use_mid_kernels(N);
   const size_t per_z = so3_ws_per_z(N, K);
   long chunk = (long)std::min<size_t>((size_t)nbatch, ws_bytes / per_z);
   if (mid) {
@@ -745,6 +784,17 @@ size_t s2c_so3_fft_workspace(long nbatch, int b_in, int b_out) {
   return per_z * (size_t)chunk;
 }
 
+size_t s2c_so3_analysis_workspace(long nbatch, int b_in, int b_out) {
+  if (nbatch < 1 || b_in < 1 || b_out < 1) return 0;
+  const int N = 2 * b_in, K = std::min(b_in, b_out);
+  return route_workspace(analysis_route(N, K, b_out, nbatch, kAnyWorkspace, kAnySize), N, K, nbatch);
+}
+size_t s2c_so3_synthesis_workspace(long nbatch, int b_in, int b_out) {
+  if (nbatch < 1 || b_in < 1 || b_out < 1) return 0;
+  const int N = 2 * b_out, K = std::min(b_in, b_out);
+  return route_workspace(synthesis_route(N, K, nbatch, kAnyWorkspace, kAnySize), N, K, nbatch);
+}
+
 int s2c_so3_rfft(const float* x, float* out, long nbatch, int b_in, int b_out, int for_grad,
                  void* ws, size_t ws_bytes, void* stream) {
   S2C_TRY(check_b(b_in, b_out));
@@ -857,8 +907,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
     return fail(S2C_ERR_UNSUPPORTED,
                 std::string(who) + ": needs 2 b <= 32, b_in <= b and b_next <= b");
   const size_t v1 = so3_mid_v_per_z(N, b_in), v2 = so3_mid_v_per_z(N, b_next);
-  if (so3_prefers_planes(kClRelay, N, b_in, b_next, nz, ws, ws_bytes, xs != nullptr) &&
-      ws_bytes >= (v1 + v2) * (size_t)std::min<long>(kWigZT, nz)) {
+  if (relay_takes_planes(N, b_in, b_next, nz, ws, ws_bytes, xs != nullptr)) {
     PanelsDev pin, pout;
     S2C_TRY(TableCache::get().panels(b_mid, b_in, b_in, false, false, pin));
     S2C_TRY(TableCache::get().panels(b_mid, b_next, b_next, true, false, pout));
@@ -925,10 +974,19 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
   return rc;
 }
 
+static size_t relay_workspace(long nbatch, int b_in, int b_mid, int b_next, bool product) {
+  const int N = 2 * b_mid;
+  if (nbatch < 1 || b_in < 1 || b_next < 1 || N > kFusedMaxN || b_in > b_mid || b_next > b_mid ||
+      !relay_takes_planes(N, b_in, b_next, nbatch, kAnyWorkspace, kAnySize, product))
+    return 0;
+  const size_t v = so3_mid_v_per_z(N, b_in) + so3_mid_v_per_z(N, b_next);
+  return v * (size_t)chunk_signals(nbatch, v);
+}
 size_t s2c_so3_relay_workspace(long nbatch, int b_in, int b_mid, int b_next) {
-  if (!small_supported(2 * b_mid) || b_in < 1 || b_next < 1) return 16;
-  const size_t v = so3_mid_v_per_z(2 * b_mid, b_in) + so3_mid_v_per_z(2 * b_mid, b_next);
-  return v * (size_t)chunk_signals(std::max(1L, nbatch), v);
+  return relay_workspace(nbatch, b_in, b_mid, b_next, false);
+}
+size_t s2c_s2_conv_relu_so3_rfft_workspace(int nbatch, int f_out, int b, int b_next) {
+  return relay_workspace((long)nbatch * f_out, b, b, b_next, true);
 }
 
 int s2c_s2_conv_relu_so3_rfft_ws(const float* xs, const float* ys, float* out, int nbatch, int f_in,
@@ -970,10 +1028,11 @@ static bool s2_product_in_wigner(int b) {
 }
 
 size_t s2c_s2_conv_synthesis_workspace(int nbatch, int f_out, int b) {
-  if (so3_synthesis_is_fused(b, b))
-    return small_supported(2 * b) ? s2c_so3_fft_workspace((long)nbatch * f_out, b, b) : 16;
-  const size_t z_bytes = (size_t)so3_nspec(b) * nbatch * f_out * sizeof(float2);
-  return z_bytes + s2c_so3_fft_workspace((long)nbatch * f_out, b, b);
+  if (nbatch < 1 || f_out < 1 || b < 1) return 0;
+  const long nz = (long)nbatch * f_out;
+  const bool product = so3_synthesis_is_fused(b, b) || s2_product_in_wigner(b);
+  const size_t z_bytes = product ? 0 : (size_t)so3_nspec(b) * nz * sizeof(float2);
+  return z_bytes + route_workspace(synthesis_route(2 * b, b, nz, kAnyWorkspace, kAnySize, product), 2 * b, b, nz);
 }
 
 int s2c_s2_conv_synthesis(const float* xs, const float* ys, float* out, int nbatch, int f_in,

@@ -76,8 +76,8 @@ long s2_bandwidth(long nspec) {
 
 // ---- one build of the library ---------------------------------------------------------------------
 #define S2C_API(X)                                                                                 \
-  X(last_error) X(is_cuda_build) X(tables_computed) X(so3_fft_workspace) X(so3_rfft)               \
-  X(so3_rfft_relu) X(so3_rfft_sums_ws) X(so3_relay_workspace) X(s2_conv_relu_so3_rfft_ws) X(so3_rifft_relu_rfft_ws) X(so3_rifft_relu_grad_ws) X(so3_fft) X(so3_rifft)                 \
+  X(last_error) X(is_cuda_build) X(tables_computed) X(so3_analysis_workspace) X(so3_synthesis_workspace) X(so3_rfft)               \
+  X(so3_rfft_relu) X(so3_rfft_sums_ws) X(so3_relay_workspace) X(s2_conv_relu_so3_rfft_workspace) X(s2_conv_relu_so3_rfft_ws) X(so3_rifft_relu_rfft_ws) X(so3_rifft_relu_grad_ws) X(so3_fft) X(so3_rifft)                 \
   X(so3_rifft_relu_integrate)                      \
   X(s2_conv_synthesis_workspace) X(s2_conv_synthesis) X(so3_ifft) X(s2_fft_workspace) X(s2_fft)    \
   X(s2_ifft) X(so3_mm) X(so3_mm_gradx_ws) X(so3_mm_gradx_workspace) X(so3_mm_grady_ws) X(so3_mm_grady_workspace) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
@@ -183,9 +183,17 @@ struct Ops {
     return s;
   }
   static Tensor empty_like_shape(const Tensor& like, at::IntArrayRef shape) { return at::empty(shape, like.options()); }
-  static Tensor workspace(size_t bytes, const Tensor& like) {
-    return at::empty({(int64_t)(bytes < 16 ? 16 : bytes)}, like.options().dtype(at::kByte));
-  }
+  // scratch space of one call; none where the kernels it will take need none
+  struct Scratch {
+    Tensor keep;
+    void* p = nullptr;
+    size_t n = 0;
+    Scratch(size_t bytes, const Tensor& like) : n(bytes) {
+      if (!bytes) return;
+      keep = at::empty({(int64_t)bytes}, like.options().dtype(at::kByte));
+      p = keep.mutable_data_ptr();
+    }
+  };
   // bias -> (contiguous flat tensor kept alive, pointer, count); the feature axis is the last of `lead`
   static const float* bias_ptr(const OptTensor& bias, Tensor& keep, int& nfeat) {
     nfeat = 0;
@@ -216,12 +224,12 @@ struct Ops {
     const long nb = lead_numel(lead);
     Tensor out = empty_like_shape(x, spectrum_shape(so3_nspec(b_out), lead));
     Ctx c(*this, x);
-    const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
+    const Scratch ws(so3_analysis_workspace_(nb, b_in, b_out), x);
     if (relu) {
       check(!for_grad, "so3_rfft: relu goes with the forward weighting");
-      S2C_CALL(so3_rfft_relu, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+      S2C_CALL(so3_rfft_relu, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, ws.p, ws.n, c.stream);
     } else {
-      S2C_CALL(so3_rfft, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+      S2C_CALL(so3_rfft, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, ws.p, ws.n, c.stream);
     }
     log_new_tables("so3_rfft", b_in, b_out);
     return out;
@@ -237,9 +245,9 @@ struct Ops {
       Tensor out = empty_like_shape(x, spectrum_shape(so3_nspec(b_out), lead));
       Tensor sums = empty_like_shape(x, lead);
       Ctx c(*this, x);
-      const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
+      const Scratch ws(so3_analysis_workspace_(nb, b_in, b_out), x);
       const int rc = call_rc("s2c_so3_rfft_sums_ws", so3_rfft_sums_ws_, cptr(x), ptr(out), ptr(sums), nb, (int)b_in,
-                             (int)b_out, (int)for_grad, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+                             (int)b_out, (int)for_grad, ws.p, ws.n, c.stream);
       if (rc == 0) {
         log_new_tables("so3_rfft", b_in, b_out);
         return {out, sums};
@@ -259,8 +267,8 @@ struct Ops {
     const long nb = lead_numel(lead);
     Tensor out = empty_like_shape(x, spectrum_shape(so3_nspec(b_out), lead));
     Ctx c(*this, x);
-    const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
-    S2C_CALL(so3_fft, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(so3_analysis_workspace_(nb, b_in, b_out), x);
+    S2C_CALL(so3_fft, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -277,8 +285,8 @@ struct Ops {
     const float* bp = bias_ptr(bias, keep, nfeat);
     check(!bp || (!lead.empty() && lead.back() == nfeat), "so3_rifft: one bias per feature (last leading axis)");
     Ctx c(*this, x);
-    const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
-    S2C_CALL(so3_rifft, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, bp, nfeat, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(so3_synthesis_workspace_(nb, b_in, b_out), x);
+    S2C_CALL(so3_rifft, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, bp, nfeat, ws.p, ws.n, c.stream);
     log_new_tables("so3_rifft", b_in, b_out);
     return out;
   }
@@ -293,8 +301,8 @@ struct Ops {
     Tensor out = at::empty_like(act);
     Ctx c(*this, x);
     const long nb = lead_numel(lead);
-    const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
-    S2C_CALL(so3_rifft_relu_grad_ws, cptr(x), cptr(act), ptr(out), nb, (int)b_in, (int)b_out, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(so3_synthesis_workspace_(nb, b_in, b_out), x);
+    S2C_CALL(so3_rifft_relu_grad_ws, cptr(x), cptr(act), ptr(out), nb, (int)b_in, (int)b_out, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -333,8 +341,8 @@ struct Ops {
     check(!bp || nfeat == d.fo, "s2_conv_relu_so3_rfft: one bias per output feature");
     Tensor out = empty_like_shape(xs, {so3_nspec(b_next), d.nb, d.fo, 2});
     Ctx c(*this, xs);
-    const Tensor ws = workspace(so3_relay_workspace_(d.nb * d.fo, (int)d.b, (int)d.b, (int)b_next), xs);
-    S2C_CALL(s2_conv_relu_so3_rfft_ws, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, (int)b_next, bp, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(s2_conv_relu_so3_rfft_workspace_((int)d.nb, (int)d.fo, (int)d.b, (int)b_next), xs);
+    S2C_CALL(s2_conv_relu_so3_rfft_ws, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, (int)b_next, bp, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -352,8 +360,8 @@ struct Ops {
     Tensor out = empty_like_shape(x, spectrum_shape(so3_nspec(b_next), lead));
     Ctx c(*this, x);
     const long nb = lead_numel(lead);
-    const Tensor ws = workspace(so3_relay_workspace_(nb, (int)b_in, (int)b_mid, (int)b_next), x);
-    S2C_CALL(so3_rifft_relu_rfft_ws, cptr(x), ptr(out), nb, (int)b_in, (int)b_mid, (int)b_next, bp, nfeat, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(so3_relay_workspace_(nb, (int)b_in, (int)b_mid, (int)b_next), x);
+    S2C_CALL(so3_rifft_relu_rfft_ws, cptr(x), ptr(out), nb, (int)b_in, (int)b_mid, (int)b_next, bp, nfeat, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -368,8 +376,8 @@ struct Ops {
     const long n = 2 * d.b;
     Tensor out = empty_like_shape(xs, {d.nb, d.fo, n, n, n});
     Ctx c(*this, xs);
-    const Tensor ws = workspace(s2_conv_synthesis_workspace_((int)d.nb, (int)d.fo, (int)d.b), xs);
-    S2C_CALL(s2_conv_synthesis, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, bp, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(s2_conv_synthesis_workspace_((int)d.nb, (int)d.fo, (int)d.b), xs);
+    S2C_CALL(s2_conv_synthesis, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, bp, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -382,8 +390,8 @@ struct Ops {
     const long nb = lead_numel(lead);
     Tensor out = empty_like_shape(x, signal_shape(lead, 2 * b_out, 3, true));
     Ctx c(*this, x);
-    const Tensor ws = workspace(so3_fft_workspace_(nb, b_in, b_out), x);
-    S2C_CALL(so3_ifft, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(so3_synthesis_workspace_(nb, b_in, b_out), x);
+    S2C_CALL(so3_ifft, cptr(x), ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -401,8 +409,8 @@ struct Ops {
     const long nb = lead_numel(lead);
     Tensor out = empty_like_shape(x, spectrum_shape(b_out * b_out, lead));
     Ctx c(*this, x);
-    const Tensor ws = workspace(s2_fft_workspace_(nb, b_in, b_out), x);
-    S2C_CALL(s2_fft, cptr(x), (int)x_is_real, ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(s2_fft_workspace_(nb, b_in, b_out), x);
+    S2C_CALL(s2_fft, cptr(x), (int)x_is_real, ptr(out), nb, (int)b_in, (int)b_out, (int)for_grad, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -416,8 +424,8 @@ struct Ops {
     const long nb = lead_numel(lead);
     Tensor out = empty_like_shape(x, signal_shape(lead, 2 * b_out, 2, !out_is_real));
     Ctx c(*this, x);
-    const Tensor ws = workspace(s2_fft_workspace_(nb, b_in, b_out), x);
-    S2C_CALL(s2_ifft, cptr(x), ptr(out), (int)out_is_real, nb, (int)b_in, (int)b_out, (int)for_grad, ws.mutable_data_ptr(), (size_t)ws.numel(), c.stream);
+    const Scratch ws(s2_fft_workspace_(nb, b_in, b_out), x);
+    S2C_CALL(s2_ifft, cptr(x), ptr(out), (int)out_is_real, nb, (int)b_in, (int)b_out, (int)for_grad, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -441,10 +449,8 @@ struct Ops {
     const Tensor a = a_.contiguous(), b = b_.contiguous();
     Tensor out = empty_like_shape(a, shape);
     Ctx c(*this, a);
-    const size_t bytes = workspace_bytes((int)nl, (int)nb, (int)fi, (int)fo);
-    Tensor ws;
-    if (bytes) ws = workspace(bytes, a);
-    call(name, fn, cptr(a), cptr(b), ptr(out), (int)nl, (int)nb, (int)fi, (int)fo, bytes ? ws.mutable_data_ptr() : nullptr, bytes, c.stream);
+    const Scratch ws(workspace_bytes((int)nl, (int)nb, (int)fi, (int)fo), a);
+    call(name, fn, cptr(a), cptr(b), ptr(out), (int)nl, (int)nb, (int)fi, (int)fo, ws.p, ws.n, c.stream);
     if (check_tc) check_tensor_core_status();
     return out;
   }
@@ -534,10 +540,8 @@ struct Ops {
     const Tensor g = g_.contiguous(), F = F_.contiguous();
     Tensor out = empty_like_shape(g, {nf, ng});
     Ctx c(*this, g);
-    const size_t bytes = rft_backward_workspace_((int)nf, (int)ng, (int)ns);
-    Tensor ws;
-    if (bytes) ws = workspace(bytes, g);
-    S2C_CALL(rft_backward_scaled, cptr(g), cptr(F), ptr(out), (int)nf, (int)ng, (int)ns, (float)scale, bytes ? ws.mutable_data_ptr() : nullptr, bytes, c.stream);
+    const Scratch ws(rft_backward_workspace_((int)nf, (int)ng, (int)ns), g);
+    S2C_CALL(rft_backward_scaled, cptr(g), cptr(F), ptr(out), (int)nf, (int)ng, (int)ns, (float)scale, ws.p, ws.n, c.stream);
     return out;
   }
 
