@@ -734,19 +734,20 @@ struct SpectralMm : torch::autograd::Function<SpectralMm<SO3>> {
   }
 };
 // scale * kernel [..., n_grid] -> [nspec, ..., 2]: the einsum of s2cnn/s2_ft.py:22 and s2cnn/so3_ft.py:22,
-// with the layers' constant scaling of the kernel; `Fg` is the matrix of the gradient (scale * F)
+// with the layers' constant scaling of the kernel
 struct Rft : torch::autograd::Function<Rft> {
-  static Tensor forward(AutogradContext* ctx, int64_t ops, const Tensor& x, const Tensor& F, const OptTensor& Ft, double scale, const Tensor& Fg) {
+  static Tensor forward(AutogradContext* ctx, int64_t ops, const Tensor& x, const Tensor& F, const OptTensor& Ft, double scale) {
     keep_ops(ctx, ops);
-    ctx->save_for_backward({Fg});
+    ctx->save_for_backward({F});
     ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["scale"] = scale;
     return reinterpret_cast<Ops*>(ops)->rft_forward_scaled(x, F, Ft, scale);
   }
   static tensor_list backward(AutogradContext* ctx, tensor_list g) {
     const auto saved = ctx->get_saved_variables();
     const Tensor& F = saved[0];
-    const Tensor gx = ops_of(ctx)->rft_backward(g[0].contiguous().view({F.size(1), -1, 2}), F, 1.0);
-    return {Variable(), gx.view(ctx->saved_data["shape"].toIntVector()), Variable(), Variable(), Variable(), Variable()};
+    const Tensor gx = ops_of(ctx)->rft_backward(g[0].contiguous().view({F.size(1), -1, 2}), F, ctx->saved_data["scale"].toDouble());
+    return {Variable(), gx.view(ctx->saved_data["shape"].toIntVector()), Variable(), Variable(), Variable()};
   }
 };
 // s2cnn/soft/so3_integrate.py:7-29, optionally of max(x, 0)
@@ -874,10 +875,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
             S2C_TRACED("ag_s2_mm", x, y);
             return wants_grad(x, y) ? SpectralMm<false>::apply(id(o), x, y) : o.s2_mm(x, y);
           }, "x"_a, "y"_a, nogil)
-      .def("ag_rft", [](Ops& o, const Tensor& x, const Tensor& F, const OptTensor& Ft, double scale, const OptTensor& Fg) {
-            S2C_TRACED("ag_rft", x, F, Ft, scale, Fg);
-            return wants_grad(x) ? Rft::apply(id(o), x, F, Ft, scale, Fg ? *Fg : F) : o.rft_forward_scaled(x, F, Ft, scale);
-          }, "x"_a, "F"_a, "Ft"_a = none, "scale"_a = 1.0, "Fg"_a = none, nogil)
+      .def("ag_rft", [](Ops& o, const Tensor& x, const Tensor& F, const OptTensor& Ft, double scale) {
+            S2C_TRACED("ag_rft", x, F, Ft, scale);
+            return wants_grad(x) ? Rft::apply(id(o), x, F, Ft, scale) : o.rft_forward_scaled(x, F, Ft, scale);
+          }, "x"_a, "F"_a, "Ft"_a = none, "scale"_a = 1.0, nogil)
       .def("ag_so3_integrate", [](Ops& o, const Tensor& x, bool relu) {
             S2C_TRACED("ag_so3_integrate", x, relu);
             return wants_grad(x) ? So3Integrate::apply(id(o), x, relu) : o.so3_integrate(x, relu);

@@ -7,9 +7,9 @@ every forward pass (s2cnn/soft/s2_conv.py:41, so3_conv.py:47).
   tensor pass after pass; the cache keeps it while the parameter has not been written to (its version
   counter, storage and device are unchanged) and no gradient with respect to it is being recorded.
   During training the transform runs every time, as autograd needs it in the graph.
-* ``FourierMatrices``: the Fourier matrices of the layer's grid, and the one of the gradient with the
-  layer's constant scaling multiplied in; the forward product scales the kernel while it reads it, so
-  neither ``kernel * scaling`` nor its gradient is a pass of its own.
+* ``FourierMatrices``: the Fourier matrices of the layer's grid; the products scale the kernel while
+  they read it and its gradient while they write it, so neither ``kernel * scaling`` nor its gradient is
+  a pass, or a matrix, of its own.
 
 Each keeps one entry as a single tuple: replaced in one assignment, so a reader in another thread
 never sees half of one entry and half of another.  Copies and pickles of a module start empty.
@@ -46,13 +46,13 @@ class KernelSpectrumCache(_OneEntry):
 
 class FourierMatrices(_OneEntry):
     def get(self, setup, b, grid, scaling, device):
-        """``setup(b, grid, device_type, device_index)`` -> (F, Ft); returns (F, Ft, scaling, scaling * F),
-        the arguments of ``ag_rft``.  The grid (a tuple of hundreds of angles, costly to hash) is
+        """``setup(b, grid, device_type, device_index)`` -> (F, Ft); returns (F, Ft, scaling), the
+        arguments of ``ag_rft``.  The grid (a tuple of hundreds of angles, costly to hash) is
         compared by identity first."""
         entry = self._entry
         key = (b, scaling, device)
         if entry is None or entry[0] is not grid or entry[1] != key:
             F, Ft = setup(b, grid, device_type=device.type, device_index=device.index)
-            entry = (grid, key, (F, Ft, scaling, F * scaling))
+            entry = (grid, key, (F, Ft, scaling))
             self._entry = entry
         return entry[2]
