@@ -26,6 +26,10 @@ class GraphedForward:
         self.graph = torch.cuda.CUDAGraph()
         with torch.no_grad(), torch.cuda.graph(self.graph):
             self.static_out = module(self.static_in)
+        # the graph reads the layers' kept spectra and matrices where they lie: they stay, also when the
+        # module replaces its own (weights written after the capture)
+        self._read = [cache._entry for m in module.modules() for cache in
+                      (getattr(m, "_spectrum_cache", None), getattr(m, "_fourier", None)) if cache is not None]
 
     def __call__(self, x):
         """Copies ``x`` (device or pinned host tensor of the captured shape) into the graph's input

@@ -12,13 +12,42 @@ import torch
 from .ops import cuda_ops
 
 
+def _raw_stream(t):
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
+
+
+def made_on_current_stream(*tensors):
+    """Notes, on tensors that will be kept between calls, the stream they were allocated on."""
+    for t in tensors:
+        if t is not None and t.is_cuda:
+            t._made_on = _raw_stream(t)
+
+
+def read_on_current_stream(*tensors, event=None):
+    """Kept tensors are about to be read on the current stream: where that is not their own it waits
+    for ``event`` (recorded after they were written; None: they were complete before they were kept),
+    and the allocator does not hand their memory on before the reader is done, whoever drops them."""
+    for t in tensors:
+        if t is None or not t.is_cuda or t._made_on == _raw_stream(t):
+            continue
+        if torch.cuda.is_current_stream_capturing():   # the graph keeps them (GraphedForward)
+            continue
+        stream = torch.cuda.current_stream(t.device)
+        if event is not None:
+            stream.wait_event(event)
+        t.record_stream(stream)
+
+
 def fourier_matrices(F_host, device):
-    """(F, Ft) on the device: Ft only for a CUDA device and an even number of grid points (the
-    tensor-core product works on pairs along the contraction)."""
+    """(F, Ft) on the device, complete for every stream: Ft only for a CUDA device and an even number
+    of grid points (the tensor-core product works on pairs along the contraction)."""
     F = torch.from_numpy(F_host).to(device)
     Ft = None
-    if F.is_cuda and F.size(0) % 2 == 0:
-        Ft = F.permute(1, 2, 0).contiguous()
+    if F.is_cuda:
+        if F.size(0) % 2 == 0:
+            Ft = F.permute(1, 2, 0).contiguous()
+            torch.cuda.current_stream(device).synchronize()   # once per grid; the copy above has waited too
+        made_on_current_stream(F, Ft)
     return F, Ft
 
 
@@ -38,4 +67,5 @@ def s2_rft(x, b, grid):
     """
     F, Ft = _setup_s2_ft(b, grid, device_type=x.device.type, device_index=x.device.index)
     assert x.size(-1) == F.size(0)
+    read_on_current_stream(F, Ft)
     return cuda_ops().ag_rft(x, F, Ft)

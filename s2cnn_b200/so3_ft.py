@@ -9,7 +9,7 @@ from functools import lru_cache
 import torch
 
 from .ops import cuda_ops
-from .s2_ft import fourier_matrices
+from .s2_ft import fourier_matrices, read_on_current_stream
 
 
 @lru_cache(maxsize=32)
@@ -28,4 +28,5 @@ def so3_rft(x, b, grid):
     """
     F, Ft = _setup_so3_ft(b, grid, device_type=x.device.type, device_index=x.device.index)
     assert x.size(-1) == F.size(0)
+    read_on_current_stream(F, Ft)
     return cuda_ops().ag_rft(x, F, Ft)

@@ -13,8 +13,15 @@ every forward pass (s2cnn/soft/s2_conv.py:41, so3_conv.py:47).
 
 Each keeps one entry as a single tuple: replaced in one assignment, so a reader in another thread
 never sees half of one entry and half of another.  Copies and pickles of a module start empty.
+
+Passes may run on any stream: a spectrum is read elsewhere only after the event that follows its
+making, and the allocator learns which streams read a kept tensor (``s2_ft.read_on_current_stream``).
+A pass under capture reads what was there before (``torch.cuda.graph`` synchronizes the device before
+it captures) and leaves nothing: what it makes itself is filled by the replays only.
 """
 import torch
+
+from ..s2_ft import made_on_current_stream, read_on_current_stream
 
 
 class _OneEntry:
@@ -37,11 +44,19 @@ class KernelSpectrumCache(_OneEntry):
             return transform(kernel)
         key = (kernel._version, kernel.data_ptr(), kernel.device, kernel.shape)
         entry = self._entry
-        if entry is None or entry[0] != key:
-            with torch.no_grad():
-                entry = (key, transform(kernel))
-            self._entry = entry
-        return entry[1]
+        if entry is not None and entry[0] == key:
+            read_on_current_stream(entry[1], event=entry[2])
+            return entry[1]
+        with torch.no_grad():
+            value = transform(kernel)
+        event = None
+        if value.is_cuda:
+            if torch.cuda.is_current_stream_capturing():
+                return value
+            event = torch.cuda.current_stream(value.device).record_event()
+            made_on_current_stream(value)
+        self._entry = (key, value, event)
+        return value
 
 
 class FourierMatrices(_OneEntry):
@@ -55,4 +70,5 @@ class FourierMatrices(_OneEntry):
             F, Ft = setup(b, grid, device_type=device.type, device_index=device.index)
             entry = (grid, key, (F, Ft, scaling))
             self._entry = entry
+        read_on_current_stream(entry[2][0], entry[2][1])
         return entry[2]

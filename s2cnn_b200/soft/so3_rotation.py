@@ -8,6 +8,7 @@ from functools import lru_cache
 import torch
 
 from ..ops import cuda_ops
+from ..s2_ft import made_on_current_stream, read_on_current_stream
 from .so3_fft import SO3_fft_real, SO3_ifft_real
 
 
@@ -19,7 +20,9 @@ def _setup_so3_rotation(b, alpha, beta, gamma, device_type, device_index):
     (s2cnn/soft/so3_rotation.py:51-73); here the library's host recurrence produces them.
     """
     U = cuda_ops().so3_rotation_matrices(b, alpha, beta, gamma)
-    return torch.from_numpy(U).to(torch.device(device_type, device_index))
+    U = torch.from_numpy(U).to(torch.device(device_type, device_index))   # waits for the copy
+    made_on_current_stream(U)
+    return U
 
 
 def so3_rotation(x, alpha, beta, gamma):
@@ -30,6 +33,7 @@ def so3_rotation(x, alpha, beta, gamma):
     x_size = x.size()
     U = _setup_so3_rotation(b, float(alpha), float(beta), float(gamma),
                             device_type=x.device.type, device_index=x.device.index)
+    read_on_current_stream(U)
     x = SO3_fft_real.apply(x)          # [l * m * n, ..., complex]
     z = cuda_ops().ag_rotate_spectrum(x, U, b)
     z = SO3_ifft_real.apply(z)
