@@ -12,15 +12,16 @@ import torch
 from .ops import cuda_ops
 
 
-def _raw_stream(t):
-    return torch._C._cuda_getCurrentRawStream(t.device.index)
+def _raw_stream(index):
+    """The current stream of a CUDA device, as a number (a stream object costs a microsecond)."""
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 def made_on_current_stream(*tensors):
     """Notes, on tensors that will be kept between calls, the stream they were allocated on."""
     for t in tensors:
         if t is not None and t.is_cuda:
-            t._made_on = _raw_stream(t)
+            t._made_on = _raw_stream(t.get_device())
 
 
 def read_on_current_stream(*tensors, event=None):
@@ -28,7 +29,7 @@ def read_on_current_stream(*tensors, event=None):
     for ``event`` (recorded after they were written; None: they were complete before they were kept),
     and the allocator does not hand their memory on before the reader is done, whoever drops them."""
     for t in tensors:
-        if t is None or not t.is_cuda or t._made_on == _raw_stream(t):
+        if t is None or not t.is_cuda or t._made_on == _raw_stream(t.get_device()):
             continue
         if torch.cuda.is_current_stream_capturing():   # the graph keeps them (GraphedForward)
             continue

@@ -21,7 +21,7 @@ it captures) and leaves nothing: what it makes itself is filled by the replays o
 """
 import torch
 
-from ..s2_ft import made_on_current_stream, read_on_current_stream
+from ..s2_ft import _raw_stream, made_on_current_stream, read_on_current_stream
 
 
 class _OneEntry:
@@ -45,17 +45,21 @@ class KernelSpectrumCache(_OneEntry):
         key = (kernel._version, kernel.data_ptr(), kernel.device, kernel.shape)
         entry = self._entry
         if entry is not None and entry[0] == key:
-            read_on_current_stream(entry[1], event=entry[2])
-            return entry[1]
+            _, value, event, index, stream = entry
+            if event is not None and stream != _raw_stream(index):
+                read_on_current_stream(value, event=event)
+            return value
         with torch.no_grad():
             value = transform(kernel)
-        event = None
+        event = index = stream = None
         if value.is_cuda:
             if torch.cuda.is_current_stream_capturing():
                 return value
             event = torch.cuda.current_stream(value.device).record_event()
             made_on_current_stream(value)
-        self._entry = (key, value, event)
+            index = value.device.index
+            stream = _raw_stream(index)
+        self._entry = (key, value, event, index, stream)
         return value
 
 
