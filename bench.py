@@ -147,26 +147,26 @@ def reference_net(seed=0):
 
 def kernel_bytes(B):
     """Per forward pass, per kernel name: bytes the kernel has to move once - its own inputs and
-    outputs, constant tables excluded - summed over its launches in the pass.  Fused kernels are
-    charged the bytes of the module boundaries they cover - the tensor each reference module writes
-    once and the next one reads once (the per-sample figure of the workload: 14,400 + 2 * 640,000 +
-    2 * 276,480 B) - although they keep those tensors on chip; `traffic` in the roofline object is
-    what actually crosses DRAM."""
+    outputs, constant tables excluded - summed over its launches in the pass.  Tensors that a fused
+    kernel keeps on chip are not charged (``roofline.whole_pass`` relates the whole pass to the
+    module boundaries); `traffic` in the roofline object is what actually crosses DRAM."""
     b0, b1, b2, f0, f1, f2 = (NET[k] for k in ("b0", "b1", "b2", "f0", "f1", "f2"))
     c = 8  # bytes per complex
-    sig1 = B * f1 * (2 * b1) ** 3 * 4   # conv1 output / conv2 input signal
+    product_in = b1 * b1 * (B * f0 + f0 * f1) * c       # the two S2 spectra of conv1
+    spec2 = n3(b2) * B * f1 * c                         # conv2's input spectrum
+    v1, v2 = (B * f1 * k * (2 * k - 1) * 2 * b1 * c for k in (b1, b2))   # the plane kernels' scratch array
     out = {}
     N0 = 2 * b0
-    out["s2_fwd_fused"] = B * f0 * N0 * N0 * 4 + b1 * b1 * B * f0 * c
+    out["s2_fwd_fused<%d>" % N0] = B * f0 * N0 * N0 * 4 + b1 * b1 * B * f0 * c
     out["rft_forward"] = (f0 * f1 * 24 * 4 + b1 * b1 * f0 * f1 * c) + (f1 * f2 * 192 * 4 + n3(b2) * f1 * f2 * c)
-    out["so3_relay_fused<%d>" % (2 * b1)] = (b1 * b1 * (B * f0 + f0 * f1) * c + 2 * sig1 +
-                                               n3(b2) * B * f1 * c)
-    # the same boundary when the batch takes the plane kernels
-    out["so3_inv_wigner_col_s2"] = b1 * b1 * (B * f0 + f0 * f1) * c
-    out["so3_relay_small<%d>" % (2 * b1)] = 2 * sig1
-    out["so3_fwd_wigner_col"] = n3(b2) * B * f1 * c
-    sig2 = B * f2 * (2 * b2) ** 3 * 4
-    out["so3_inv_fused<%d>" % (2 * b2)] = n3(b2) * B * f2 * c + 2 * sig2 + B * f2 * 4
+    # batches below the plane kernels' line: one kernel from the S2 spectra to conv2's input spectrum
+    for name in ("so3_relay_cl<%d>", "so3_relay_fused<%d>"):
+        out[name % (2 * b1)] = product_in + spec2
+    out["so3_inv_wigner_col_s2"] = product_in + v1
+    out["so3_relay_small<%d>" % (2 * b1)] = v1 + v2
+    out["so3_fwd_wigner_col"] = v2 + spec2
+    for name in ("so3_inv_cl<%d>", "so3_inv_fused<%d>"):   # conv2's synthesis with the integral
+        out[name % (2 * b2)] = n3(b2) * B * f2 * c + B * f2 * 4
     out["so3_mm_tc_kernel"] = n3(b2) * (B * f1 + f1 * f2 + B * f2) * c
     return out
 
@@ -825,11 +825,10 @@ def run_ours(args):
                     "peak_source": peak_kind,
                     "alg_bytes_per_launch": top["alg_bytes_per_batch"] / max(top["launches_per_batch"], 1),
                     "launches_per_batch": top["launches_per_batch"],
-                    "note": "algorithmic bytes of a fused kernel are those of the module boundaries "
-                            "it covers (tensors it keeps on chip); `traffic` is what crosses DRAM "
-                            "per launch in the committed ncu summary, `dram_frac` that figure over "
-                            "the launch time and the peak - the kernel is bound by instruction "
-                            "issue, not by HBM"}
+                    "note": "algorithmic bytes are the kernel's own inputs and outputs, once (a "
+                            "scratch array between two kernels counts for both, wherever it is cached); "
+                            "`traffic` is what crosses DRAM per launch in the committed ncu summary, "
+                            "`dram_frac` that figure over the launch time and the peak"}
         if traffic:
             roofline["dram_frac"] = traffic / (top["avg_launch_ms"] * 1e-3) / 1e9 / hbm_gbs
             roofline["traffic_source"] = os.path.relpath(TRAFFIC_PROFILE, ROOT)
@@ -844,7 +843,8 @@ def run_ours(args):
 
     cfg = workload_config(world, M)
     cfg.update({
-        "fusion": "s2_mm + conv1 synthesis + ReLU + conv2 analysis in one kernel; second ReLU and "
+        "fusion": "s2_mm + conv1 synthesis + ReLU + conv2 analysis in one call (the signal between the "
+                  "layers stays on chip); second ReLU and "
                   "so3_integrate inside conv2's synthesis kernel (s2cnn_b200.fuse on a plain Sequential)",
         "launch": "eager" if args.no_graph else (
             "CUDA graph replay (s2cnn_b200.graph.GraphedForward)" if args.lanes < 2 else

@@ -5,16 +5,20 @@
 Each case runs one op a few times on seeded synthetic data sized for a capture that ends by itself
 within a minute (inputs above the 126 MB L2 where DRAM figures matter, a few hundred MB at most):
 
-    inv10   so3_rifft, b = 10, 5120 signals          (kernel so3_inv_fused<20>)
-    fwd10   so3_rfft,  b = 10 -> 6, 5120 signals     (kernel so3_fwd_fused<20>)
-    inv16   so3_rifft, b = 16, 1600 signals          (kernel so3_inv_fused<32>, 512-thread blocks)
-    fwd16   so3_rfft,  b = 16, 1600 signals          (kernel so3_fwd_fused<32>, 512-thread blocks)
+    inv10   so3_rifft, b = 10, 5120 signals          (so3_inv_wigner_col, so3_inv_small<20>)
+    fwd10   so3_rfft,  b = 10 -> 6, 5120 signals     (so3_fwd_small<20>, so3_fwd_wigner_col)
+    inv16   so3_rifft, b = 16, 1600 signals          (so3_inv_wigner_col, so3_inv_small<32>)
+    fwd16   so3_rfft,  b = 16, 1600 signals          (so3_fwd_small<32>, so3_fwd_wigner_col)
     relay10 s2_mm + so3_rifft (b = 10) + bias + ReLU + so3_rfft (-> b = 6), batch 256, 1 -> 20
-            features = 5120 signals                  (kernel so3_relay_fused<20>)
+            features = 5120 signals                  (so3_inv_wigner_col_s2, so3_relay_small<20>,
+                                                      so3_fwd_wigner_col)
     mm      so3_mm, nl = 6, batch 256, 20 -> 40      (kernel so3_mm_tc_kernel)
     mm_c4   so3_mm, nl = 10, batch 32, 100 -> 100    (kernel so3_mm_tc_kernel at a GEMM-sized case)
     fft64   so3_rfft + so3_rifft, b = 64, 8 signals  (plane kernels + Wigner contraction)
     fft64_three_pass   the same through the three separate passes (the path 2b = 256 takes)
+
+With ``walking`` after the name the b <= 16 cases take the kernels whose blocks walk beta
+(so3_inv_fused, so3_fwd_fused, so3_relay_fused) instead.
 """
 import sys
 
@@ -23,8 +27,9 @@ import torch
 from .ops import cuda_ops, so3_nspec
 
 
-def main(which):
+def main(which, walking=False):
     ops = cuda_ops()
+    ops.lib.s2c_debug_cluster(2 if walking else 0)
     dev = torch.device("cuda:0")
     torch.manual_seed(0)
     if which == "inv10":
@@ -72,4 +77,4 @@ def main(which):
 
 
 if __name__ == "__main__":
-    main(sys.argv[1] if len(sys.argv) > 1 else "")
+    main(sys.argv[1] if len(sys.argv) > 1 else "", "walking" in sys.argv[2:])

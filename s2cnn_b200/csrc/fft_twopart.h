@@ -55,8 +55,9 @@ S2C_HD constexpr int two_freq_block(int n, int r1, int f) {
 // a * w^DIR with the roundings spelled out: which of the two products of a component is fused into the
 // addition is the compiler's choice in ctw() (and changes with constant operands), but it decides the last
 // bit, and a training step of a deep network amplifies last bits through its ReLUs and batch
-// normalisation.  This is the choice fft_dif_inplace is compiled to; in the general prime radices (PRIME:
-// 7 and above) the imaginary part of the inverse direction is fused the other way round.
+// normalisation.  With this choice - in the general prime radices (PRIME: 7 and above) the imaginary part of
+// the inverse direction fused the other way round - the outputs equal those of the three-pass kernels, whose
+// stages call fft_dif_inplace, bit for bit on the GPU (tests/test_mid_bandwidths.py).
 #ifndef S2C_EMUL
 __device__ __forceinline__ float two_mul(float a, float b) { return __fmul_rn(a, b); }
 #else
