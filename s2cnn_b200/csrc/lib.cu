@@ -764,6 +764,7 @@ int s2c_s2_ft_matrix(int b, const double* grid, int n_grid, float* F) {
 
 // ---- SO(3) transforms ----------------------------------------------------------------------------
 size_t s2c_so3_fft_workspace_min(int b_in, int b_out) {
+  if (b_in < 1 || b_out < 1) return 0;
   // the beta grid is b_in's for analysis and b_out's for synthesis; take the larger of the two
   const int K = std::min(b_in, b_out);
   return std::max(so3_ws_per_z(2 * b_in, K), so3_ws_per_z(2 * b_out, K));
@@ -771,6 +772,7 @@ size_t s2c_so3_fft_workspace_min(int b_in, int b_out) {
 
 size_t s2c_so3_fft_workspace(long nbatch, int b_in, int b_out) {
   const size_t per_z = s2c_so3_fft_workspace_min(b_in, b_out);
+  if (!per_z) return 0;
   if (plane_supported(2 * b_in) && plane_supported(2 * b_out)) {
     // large-bandwidth path: one chunk of the scratch array V (sized to stay in L2); never less than
     // one signal of the three-pass organisation, which the test switches can select instead
@@ -1078,6 +1080,7 @@ int s2c_so3_ifft(const float* x, float* out, long nbatch, int b_in, int b_out, i
 
 // ---- S2 transforms -------------------------------------------------------------------------------
 size_t s2c_s2_fft_workspace(long nbatch, int b_in, int b_out) {
+  if (b_in < 1 || b_out < 1) return 0;
   const int K = std::min(b_in, b_out), N = 2 * std::max(b_in, b_out);
   return s2_ws_per_z(N, K) * (size_t)std::max(1L, nbatch);
 }

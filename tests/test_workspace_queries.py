@@ -33,6 +33,17 @@ def test_single_kernel_paths_need_no_workspace(backend):
 
 
 @pytest.mark.parametrize("backend", backends.BACKENDS)
+def test_queries_answer_nonsense_with_nothing(backend):
+    lib = backends.get(backend)[0].lib
+    for name in ("so3_fft", "so3_analysis", "so3_synthesis", "s2_fft"):
+        for bad in ((4, 0, 3), (4, 3, 0), (4, -2, 3), (4, 3, -1)):
+            assert getattr(lib, "s2c_%s_workspace" % name)(*bad) == 0, (name, bad)
+    assert lib.s2c_so3_relay_workspace(0, 3, 3, 3) == 0 and lib.s2c_so3_relay_workspace(5, 3, 0, 3) == 0
+    assert lib.s2c_s2_conv_synthesis_workspace(2, 3, 0) == 0 and lib.s2c_s2_conv_synthesis_workspace(0, 3, 3) == 0
+    assert lib.s2c_so3_mm_gradx_workspace(0, 1, 1, 1) == 0 and lib.s2c_rft_backward_workspace(3, 0, 5) == 0
+
+
+@pytest.mark.parametrize("backend", backends.BACKENDS)
 @pytest.mark.parametrize("b,b_spec,nb", [(4, 6, 3), (9, 9, 2), (13, 13, 130), (17, 5, 3), (18, 18, 2), (33, 7, 1)])
 def test_calls_run_with_what_the_query_says(backend, b, b_spec, nb):
     ops, dev = backends.get(backend)
