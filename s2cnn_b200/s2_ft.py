@@ -24,19 +24,21 @@ def made_on_current_stream(*tensors):
             t._made_on = _raw_stream(t.get_device())
 
 
-def read_on_current_stream(*tensors, event=None):
-    """Kept tensors are about to be read on the current stream: where that is not their own it waits
-    for ``event`` (recorded after they were written; None: they were complete before they were kept),
-    and the allocator does not hand their memory on before the reader is done, whoever drops them."""
-    for t in tensors:
-        if t is None or not t.is_cuda or t._made_on == _raw_stream(t.get_device()):
-            continue
-        if torch.cuda.is_current_stream_capturing():   # the graph keeps them (GraphedForward)
-            continue
-        stream = torch.cuda.current_stream(t.device)
-        if event is not None:
-            stream.wait_event(event)
-        t.record_stream(stream)
+def read_on_current_stream(first, *others, event=None):
+    """Kept tensors, made together, are about to be read on the current stream: where that is not their
+    own it waits for ``event`` (recorded after they were written; None: they were complete before they
+    were kept), and the allocator does not hand their memory on before the reader is done, whoever drops
+    them."""
+    if not first.is_cuda or first._made_on == _raw_stream(first.get_device()):
+        return
+    if torch.cuda.is_current_stream_capturing():   # the graph keeps them (GraphedForward)
+        return
+    stream = torch.cuda.current_stream(first.device)
+    if event is not None:
+        stream.wait_event(event)
+    for t in (first,) + others:
+        if t is not None:
+            t.record_stream(stream)
 
 
 def fourier_matrices(F_host, device):
