@@ -798,7 +798,9 @@ struct TcShare {
 // blocks on top of its own (set-up, pipeline fill, epilogue: about 6 us against 0.6 us a block), sharing within a
 // cluster another kShare and between clusters another kGather.  kSlots: clusters resident on the chip, by size
 // (cudaOccupancyMaxActiveClusters).  The split is taken only where the estimate drops by a tenth, so that large
-// products keep one CTA per tile.
+// products keep one CTA per tile.  One CTA per tile -> shared (us): 100 -> 255 channels, nl 5, batch 32, grad-x 123 -> 86;
+// 20 -> 40, nl 6, batch 32, grad-x 29 -> 14, grad-y 22 -> 14; 13 -> 9, nl 7, batch 5, grad-x 14 -> 9; kernel gradients
+// (rows x grid x spectrum) 800 x 192 x 286 26 -> 11, 10000 x 192 x 1330 137 -> 115, 128 x 36 x 4495 (15 clusters) 189 -> 16.
 inline TcShare tc_pick_share(int op, int nl, int nb, int fi, int fo, int nblk, bool several_clusters) {
   constexpr double kCta = 8, kShare = 4, kGather = 6;
   constexpr int kSlots[kTcMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
