@@ -232,6 +232,14 @@ int s2c_so3_mm_gradx_ws(const float* gz, const float* y, float* gx, int nl, int 
                         int f_out, void* workspace, size_t workspace_bytes, void* stream);
 int s2c_so3_mm_grady_ws(const float* gz, const float* x, float* gy, int nl, int nbatch, int f_in,
                         int f_out, void* workspace, size_t workspace_bytes, void* stream);
+/* The same three products for spectra of REAL signals and kernels, which a layer's products are:
+ * X[l,-m,-n] = (-1)^(m-n) conj X[l,m,n] for both operands and so for the result.  One half of the result is
+ * computed, the other written as its mirror; operands without the symmetry give one-sided results.
+ *   op 0: u = x, v = y, out = z     op 1: u = gz, v = y, out = gx     op 2: u = gz, v = x, out = gy
+ * Workspace as for the gradients above (0 for op 0). */
+size_t s2c_so3_mm_real_workspace(int op, int nl, int nbatch, int f_in, int f_out);
+int s2c_so3_mm_real(int op, const float* u, const float* v, float* out, int nl, int nbatch, int f_in, int f_out,
+                    void* workspace, size_t workspace_bytes, void* stream);
 /* z[l,m,n,i,j] = sum_k x[l,m,i,k] conj(y[l,n,k,j]);  x [nl^2, nbatch, f_in, 2],
  * y [nl^2, f_in, f_out, 2], z [nspec(nl), nbatch, f_out, 2].
  * Replaces s2_mm / _cuda_s2_mm, s2cnn/s2_mm.py:10-28,104-137 (+ kernel s2mm.cu :140-198). */

@@ -75,6 +75,8 @@ _SIGNATURES = {
     "s2c_so3_mm_grady_workspace": (c_size_t, [c_int, c_int, c_int, c_int]),
     "s2c_so3_mm_gradx_ws": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
     "s2c_so3_mm_grady_ws": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
+    "s2c_so3_mm_real_workspace": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "s2c_so3_mm_real": (c_int, [c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
     "s2c_s2_mm": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_s2_mm_gradx": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_s2_mm_grady": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),

@@ -1248,34 +1248,36 @@ static bool tc_flush(const MmTcParams& p, long blocks, int ns) {
 static int tc_run(int op, int nb, int fi, int fo) { return 2 * (op == kTcFwd ? fi : op == kTcGradX ? fo : nb); }
 // CTAs per tile; several clusters to a tile only with the workspace they meet in
 static int tc_share(MmTcParams& p, int op, long tiles, void* ws, size_t ws_bytes, stream_t st) {
-  TcShare s = tc_pick_share(op, p.nl, p.nb, p.fi, p.fo, p.nblk, true);
+  TcShare s = tc_pick_share(op, p.half, p.nl, p.nb, p.fi, p.fo, p.nblk, true);
   if (s.groups > 1 && (!ws || (uintptr_t)ws % 16 != 0 || ws_bytes < tc_share_bytes(tiles, s.groups)))
-    s = tc_pick_share(op, p.nl, p.nb, p.fi, p.fo, p.nblk, false);
+    s = tc_pick_share(op, p.half, p.nl, p.nb, p.fi, p.fo, p.nblk, false);
   p.csize = s.csize; p.groups = s.groups;
   if (s.groups == 1) return S2C_OK;
   p.count = (int*)ws;
   p.part = (float*)((unsigned char*)ws + tc_count_bytes(tiles));
   return cuda_check(cudaMemsetAsync(ws, 0, tc_count_bytes(tiles), st), "counters of the shared tiles");
 }
-static size_t tc_share_workspace(int op, int nl, int nb, int fi, int fo, int run) {
+static size_t tc_share_workspace(int op, int half, int nl, int nb, int fi, int fo, int run) {
   if (g_force_general) return 0;
   MmTcParams p;
   p.run = run;
   tc_blocks(p);
-  return tc_share_bytes(so3_mm_tc_tiles(op, nl, nb, fi, fo), tc_pick_share(op, nl, nb, fi, fo, p.nblk, true).groups);
+  return tc_share_bytes(so3_mm_tc_tiles(op, half, nl, nb, fi, fo),
+                        tc_pick_share(op, half, nl, nb, fi, fo, p.nblk, true).groups);
 }
-// so3_mm or one of its gradients on the tensor cores; `handled` tells whether the shape qualified.
-static int so3_mm_tc_launch(int op, const float* a, const float* b, float* c, int nl, int nb, int fi,
+// so3_mm or one of its gradients on the tensor cores, `half` of it where the operands are spectra of real signals;
+// `handled` tells whether the shape qualified.
+static int so3_mm_tc_launch(int op, int half, const float* a, const float* b, float* c, int nl, int nb, int fi,
                             int fo, void* ws, size_t ws_bytes, stream_t st, bool* handled) {
   *handled = !g_force_general;
   if (!*handled) return S2C_OK;
   MmTcParams p;
   p.a = a; p.b = b; p.c = c;
-  p.nl = nl; p.nb = nb; p.fi = fi; p.fo = fo;
+  p.nl = nl; p.nb = nb; p.fi = fi; p.fo = fo; p.half = half;
   p.run = tc_run(op, nb, fi, fo);
   tc_blocks(p);
   S2C_TRY(tc_err_flag(&p.err));
-  const long tiles = so3_mm_tc_tiles(op, nl, nb, fi, fo);
+  const long tiles = so3_mm_tc_tiles(op, half, nl, nb, fi, fo);
   p.csize = p.groups = 1;
   p.part = nullptr; p.count = nullptr;
   // The forward product always runs one CTA per tile: its rounding is then the same whatever the batch.
@@ -1296,7 +1298,7 @@ static int plain_tc_launch(bool a_strided, const float* a, const float* b, float
                            float scale, void* ws, size_t ws_bytes, stream_t st) {
   MmTcParams p;
   p.a = a; p.b = b; p.c = c;
-  p.nl = 1; p.nb = (int)M; p.fi = (int)(K / 2); p.fo = (int)(N / 2);
+  p.nl = 1; p.nb = (int)M; p.fi = (int)(K / 2); p.fo = (int)(N / 2); p.half = 0;
   p.run = (int)K;
   tc_blocks(p);
   p.a_rs = a_rs; p.a_ps = a_ps; p.b_rs = b_rs; p.b_ps = b_ps; p.c_rs = c_rs; p.c_ps = c_ps;
@@ -1304,7 +1306,7 @@ static int plain_tc_launch(bool a_strided, const float* a, const float* b, float
   S2C_TRY(tc_err_flag(&p.err));
   // (one degree, l = 0, with M rows and N columns in the spectral geometry; the forward transform has a
   // short contraction and is not split)
-  const long tiles = so3_mm_tc_tiles(kTcPlainSC, 1, (int)M, p.fi, p.fo);
+  const long tiles = so3_mm_tc_tiles(kTcPlainSC, 0, 1, (int)M, p.fi, p.fo);
   p.csize = p.groups = 1;
   p.part = nullptr; p.count = nullptr;
   if (a_strided) S2C_TRY(tc_share(p, kTcPlainSC, tiles, ws, ws_bytes, st));
@@ -1323,7 +1325,7 @@ int s2c_so3_mm(const float* x, const float* y, float* z, int nl, int nb, int fi,
   if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
 #ifndef S2C_EMUL
   bool handled = false;
-  S2C_TRY(so3_mm_tc_launch(kTcFwd, x, y, z, nl, nb, fi, fo, nullptr, 0, as_stream(st), &handled));
+  S2C_TRY(so3_mm_tc_launch(kTcFwd, 0, x, y, z, nl, nb, fi, fo, nullptr, 0, as_stream(st), &handled));
   if (handled) return S2C_OK;
 #endif
   return mm_dispatch(true, kMmFwd, x, y, z, nl, nb, fi, fo, as_stream(st));
@@ -1344,7 +1346,7 @@ int s2c_so3_mm_tc_status(void) {
 size_t s2c_so3_mm_gradx_workspace(int nl, int nb, int fi, int fo) {
 #ifndef S2C_EMUL
   if (nl >= 1 && nb >= 1 && fi >= 1 && fo >= 1)
-    return tc_share_workspace(kTcGradX, nl, nb, fi, fo, tc_run(kTcGradX, nb, fi, fo));
+    return tc_share_workspace(kTcGradX, 0, nl, nb, fi, fo, tc_run(kTcGradX, nb, fi, fo));
 #endif
   return 0;
 }
@@ -1354,7 +1356,7 @@ int s2c_so3_mm_gradx_ws(const float* gz, const float* y, float* gx, int nl, int 
   if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
 #ifndef S2C_EMUL
   bool handled = false;
-  S2C_TRY(so3_mm_tc_launch(kTcGradX, gz, y, gx, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
+  S2C_TRY(so3_mm_tc_launch(kTcGradX, 0, gz, y, gx, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
   if (handled) return S2C_OK;
 #endif
   return mm_dispatch(true, kMmGradX, gz, y, gx, nl, nb, fi, fo, as_stream(st));
@@ -1365,7 +1367,7 @@ int s2c_so3_mm_gradx(const float* gz, const float* y, float* gx, int nl, int nb,
 size_t s2c_so3_mm_grady_workspace(int nl, int nb, int fi, int fo) {
 #ifndef S2C_EMUL
   if (nl >= 1 && nb >= 1 && fi >= 1 && fo >= 1)
-    return tc_share_workspace(kTcGradY, nl, nb, fi, fo, tc_run(kTcGradY, nb, fi, fo));
+    return tc_share_workspace(kTcGradY, 0, nl, nb, fi, fo, tc_run(kTcGradY, nb, fi, fo));
 #endif
   return 0;
 }
@@ -1375,13 +1377,40 @@ int s2c_so3_mm_grady_ws(const float* gz, const float* x, float* gy, int nl, int 
   if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
 #ifndef S2C_EMUL
   bool handled = false;
-  S2C_TRY(so3_mm_tc_launch(kTcGradY, x, gz, gy, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
+  S2C_TRY(so3_mm_tc_launch(kTcGradY, 0, x, gz, gy, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
   if (handled) return S2C_OK;
 #endif
   return mm_dispatch(true, kMmGradY, x, gz, gy, nl, nb, fi, fo, as_stream(st));
 }
 int s2c_so3_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo, void* st) {
   return s2c_so3_mm_grady_ws(gz, x, gy, nl, nb, fi, fo, nullptr, 0, st);
+}
+// Products of spectra of real signals.  X[l,-m,-n] = (-1)^(m-n) conj X[l,m,n] holds for the operands and so for the
+// result: the tensor cores compute the rows of outer index l .. 2l (m >= 0; the kernel index for the gradient of y), half
+// of the multiply-adds, and write each coefficient and its mirror.  us on one B200, all rows -> half, for z, gx
+// and gy: 100 -> 100 channels, nl = 10, batch 32: 314, 325, 314 -> 205, 211, 203; 16 -> 16, nl = 15, batch 32: 77, 80, 65 -> 50,
+// 52, 51; 20 -> 40, nl = 6, batch 256: 46, 50, 52 -> 33, 33, 36.  Calls of one tile row (batch 1) take the time they took.
+size_t s2c_so3_mm_real_workspace(int op, int nl, int nb, int fi, int fo) {
+#ifndef S2C_EMUL
+  if ((op == kTcGradX || op == kTcGradY) && nl >= 1 && nb >= 1 && fi >= 1 && fo >= 1)
+    return tc_share_workspace(op, 1, nl, nb, fi, fo, tc_run(op, nb, fi, fo));
+#endif
+  return 0;
+}
+int s2c_so3_mm_real(int op, const float* u, const float* v, float* out, int nl, int nb, int fi, int fo, void* ws,
+                    size_t ws_bytes, void* st) {
+  if (op < 0 || op > 2) return fail(S2C_ERR_BAD_ARG, "s2c_so3_mm_real: op is 0, 1 or 2");
+  if (!u || !v || !out) return fail(S2C_ERR_BAD_ARG, "s2c_so3_mm_real: null pointer");
+  if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
+  const float *a = op == 2 ? v : u, *b = op == 2 ? u : v;     // the gradient of y: rows from x
+#ifndef S2C_EMUL
+  static_assert((int)kTcFwd == 0 && (int)kTcGradX == 1 && (int)kTcGradY == 2, "op codes");
+  bool handled = false;
+  S2C_TRY(so3_mm_tc_launch(op, 1, a, b, out, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
+  if (handled) return S2C_OK;
+#endif
+  static_assert(kMmFwd == 0 && kMmGradX == 1 && kMmGradY == 2, "op codes");
+  return mm_dispatch(true, op, a, b, out, nl, nb, fi, fo, as_stream(st));
 }
 int s2c_s2_mm(const float* x, const float* y, float* z, int nl, int nb, int fi, int fo, void* st) {
   if (!x || !y || !z) return fail(S2C_ERR_BAD_ARG, "s2c_s2_mm: null pointer");
@@ -1454,7 +1483,7 @@ int s2c_rft_forward_scaled(const float* x, const float* F, const float* Ft, floa
 
 size_t s2c_rft_backward_workspace(int nf, int ng, int ns) {
 #ifndef S2C_EMUL
-  if (nf >= 1 && ng >= 1 && ns >= 1 && ng % 2 == 0) return tc_share_workspace(kTcPlainSC, 1, nf, ns, ng / 2, 2 * ns);
+  if (nf >= 1 && ng >= 1 && ns >= 1 && ng % 2 == 0) return tc_share_workspace(kTcPlainSC, 0, 1, nf, ns, ng / 2, 2 * ns);
 #endif
   return 0;
 }

@@ -85,6 +85,7 @@ struct MmTcParams {
   const float* b;   // operand read along the output columns
   float* c;         // output
   int nl, nb, fi, fo;
+  int half;         // spectra of real signals: rows of outer index l .. 2l only, the others are their mirrors
   int run;          // floats per outer contraction index: 2 fi (fwd), 2 fo (grad x), 2 nb (grad y)
   int kblk;         // floats per K block (multiple of 8, <= kTcKMax)
   int nblk;         // K blocks per run
@@ -127,10 +128,14 @@ constexpr int kTcFirstProducer = 32 * (1 + kTcCollectorWarps);  // thread index 
 constexpr int kTcThreads = 32 * (1 + kTcCollectorWarps + kTcProducerWarps);
 // K blocks accumulated by the tensor core before the partial sum is added, in FP32 with rounding,
 // into the sum region (bounds the length of the tensor core's own accumulation chain, whose
-// additions truncate): 8 blocks = 72 MMAs per chain.
+// additions truncate): 8 blocks = 72 MMAs per chain.  Half products flush every 7: a coefficient and its mirror are then no
+// longer two sums of which the synthesis takes the mean, and the shorter chain makes up for that (relative error of the
+// symmetric part, nl = 10, 100 -> 100, batch 32: 1.69e-6 full, 1.75e-6 half with 8, 1.58e-6 with 7).
 constexpr int kTcFlushBlocks = 8;
-// longest chain (in MMAs) left to the tensor core's own accumulation without partial sums: its
-// truncation bias stays below about 1e-5 relative
+// longest chain (in MMAs) left to the tensor core's own accumulation without partial sums: its truncation bias stays
+// below about 1e-5 relative.  The second accumulator is then free; in half products it takes the products with a lo part:
+// they are 2^-11 of the others, so their truncations do not count, and a third of the chain's remain (198 MMAs, nl = 6,
+// 20 -> 40: relative error 3.3e-6 in one accumulator, 1.2e-6 in two).  Full products stay as they were, to the bit.
 constexpr int kTcChainMax = 200;
 // tensor-memory columns: two alternating accumulators, the FP32 sum region and two stages of the row operand
 // (hi in columns 0 - 23, lo in 32 - 55 of each)
@@ -291,10 +296,10 @@ __device__ __forceinline__ void tc_st8(uint32_t taddr, const float (&v)[8]) {
 // lower 13 bits of its inputs, so lo = v - hi needs no further rounding)
 __device__ __forceinline__ float tc_hi(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFFE000u); }
 
-__host__ __device__ __forceinline__ long tc_tiles_for(int op, int nb, int fi, int fo, int l) {
+__host__ __device__ __forceinline__ long tc_tiles_for(int op, int half, int nb, int fi, int fo, int l) {
   const TcGeom g = tc_geom(op, nb, fi, fo);
   const long L = 2 * l + 1;
-  const long M = L * g.RI, N = L * g.CW;
+  const long M = (half ? l + 1 : L) * g.RI, N = L * g.CW;
   return ((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);
 }
 
@@ -321,7 +326,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   int l = p.nl - 1;
   long t = blockIdx.x;
   for (;; --l) {
-    const long c = tc_tiles_for(OP, p.nb, p.fi, p.fo, l) * nsplit;
+    const long c = tc_tiles_for(OP, p.half, p.nb, p.fi, p.fo, l) * nsplit;
     if (t < c) break;
     t -= c;
   }
@@ -333,14 +338,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   const int o_lo = it_lo / p.nblk, kb_lo = it_lo - o_lo * p.nblk;
   const TcGeom geo = tc_geom(OP, p.nb, p.fi, p.fo);
   const int RI = geo.RI, CW = geo.CW;
-  const int M = L * RI, Np = L * CW;
+  const int ro0 = p.half ? l : 0;                         // outer index of the first row
+  const int M = (L - ro0) * RI, Np = L * CW;
   const int tiles_n = (Np + kTcBN - 1) / kTcBN;
   const int row0 = (int)(t / tiles_n) * kTcBM, col0 = (int)(t % tiles_n) * kTcBN;
   const long spec0 = (long)l * (4L * l * l - 1) / 3;
   const int fi2 = 2 * p.fi, fo2 = 2 * p.fo;
   const int nit = it_hi - it_lo;                          // K blocks of this CTA (a shared tile: possibly none)
+  const bool two_accs = !FLUSH && p.half;
   // accumulator groups (one when the whole chain stays in the tensor core's accumulator)
-  const int ngroups = FLUSH ? (nit + kTcFlushBlocks - 1) / kTcFlushBlocks : 1;
+  const int flush_blocks = p.half ? kTcFlushBlocks - 1 : kTcFlushBlocks;
+  const int ngroups = FLUSH ? (nit + flush_blocks - 1) / flush_blocks : 1;
 
   // ---- set-up: barriers, tensor memory ------------------------------------------------------
   if (tid == 0) {
@@ -408,18 +416,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
           if (ks < ksteps) {
             const uint64_t dbh = db + ks * kDStep, dbl = dbh + kDBuf;
             const uint32_t tah = ta + 8 * ks, tal = tah + kTcALo;
-            tc_mma_tf32(acc, tah, dbh, idesc, ((FLUSH ? ing == 0 : it == 0) && ks == 0) ? 0u : 1u);
-            tc_mma_tf32(acc, tal, dbh, idesc, 1u);
-            tc_mma_tf32(acc, tah, dbl, idesc, 1u);
+            const uint32_t acc_lo = two_accs ? acc + kTcBN : acc;
+            const uint32_t first = ((FLUSH ? ing == 0 : it == 0) && ks == 0) ? 0u : 1u;
+            tc_mma_tf32(acc, tah, dbh, idesc, first);
+            tc_mma_tf32(acc_lo, tal, dbh, idesc, two_accs ? first : 1u);
+            tc_mma_tf32(acc_lo, tah, dbl, idesc, 1u);
           }
         }
         tc_commit(&empty[s]);     // arrives when these MMAs have read the stage
-        if ((FLUSH && ing + 1 == kTcFlushBlocks) || it + 1 == nit) tc_commit(&accdone[g & 1]);
+        if ((FLUSH && ing + 1 == flush_blocks) || it + 1 == nit) tc_commit(&accdone[g & 1]);
       }
       __syncwarp();
       if (++kb == p.nblk) kb = 0;
       if (++s == kTcStages) { s = 0; full_par ^= 1u; }
-      if (FLUSH && ++ing == kTcFlushBlocks) { ing = 0; ++g; }
+      if (FLUSH && ++ing == flush_blocks) { ing = 0; ++g; }
     }
   } else if (warp <= kTcCollectorWarps) {
     // ================================ collectors ================================================
@@ -469,7 +479,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     const float* gA = nullptr;
     {
       const int gr = row0 + 32 * (warp & 3) + lane;
-      const int ro = gr / RI, ri = gr - ro * RI;
+      const int rq = gr / RI, ri = gr - rq * RI, ro = ro0 + rq;
       long base;
       if (OP == kTcFwd)        base = ((spec0 + (long)ro * L) * p.nb + ri) * fi2;
       else if (OP == kTcGradX) base = ((spec0 + (long)ro * L) * p.nb + ri) * fo2;
@@ -645,32 +655,42 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
       }
     };
     load_columns(last_acc, v);
-    if (FLUSH && ngroups > 1) {
+    if (two_accs || (FLUSH && ngroups > 1)) {     // the products with a lo part, or the earlier groups' sum
       float w[32];
-      load_columns((uint32_t)kTcSumCol, w);
+      load_columns((uint32_t)(FLUSH ? kTcSumCol : kTcBN), w);
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] += w[i];
     }
   }
-  const int ro = r / RI, ri = r - ro * RI;
-  // c[((spec0 + ro * sro + co * sco) * RI + ri) * CW + rem]
+  const int rq = r / RI, ri = r - rq * RI, ro = ro0 + rq;
+  // spectral products: coefficient q = ro * sro + co * sco of the degree is c[((spec0 + q) * RI + ri) * CW + rem]; its
+  // mirror (-m, -n) is coefficient L * L - 1 - q, (-1)^(m - n) = (-1)^q times the conjugate (L is odd)
+  constexpr bool kPlain = OP == kTcPlainCC || OP == kTcPlainSC;
   const int sro = OP == kTcGradY ? 1 : L, sco = OP == kTcGradY ? L : 1;
+  const bool mirror = !kPlain && p.half && rq > 0;
+  auto at_coefficient = [&](int q, int rem) { return p.c + ((spec0 + q) * RI + ri) * CW + rem; };
+  auto mirrored = [](float4 o, float s) { return make_float4(s * o.x, -s * o.y, s * o.z, -s * o.w); };
   // two columns (one complex number: never straddles an outer column index), four with VEC
   auto store2 = [&](int gcol, float a, float b) {
     if (gcol >= Np) return;
-    if constexpr (OP == kTcPlainCC || OP == kTcPlainSC) {
+    if constexpr (kPlain) {
       if (OP == kTcPlainSC) { a *= p.scale; b *= p.scale; }
       *reinterpret_cast<float2*>(p.c + (long)r * p.c_rs + (long)(gcol >> 1) * p.c_ps) = make_float2(a, b);
     } else {
-      const int co = gcol / CW, rem = gcol - co * CW;
-      *reinterpret_cast<float2*>(p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem) = make_float2(a, b);
+      const int co = gcol / CW, rem = gcol - co * CW, q = ro * sro + co * sco;
+      *reinterpret_cast<float2*>(at_coefficient(q, rem)) = make_float2(a, b);
+      if (mirror) {
+        const float s = (q & 1) ? -1.f : 1.f;
+        *reinterpret_cast<float2*>(at_coefficient(L * L - 1 - q, rem)) = make_float2(s * a, -s * b);
+      }
     }
   };
   auto store4 = [&](int gcol, float4 o) {
-    if constexpr (VEC && OP != kTcPlainCC && OP != kTcPlainSC) {
+    if constexpr (VEC && !kPlain) {
       if (gcol >= Np) return;     // CW is a multiple of 4, so a group of 4 is all in or all out
-      const int co = gcol / CW, rem = gcol - co * CW;
-      *reinterpret_cast<float4*>(p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem) = o;
+      const int co = gcol / CW, rem = gcol - co * CW, q = ro * sro + co * sco;
+      *reinterpret_cast<float4*>(at_coefficient(q, rem)) = o;
+      if (mirror) *reinterpret_cast<float4*>(at_coefficient(L * L - 1 - q, rem)) = mirrored(o, (q & 1) ? -1.f : 1.f);
     } else {
       store2(gcol, o.x, o.y);
       store2(gcol + 2, o.z, o.w);
@@ -721,19 +741,24 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     }
     tc_cluster_sync();     // the others have read this CTA's part
   } else if (ok && warp != 0 && r < M) {
-    if (VEC && OP != kTcPlainCC && OP != kTcPlainSC && CW % 8 == 0 && reinterpret_cast<unsigned long long>(p.c) % 32 == 0) {
+    if (VEC && !kPlain && CW % 8 == 0 && reinterpret_cast<unsigned long long>(p.c) % 32 == 0) {
       // a lane owns a row: 32-byte stores write whole sectors (16-byte ones would send every
       // sector to L2 in two halves); CW % 8 == 0 keeps a group of 8 inside one outer column index
 #pragma unroll
       for (int c8 = 0; c8 < 4; ++c8) {
         const int gcol = col0 + cbase + 8 * c8;
         if (gcol < Np) {
-          const int co = gcol / CW, rem = gcol - co * CW;
-          float* dst = p.c + ((spec0 + (long)ro * sro + (long)co * sco) * RI + ri) * CW + rem;
+          const int co = gcol / CW, rem = gcol - co * CW, q = ro * sro + co * sco;
           float8 o;
           o.lo = make_float4(v[8 * c8], v[8 * c8 + 1], v[8 * c8 + 2], v[8 * c8 + 3]);
           o.hi = make_float4(v[8 * c8 + 4], v[8 * c8 + 5], v[8 * c8 + 6], v[8 * c8 + 7]);
-          st_global_256(dst, o);
+          st_global_256(at_coefficient(q, rem), o);
+          if (mirror) {
+            const float s = (q & 1) ? -1.f : 1.f;
+            o.lo = mirrored(o.lo, s);
+            o.hi = mirrored(o.hi, s);
+            st_global_256(at_coefficient(L * L - 1 - q, rem), o);
+          }
         }
       }
     } else {
@@ -777,9 +802,9 @@ inline bool so3_mm_tc_vec16(int op, int nb, int fi, int fo) {
   return (fi % 2 == 0) && (fo % 2 == 0);
 }
 
-inline long so3_mm_tc_tiles(int op, int nl, int nb, int fi, int fo) {
+inline long so3_mm_tc_tiles(int op, int half, int nl, int nb, int fi, int fo) {
   long t = 0;
-  for (int l = 0; l < nl; ++l) t += tc_tiles_for(op, nb, fi, fo, l);
+  for (int l = 0; l < nl; ++l) t += tc_tiles_for(op, half, nb, fi, fo, l);
   return t;
 }
 inline size_t tc_count_bytes(long tiles) { return align_up((size_t)tiles * kTcMaxCluster * sizeof(int), 256); }
@@ -801,10 +826,10 @@ struct TcShare {
 // products keep one CTA per tile.  One CTA per tile -> shared (us): 100 -> 255 channels, nl 5, batch 32, grad-x 123 -> 86;
 // 20 -> 40, nl 6, batch 32, grad-x 29 -> 14, grad-y 22 -> 14; 13 -> 9, nl 7, batch 5, grad-x 14 -> 9; kernel gradients
 // (rows x grid x spectrum) 800 x 192 x 286 26 -> 11, 10000 x 192 x 1330 137 -> 115, 128 x 36 x 4495 (15 clusters) 189 -> 16.
-inline TcShare tc_pick_share(int op, int nl, int nb, int fi, int fo, int nblk, bool several_clusters) {
+inline TcShare tc_pick_share(int op, int half, int nl, int nb, int fi, int fo, int nblk, bool several_clusters) {
   constexpr double kCta = 8, kShare = 4, kGather = 6;
   constexpr int kSlots[kTcMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
-  const long tiles = so3_mm_tc_tiles(op, nl, nb, fi, fo);
+  const long tiles = so3_mm_tc_tiles(op, half, nl, nb, fi, fo);
   auto estimate = [&](int c, int groups) {
     const int ns = c * groups;
     double load = 0, shortest = 0, longest = 0;
@@ -812,7 +837,7 @@ inline TcShare tc_pick_share(int op, int nl, int nb, int fi, int fo, int nblk, b
       const int blocks = (2 * l + 1) * nblk;
       shortest = (blocks + ns - 1) / ns + kCta + (ns > 1 ? kShare : 0) + (groups > 1 ? kGather : 0);
       longest = std::max(longest, shortest);
-      load += (double)tc_tiles_for(op, nb, fi, fo, l) * groups * shortest;
+      load += (double)tc_tiles_for(op, half, nb, fi, fo, l) * groups * shortest;
     }
     return tiles * groups <= kSlots[c] ? longest : std::max(longest, load / kSlots[c] + shortest);
   };

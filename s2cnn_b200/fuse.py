@@ -8,7 +8,8 @@ memory.  ``fuse`` traces the model once (``torch.fx``; the convolution modules a
 keyword arguments of this package's modules that select the fused kernels; everything else in the
 model is left as traced.  The result computes the same function.
 
-    conv_a -> relu -> SO3Convolution b     conv_a(x, relu_so3_fft=b.b_out); b(.., input_spectrum=True)
+    conv_a -> relu -> SO3Convolution b     conv_a(x, relu_so3_fft=b.b_out); b(.., input_spectrum=True,
+                                             real_spectrum=True)
                                            (synthesis, bias, ReLU and the next analysis in one kernel)
     conv -> BatchNorm3d (eval mode)        conv(x, channel_scale=s, bias=t): the normalisation is a
                                            per-channel affine map, folded into the kernel's spectrum
@@ -78,7 +79,7 @@ class _RecordedCalls:
 
 
 _OWN_KEYWORDS = {"relu_input", "relu_integrate", "input_spectrum", "relu_so3_fft", "channel_scale",
-                 "bias"}
+                 "bias", "real_spectrum"}
 
 
 def _fold_batchnorm(conv_bias, mean, var, weight, bias, eps):
@@ -177,7 +178,7 @@ def fuse(model):
                 # synthesis + bias + ReLU + the next layer's analysis in one kernel
                 src.kwargs = dict(src.kwargs, relu_so3_fft=consumer.b_out)
                 dst.args = (src,)
-                dst.kwargs = dict(dst.kwargs, input_spectrum=True)
+                dst.kwargs = dict(dst.kwargs, input_spectrum=True, real_spectrum=True)
                 graph.erase_node(node)
             elif 2 * consumer.b_in < 64:
                 dst.args = (src,)

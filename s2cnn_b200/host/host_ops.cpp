@@ -80,7 +80,7 @@ long s2_bandwidth(long nspec) {
   X(so3_rfft_relu) X(so3_rfft_sums_ws) X(so3_relay_workspace) X(s2_conv_relu_so3_rfft_workspace) X(s2_conv_relu_so3_rfft_ws) X(so3_rifft_relu_rfft_ws) X(so3_rifft_relu_grad_ws) X(so3_fft) X(so3_rifft)                 \
   X(so3_rifft_relu_integrate)                      \
   X(s2_conv_synthesis_workspace) X(s2_conv_synthesis) X(so3_ifft) X(s2_fft_workspace) X(s2_fft)    \
-  X(s2_ifft) X(so3_mm) X(so3_mm_gradx_ws) X(so3_mm_gradx_workspace) X(so3_mm_grady_ws) X(so3_mm_grady_workspace) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
+  X(s2_ifft) X(so3_mm) X(so3_mm_gradx_ws) X(so3_mm_gradx_workspace) X(so3_mm_grady_ws) X(so3_mm_grady_workspace) X(so3_mm_real) X(so3_mm_real_workspace) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
   X(s2_mm_grady) X(rft_forward) X(rft_forward_t) X(rft_forward_scaled) X(rft_backward_scaled) X(rft_backward_workspace) X(so3_integrate)                  \
   X(so3_integrate_backward) X(so3_rotate_spectrum) X(project_on_sphere)
 
@@ -476,6 +476,32 @@ struct Ops {
     const long nl = so3_bandwidth(x.size(0)), nb = x.size(1), fi = x.size(2);
     return mm_grad("s2c_so3_mm_grady", so3_mm_grady_ws_, so3_mm_grady_workspace_, gz, x, {so3_nspec(nl), fi, fo, 2}, nl, nb, fi, fo);
   }
+  // products of spectra of real signals; op as in s2c_so3_mm_real
+  Tensor mm_real(int op, const Tensor& u_, const Tensor& v_, at::IntArrayRef shape, long nl, long nb, long fi, long fo) {
+    prep(u_);
+    prep(v_);
+    const Tensor u = u_.contiguous(), v = v_.contiguous();
+    Tensor out = empty_like_shape(u, shape);
+    Ctx c(*this, u);
+    const Scratch ws(so3_mm_real_workspace_(op, (int)nl, (int)nb, (int)fi, (int)fo), u);
+    S2C_CALL(so3_mm_real, op, cptr(u), cptr(v), ptr(out), (int)nl, (int)nb, (int)fi, (int)fo, ws.p, ws.n, c.stream);
+    if (check_tc) check_tensor_core_status();
+    return out;
+  }
+  Tensor so3_mm_real(const Tensor& x, const Tensor& y) {
+    check(x.dim() == 4 && y.dim() == 4 && x.size(3) == 2 && y.size(3) == 2 && y.size(1) == x.size(2) && y.size(0) == x.size(0),
+          "so3_mm: x [l * m * n, batch, f_in, 2] and y [l * m * n, f_in, f_out, 2]");
+    const long nl = so3_bandwidth(x.size(0)), nb = x.size(1), fi = x.size(2), fo = y.size(2);
+    return mm_real(0, x, y, {so3_nspec(nl), nb, fo, 2}, nl, nb, fi, fo);
+  }
+  Tensor so3_mm_real_gradx(const Tensor& gz, const Tensor& y, int64_t nb, int64_t fi) {
+    const long nl = so3_bandwidth(y.size(0)), fo = y.size(2);
+    return mm_real(1, gz, y, {so3_nspec(nl), nb, fi, 2}, nl, nb, fi, fo);
+  }
+  Tensor so3_mm_real_grady(const Tensor& gz, const Tensor& x, int64_t fo) {
+    const long nl = so3_bandwidth(x.size(0)), nb = x.size(1), fi = x.size(2);
+    return mm_real(2, gz, x, {so3_nspec(nl), fi, fo, 2}, nl, nb, fi, fo);
+  }
   Tensor s2_mm(const Tensor& x, const Tensor& y) {
     const S2Product d = s2_product_dims(x, y);
     return mm("s2c_s2_mm", s2_mm_, x, y, {so3_nspec(d.b), d.nb, d.fo, 2}, d.b, d.nb, d.fi, d.fo);
@@ -714,13 +740,16 @@ struct S2ProductSynthesis : torch::autograd::Function<S2ProductSynthesis> {
   }
 };
 // s2cnn/so3_mm.py:95-122 and s2cnn/s2_mm.py:67-101
-template <bool SO3>
-struct SpectralMm : torch::autograd::Function<SpectralMm<SO3>> {
+enum MmKind { kSo3Mm, kSo3MmReal, kS2Mm };
+template <MmKind KIND>
+struct SpectralMm : torch::autograd::Function<SpectralMm<KIND>> {
   static Tensor forward(AutogradContext* ctx, int64_t ops, const Tensor& x, const Tensor& y) {
     keep_ops(ctx, ops);
     ctx->save_for_backward({x, y});
     Ops* o = reinterpret_cast<Ops*>(ops);
-    return SO3 ? o->so3_mm(x, y) : o->s2_mm(x, y);
+    // The forward product of a recorded pass stays the full one: the half product rounds differently, and through the
+    // ReLUs that follow a changed last bit of an activation moves a deep network's gradients by 1e-4 and more.
+    return KIND == kS2Mm ? o->s2_mm(x, y) : o->so3_mm(x, y);
   }
   static tensor_list backward(AutogradContext* ctx, tensor_list g) {
     const auto saved = ctx->get_saved_variables();
@@ -728,8 +757,11 @@ struct SpectralMm : torch::autograd::Function<SpectralMm<SO3>> {
     Ops* o = ops_of(ctx);
     Tensor gx, gy;
     const Tensor gz = g[0].contiguous();
-    if (ctx->needs_input_grad(0)) gx = SO3 ? o->so3_mm_gradx(gz, y, x.size(1), x.size(2)) : o->s2_mm_gradx(gz, y, x.size(1), x.size(2));
-    if (ctx->needs_input_grad(1)) gy = SO3 ? o->so3_mm_grady(gz, x, y.size(2)) : o->s2_mm_grady(gz, x, y.size(2));
+    const long nb = x.size(1), fi = x.size(2), fo = y.size(2);
+    if (ctx->needs_input_grad(0))
+      gx = KIND == kSo3Mm ? o->so3_mm_gradx(gz, y, nb, fi) : KIND == kSo3MmReal ? o->so3_mm_real_gradx(gz, y, nb, fi) : o->s2_mm_gradx(gz, y, nb, fi);
+    if (ctx->needs_input_grad(1))
+      gy = KIND == kSo3Mm ? o->so3_mm_grady(gz, x, fo) : KIND == kSo3MmReal ? o->so3_mm_real_grady(gz, x, fo) : o->s2_mm_grady(gz, x, fo);
     return {Variable(), gx, gy};
   }
 };
@@ -832,6 +864,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("so3_mm", &Ops::so3_mm, "x"_a, "y"_a, nogil)
       .def("so3_mm_gradx", &Ops::so3_mm_gradx, "gz"_a, "y"_a, "nb"_a, "fi"_a, nogil)
       .def("so3_mm_grady", &Ops::so3_mm_grady, "gz"_a, "x"_a, "fo"_a, nogil)
+      .def("so3_mm_real", &Ops::so3_mm_real, "x"_a, "y"_a, nogil)
+      .def("so3_mm_real_gradx", &Ops::so3_mm_real_gradx, "gz"_a, "y"_a, "nb"_a, "fi"_a, nogil)
+      .def("so3_mm_real_grady", &Ops::so3_mm_real_grady, "gz"_a, "x"_a, "fo"_a, nogil)
       .def("s2_mm", &Ops::s2_mm, "x"_a, "y"_a, nogil)
       .def("s2_mm_gradx", &Ops::s2_mm_gradx, "gz"_a, "y"_a, "nb"_a, "fi"_a, nogil)
       .def("s2_mm_grady", &Ops::s2_mm_grady, "gz"_a, "x"_a, "fo"_a, nogil)
@@ -869,11 +904,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           }, "x"_a, "y"_a, "bias"_a, nogil)
       .def("ag_so3_mm", [](Ops& o, const Tensor& x, const Tensor& y) {
             S2C_TRACED("ag_so3_mm", x, y);
-            return wants_grad(x, y) ? SpectralMm<true>::apply(id(o), x, y) : o.so3_mm(x, y);
+            return wants_grad(x, y) ? SpectralMm<kSo3Mm>::apply(id(o), x, y) : o.so3_mm(x, y);
+          }, "x"_a, "y"_a, nogil)
+      .def("ag_so3_mm_real", [](Ops& o, const Tensor& x, const Tensor& y) {
+            S2C_TRACED("ag_so3_mm_real", x, y);
+            return wants_grad(x, y) ? SpectralMm<kSo3MmReal>::apply(id(o), x, y) : o.so3_mm_real(x, y);
           }, "x"_a, "y"_a, nogil)
       .def("ag_s2_mm", [](Ops& o, const Tensor& x, const Tensor& y) {
             S2C_TRACED("ag_s2_mm", x, y);
-            return wants_grad(x, y) ? SpectralMm<false>::apply(id(o), x, y) : o.s2_mm(x, y);
+            return wants_grad(x, y) ? SpectralMm<kS2Mm>::apply(id(o), x, y) : o.s2_mm(x, y);
           }, "x"_a, "y"_a, nogil)
       .def("ag_rft", [](Ops& o, const Tensor& x, const Tensor& F, const OptTensor& Ft, double scale) {
             S2C_TRACED("ag_rft", x, F, Ft, scale);

@@ -44,11 +44,14 @@ class SO3Convolution(Module):
                                                             kernel.device))
 
     def forward(self, x, relu_input=False, relu_integrate=False, input_spectrum=False,
-                relu_so3_fft=None, channel_scale=None, bias=None):
+                relu_so3_fft=None, channel_scale=None, bias=None, real_spectrum=False):
         '''
         :x:      [batch, feature_in,  beta, alpha, gamma]
         :input_spectrum: (extension) x is already SO3_fft_real(signal, b_out), as returned by
                          ``S2Convolution.forward(..., relu_so3_fft=b_out)``
+        :real_spectrum: (extension, with input_spectrum) the caller has made x from a real signal, so that
+                         X[l,-m,-n] = (-1)^(m-n) conj X[l,m,n]; half of the spectral product is then computed
+                         and the other half mirrored, as for a signal given as x
         :relu_so3_fft: (extension) bandwidth b_next of the SO3Convolution that follows: return that
                        layer's input spectrum SO3_fft_real(relu(conv(x)), b_next) (see S2Convolution)
         :relu_input: (extension) compute conv(relu(x)); the activation is applied while x is read
@@ -80,7 +83,9 @@ class SO3Convolution(Module):
         own_bias = self.bias if bias is None else bias
         assert x.size(0) == y.size(0)
         assert x.size(2) == y.size(1)
-        z = so3_mm(x, y)  # [l * m * n, batch, feature_out, complex]
+        # [l * m * n, batch, feature_out, complex].  y is the spectrum of a real kernel: half products where x has
+        # the symmetry, too (without autograd, and for the gradients)
+        z = so3_mm(x, y) if input_spectrum and not real_spectrum else cuda_ops().ag_so3_mm_real(x, y)
         needs_grad = torch.is_grad_enabled() and (z.requires_grad or own_bias.requires_grad)
         opt_in = getattr(self, "fused_training", False)
         if relu_so3_fft is not None:

@@ -1,0 +1,100 @@
+"""Spectral products of real signals (``so3_mm_real`` and its gradients): half of the result is computed, the
+other half is its mirror.  Checked against the full product in float64 on spectra with the symmetry
+X[l,-m,-n] = (-1)^(m-n) conj X[l,m,n], at row counts around the 128-row tiles, odd sizes, one degree, and tiles
+shared by several thread blocks.  A spectrum that a caller hands to a layer keeps the full product unless the
+caller vouches for the symmetry."""
+import numpy as np
+import pytest
+import torch
+
+import s2cnn_b200 as S
+import backends
+from oracle import s2cnn_oracle as O
+from util import assert_close
+
+n3 = O.so3_nspec
+
+
+def mirrored(x, nl):
+    """(-1)^(m-n) conj X[l,-m,-n]; within a degree the mirror reverses the order and the sign alternates."""
+    out = torch.empty_like(x)
+    for l in range(nl):
+        s = slice(n3(l), n3(l + 1))
+        q = torch.arange((2 * l + 1) ** 2)
+        sign = (1.0 - 2.0 * (q % 2)).view(-1, 1, 1, 1).to(x.dtype)
+        out[s] = x[s].flip(0) * sign * torch.tensor([1.0, -1.0], dtype=x.dtype)
+    return out
+
+
+def real_spectrum(nl, *shape, gen):
+    x = torch.randn(n3(nl), *shape, 2, generator=gen)
+    return (x + mirrored(x, nl)) / 2
+
+
+def products64(x, y, gz, nl):
+    xc, yc, gc = (torch.view_as_complex(t.double()) for t in (x, y, gz))
+    z, gx, gy = torch.zeros_like(gc), torch.zeros_like(xc), torch.zeros_like(yc)
+    for l in range(nl):
+        L, s = 2 * l + 1, slice(n3(l), n3(l + 1))
+        xl, yl, gl = (t[s].reshape(L, L, *t.shape[1:]) for t in (xc, yc, gc))
+        z[s] = torch.einsum("mpik,npkj->mnij", xl, yl.conj()).reshape(L * L, *z.shape[1:])
+        gx[s] = torch.einsum("mnij,npkj->mpik", gl, yl).reshape(L * L, *gx.shape[1:])
+        gy[s] = torch.einsum("mnij,mpik->npkj", gl.conj(), xl).reshape(L * L, *gy.shape[1:])
+    return [torch.view_as_real(t) for t in (z, gx, gy)]
+
+
+@pytest.mark.parametrize("backend", backends.BACKENDS)
+@pytest.mark.parametrize("nl,nb,fi,fo", [(1, 1, 2, 2), (4, 32, 4, 6), (4, 33, 3, 5), (2, 64, 8, 12), (2, 65, 2, 3),
+                                         (7, 1, 20, 8), (9, 2, 1, 1), (3, 128, 26, 10), (6, 3, 24, 16)])
+def test_half_products_match_the_full_ones(backend, nl, nb, fi, fo):
+    ops, dev = backends.get(backend)
+    gen = torch.Generator().manual_seed(nl * 31 + nb)
+    x, y, gz = (real_spectrum(nl, *s, gen=gen) for s in ((nb, fi), (fi, fo), (nb, fo)))
+    want = products64(x, y, gz, nl)
+    xd, yd, gd = x.to(dev), y.to(dev), gz.to(dev)
+    got = [ops.so3_mm_real(xd, yd), ops.so3_mm_real_gradx(gd, yd, nb, fi), ops.so3_mm_real_grady(gd, xd, fo)]
+    full = [ops.so3_mm(xd, yd), ops.so3_mm_gradx(gd, yd, nb, fi), ops.so3_mm_grady(gd, xd, fo)]
+    for name, g, f, w in zip(("z", "gx", "gy"), got, full, want):
+        g, f = g.cpu(), f.cpu()
+        # 3xTF32: 2^-22 for the split and at most 2^-23 per truncated addition of a chain of 66: below 1e-5
+        err = [((t.double() - w).norm() / w.norm()).item() for t in (g, f)]
+        assert err[0] < 1e-5, (name, err)
+        assert_close(g, f, name)
+        if backend == "cuda":     # the halves mirror each other exactly (m = 0 is its own half: computed as a whole)
+            m0 = torch.cat([(torch.arange((2 * l + 1) ** 2) // (2 * l + 1) == l) if name != "gy" else
+                            (torch.arange((2 * l + 1) ** 2) % (2 * l + 1) == l) for l in range(nl)])
+            assert torch.equal(g[~m0], mirrored(g, nl)[~m0]), name
+    if backend == "cuda":
+        from s2cnn_b200 import _lib
+        assert _lib.cuda_lib().s2c_so3_mm_tc_status() == 0
+
+
+@pytest.mark.gpu
+def test_a_given_spectrum_keeps_the_full_product():
+    torch.manual_seed(3)
+    conv = S.SO3Convolution(3, 4, 5, 4, S.so3_near_identity_grid()).cuda()
+    x = torch.randn(n3(4), 2, 3, 2)                      # no symmetry
+    y = O.so3_rft(conv.kernel.detach().cpu() * conv.scaling, 4, conv.grid)
+    want = O.so3_rifft(O.so3_mm(x, y))                  # the synthesis takes the symmetric part of the product
+    with torch.no_grad():
+        assert_close(conv(x.cuda(), input_spectrum=True), want, "given spectrum")
+        xs = real_spectrum(4, 2, 3, gen=torch.Generator().manual_seed(1))
+        a = conv(xs.cuda(), input_spectrum=True)
+        b = conv(xs.cuda(), input_spectrum=True, real_spectrum=True)
+    assert_close(b, a, "real spectrum")
+
+
+@pytest.mark.gpu
+def test_layer_gradients_with_half_products():
+    """SO3Convolution forward and backward against the oracle in float64 (odd channel counts, b_out < b_in)."""
+    torch.manual_seed(4)
+    grid = S.so3_near_identity_grid(max_beta=np.pi / 8, n_alpha=4, n_beta=2, n_gamma=3)
+    conv = S.SO3Convolution(5, 3, 6, 4, grid)
+    x, gy = torch.randn(3, 5, 12, 12, 12), torch.randn(3, 3, 8, 8, 8)
+    xo, ko = x.clone().requires_grad_(True), conv.kernel.detach().clone().requires_grad_(True)
+    O.so3_convolution(xo, ko, conv.bias.detach(), 6, 4, grid).backward(gy)
+    conv = conv.cuda()
+    xd = x.cuda().requires_grad_(True)
+    conv(xd).backward(gy.cuda())
+    assert_close(xd.grad, xo.grad, "gx")
+    assert_close(conv.kernel.grad, ko.grad, "gkernel")
