@@ -92,6 +92,16 @@ inline int dev_memset_async(void* p, int v, size_t bytes, stream_t s) {
 }
 // Per-device values the host looks up on every call, remembered after the first (0 = not yet known).
 constexpr int kMaxDevices = 64;
+inline int dev_sm_count() {
+  static std::atomic<int> known[kMaxDevices];
+  const int dev = dev_current();
+  int n = dev < kMaxDevices ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+    if (dev < kMaxDevices) known[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
 inline int dev_smem_limit() {
   static std::atomic<int> known[kMaxDevices];
   const int dev = dev_current();
@@ -231,6 +241,15 @@ __device__ __forceinline__ void bulk_load_issue(void* dst, const void* src, unsi
           smem_u32(dst)),
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+// Shared -> global by the same engine, issued by one thread after bulk_store_fence() of every thread that wrote the
+// shared memory and a block barrier; bulk_store_wait() before the shared memory is given up.  16-byte aligned.
+__device__ __forceinline__ void bulk_store_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_issue(void* dst, const void* src, unsigned bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_store_wait() {
+  asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 // two independent single-precision operations in one instruction, each rounded as the scalar one
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -432,6 +451,7 @@ inline int dev_memset_async(void* p, int v, size_t bytes, stream_t) {
   return S2C_OK;
 }
 inline int dev_smem_limit() { return 227 * 1024; }
+inline int dev_sm_count() { return 3; }
 
 extern thread_local long g_launch_count;
 
@@ -484,6 +504,9 @@ inline void bulk_barrier_init(unsigned long long*) {}
 inline void bulk_load_issue(void* dst, const void* src, unsigned bytes, unsigned long long*) {
   std::memcpy(dst, src, bytes);
 }
+inline void bulk_store_fence() {}
+inline void bulk_store_issue(void* dst, const void* src, unsigned bytes) { std::memcpy(dst, src, bytes); }
+inline void bulk_store_wait() {}
 inline float2 fma2(float2 a, float2 b, float2 c) { return make_float2(std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)); }
 inline float relu(float v) { return v <= 0.f ? 0.f : v; }
 struct float8 {

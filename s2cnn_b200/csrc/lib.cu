@@ -7,6 +7,9 @@
 #include <algorithm>
 #include <atomic>
 #include <complex>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 #include "backend.h"
 #include "host_math.h"
@@ -62,9 +65,8 @@ static size_t so3_ws_per_z(int N, int K) {
 static size_t s2_ws_per_z(int N, int K) { return (size_t)(2 * K - 1) * N * sizeof(float2); }
 
 // Large-bandwidth path for N = 64 and 128: a plane kernel (both row transforms of a (z, beta)
-// plane) and a Wigner kernel per direction, through the scratch array V[n][z][beta][f] of
-// 8 K N^2 bytes per signal, in chunks of at most kRowsZC signals so that V stays in L2 between the
-// two kernels (b = 64: 8.4 MB per signal, 67 MB per chunk of the 126 MB).
+// plane) and a Wigner kernel per direction, through the scratch array V of
+// 8 K N^2 bytes per signal (8.4 MB at b = 64), in chunks of at most rows_zc(N) signals.
 static size_t so3_v_per_z(int N, int K) { return (size_t)K * N * N * sizeof(float2); }
 static bool use_plane_kernels(int N) { return plane_supported(N) && g_force_general < 2; }
 static int launch_fwd_plane(int N, long zc, stream_t st, const FwdPlaneParams& f) {
@@ -77,19 +79,50 @@ static int launch_inv_plane(int N, long zc, stream_t st, const InvPlaneParams& f
   if (N == 128) return S2C_LAUNCH_PLANE(so3_inv_plane, 128, grid, st, f);
   return S2C_LAUNCH_PLANE(so3_inv_plane, 64, grid, st, f);
 }
-static int launch_fwd_rows(int N, stream_t st, const FwdRowsParams& f) {
-  if (N == 128) return S2C_LAUNCH_ROWS(so3_fwd_wigner_r, 128, rows_grid(f.K, f.zc), st, f);
-  return S2C_LAUNCH_ROWS(so3_fwd_wigner_r, 64, rows_grid(f.K, f.zc), st, f);
+// The order in which the analysis' Wigner kernel takes its items, one block per SM (two at N = 64) walking its share:
+// sorted by their table rows and dealt out forwards and backwards in turn, so that the shares are equal to a few percent.
+// (In the order of n and m a quarter of the SM time was idle at b = 64: 48 us per 8 signals instead of 39.)
+static void rows_order(int nl, int K, RowsOrder* out) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, RowsOrder> known;
+  std::lock_guard<std::mutex> g(mu);
+  auto it = known.find({nl, K});
+  if (it == known.end()) {
+    if (known.size() >= 64) known.clear();
+    std::vector<std::pair<int, int>> pairs;      // (-rows, pair)
+    for (int n = 0; n < K; ++n)
+      for (int m0 = 0; m0 < K; m0 += kRowsMG) {
+        int rows = 0;
+        for (int m = m0; m < std::min(m0 + kRowsMG, K); ++m)
+          rows += std::max(0, nl - std::max(m, n) + kRowsStep - 1) / kRowsStep * kRowsStep;
+        pairs.push_back({-rows, n * kRowsMG + m0 / kRowsMG});
+      }
+    std::sort(pairs.begin(), pairs.end());
+    RowsOrder o{};
+    for (size_t i = 0; i < pairs.size(); ++i) o.pair[i] = (unsigned short)pairs[i].second;
+    it = known.emplace(std::make_pair(nl, K), o).first;
+  }
+  *out = it->second;
 }
+static int launch_fwd_rows(int N, stream_t st, FwdRowsParams& f) {
+  rows_order(f.nl, f.K, &f.order);
+  const long grid = std::min<long>(rows_items(f.K, f.zc), (N == 128 ? 1 : 2) * (long)dev_sm_count());
+  if (N == 128) return S2C_LAUNCH_FWD_ROWS(128, grid, st, f);
+  return S2C_LAUNCH_FWD_ROWS(64, grid, st, f);
+}
+// eight batch elements to a warp (a table value is then loaded once for eight numbers) where there are more than four
 static int launch_inv_rows(int N, stream_t st, const InvRowsParams& f) {
-  if (N == 128) return S2C_LAUNCH_ROWS(so3_inv_wigner_r, 128, rows_grid(f.K, f.zc), st, f);
-  return S2C_LAUNCH_ROWS(so3_inv_wigner_r, 64, rows_grid(f.K, f.zc), st, f);
+  const long grid = (long)f.K * ((f.K + kRowsMGI - 1) / kRowsMGI) * ((f.zc + 7) / 8);     // (one or two fours: the same)
+  if (f.zc > 4) {
+    if (N == 128) return S2C_LAUNCH_INV_ROWS(128, 8, grid, st, f);
+    return S2C_LAUNCH_INV_ROWS(64, 8, grid, st, f);
+  }
+  if (N == 128) return S2C_LAUNCH_INV_ROWS(128, 4, grid, st, f);
+  return S2C_LAUNCH_INV_ROWS(64, 4, grid, st, f);
 }
 
 // Runs `first(z0, zc, buffer, stream)` then `second(z0, zc, buffer, stream)` for every chunk of the
-// batch, in order on the caller's stream, through one scratch buffer.  (Running the two kernel
-// kinds of neighbouring chunks concurrently on two streams through two half-size buffers was
-// measured slower: both kinds are limited by the same shared-memory / L1 data path.)
+// batch, in order on the caller's stream, through one scratch buffer.
 template <class F1, class F2>
 static int plane_pipeline(long nbatch, int N, int K, void* ws, size_t ws_bytes, stream_t st,
                           F1 first, F2 second) {
@@ -99,8 +132,12 @@ static int plane_pipeline(long nbatch, int N, int K, void* ws, size_t ws_bytes, 
   if (fit < 1 || ws == nullptr)
     return fail(S2C_ERR_WORKSPACE, "workspace smaller than one batch element (" + std::to_string(vz) +
                                        " bytes needed)");
-  long chunk = (want >= 1 && want <= kRowsZC) ? want : kRowsZC;
+  long chunk = (want >= 1 && want <= rows_zc(N)) ? want : rows_zc(N);
   chunk = std::min(std::min(chunk, fit), nbatch);
+  if (want < 1) {      // equal chunks, of whole eights: the last one is not a fraction
+    const long parts = (nbatch + chunk - 1) / chunk;
+    chunk = std::min(chunk, ((nbatch + parts - 1) / parts + 7) / 8 * 8);
+  }
   for (long z0 = 0; z0 < nbatch; z0 += chunk) {
     const long zc = std::min(chunk, nbatch - z0);
     S2C_TRY(first(z0, zc, (float2*)ws, st));
@@ -215,7 +252,7 @@ constexpr size_t kAnySize = ~(size_t)0 / 2;
 // scratch that a route uses up in full (every transform also works with less, in shorter chunks)
 static size_t route_workspace(So3Route r, int N, int K, long nbatch) {
   if (r == kPlanes || r == kMid) return so3_mid_v_per_z(N, K) * (size_t)chunk_signals(nbatch, so3_mid_v_per_z(N, K));
-  if (r == kRows) return so3_v_per_z(N, K) * (size_t)std::min<long>(kRowsZC, nbatch);
+  if (r == kRows) return so3_v_per_z(N, K) * (size_t)std::min<long>(rows_zc(N), nbatch);
   if (r == kPasses) {
     const size_t per_z = so3_ws_per_z(N, K);
     return per_z * (size_t)std::min((long)std::max<size_t>(32, ((size_t)256 << 20) / per_z), nbatch);
@@ -778,7 +815,7 @@ size_t s2c_so3_fft_workspace(long nbatch, int b_in, int b_out) {
     // one signal of the three-pass organisation, which the test switches can select instead
     const int K = std::min(b_in, b_out);
     const size_t v = std::max(so3_v_per_z(2 * b_in, K), so3_v_per_z(2 * b_out, K));
-    return std::max(per_z, v * (size_t)std::min<long>(kRowsZC, std::max(1L, nbatch)));
+    return std::max(per_z, v * (size_t)std::min<long>(rows_zc(2 * b_in), std::max(1L, nbatch)));
   }
   const size_t target = (size_t)256 << 20;
   long chunk = (long)std::max<size_t>(32, target / per_z);

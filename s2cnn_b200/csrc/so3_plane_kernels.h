@@ -8,13 +8,9 @@
 //   synthesis (so3_inv_plane): the same steps reversed, ending with + bias and the store of the
 //       real plane.
 //
-// Scratch layout, chosen for THESE kernels:  V[n < K][z < zc][beta < N][f < N]  (complex), f the
-// raw FFT bin of the alpha transform (frequency m at f = m mod N).  A block that owns one plane
-// therefore reads / writes, for every kept n, one contiguous row of N complex numbers (1 KB at
-// b = 64), 64 aligned bytes per 8 lanes.  The Wigner kernels (wigner_rows.h) do the transposition to
-// "beta innermost" on their side, through shared memory, 32 bytes (one sector) at a time.  The batch
-// is processed in chunks of zc signals sized so that V (8 K N^2 bytes per signal) stays in L2
-// between the two kernels; the signal itself is read / written with streaming (evict-first) hints.
+// Scratch layout: wigner_rows.h's.  A block that owns one plane writes / reads, for every kept n, lines of 128 bytes
+// (sixteen frequencies); what an item of the Wigner kernels wants is one run of memory per sign.  The signal
+// itself is read / written with streaming (evict-first) hints.
 //
 // Every 1-D transform is a two-step register FFT (N = R1 * R2: R1-point transforms, twiddle,
 // transpose through a small buffer, R2-point transforms, natural order out) run by ONE WARP on four
@@ -34,6 +30,7 @@
 #include "backend.h"
 #include "fft_device.h"
 #include "fft_reg.h"
+#include "wigner_rows.h"
 
 namespace s2c {
 
@@ -51,13 +48,13 @@ inline void plane_st_stream(float* p, float v) { *p = v; }
 struct FwdPlaneParams {
   const float* x;     // real signal, element e at x[e * in_stride + in_off]
   long in_stride, in_off;
-  float2* v;          // [n < K][z < nbatch][beta][f < N]
+  float2* v;          // laid out as wigner_rows.h says
   const float2* tw;   // exp(+2 pi i k / N), k < N
   int nbatch, K;      // nbatch = signals of this chunk
 };
 
 struct InvPlaneParams {
-  const float2* s;    // [n < K][z < nbatch][beta][f < N]
+  const float2* s;    // laid out as wigner_rows.h says
   float* out;         // real signal, element e at out[e * out_stride + out_off]
   long out_stride, out_off;
   const float* bias;  // optional [nfeat]; feature of signal z is (z0 + z) % nfeat
@@ -92,14 +89,23 @@ S2C_HD constexpr int plane_col0(int RW, int warp) { return (warp % 8) + 8 * RW *
 S2C_HD constexpr int plane_col_warp(int RW, int nl) { return (nl % 8) + 8 * (nl / (8 * RW)); }
 S2C_HD constexpr int plane_col_row(int RW, int nl) { return (nl / 8) % RW; }
 
-// step 1 output: frequency pc of the R1-point transform, times W_N^(j pc), to dst[pc * (R2 + 1)]
-template <int R1, int R2, int DIR>
-S2C_D void plane_put_step1(float2 (&v)[R1], float2* dst, int j, const float2* tw) {
-  static_for<0, R1>([&](auto pc_) {
+// step 1 output: frequency pc of the 8-point transform, times W_N^(j pc), to dst[pc * (R2 + 1)].  A lane's j = lane % RB is
+// the same in every transform it takes part in, so its seven factors stay in registers (loaded from shared memory at
+// every use they were a third of the kernel's shared-memory wavefronts, bank conflicts of their strides included)
+struct PlaneTw {
+  float2 w[8];
+  S2C_D PlaneTw(const float2* tw, int j) {
+#pragma unroll
+    for (int pc = 1; pc < 8; ++pc) w[pc] = tw[j * pc];
+  }
+};
+template <int R2, int DIR>
+S2C_D void plane_put_step1(float2 (&v)[8], float2* dst, const PlaneTw& tw) {
+  static_for<0, 8>([&](auto pc_) {
     constexpr int pc = decltype(pc_)::value;
-    constexpr int pp = fft_reg_pos<R1>(pc);
+    constexpr int pp = fft_reg_pos<8>(pc);
     if constexpr (pc == 0) dst[0] = v[pp];
-    else dst[pc * (R2 + 1)] = ctw<DIR>(v[pp], tw[j * pc]);
+    else dst[pc * (R2 + 1)] = ctw<DIR>(v[pp], tw.w[pc]);
   });
 }
 
@@ -152,6 +158,7 @@ struct so3_fwd_plane_impl {
 #endif
     for (int i = ctx.tid; i < N; i += ctx.nthr) tw[i] = p.tw[i];
     ctx.sync();
+    const PlaneTw step_tw(tw, lane % RB);
 #pragma unroll
     for (int gi = 0; gi < NG; ++gi) {
       const int g = gi * NW + warp;
@@ -164,7 +171,7 @@ struct so3_fwd_plane_impl {
         if (gi * IT + ii + 1 < NG * IT) load_batch(gi * IT + ii + 1, vnext);
         if (RW * RB < 32 && it >= RW * RB) continue;
         fft_reg<8, -1>(v, tw);
-        plane_put_step1<8, RB, -1>(v, wtmp + tl * LDT + j, j, tw);
+        plane_put_step1<RB, -1>(v, wtmp + tl * LDT + j, step_tw);
       }
       ctx.sync_warp();
       if (lane < RW * 8) {
@@ -203,7 +210,7 @@ struct so3_fwd_plane_impl {
             v[kk + 4] = make_float2(0.5f * (a.y + cc.y), -0.5f * (a.x - cc.x));     // row t + N/2
           }
           fft_reg<8, -1>(v, tw);
-          plane_put_step1<8, RB, -1>(v, wtmp + i * LDT + j, j, tw);
+          plane_put_step1<RB, -1>(v, wtmp + i * LDT + j, step_tw);
         }
       }
       ctx.sync_warp();
@@ -215,13 +222,17 @@ struct so3_fwd_plane_impl {
 #pragma unroll
         for (int j = 0; j < RB; ++j) u[j] = src[j];
         fft_reg<RB, -1>(u, tw);
-        // row of this (n, z, beta): bins pq + 8 q; eight neighbouring lanes write 64 aligned bytes
-        float2* vrow = p.v + (((long)n * p.nbatch + z) * N + beta) * N + pq;
+        // bins f = pq + 8 q of this (n, z, beta): eight neighbouring lanes write half a line.  f = N/2 is |m| = N/2 >= K:
+        // never read
+        const RowsBins<8> bins(N, p.nbatch, (int)z, beta, pq);
+        float2* vn = p.v + (long)n * 2 * rows_groups(N) * bins.gs;
         static_for<0, RB>([&](auto q_) {
           constexpr int q = decltype(q_)::value;
-          const int f = pq + 8 * q;
-          const int m = f < N / 2 ? f : f - N;       // f = N/2 is |m| = N/2 >= K: never read
-          if (m > -K && m < K) vrow[8 * q] = u[fft_reg_pos<RB>(q)];
+          if constexpr (q < RB / 2) {
+            if (pq + 8 * q < K) vn[bins.pos(q)] = u[fft_reg_pos<RB>(q)];
+          } else {
+            if (8 * (RB - q) - pq < K) vn[bins.neg(RB - q)] = u[fft_reg_pos<RB>(q)];
+          }
         });
       }
       ctx.sync_warp();
@@ -255,14 +266,17 @@ struct so3_inv_plane_impl {
       const int it = (bi % IT) * 32 + lane, i = it / RB, j = it % RB;
       const int n = (RW * RB < 32 && it >= RW * RB) ? K : n0 + 8 * i;
       if (n < K) {
-        // bins j + RB k of the row of this (n, z, beta): RB neighbouring lanes read RB * 8
-        // contiguous bytes per k
-        const float2* srow = p.s + (((long)n * p.nbatch + z) * N + beta) * N + j;
+        // bins j + RB k of this (n, z, beta): RB neighbouring lanes read RB * 8 contiguous bytes per k
+        const RowsBins<RB> bins(N, p.nbatch, (int)z, beta, j);
+        const float2* sn = p.s + (long)n * 2 * rows_groups(N) * bins.gs;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const int f = j + RB * k;
-          const int m = f < N / 2 ? f : f - N;
-          v[k] = (m > -K && m < K) ? srow[RB * k] : make_float2(0.f, 0.f);
+          v[k] = make_float2(0.f, 0.f);
+          if (k < 4) {
+            if (j + RB * k < K) v[k] = sn[bins.pos(k)];
+          } else {
+            if (RB * (8 - k) - j < K) v[k] = sn[bins.neg(8 - k)];
+          }
         }
       }
     };
@@ -277,6 +291,7 @@ struct so3_inv_plane_impl {
       }
     }
     ctx.sync();
+    const PlaneTw step_tw(tw, lane % RB);
     for (int c = 0; c < nchunks; ++c) {
       const int n0 = c * 32 + plane_col0(RW, warp);
 #pragma unroll
@@ -289,7 +304,7 @@ struct so3_inv_plane_impl {
         if (c * IT + ii + 1 < nchunks * IT) load_batch(c * IT + ii + 1, vnext);
         if (n < K) {
           fft_reg<8, +1>(v, tw);
-          plane_put_step1<8, RB, +1>(v, wtmp + i * LDA + j, j, tw);
+          plane_put_step1<RB, +1>(v, wtmp + i * LDA + j, step_tw);
         }
       }
       ctx.sync_warp();
@@ -336,7 +351,7 @@ struct so3_inv_plane_impl {
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = src[RB * k];
         fft_reg<8, +1>(v, tw);
-        plane_put_step1<8, RB, +1>(v, wtmp + tl * LDG + j, j, tw);
+        plane_put_step1<RB, +1>(v, wtmp + tl * LDG + j, step_tw);
       }
       ctx.sync_warp();
       if (lane < RW * 8) {

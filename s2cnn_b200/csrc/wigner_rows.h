@@ -1,44 +1,91 @@
-// Wigner-d contractions of the large-bandwidth SO(3) path (N = 2b in {64, 128}), written for SMALL
-// batch chunks: the scratch array V between the plane kernels (so3_plane_kernels.h) and these
-// kernels must stay in L2, so a launch sees only a handful of signals and a tile that reuses a
-// staged Wigner panel over many batch elements (wigner_tiled.h) has nothing to reuse it over.
+// Wigner-d contractions of the large-bandwidth SO(3) path (N = 2b in {64, 128}), between the spectrum and the scratch
+// array V of the plane kernels (so3_plane_kernels.h).
 //
 // Same arithmetic as so3_fwd_wigner / so3_inv_wigner (so3_kernels.h), i.e. the beta / l contraction
 // of the reference's so3fft.cu / so3ifft.cu tile loops (s2cnn/soft/so3_fft.py:296-336, :391-431).
 //
-// Organisation: the 32 lanes of a warp split the BETA axis; a warp owns the frequency pair
-// (+m, n) and (-m, n) for four batch elements, a block of 8 warps eight consecutive values of |m|.
+// Organisation: a warp owns the frequency pair (+m, n) and (-m, n).  Analysis: for four batch elements, a block of 16
+// warps sixteen consecutive values of |m|, and one block per SM walks its share of these items.  Synthesis: for eight
+// batch elements (four where there are no more), a block of 4 warps.
 //   * The table holds only the first half of the beta range (TableCache::half_panels): the
 //     SOFT grid maps onto itself under beta -> pi - beta and
 //         d^l_{m,n}(pi - beta_j) = (-1)^(l+n) d^l_{-m,n}(beta_j),
 //     so the second half of panel (m, n) is the first half of panel (-m, n) up to that sign.  A warp
 //     reads row l of both half panels once and uses each for both members of its pair.
-//   * Panel rows reach a warp through a private ring in shared memory filled by 16-byte
-//     asynchronous copies (cp.async), kRowsDepth - 1 steps ahead of their use: with one outstanding
-//     row per warp the kernels ran at the latency, not the bandwidth, of L2 / HBM.  (Copies of 4 or
-//     8 bytes per lane cost about six times the shared-memory wavefronts of 16-byte ones, so a lane
-//     copies 16 bytes and reads the 4 or 8 bytes it needs after a warp barrier.)
-//   * analysis: the warp keeps its slice of V in registers for the whole pair and streams the
-//     panel rows; every two degrees end with a sum over the lanes (a 32-value transpose-reduce by
-//     shuffles, after which lane i holds value i).
-//   * synthesis: the accumulators (one beta slice of four signals per lane) stay in registers
-//     while the rows stream; no cross-lane traffic at all.
-//   * V is [n][z][beta][f] (f = alpha-frequency bin, see so3_plane_kernels.h): rows of one (z, beta)
-//     are 8 N bytes apart, so the block moves its 16 columns (+-m) between global and shared memory
-//     as 64-byte runs - four neighbouring lanes, 16 bytes each, per run - and the lanes read / write
-//     the transposed tile [column][z][beta] without bank conflicts.
+//   * The 32 lanes are 8 slices of the half beta range (lane b owns the runs of four 4 b .. and, at N = 128,
+//     32 + 4 b ..: 16-byte pieces of a table row) times 4 quarters of the numbers of a beta: one member of the pair
+//     and half of the batch elements each.  A lane has 16 (8) betas of its four or eight numbers in registers - V in the analysis,
+//     the sums in the synthesis - and pairs of neighbouring betas are the two halves of the packed multiply-adds, so
+//     that no table value is duplicated into a register pair.
+//   * Panel rows reach a warp through a private ring in shared memory filled by 16-byte asynchronous copies
+//     (cp.async), four rows a step.
+//   * analysis: an output is the sum over the 8 slices.  In step r of four rows lane b works on row r XOR (b % 4), so
+//     that what two lanes exchange sits in the same register of both: 4 shuffles and additions for 4 rows and each of a
+//     lane's numbers, no selects; lanes b and b + 4 end up with row b and write it and its mirror.
+//   * analysis: V comes as bulk copies, see below; an item's part is fetched while the one before is worked on (its
+//     numbers are in registers then).
+//   * synthesis: the accumulators stay in registers while the rows stream; they leave as runs of 32 bytes.
+//
+// Bound by latency and the shared-memory pipe (analysis: a lane loads 16 floats of table for 64 multiply-adds, 16 + 4 (ring)
+// + 4 (shuffles) clocks of the pipe per row; issue 49 %, packed multiply-adds 45 % of the time).  64 signals at b = 64:
+// analysis 275 us, synthesis 309; with one slice of V per lane of 32, staged through registers (124 instructions of
+// sums for 64 multiply-adds, V fetched in 64-byte pieces), in chunks of 8 signals: 407 and 390.  Eight batch elements to a
+// warp in the analysis, V in pieces of 32 bytes: 8 warps per SM, 35 instead of 39 us per 8 signals, which the plane
+// kernels lost to the shorter pieces.  The synthesis as one walking block of 16 warps and bulk stores: 50 us instead of 46.
 #pragma once
 
 #include "backend.h"
+#include "fft_reg.h"
 #include "so3_kernels.h"
 
 namespace s2c {
 
-constexpr int kRowsMG = 8;      // values of |m| per block = warps per block
-constexpr int kRowsZQ = 4;      // batch elements per block (and per warp)
-constexpr int kRowsZC = 8;      // batch elements per chunk (what the host sizes V for)
+// Batch elements per chunk, 256 MB of V.  That is more than L2 holds: long launches weigh more than keeping V in L2 (64
+// signals at b = 64, analysis / synthesis: 651 / 699 us in chunks of 8 (67 MB), 603 / 637 of 16, 589 / 615 of 32, 581 / 602
+// of 64; 512 signals at b = 32: 1190 / 1188 us of 8, 632 / 666 of 32, 576 / 617 of 64, 525 / 602 of 128, 500 / 574 of 256).
+S2C_HD constexpr int rows_zc(int N) { return N == 128 ? 32 : 256; }
+constexpr int kRowsZQ = 4;      // batch elements per item
+constexpr int kRowsMG = 16;     // values of |m| per item = warps per block
 constexpr int kRowsThreads = 32 * kRowsMG;
-constexpr int kRowsDepth = 8;   // ring slots per warp
+constexpr int kRowsStep = 4;    // table rows per ring step
+#ifndef S2C_EMUL
+constexpr int kRowsSlotsF = 3;  // ring steps per warp: analysis
+#else
+constexpr int kRowsSlotsF = 2;  // (the exchange buffer needs the room)
+#endif
+// the synthesis: four values of |m| (warps) and up to ZQ = 8 or 4 batch elements per block
+constexpr int kRowsMGI = 4, kRowsThreadsI = 32 * kRowsMGI, kRowsSlotsI = 4;
+
+// V between the plane kernels and these: [n < K][sign of m][|m| / 16][z < zc][beta][|m| % 16], so that the plane kernels
+// see lines of 128 bytes and an item's part is one run per sign (a bulk copy).  Within a line the order is XOR-ed with a
+// number of four bits: the lanes of a half warp, which hold betas four apart of two halves of the batch elements, then
+// touch all banks at once.
+S2C_HD constexpr int rows_groups(int N) { return N / (2 * kRowsMG); }      // per sign
+S2C_HD constexpr long rows_group_stride(int N, int zc) { return (long)zc * N * kRowsMG; }
+S2C_HD constexpr int rows_swizzle(int z, int beta) { return ((beta >> 2) & 7) | (((z >> 1) & 1) << 3); }
+// Where the bins of one (n, z, beta) lie that a lane handles in a transform over f: f = j + step q for the frequencies
+// m = f in the first half, and m = -(step M - j) in the second; step 8 or 16, j < step.
+template <int STEP>
+struct RowsBins {
+  long gs;
+  int pos0, pos1;        // step 8: even / odd q
+  long neg0, neg1;       // even / odd M
+  S2C_D RowsBins(int N, int zc, int z, int beta, int j) : gs(rows_group_stride(N, zc)) {
+    const int at = z * N * kRowsMG, line = beta * kRowsMG, h = rows_swizzle(z, beta);
+    pos0 = at + ((line + j) ^ h);
+    const long ng = rows_groups(N) * gs + at;
+    if (STEP == 16) {
+      pos1 = pos0;
+      neg0 = neg1 = j == 0 ? ng + (line ^ h) : ng - gs + ((line + 16 - j) ^ h);
+    } else {
+      pos1 = at + ((line + 8 + j) ^ h);
+      neg0 = j == 0 ? ng + (line ^ h) : ng - gs + ((line + 16 - j) ^ h);
+      neg1 = ng + (j == 0 ? ((line + 8) ^ h) : ((line + 8 - j) ^ h));
+    }
+  }
+  S2C_D long pos(int q) const { return STEP == 16 ? pos0 + q * gs : (q & 1 ? pos1 : pos0) + (q >> 1) * gs; }
+  S2C_D long neg(int M) const { return STEP == 16 ? neg0 + M * gs : (M & 1 ? neg1 : neg0) + (M >> 1) * gs; }
+};
 
 struct HalfPanelsDev {
   int nbeta;                // N = 2 b of the beta grid
@@ -47,44 +94,46 @@ struct HalfPanelsDev {
   const long long* off;     // npairs + 1 offsets in floats
 };
 
+// The pairs (n, sixteen values of |m|) of the analysis' items, those with the longest rows first: 16 n + m / 16.  Item i is
+// pair i / nzq and the batch elements from 4 (i % nzq); block b of G walks the items b, 2 G - 1 - b, 2 G + b, 4 G - 1 - b, ...
+constexpr int kRowsMaxPairs = 64 * 4;
+struct RowsOrder {
+  unsigned short pair[kRowsMaxPairs];
+};
+
 struct FwdRowsParams {
-  const float2* v;      // [n < K][z < zc][beta][f]
+  const float2* v;      // (see rows_swizzle)
   float2* out;          // spectrum rows of out_zstride complex, already offset to the chunk's z0
   long out_zstride;
   HalfPanelsDev pan;
-  int zc, K, nl, mode;  // mode: kSo3Real or kSo3AccumI
+  int zc, K, nl, mode;  // zc <= rows_zc(N) batch elements; mode: kSo3Real or kSo3AccumI
+  RowsOrder order;
 };
 
 struct InvRowsParams {
   const float2* x;      // spectrum rows of x_zstride complex, offset to the chunk's z0
   long x_zstride;
-  float2* s;            // [n < K][z < zc][beta][f]
+  float2* s;            // (see rows_swizzle)
   HalfPanelsDev pan;
   int zc, K, mode;      // mode: kSo3Real or kSo3RotI
 };
 
-// Shared memory: the tile [16 columns][4 z][N beta] of complex numbers with a column stride of
-// 4 N + 2 (so that four lanes storing to four columns hit four different bank groups).  The rings
-// [warp][depth][rows per step][A, B][N / 2] live inside it: the analysis is done with the tile once
-// every warp has its slice of V in registers (8 rings of depth 8 x 2 rows fill it), the synthesis
-// keeps the symmetrised spectrum rows in the lower half until the tile is written and its rings
-// (depth 8 x 1 row) in the upper half.  (+ in the host-emulation build a per-warp exchange buffer
-// that stands in for the shuffles.)
-template <int N>
-S2C_HD constexpr int rows_cs() { return kRowsZQ * N + 2; }
-template <int N>
-S2C_HD constexpr int rows_tile_floats() { return 2 * kRowsMG * rows_cs<N>() * 2; }
-template <int N>
-S2C_HD constexpr int rows_ring_floats(int rows_per_step) { return kRowsDepth * rows_per_step * 2 * (N / 2); }
-template <int N>
-inline size_t rows_smem_bytes() {
-  static_assert(kRowsMG * rows_ring_floats<N>(2) <= rows_tile_floats<N>(), "analysis rings");
-  static_assert(kRowsMG * rows_ring_floats<N>(1) <= rows_tile_floats<N>() / 2, "synthesis rings");
-  size_t b = (size_t)rows_tile_floats<N>() * sizeof(float);
+// Shared memory.  Analysis: the item's part of V, [sign][4 z][N beta][16], and behind it the rings
+// [warp][slot][row][A, B][N / 2].  Synthesis: the block's part of V, [sign][ZQ z][N beta][4] (before it the symmetrised
+// spectrum rows [8 columns][degree][ZQ z]), and the rings.  (+ in the host-emulation build a per-warp exchange buffer that
+// stands in for the shuffles.)
+S2C_HD constexpr int rows_tile_floats(int N) { return 2 * kRowsZQ * N * kRowsMG * 2; }
+S2C_HD constexpr int rows_ring_floats(int N, int slots) { return slots * kRowsStep * N; }      // per warp
+S2C_HD constexpr size_t rows_fwd_smem(int N) {
+  size_t b = (rows_tile_floats(N) + kRowsMG * rows_ring_floats(N, kRowsSlotsF)) * sizeof(float) + 32;
 #ifdef S2C_EMUL
-  b += (size_t)kRowsMG * 32 * 33 * sizeof(float);
+  b += (size_t)kRowsMG * 32 * 17 * sizeof(float);
 #endif
   return b;
+}
+S2C_HD constexpr int rows_inv_tile_floats(int N, int ZQ) { return 2 * ZQ * N * kRowsMGI * 2; }
+S2C_HD constexpr size_t rows_inv_smem(int N, int ZQ) {
+  return (rows_inv_tile_floats(N, ZQ) + kRowsMGI * rows_ring_floats(N, kRowsSlotsI)) * sizeof(float);
 }
 
 // 16 bytes global -> shared, asynchronously; groups complete in issue order
@@ -93,74 +142,86 @@ S2C_D void rows_copy16_async(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 S2C_D void rows_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// kRowsDepth - 1 steps are in flight: wait until at most kRowsDepth - 2 of this thread's copy
-// groups are pending, i.e. the oldest has landed.  (The step issued next goes into the slot that
-// was read one iteration earlier, never into the one being read.)
-S2C_D void rows_wait_oldest() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(kRowsDepth - 2) : "memory");
+// Of this thread's SLOTS copy groups all but the oldest may be pending.
+template <int SLOTS>
+S2C_D void rows_wait_oldest() { asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS - 1) : "memory"); }
+S2C_D float2 rows_mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
 }
 #else
 inline void rows_copy16_async(float* dst, const float* src) {
   for (int i = 0; i < 4; ++i) dst[i] = src[i];
 }
 inline void rows_commit() {}
+template <int SLOTS>
 inline void rows_wait_oldest() {}
+inline float2 rows_mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 #endif
 
-// ---- sum over the lanes of a warp: v[i] of every lane -> lane i -------------------------------
+// ---- four rows, summed over the 8 beta slices of a warp ------------------------------------------
+// part(r) is this lane's part (two complex numbers) of row r XOR (b % 4), b = lane % 8; returns the sum of row b % 4 over
+// the 8 lanes of its quarter.  After the exchange over bit 2 lane b holds rows r XOR (b % 4), r < 2, and so on.
 #ifndef S2C_EMUL
-S2C_D float rows_reduce32(const Ctx&, float (&v)[32], int lane, float*) {
-#pragma unroll
-  for (int step = 16; step >= 1; step >>= 1) {
-    const bool upper = (lane & step) != 0;
-#pragma unroll
-    for (int k = 0; k < step; ++k) {
-      const float send = upper ? v[k] : v[k + step];
-      const float keep = upper ? v[k + step] : v[k];
-      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, step);
-    }
-  }
-  return v[0];
+S2C_D float4 rows_add_from(float4 v, float4 w, int bit) {
+  v.x += __shfl_xor_sync(0xffffffffu, w.x, bit);
+  v.y += __shfl_xor_sync(0xffffffffu, w.y, bit);
+  v.z += __shfl_xor_sync(0xffffffffu, w.z, bit);
+  v.w += __shfl_xor_sync(0xffffffffu, w.w, bit);
+  return v;
 }
-S2C_D float rows_partner(const Ctx&, float v, int, float*) {
-  return __shfl_xor_sync(0xffffffffu, v, 1);
+template <class Part>
+S2C_D float4 rows_sum4(const Ctx&, Part part, int, float*) {
+  float4 v0 = part(std::integral_constant<int, 0>{}), v1 = part(std::integral_constant<int, 1>{});
+  v0 = rows_add_from(v0, part(std::integral_constant<int, 2>{}), 2);
+  v1 = rows_add_from(v1, part(std::integral_constant<int, 3>{}), 2);
+  v0 = rows_add_from(v0, v1, 1);
+  return rows_add_from(v0, v0, 4);
 }
 #else
-// every warp of the block calls these equally often (a warp barrier is a block barrier here)
-inline float rows_reduce32(const Ctx& ctx, float (&v)[32], int lane, float* xch) {
-  for (int k = 0; k < 32; ++k) xch[lane * 33 + k] = v[k];
+// every warp of the block calls this equally often (a warp barrier is a block barrier here)
+template <class Part>
+inline float4 rows_sum4(const Ctx& ctx, Part part, int lane, float* xch) {
+  const int b = lane & 3;
+  static_for<0, 4>([&](auto r) {
+    constexpr int k = decltype(r)::value;
+    const float4 v = part(std::integral_constant<int, k>{});
+    float* dst = xch + lane * 17 + (k ^ b) * 4;
+    dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
+  });
   ctx.sync_warp();
-  float s = 0.f;
-  for (int t = 0; t < 32; ++t) s += xch[t * 33 + lane];
+  float o[4];
+  for (int c = 0; c < 4; ++c) {     // the order of the shuffles: bits 2, 1, 4
+    auto at = [&](int x) { return xch[(lane ^ x) * 17 + b * 4 + c]; };
+    auto two = [&](int x) { return at(x) + at(x ^ 2); };
+    auto four = [&](int x) { return two(x) + two(x ^ 1); };
+    o[c] = four(0) + four(4);
+  }
   ctx.sync_warp();
-  return s;
-}
-inline float rows_partner(const Ctx& ctx, float v, int lane, float* xch) {
-  xch[lane] = v;
-  ctx.sync_warp();
-  const float r = xch[lane ^ 1];
-  ctx.sync_warp();
-  return r;
+  return make_float4(o[0], o[1], o[2], o[3]);
 }
 #endif
 
-// which (n, |m| group, z quad) a block owns, and the columns of its tile:
-//   c < 8:   frequency +(m0 + c)      at bin f = m0 + c
-//   c >= 8:  frequency -(m0 + c - 8)  at bin f = N - (m0 + c - 8)      (not for m = 0)
 struct RowsGeom {
-  int n, m0, zq;
+  int n, m0, zbase, nz;      // nz: batch elements there are, up to 4
 };
-S2C_D RowsGeom rows_geom(int bid, int K, int zc) {
-  const int ngroups = (K + kRowsMG - 1) / kRowsMG, nzq = (zc + kRowsZQ - 1) / kRowsZQ;
+S2C_D RowsGeom rows_geom(const RowsOrder& order, int item, int zc) {
+  const int nzq = (zc + kRowsZQ - 1) / kRowsZQ, pair = order.pair[item / nzq];
   RowsGeom g;
-  g.zq = bid % nzq;
-  const int t = bid / nzq;
-  g.n = t / ngroups;
-  g.m0 = (t - g.n * ngroups) * kRowsMG;
+  g.n = pair / kRowsMG;
+  g.m0 = pair % kRowsMG * kRowsMG;
+  g.zbase = item % nzq * kRowsZQ;
+  g.nz = zc - g.zbase < kRowsZQ ? zc - g.zbase : kRowsZQ;
   return g;
 }
-inline long rows_grid(int K, int zc) {
-  return (long)K * ((K + kRowsMG - 1) / kRowsMG) * ((zc + kRowsZQ - 1) / kRowsZQ);
+S2C_HD int rows_items(int K, int zc) { return K * ((K + kRowsMG - 1) / kRowsMG) * ((zc + kRowsZQ - 1) / kRowsZQ); }
+// an item's part of V for sign s, [z][beta][16]
+S2C_D long rows_part(int N, int zc, const RowsGeom& g, int s) {
+  return (((long)g.n * 2 + s) * rows_groups(N) + g.m0 / kRowsMG) * rows_group_stride(N, zc) + (long)g.zbase * N * kRowsMG;
 }
 
 // half-panel rows of the pair (+m, n) and (-m, n); for n = 0 only m >= 0 is stored and
@@ -183,27 +244,38 @@ S2C_D RowsPanels rows_panels(const HalfPanelsDev& pan, int m, int n) {
   return r;
 }
 
-// One ring step = S rows of both half panels: [row][A, B][NH] floats, copied 16 bytes per lane.
-template <int N, int S>
-S2C_D void rows_issue(float* ring, int t, const float* pa, const float* pb, int L, int lane) {
-  constexpr int NH = N / 2, P = NH / 4;      // 16-byte pieces per half-panel row
-  float* slot = ring + (t % kRowsDepth) * (S * 2 * NH);
-#pragma unroll
-  for (int piece = lane; piece < S * 2 * P; piece += 32) {
-    const int r = piece / (2 * P), rem = piece - r * 2 * P, ab = rem / P, q = rem - ab * P;
-    const int row = S * t + r;
-    if (row < L)
-      rows_copy16_async(slot + (r * 2 + ab) * NH + 4 * q, (ab ? pb : pa) + (long)row * NH + 4 * q);
+// A warp's ring: a step is kRowsStep rows of both half panels, [row][A, B][NH] floats, copied 16 bytes per lane.  A lane
+// copies the same piece of every row (N = 64: of every other row).
+template <int N, int SLOTS>
+struct RowsRing {
+  static constexpr int NH = N / 2, kPieces = N / 4, kRowsAtOnce = 32 / kPieces;
+  float* base;
+  const float* src;
+  int row0, L, dst, lane_row;
+  S2C_D RowsRing(float* ring, const RowsPanels& pn, int lane, int rows) : base(ring), L(rows) {
+    const int piece = lane % kPieces, ab = piece / (kPieces / 2), q = piece - ab * (kPieces / 2);
+    lane_row = lane / kPieces;
+    row0 = lane_row;
+    src = (ab ? pn.b : pn.a) + (long)lane_row * NH + 4 * q;
+    dst = lane_row * 2 * NH + 4 * piece;
   }
-  rows_commit();   // one group per step, empty or not, so that the wait counts steps
-}
+  S2C_D const float* slot(int t) const { return base + (t % SLOTS) * (kRowsStep * 2 * NH); }
+  S2C_D void issue(int t) {     // the next step, into slot t
+    float* d = base + (t % SLOTS) * (kRowsStep * 2 * NH) + dst;
+#pragma unroll
+    for (int r = 0; r < kRowsStep; r += kRowsAtOnce)
+      if (row0 + r < L) rows_copy16_async(d + r * 2 * NH, src + (long)r * NH);
+    row0 += kRowsStep;
+    src += kRowsStep * NH;
+    rows_commit();   // one group per step, empty or not, so that the wait counts steps
+  }
+};
 
-// The tile rows a thread moves: thread = (run piece q < 4, row r0 < 64), rows r0 + 64 k.
-template <int N>
-struct RowsTileMap {
-  static constexpr int kPasses = kRowsZQ * N / 64;
-  int q, r0;
-  S2C_D explicit RowsTileMap(int tid) : q(tid & 3), r0(tid >> 2) {}
+// Lane = 8 * quarter + b.  Quarter: the pair's member s (0: +m, 1: -m) and two of the four batch elements, from zp.
+// The lane's betas are j = 4 b + 32 p + i (p < N / 64, i < 4) and N - 1 - j.
+struct RowsLane {
+  int b, s, zp;
+  S2C_D explicit RowsLane(int lane) : b(lane & 7), s(lane >> 4), zp(2 * ((lane >> 3) & 1)) {}
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -212,167 +284,161 @@ struct RowsTileMap {
 template <int N>
 struct so3_fwd_wigner_r_impl {
   static S2C_D void run(const Ctx& ctx, const FwdRowsParams& p, unsigned char* smem) {
-    constexpr int NH = N / 2, JL = NH / 32;           // betas of the half range per lane
-    constexpr int ZS = N, CS = rows_cs<N>();          // tile strides (complex): z, column
-    float2* tile = reinterpret_cast<float2*>(smem);   // [16][4][N] (column stride CS)
+    constexpr int NH = N / 2, NP = NH / 32;                       // pieces of a half row per lane
+    constexpr int kRing = rows_ring_floats(N, kRowsSlotsF);
+    float2* tile = reinterpret_cast<float2*>(smem);               // [sign][z][N * 16]
     const int warp = ctx.tid >> 5, lane = ctx.tid & 31;
-    // ring step = two degrees: [depth][row 0 / 1][A / B][NH]; reuses the tile's memory (see below)
-    float* ring = reinterpret_cast<float*>(smem) + warp * rows_ring_floats<N>(2);
-    float* xch = reinterpret_cast<float*>(smem) + rows_tile_floats<N>() + warp * 32 * 33;
-    const int K = p.K, zc = p.zc;
-    const RowsGeom g = rows_geom(ctx.bid, K, zc);
-    const int n = g.n, m0 = g.m0, zbase = g.zq * kRowsZQ;
+    float* rings = reinterpret_cast<float*>(smem) + rows_tile_floats(N);
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(rings + kRowsMG * kRing);     // [sign]
+    int* readers = reinterpret_cast<int*>(bar + 2);
+    float* xch = reinterpret_cast<float*>(bar + 4) + warp * 32 * 17;
+    const int K = p.K, zc = p.zc, items = rows_items(K, zc);
+    const RowsLane ln(lane);
+    auto next = [&](int round) { return round * ctx.nblk + (round & 1 ? ctx.nblk - 1 - ctx.bid : ctx.bid); };
 
-    // ---- stage the block's columns of V: tile[c][z][beta] ----------------------------------------
-    // Per (z, beta) row: bins m0 .. m0+7 (64 aligned bytes) and bins N-m0-7 .. N-m0, read as the
-    // aligned run N-m0-8 .. N-m0-1 plus the single bin N-m0.  All loads of a thread are issued
-    // before the first value is used.
-    {
-      const RowsTileMap<N> tm(ctx.tid);
-      constexpr int kP = RowsTileMap<N>::kPasses;
-      const float2* vn = p.v + ((long)n * zc + zbase) * N * N;
-      float4 pos[kP], neg[kP];
-      float2 one[kP];
-#pragma unroll
-      for (int k = 0; k < kP; ++k) {
-        const int r = tm.r0 + 64 * k, z = r / N;
-        pos[k] = neg[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        one[k] = make_float2(0.f, 0.f);
-        if (zbase + z < zc) {
-          const float2* row = vn + (long)r * N;           // r = z * N + beta
-          pos[k] = *reinterpret_cast<const float4*>(row + m0 + 2 * tm.q);
-          neg[k] = *reinterpret_cast<const float4*>(row + N - m0 - 8 + 2 * tm.q);
-          if (tm.q == 0 && m0 > 0) one[k] = row[N - m0];
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kP; ++k) {
-        const int r = tm.r0 + 64 * k, z = r / N, beta = r - z * N;
-        float2* dst = tile + z * ZS + beta;
-        dst[(2 * tm.q) * CS] = make_float2(pos[k].x, pos[k].y);
-        dst[(2 * tm.q + 1) * CS] = make_float2(pos[k].z, pos[k].w);
-        // bins N-m0-8+2q, N-m0-7+2q are the frequencies -(m0+8-2q), -(m0+7-2q)
-        if (tm.q > 0) dst[(16 - 2 * tm.q) * CS] = make_float2(neg[k].x, neg[k].y);
-        dst[(15 - 2 * tm.q) * CS] = make_float2(neg[k].z, neg[k].w);
-        if (tm.q == 0) dst[8 * CS] = one[k];
-      }
+    // the item's part of V, one copy per sign; issued by one thread once every warp has the part before in registers
+    auto fetch = [&](int item) {
+      if (item >= items) return;
+      const RowsGeom g = rows_geom(p.order, item, zc);
+      for (int s = 0; s < 2; ++s)
+        bulk_load_issue(tile + s * kRowsZQ * N * kRowsMG, p.v + rows_part(N, zc, g, s),
+                        (unsigned)(g.nz * N * kRowsMG * sizeof(float2)), bar + s);
+    };
+    if (ctx.tid == 0) {
+      bulk_barrier_init(bar);
+      bulk_barrier_init(bar + 1);
+      *readers = 0;
+      fetch(next(0));
     }
     ctx.sync();
 
-    const int m = m0 + warp;
-    const int lmin = m > n ? m : n;
-    const int L = (m < K) ? p.nl - lmin : 0;
+    for (int round = 0; next(round) < items; ++round) {
+      const RowsGeom g = rows_geom(p.order, next(round), zc);
+      const unsigned phase = round & 1;
+      const int n = g.n, m = g.m0 + warp;
+      const int lmin = m > n ? m : n;
+      const int L = (m < K) ? p.nl - lmin : 0;
 #ifdef S2C_EMUL
-    const int lmin_blk = m0 > n ? m0 : n;
-    const int Lloop = p.nl - lmin_blk > 0 ? p.nl - lmin_blk : 0;   // uniform over the block
+      const int lmin_blk = g.m0 > n ? g.m0 : n;
+      const int Lloop = p.nl - lmin_blk > 0 ? p.nl - lmin_blk : 0;   // uniform over the block
 #else
-    const int Lloop = L;
+      const int Lloop = L;
 #endif
+      RowsPanels pn;
+      pn.a = pn.b = p.pan.data;
+      pn.bsign = 1.f;
+      if (L > 0) pn = rows_panels(p.pan, m, n);
+      RowsRing<N, kRowsSlotsF> ring(rings + warp * kRing, pn, lane, L);
+      for (int t = 0; t < kRowsSlotsF; ++t) ring.issue(t);
 
-    // ---- this lane's slice of V: betas j (p) and N-1-j (q) of the columns +m and -m ----------------
-    float2 vp[2][kRowsZQ][JL], vq[2][kRowsZQ][JL];
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int z = 0; z < kRowsZQ; ++z)
-#pragma unroll
-        for (int jj = 0; jj < JL; ++jj) {
-          const int j = JL * lane + jj;
-          const float2* col = tile + (s * kRowsMG + warp) * CS + z * ZS;
-          vp[s][z][jj] = col[j];
-          vq[s][z][jj] = col[N - 1 - j];
-        }
-
-    RowsPanels pn;
-    pn.a = pn.b = p.pan.data;
-    pn.bsign = 1.f;
-    if (L > 0) pn = rows_panels(p.pan, m, n);
-    const bool self = (m == 0);
-    ctx.sync();   // every warp has its slice of V in registers: the tile's memory becomes the rings
-#ifndef S2C_EMUL
-    if (L <= 0) return;   // no block barrier below this point
-#endif
-    for (int t = 0; t < kRowsDepth - 1; ++t) rows_issue<N, 2>(ring, t, pn.a, pn.b, L, lane);
-
-    // This lane's output in every step: value lane = r * 16 + s * 8 + z * 2 + c of the transpose-
-    // reduce, i.e. degree lmin + li + r, frequency +-m, batch element z, real / imaginary part.
-    // Its spectrum row and the Hermitian mirror row advance by two degrees per step; with
-    // row(l, m, n) = l (4 l^2 - 1) / 3 + (l + m)(2 l + 1) + l + n the step is a quadratic in l, kept
-    // by differences (no multiplications or divisions in the loop).
-    const int o_r = lane >> 4, o_s = (lane >> 3) & 1, o_z = (lane >> 1) & 3, o_c = lane & 1;
-    const int o_mm = o_s ? -m : m;
-    const bool o_ok = zbase + o_z < zc && !(self && o_s == 1);
-    const float o_fudge = ((o_mm - n) & 1) ? -1.f : 1.f;
-    float* const o_base = reinterpret_cast<float*>(p.out + zbase + o_z) + o_c;
-    const long o_zs2 = 2 * p.out_zstride;
-    int o_row1 = (int)so3_row(lmin + o_r, o_mm, n), o_row2 = (int)so3_row(lmin + o_r, -o_mm, -n);
-    int o_d1 = 8 * (lmin + o_r) * (lmin + o_r) + 24 * (lmin + o_r) + 22 + 4 * o_mm;
-    int o_d2 = o_d1 - 8 * o_mm, o_dd = 32 * (lmin + o_r) + 80;
-
-    float va[2][JL], vb[2][JL];     // rows li, li + 1 of the two half panels
-    for (int li = 0; li < Lloop; li += 2) {
-      rows_wait_oldest();
-      ctx.sync_warp();              // the other lanes' pieces of this step have landed, too
+      // ---- this lane's numbers: v1 goes with the row of the first half panel, v2 with that of the second ----------------
+      //   X_{+m} = sum_j A_j V_{+m}[j] + s B_j V_{+m}[N-1-j];   X_{-m} = s (sum_j A_j V_{-m}[N-1-j] + s B_j V_{-m}[j]),
+      // s = (-1)^(l+n).  Index [2 z + re/im][pair of neighbouring betas].
+      float2 v1[4][2 * NP], v2[4][2 * NP];
       {
-        const float* slot = ring + ((li / 2) % kRowsDepth) * (4 * NH) + JL * lane;
+        const bool landed0 = bulk_wait(ctx, bar, phase), landed1 = bulk_wait(ctx, bar + 1, phase);
+        // (a copy that has not landed within the bound of the wait is read from where it comes from)
+        const bool landed = landed0 && landed1;
+        const float2* col = landed ? tile + ln.s * kRowsZQ * N * kRowsMG : p.v + rows_part(N, zc, g, ln.s);
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
+        for (int z = 0; z < 2; ++z) {
+          const int zz = ln.zp + z;
+          const bool there = landed || zz < g.nz;
+          auto number = [&](int beta) {
+            return there ? col[zz * N * kRowsMG + ((beta * kRowsMG + warp) ^ rows_swizzle(zz, beta))] : make_float2(0.f, 0.f);
+          };
 #pragma unroll
-          for (int jj = 0; jj < JL; ++jj) {
-            const bool ok = li + r < L;
-            va[r][jj] = ok ? slot[(2 * r) * NH + jj] : 0.f;
-            vb[r][jj] = ok ? pn.bsign * slot[(2 * r + 1) * NH + jj] : 0.f;
+          for (int k = 0; k < 2 * NP; ++k) {
+            const int j = 4 * ln.b + 32 * (k / 2) + 2 * (k % 2);
+            const float2 j0 = number(j), j1 = number(j + 1), q0 = number(N - 1 - j), q1 = number(N - 2 - j);
+            const float2 jr = make_float2(j0.x, j1.x), ji = make_float2(j0.y, j1.y);
+            const float2 qr = make_float2(q0.x, q1.x), qi = make_float2(q0.y, q1.y);
+            v1[2 * z][k] = ln.s ? qr : jr;      v2[2 * z][k] = ln.s ? jr : qr;
+            v1[2 * z + 1][k] = ln.s ? qi : ji;  v2[2 * z + 1][k] = ln.s ? ji : qi;
           }
-      }
-      rows_issue<N, 2>(ring, li / 2 + kRowsDepth - 1, pn.a, pn.b, L, lane);
-      float val[32];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int l = lmin + li + r;
-        const float sl = ((l + n) & 1) ? -1.f : 1.f;
-#pragma unroll
-        for (int z = 0; z < kRowsZQ; ++z) {
-          float2 xp = make_float2(0.f, 0.f), xq = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int jj = 0; jj < JL; ++jj) {
-            const float a = va[r][jj], b = vb[r][jj], sa = sl * a, sb = sl * b;
-            // X_{+m} = sum A Vp_{+m} + s B Vq_{+m};   X_{-m} = sum B Vp_{-m} + s A Vq_{-m}
-            // (packed multiply-adds for two betas per lane only: with one, 64 signals at b = 32, 29 degrees, took
-            // 163 us packed and 148 scalar)
-            auto mul_add = [](float w, float2 v, float2 acc) {
-              if constexpr (JL == 1) return make_float2(fmaf(w, v.x, acc.x), fmaf(w, v.y, acc.y));
-              else return fma2(make_float2(w, w), v, acc);
-            };
-            xp = mul_add(a, vp[0][z][jj], xp);
-            xp = mul_add(sb, vq[0][z][jj], xp);
-            xq = mul_add(b, vp[1][z][jj], xq);
-            xq = mul_add(sa, vq[1][z][jj], xq);
-          }
-          val[r * 16 + 0 * 8 + z * 2 + 0] = xp.x;
-          val[r * 16 + 0 * 8 + z * 2 + 1] = xp.y;
-          val[r * 16 + 1 * 8 + z * 2 + 0] = xq.x;
-          val[r * 16 + 1 * 8 + z * 2 + 1] = xq.y;
         }
       }
-      const float mine = rows_reduce32(ctx, val, lane, xch);   // value `lane` summed over the warp
-      const float other = rows_partner(ctx, mine, lane, xch);  // the other component of the number
-      if (li + o_r < L && o_ok) {
-        float* o1 = o_base + o_row1 * o_zs2;
-        const bool mirror = n > 0;      // for n = 0 the mirror (-m, 0) is computed directly
-        float* o2 = o_base + o_row2 * o_zs2;
-        if (p.mode == kSo3Real) {
-          *o1 = mine;
-          if (mirror) *o2 = o_c ? -o_fudge * mine : o_fudge * mine;
-        } else {   // += i * (re + i im):  re -= im, im += re;   mirror += i * fudge * conj
-          *o1 += o_c ? other : -other;
-          if (mirror) *o2 += o_fudge * other;
+      // the last warp to get here starts the next copy; no warp waits for another
+#ifndef S2C_EMUL
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence_block();
+        if (atomicAdd(readers, 1) == kRowsMG - 1) {
+          *readers = 0;
+          __threadfence_block();
+          fetch(next(round + 1));
         }
       }
-      o_row1 += o_d1;
-      o_row2 += o_d2;
-      o_d1 += o_dd;
-      o_d2 += o_dd;
-      o_dd += 64;
+      __syncwarp();
+#else
+      ctx.sync();
+      if (ctx.tid == 0) fetch(next(round + 1));
+#endif
+
+      // output: row li + b % 4 (lanes b < 4) or its mirror (b >= 4), frequency +-m, batch elements from zp
+      const int o_mm = ln.s ? -m : m, o_z = g.zbase + ln.zp, o_b = ln.b & 3;
+      const float sl = ((lmin + n + o_b) & 1) ? -1.f : 1.f;      // (-1)^(l+n) of row b % 4, and of row r XOR (b % 4), r even
+      const bool o_mirror = ln.b >= 4;
+      // v = (x, y) of a number becomes (cx x, cy y), or of i times it (cx y, cy x); the mirror is (-1)^(m-n) times the conjugate
+      const float o_sign = (ln.s ? sl : 1.f) * (o_mirror && ((o_mm - n) & 1) ? -1.f : 1.f);
+      const float o_sx = p.mode == kSo3Real || o_mirror ? o_sign : -o_sign;
+      const float o_sy = p.mode == kSo3Real && o_mirror ? -o_sign : o_sign;
+      const int o_om = o_mirror ? -o_mm : o_mm, o_on = o_mirror ? -n : n;
+      // for n = 0 the mirror (-m, 0) is computed directly; m = 0 is its own partner
+      const int o_nz = (m == 0 && ln.s) || (o_mirror && n == 0) ? 0 : zc - o_z;
+      const bool o_vec = o_nz >= 2 && p.out_zstride % 2 == 0 && reinterpret_cast<unsigned long long>(p.out + o_z) % 16 == 0;
+      const float2 bs_even = make_float2(sl * pn.bsign, sl * pn.bsign), bs_odd = make_float2(-sl * pn.bsign, -sl * pn.bsign);
+
+      for (int li = 0, t = 0; li < Lloop; li += kRowsStep, ++t) {
+        rows_wait_oldest<kRowsSlotsF>();
+        ctx.sync_warp();              // the other lanes' pieces of this step have landed, too
+        const float* slot = ring.slot(t) + 4 * ln.b;
+        const float4 sum = rows_sum4(ctx, [&](auto r_) {
+          constexpr int r = decltype(r_)::value;
+          const float* row = slot + (r ^ o_b) * (2 * NH);
+          float2 acc[4];
+#pragma unroll
+          for (int pp = 0; pp < NP; ++pp) {
+            const float4 a4 = *reinterpret_cast<const float4*>(row + 32 * pp);
+            const float2 a0 = make_float2(a4.x, a4.y), a1 = make_float2(a4.z, a4.w);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              acc[c] = pp == 0 ? rows_mul2(a0, v1[c][0]) : fma2(a0, v1[c][2 * pp], acc[c]);
+              acc[c] = fma2(a1, v1[c][2 * pp + 1], acc[c]);
+            }
+          }
+#pragma unroll
+          for (int pp = 0; pp < NP; ++pp) {
+            const float4 b4 = *reinterpret_cast<const float4*>(row + NH + 32 * pp);
+            const float2 sgn = r & 1 ? bs_odd : bs_even;
+            const float2 b0 = rows_mul2(make_float2(b4.x, b4.y), sgn), b1 = rows_mul2(make_float2(b4.z, b4.w), sgn);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              acc[c] = fma2(b0, v2[c][2 * pp], acc[c]);
+              acc[c] = fma2(b1, v2[c][2 * pp + 1], acc[c]);
+            }
+          }
+          return make_float4(acc[0].x + acc[0].y, acc[1].x + acc[1].y, acc[2].x + acc[2].y, acc[3].x + acc[3].y);
+        }, lane, xch);
+        ctx.sync_warp();              // every lane has read the slot
+        ring.issue(t);
+        if (li + o_b < L && o_nz > 0) {
+          float2* o = p.out + so3_row(lmin + li + o_b, o_om, o_on) * p.out_zstride + o_z;
+          if (p.mode == kSo3Real) {
+            const float4 w = make_float4(o_sx * sum.x, o_sy * sum.y, o_sx * sum.z, o_sy * sum.w);
+            if (o_vec) {
+              *reinterpret_cast<float4*>(o) = w;
+            } else {
+              o[0] = make_float2(w.x, w.y);
+              if (o_nz > 1) o[1] = make_float2(w.z, w.w);
+            }
+          } else {   // += i * (re + i im):  re -= im, im += re;   mirror += i * (-1)^(m-n) * conj
+            o[0] = make_float2(o[0].x + o_sx * sum.y, o[0].y + o_sy * sum.x);
+            if (o_nz > 1) o[1] = make_float2(o[1].x + o_sx * sum.w, o[1].y + o_sy * sum.z);
+          }
+        }
+      }
+      ctx.sync_warp();                // the ring is free for the next item
     }
   }
 };
@@ -380,56 +446,20 @@ struct so3_fwd_wigner_r_impl {
 // ---------------------------------------------------------------------------------------------
 // synthesis:  S[z][beta] = sum_l W[l][beta] Xs[l][z],  Xs = symmetrised spectrum
 // ---------------------------------------------------------------------------------------------
-template <int N>
+template <int N, int ZQ>
 struct so3_inv_wigner_r_impl {
   static S2C_D void run(const Ctx& ctx, const InvRowsParams& p, unsigned char* smem) {
-    constexpr int NH = N / 2, JL = NH / 32;
-    constexpr int ZS = N, CS = rows_cs<N>();
-    float2* tile = reinterpret_cast<float2*>(smem);     // [16][4][N], written after the loop
-    float2* xs = tile;                                    // before: [16][Lmax][4] symmetrised rows
+    constexpr int MG = kRowsMGI, ZL = ZQ / 2, NC = 2 * ZL;       // batch elements and numbers per lane
+    constexpr int NH = N / 2, NP = NH / 32;
+    float2* tile = reinterpret_cast<float2*>(smem);              // [sign][z][N * 4], written after the loop
+    float2* xs = tile;                                             // before: [2 MG][Lmax][ZQ] symmetrised rows
     const int warp = ctx.tid >> 5, lane = ctx.tid & 31;
-    // ring step = one degree: [depth][A / B][NH], in the upper half of the tile's memory
-    float* ring = reinterpret_cast<float*>(smem) + rows_tile_floats<N>() / 2 + warp * rows_ring_floats<N>(1);
+    float* ring_base = reinterpret_cast<float*>(smem) + rows_inv_tile_floats(N, ZQ) + warp * rows_ring_floats(N, kRowsSlotsI);
     const int K = p.K, zc = p.zc, nl = p.pan.nl;
-    const RowsGeom g = rows_geom(ctx.bid, K, zc);
-    const int n = g.n, m0 = g.m0, zbase = g.zq * kRowsZQ;
+    const int ngroups = (K + MG - 1) / MG, nzq = (zc + ZQ - 1) / ZQ, zbase = ctx.bid % nzq * ZQ, nm = ctx.bid / nzq;
+    const int n = nm / ngroups, m0 = (nm - n * ngroups) * MG;
     const int lmin_blk = m0 > n ? m0 : n;
     const int Lmax = nl - lmin_blk;                      // rows of the block's longest pair (<= N/2)
-
-    // ---- symmetrised spectrum rows of the block's 16 columns: xs[c][li][z], li from lmin_blk ------
-    // thread = (z, li); the loads of all 16 columns are issued before any is used
-    {
-      const int z = ctx.tid % kRowsZQ;
-      for (int li = ctx.tid / kRowsZQ; li < Lmax; li += kRowsThreads / kRowsZQ) {
-        const int l = lmin_blk + li;
-        float2 a[2 * kRowsMG], b[2 * kRowsMG];
-#pragma unroll
-        for (int c = 0; c < 2 * kRowsMG; ++c) {
-          const int mabs = m0 + (c % kRowsMG);
-          const int mm = c < kRowsMG ? mabs : -mabs;
-          const bool ok = zbase + z < zc && mabs < K && l >= mabs && !(c >= kRowsMG && mabs == 0);
-          a[c] = b[c] = make_float2(0.f, 0.f);
-          if (ok) {
-            a[c] = p.x[so3_row(l, mm, n) * p.x_zstride + zbase + z];
-            b[c] = p.x[so3_row(l, -mm, -n) * p.x_zstride + zbase + z];
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < 2 * kRowsMG; ++c) {
-          const int mabs = m0 + (c % kRowsMG);
-          const int mm = c < kRowsMG ? mabs : -mabs;
-          float2 u = a[c], w = b[c];
-          if (p.mode == kSo3RotI) {  // multiply the spectrum by -i
-            u = make_float2(u.y, -u.x);
-            w = make_float2(w.y, -w.x);
-          }
-          const float fudge = ((mm - n) & 1) ? -1.f : 1.f;
-          xs[(c * Lmax + li) * kRowsZQ + z] =
-              make_float2(0.5f * (u.x + fudge * w.x), 0.5f * (u.y - fudge * w.y));
-        }
-      }
-    }
-    ctx.sync();
 
     const int m = m0 + warp;
     const int lmin = m > n ? m : n;
@@ -439,97 +469,147 @@ struct so3_inv_wigner_r_impl {
 #else
     const int Lloop = L;
 #endif
+    RowsPanels pn;
+    pn.a = pn.b = p.pan.data;
+    pn.bsign = 1.f;
+    if (L > 0) pn = rows_panels(p.pan, m, n);
+    RowsRing<N, kRowsSlotsI> ring(ring_base, pn, lane, L);
+    for (int t = 0; t < kRowsSlotsI; ++t) ring.issue(t);
 
-    // accumulators: betas j (p) and N-1-j (q) of the columns +m (0) and -m (1)
-    float2 sp[2][kRowsZQ][JL], sq[2][kRowsZQ][JL];
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int z = 0; z < kRowsZQ; ++z)
-#pragma unroll
-        for (int jj = 0; jj < JL; ++jj) sp[s][z][jj] = sq[s][z][jj] = make_float2(0.f, 0.f);
-
+    // ---- symmetrised spectrum rows of the block's columns: xs[c][li][z], li from lmin_blk ------
+    // thread = (z, li); the loads of all columns are issued before any is used
     {
-      RowsPanels pn;
-      pn.a = pn.b = p.pan.data;
-      pn.bsign = 1.f;
-      if (L > 0) pn = rows_panels(p.pan, m, n);
-      const int lrel = L > 0 ? lmin - lmin_blk : 0;
-      const float2* x0 = xs + ((0 * kRowsMG + warp) * Lmax + lrel) * kRowsZQ;
-      const float2* x1 = xs + ((1 * kRowsMG + warp) * Lmax + lrel) * kRowsZQ;
-      if (Lloop > 0)
-        for (int t = 0; t < kRowsDepth - 1; ++t) rows_issue<N, 1>(ring, t, pn.a, pn.b, L, lane);
-      float a[JL], b[JL];
-      for (int li = 0; li < Lloop; ++li) {
-        rows_wait_oldest();
-        ctx.sync_warp();            // the other lanes' pieces of this row have landed, too
-        const bool act = li < L;
-        {
-          const float* slot = ring + (li % kRowsDepth) * (2 * NH) + JL * lane;
+      const int z = ctx.tid % ZQ;
+      for (int li = ctx.tid / ZQ; li < Lmax; li += kRowsThreadsI / ZQ) {
+        const int l = lmin_blk + li;
+        float2 a[2 * MG], b[2 * MG];
 #pragma unroll
-          for (int jj = 0; jj < JL; ++jj) {
-            a[jj] = act ? slot[jj] : 0.f;
-            b[jj] = act ? pn.bsign * slot[NH + jj] : 0.f;
+        for (int c = 0; c < 2 * MG; ++c) {
+          const int mabs = m0 + (c % MG);
+          const int mm = c < MG ? mabs : -mabs;
+          const bool ok = zbase + z < zc && mabs < K && l >= mabs && !(c >= MG && mabs == 0);
+          a[c] = b[c] = make_float2(0.f, 0.f);
+          if (ok) {
+            a[c] = p.x[so3_row(l, mm, n) * p.x_zstride + zbase + z];
+            b[c] = p.x[so3_row(l, -mm, -n) * p.x_zstride + zbase + z];
           }
         }
-        rows_issue<N, 1>(ring, li + kRowsDepth - 1, pn.a, pn.b, L, lane);
-        if (!act) continue;
-        const int l = lmin + li;
-        const float sl = ((l + n) & 1) ? -1.f : 1.f;
 #pragma unroll
-        for (int z = 0; z < kRowsZQ; ++z) {
-          const float2 xp = x0[li * kRowsZQ + z], xm = x1[li * kRowsZQ + z];
-#pragma unroll
-          for (int jj = 0; jj < JL; ++jj) {
-            const float sa = sl * a[jj], sb = sl * b[jj];
-            // S_{+m}[j] += A X_{+m};  S_{+m}[N-1-j] += s B X_{+m};  S_{-m}[j] += B X_{-m};  S_{-m}[N-1-j] += s A X_{-m}
-            sp[0][z][jj] = fma2(make_float2(a[jj], a[jj]), xp, sp[0][z][jj]);
-            sq[0][z][jj] = fma2(make_float2(sb, sb), xp, sq[0][z][jj]);
-            sp[1][z][jj] = fma2(make_float2(b[jj], b[jj]), xm, sp[1][z][jj]);
-            sq[1][z][jj] = fma2(make_float2(sa, sa), xm, sq[1][z][jj]);
+        for (int c = 0; c < 2 * MG; ++c) {
+          const int mabs = m0 + (c % MG);
+          float2 u = a[c], w = b[c];
+          if (p.mode == kSo3RotI) {  // multiply the spectrum by -i
+            u = make_float2(u.y, -u.x);
+            w = make_float2(w.y, -w.x);
           }
+          const float fudge = ((mabs - n) & 1) ? -1.f : 1.f;
+          const float sl = c >= MG && ((l + n) & 1) ? -0.5f : 0.5f;      // (see the loop over the degrees)
+          xs[(c * Lmax + li) * ZQ + z] = make_float2(sl * (u.x + fudge * w.x), sl * (u.y - fudge * w.y));
         }
       }
     }
-    ctx.sync();   // every warp is done with the spectrum rows and its ring; the memory becomes the tile
-
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-      for (int z = 0; z < kRowsZQ; ++z)
-#pragma unroll
-        for (int jj = 0; jj < JL; ++jj) {
-          const int j = JL * lane + jj;
-          float2* col = tile + (s * kRowsMG + warp) * CS + z * ZS;
-          col[j] = sp[s][z][jj];
-          col[N - 1 - j] = sq[s][z][jj];
-        }
     ctx.sync();
 
-    // ---- tile -> V[n][z][beta][f], the transfer of the analysis reversed ----------------------------
-    // Only bins of this block's own frequencies are written: m0 .. m0+7 (all of them: bins of
-    // frequencies >= K are never read by anyone) and N - m for m0 <= m <= m0+7, 0 < m < K.
-    {
-      const RowsTileMap<N> tm(ctx.tid);
-      constexpr int kP = RowsTileMap<N>::kPasses;
-      float2* vn = p.s + ((long)n * zc + zbase) * N * N;
+    // Sums of this lane's numbers: u1 with the rows of the first half panel, u2 with those of the second.
+    //   S_{+m}[j] += A_j X, S_{+m}[N-1-j] += s B_j X;   S_{-m}[N-1-j] += A_j (s X), S_{-m}[j] += s B_j (s X),   s = (-1)^(l+n),
+    // and the spectrum rows of -m are kept times s.  Index [2 z + re/im][pair of neighbouring betas].
+    const int b = lane & 7, s = lane >> 4, zp = ZL * ((lane >> 3) & 1);
+    float2 u1[NC][2 * NP], u2[NC][2 * NP];
 #pragma unroll
-      for (int k = 0; k < kP; ++k) {
-        const int r = tm.r0 + 64 * k, z = r / N, beta = r - z * N;
-        if (zbase + z >= zc) continue;
-        const float2* src = tile + z * ZS + beta;
-        float2* row = vn + (long)r * N;
-        const float2 c0 = src[(2 * tm.q) * CS], c1 = src[(2 * tm.q + 1) * CS];
-        *reinterpret_cast<float4*>(row + m0 + 2 * tm.q) = make_float4(c0.x, c0.y, c1.x, c1.y);
-        const int m_hi = m0 + 8 - 2 * tm.q, m_lo = m0 + 7 - 2 * tm.q;   // bins N-m0-8+2q and the next
-        const float2 d_lo = src[(15 - 2 * tm.q) * CS];
-        if (tm.q > 0 && m_hi < K) {
-          const float2 d_hi = src[(16 - 2 * tm.q) * CS];
-          *reinterpret_cast<float4*>(row + N - m_hi) = make_float4(d_hi.x, d_hi.y, d_lo.x, d_lo.y);
-        } else if (m_lo < K) {
-          row[N - m_lo] = d_lo;
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int k = 0; k < 2 * NP; ++k) u1[c][k] = u2[c][k] = make_float2(0.f, 0.f);
+    {
+      const int lrel = L > 0 ? lmin - lmin_blk : 0;
+      const float2* x = xs + ((s * MG + warp) * Lmax + lrel) * ZQ + zp;
+      const float s0 = (((lmin + n) & 1) ? -1.f : 1.f) * pn.bsign;
+      for (int li = 0, t = 0; li < Lloop; li += kRowsStep, ++t) {
+        rows_wait_oldest<kRowsSlotsI>();
+        ctx.sync_warp();            // the other lanes' pieces of these rows have landed, too
+        const float* slot = ring.slot(t) + 4 * b;
+#pragma unroll
+        for (int r = 0; r < kRowsStep; ++r) {
+          if (li + r >= L) break;
+          float2 y[NC];
+#pragma unroll
+          for (int z = 0; z < ZL; z += 2) {
+            const float4 x4 = *reinterpret_cast<const float4*>(x + (li + r) * ZQ + z);
+            y[2 * z] = make_float2(x4.x, x4.x);
+            y[2 * z + 1] = make_float2(x4.y, x4.y);
+            y[2 * z + 2] = make_float2(x4.z, x4.z);
+            y[2 * z + 3] = make_float2(x4.w, x4.w);
+          }
+          const float2 s2 = r & 1 ? make_float2(-s0, -s0) : make_float2(s0, s0);
+          const float* row = slot + r * (2 * NH);
+#pragma unroll
+          for (int pp = 0; pp < NP; ++pp) {
+            const float4 a4 = *reinterpret_cast<const float4*>(row + 32 * pp);
+            const float2 a0 = make_float2(a4.x, a4.y), a1 = make_float2(a4.z, a4.w);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              u1[c][2 * pp] = fma2(a0, y[c], u1[c][2 * pp]);
+              u1[c][2 * pp + 1] = fma2(a1, y[c], u1[c][2 * pp + 1]);
+            }
+          }
+#pragma unroll
+          for (int pp = 0; pp < NP; ++pp) {
+            const float4 b4 = *reinterpret_cast<const float4*>(row + NH + 32 * pp);
+            const float2 b0 = rows_mul2(make_float2(b4.x, b4.y), s2), b1 = rows_mul2(make_float2(b4.z, b4.w), s2);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              u2[c][2 * pp] = fma2(b0, y[c], u2[c][2 * pp]);
+              u2[c][2 * pp + 1] = fma2(b1, y[c], u2[c][2 * pp + 1]);
+            }
+          }
         }
-        if (tm.q == 0 && m0 > 0 && m0 < K) row[N - m0] = src[8 * CS];
+        ctx.sync_warp();            // every lane has read the slot
+        ring.issue(t);
+      }
+    }
+    ctx.sync();   // every warp is done with the spectrum rows; the memory becomes the block's part of V
+
+    // [sign][z][beta][4], within a line of 16 numbers in the order that spreads a half warp over all banks; a run of four
+    // is in memory's order (rows_swizzle, whose two low bits are these)
+    auto swizzle = [](int z, int beta) { return ((beta >> 2) & 7) | ((z / ZL & 1) << 3); };
+#pragma unroll
+    for (int z = 0; z < ZL; ++z) {
+      float2* col = tile + (s * ZQ + zp + z) * N * MG;
+      auto number = [&](int beta) -> float2& { return col[(beta * MG + warp) ^ swizzle(zp + z, beta)]; };
+#pragma unroll
+      for (int k = 0; k < 2 * NP; ++k) {
+        const int j = 4 * b + 32 * (k / 2) + 2 * (k % 2);
+        const float2 jr = s ? u2[2 * z][k] : u1[2 * z][k], ji = s ? u2[2 * z + 1][k] : u1[2 * z + 1][k];
+        const float2 qr = s ? u1[2 * z][k] : u2[2 * z][k], qi = s ? u1[2 * z + 1][k] : u2[2 * z + 1][k];
+        number(j) = make_float2(jr.x, ji.x);
+        number(j + 1) = make_float2(jr.y, ji.y);
+        number(N - 1 - j) = make_float2(qr.x, qi.x);
+        number(N - 2 - j) = make_float2(qr.y, qi.y);
+      }
+    }
+    ctx.sync();
+    // runs of four numbers, 32 bytes, to their places in the lines of V (numbers of frequencies >= K are never read)
+    const long gs = rows_group_stride(N, zc);
+    float2* dst = p.s + ((long)n * 2 * rows_groups(N) + m0 / kRowsMG) * gs;
+    const int run = m0 / MG % (kRowsMG / MG);
+    const bool wide = reinterpret_cast<unsigned long long>(p.s) % 32 == 0;
+    // (two numbers at a time, lanes 4 - 7 of eight the second pair first: 32-byte steps would meet in half the banks)
+    const int up = ctx.tid >> 2 & 1;
+#pragma unroll 4
+    for (int i = ctx.tid; i < 2 * ZQ * N; i += kRowsThreadsI) {
+      const int beta = i % N, zs = i / N, z = zs % ZQ, sg = zs / ZQ;
+      if (zbase + z >= zc) continue;
+      const float4* src = reinterpret_cast<const float4*>(tile + zs * N * MG + ((beta * MG) ^ (swizzle(z, beta) & 12)));
+      float* out = reinterpret_cast<float*>(dst + sg * rows_groups(N) * gs + (long)(zbase + z) * N * kRowsMG +
+                                            ((beta * kRowsMG + run * MG) ^ (rows_swizzle(z, beta) & 12)));
+      const float4 first = src[up], second = src[1 - up];
+      float8 v;
+      v.lo = up ? second : first;
+      v.hi = up ? first : second;
+      if (wide) {
+        st_global_256(out, v);
+      } else {
+        reinterpret_cast<float4*>(out)[0] = v.lo;
+        reinterpret_cast<float4*>(out)[1] = v.hi;
       }
     }
   }
@@ -537,24 +617,29 @@ struct so3_inv_wigner_r_impl {
 
 #ifndef S2C_EMUL
 template <int N>
-__global__ void __launch_bounds__(kRowsThreads, 2) so3_fwd_wigner_r(const FwdRowsParams p) {
+__global__ void __launch_bounds__(kRowsThreads, 1) so3_fwd_wigner_r(const FwdRowsParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
   so3_fwd_wigner_r_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
 }
-template <int N>
-__global__ void __launch_bounds__(kRowsThreads, 2) so3_inv_wigner_r(const InvRowsParams p) {
+template <int N, int ZQ>
+__global__ void __launch_bounds__(kRowsThreadsI, 2) so3_inv_wigner_r(const InvRowsParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
-  so3_inv_wigner_r_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  so3_inv_wigner_r_impl<N, ZQ>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
 }
-#define S2C_LAUNCH_ROWS(name, N, grid, stream, params)                                         \
-  s2c::launch_impl<name<N>>(#name, (long)(grid), s2c::kRowsThreads, s2c::rows_smem_bytes<N>(), \
-                   stream, params)
+#define S2C_LAUNCH_FWD_ROWS(N, grid, stream, params)                                                             \
+  s2c::launch_impl<so3_fwd_wigner_r<N>>("so3_fwd_wigner_r", (long)(grid), s2c::kRowsThreads, s2c::rows_fwd_smem(N), \
+                                        stream, params)
+#define S2C_LAUNCH_INV_ROWS(N, ZQ, grid, stream, params)                                                          \
+  s2c::launch_impl<so3_inv_wigner_r<N, ZQ>>("so3_inv_wigner_r", (long)(grid), s2c::kRowsThreadsI,                 \
+                                            s2c::rows_inv_smem(N, ZQ), stream, params)
 #else
-#define S2C_LAUNCH_ROWS(name, N, grid, stream, params)                                         \
-  s2c::emu_launch<name##_impl<N>>(#name, (long)(grid), s2c::kRowsThreads,                      \
-                                  s2c::rows_smem_bytes<N>(), params)
+#define S2C_LAUNCH_FWD_ROWS(N, grid, stream, params) \
+  s2c::emu_launch<so3_fwd_wigner_r_impl<N>>("so3_fwd_wigner_r", (long)(grid), s2c::kRowsThreads, s2c::rows_fwd_smem(N), params)
+#define S2C_LAUNCH_INV_ROWS(N, ZQ, grid, stream, params)                                                        \
+  s2c::emu_launch<so3_inv_wigner_r_impl<N, ZQ>>("so3_inv_wigner_r", (long)(grid), s2c::kRowsThreadsI,           \
+                                                s2c::rows_inv_smem(N, ZQ), params)
 #endif
 
 }  // namespace s2c
