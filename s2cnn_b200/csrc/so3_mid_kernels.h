@@ -23,18 +23,27 @@
 namespace s2c {
 
 S2C_HD constexpr bool mid_supported(int N) { return N > 32 && N < 64 && N % 2 == 0; }
-S2C_HD constexpr int mid_ld(int N) { return N % 4 == 2 ? N : N + 2; }
 S2C_HD constexpr int mid_nb(int N) { return N <= 44 ? 4 : 2; }
-// plane strides (complex): buffer A is read down columns, buffer B along rows
-S2C_HD constexpr int mid_psa(int N) { return (N / 2) * mid_ld(N) | 1; }
-S2C_HD constexpr int mid_psb(int N) {
-  int ps = (N / 2) * mid_ld(N);
+// Row strides (complex).  Odd, so that lanes that run down a column hit all banks (16 numbers of 8 bytes); where the
+// leading step of a row transform writes R2 neighbours per row, the stride is R2 modulo 16 if that costs at most four
+// numbers: lanes that go on to the next row then go on through the banks.  The synthesis reads two numbers at a time from
+// buffer B, whose stride is 2 modulo 4.
+S2C_HD constexpr int mid_lda(int N) {
+  for (int ld = N + 1; ld <= N + 4; ++ld)
+    if (ld % 2 == 1 && (ld - two_r2(N)) % 16 == 0) return ld;
+  return N + 1;
+}
+S2C_HD constexpr int mid_ldb(int N, bool synthesis) { return !synthesis ? N + 1 : N % 4 == 2 ? N : N + 2; }
+// plane strides: the planes of a block, which are the fastest index of the lanes where columns are touched, share the banks
+S2C_HD constexpr int mid_plane(int N, int ld) {
+  int ps = (N / 2) * ld;
   while (ps % 16 != 16 / mid_nb(N)) ++ps;
   return ps;
 }
 constexpr int kMidThreads = 256;
 inline size_t mid_smem_bytes(int N) {
-  return ((size_t)(N + 1) / 2 * 2 + (size_t)mid_nb(N) * (mid_psa(N) + mid_psb(N)) + 2) * sizeof(float2);
+  const int b = std::max(mid_plane(N, mid_ldb(N, false)), mid_plane(N, mid_ldb(N, true)));
+  return ((size_t)(N + 1) / 2 * 2 + (size_t)mid_nb(N) * (mid_plane(N, mid_lda(N)) + b) + 2) * sizeof(float2);
 }
 
 struct MidParams {
@@ -67,8 +76,8 @@ S2C_D void mid_ld(const float* p, float (&v)[2]) {
 template <int N>
 struct so3_fwd_mid_impl {
   static S2C_D void run(const Ctx& ctx, const MidParams& p, unsigned char* smem) {
-    constexpr int R1 = two_r1(N), R2 = two_r2(N), H = N / 2, NB = mid_nb(N), LD = mid_ld(N);
-    constexpr int PSA = mid_psa(N), PSB = mid_psb(N), G = (N + NB - 1) / NB;
+    constexpr int R1 = two_r1(N), R2 = two_r2(N), H = N / 2, NB = mid_nb(N), LD = mid_lda(N), LDB = mid_ldb(N, false);
+    constexpr int PSA = mid_plane(N, LD), PSB = mid_plane(N, LDB), G = (N + NB - 1) / NB;
     float2* tw = reinterpret_cast<float2*>(smem);
     float2* B = tw + (N + 1) / 2 * 2;
     float2* A = B + NB * PSB;
@@ -102,13 +111,14 @@ struct so3_fwd_mid_impl {
       for (int k = 0; k < R1; ++k) a[k * R2] = v[k];
     }
     ctx.sync();
-    for (int it = ctx.tid; it < bc * H * R1; it += ctx.nthr) {
-      const int b = it % R1, row = it / R1, pl = row / H, t = row - pl * H;
+    for (int it = ctx.tid; it < NB * H * R1; it += ctx.nthr) {
+      const int b = it / (NB * H), row = it % (NB * H), pl = row / H, t = row - pl * H;
+      if (pl >= bc) continue;
       const float2* a = A + pl * PSA + t * LD + b * R2;
       float2 v[R2];
 #pragma unroll
       for (int i = 0; i < R2; ++i) v[i] = a[i];
-      float2* o = B + pl * PSB + t * LD + two_block_freq(N, R1, b);
+      float2* o = B + pl * PSB + t * LDB + two_block_freq(N, R1, b);
       two_tail<N, -1>(v, tw, [&](int q, float2 val) { o[R1 * q] = val; });
     }
     ctx.sync();
@@ -122,7 +132,7 @@ struct so3_fwd_mid_impl {
 #pragma unroll
       for (int k = 0; k < R1; ++k) {
         const int al = j + k * R2;                          // alpha: row 2 t (even) or 2 t + 1 (odd)
-        const float2 zk = bk[(al >> 1) * LD], zc = bq[(al >> 1) * LD];
+        const float2 zk = bk[(al >> 1) * LDB], zc = bq[(al >> 1) * LDB];
         v[k] = (al & 1) ? make_float2(0.5f * (zk.y + zc.y), -0.5f * (zk.x - zc.x))
                         : make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y - zc.y));
       }
@@ -153,8 +163,8 @@ struct so3_fwd_mid_impl {
 template <int N>
 struct so3_inv_mid_impl {
   static S2C_D void run(const Ctx& ctx, const MidParams& p, unsigned char* smem) {
-    constexpr int R1 = two_r1(N), R2 = two_r2(N), H = N / 2, NB = mid_nb(N), LD = mid_ld(N);
-    constexpr int PSA = mid_psa(N), PSB = mid_psb(N), G = (N + NB - 1) / NB;
+    constexpr int R1 = two_r1(N), R2 = two_r2(N), H = N / 2, NB = mid_nb(N), LD = mid_lda(N), LDB = mid_ldb(N, true);
+    constexpr int PSA = mid_plane(N, LD), PSB = mid_plane(N, LDB), G = (N + NB - 1) / NB;
     float2* tw = reinterpret_cast<float2*>(smem);
     float2* B = tw + (N + 1) / 2 * 2;                        // 16-byte aligned: read two numbers at a time
     float2* A = B + NB * PSB;
@@ -196,7 +206,7 @@ struct so3_inv_mid_impl {
       float2 v[R2];
 #pragma unroll
       for (int i = 0; i < R2; ++i) v[i] = a[i];
-      float2* o = B + pl * PSB + n * LD + two_block_freq(N, R1, b);
+      float2* o = B + pl * PSB + n * LDB + two_block_freq(N, R1, b);
       if (pl < bc) two_tail<N, +1>(v, tw, [&](int q, float2 val) { o[R1 * q] = val; });
     }
     ctx.sync();
@@ -209,11 +219,11 @@ struct so3_inv_mid_impl {
       for (int k = 0; k < R1; ++k) {
         const int n = j + k * R2;
         if (n < K) {
-          const float4 u = *reinterpret_cast<const float4*>(src + n * LD);         // alpha = 2 t, 2 t + 1
+          const float4 u = *reinterpret_cast<const float4*>(src + n * LDB);        // alpha = 2 t, 2 t + 1
           // T[alpha][0] is real for a Hermitian spectrum; its rounding-level imaginary part is dropped
           v[k] = n == 0 ? make_float2(u.x, u.z) : make_float2(u.x - u.w, u.y + u.z);   // T1 + i T2
         } else if (N - n < K) {
-          const float4 u = *reinterpret_cast<const float4*>(src + (N - n) * LD);
+          const float4 u = *reinterpret_cast<const float4*>(src + (N - n) * LDB);
           v[k] = make_float2(u.x + u.w, u.z - u.y);                                    // conj(T1) + i conj(T2)
         } else {
           v[k] = make_float2(0.f, 0.f);
@@ -225,13 +235,14 @@ struct so3_inv_mid_impl {
       for (int k = 0; k < R1; ++k) a[k * R2] = v[k];
     }
     ctx.sync();
-    for (int it = ctx.tid; it < bc * H * R1; it += ctx.nthr) {
-      const int b = it % R1, row = it / R1, pl = row / H, t = row - pl * H;
+    for (int it = ctx.tid; it < NB * H * R1; it += ctx.nthr) {
+      const int b = it / (NB * H), row = it % (NB * H), pl = row / H, t = row - pl * H;
+      if (pl >= bc) continue;
       const float2* a = A + pl * PSA + t * LD + b * R2;
       float2 v[R2];
 #pragma unroll
       for (int i = 0; i < R2; ++i) v[i] = a[i];
-      float2* o = B + pl * PSB + t * LD + two_block_freq(N, R1, b);
+      float2* o = B + pl * PSB + t * LDB + two_block_freq(N, R1, b);
       two_tail<N, +1>(v, tw, [&](int q, float2 val) { o[R1 * q] = val; });
     }
     ctx.sync();
@@ -261,7 +272,7 @@ struct so3_inv_mid_impl {
         const int it = base + u * ctx.nthr;
         if (it >= total) break;
         const int c = it % PR, row = it / PR, pl = row / H, t = row - pl * H;
-        const float4* src = reinterpret_cast<const float4*>(B + pl * PSB + t * LD + c * W);
+        const float4* src = reinterpret_cast<const float4*>(B + pl * PSB + t * LDB + c * W);
         const long e0 = e00 + (long)row * 2 * N + c * W;
         float r0[W], r1[W];
 #pragma unroll
