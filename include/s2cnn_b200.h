@@ -188,6 +188,13 @@ size_t s2c_s2_conv_synthesis_workspace(int nbatch, int f_out, int b);
 int s2c_s2_conv_synthesis(const float* xs, const float* ys, float* out, int nbatch, int f_in,
                           int f_out, int b, const float* bias, void* workspace,
                           size_t workspace_bytes, void* stream);
+/* The same, and s2c_s2_conv_relu_so3_rfft_ws (same workspace), for spectra of REAL signals and kernels, as a layer's are:
+ * x[l,-m] = (-1)^m conj x[l,m] for both factors, so that half of the product is the mirror of the other half. */
+size_t s2c_s2_conv_real_synthesis_workspace(int nbatch, int f_out, int b);
+int s2c_s2_conv_real_synthesis(const float* xs, const float* ys, float* out, int nbatch, int f_in, int f_out, int b,
+                               const float* bias, void* workspace, size_t workspace_bytes, void* stream);
+int s2c_s2_conv_real_relu_so3_rfft(const float* xs, const float* ys, float* out, int nbatch, int f_in, int f_out, int b,
+                                   int b_next, const float* bias, void* workspace, size_t workspace_bytes, void* stream);
 /* x [nspec(b_in), nbatch, 2] -> out [nbatch, 2b_out, 2b_out, 2b_out, 2] complex.
  * Replaces so3_ifft, s2cnn/soft/so3_fft.py:115-155. */
 int s2c_so3_ifft(const float* x, float* out, long nbatch, int b_in, int b_out, int for_grad,

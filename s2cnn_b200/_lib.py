@@ -63,6 +63,9 @@ _SIGNATURES = {
     "s2c_so3_rifft_static_max_bytes": (c_size_t, []),
     "s2c_s2_conv_synthesis_workspace": (c_size_t, [c_int, c_int, c_int]),
     "s2c_s2_conv_synthesis": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, c_size_t, _P]),
+    "s2c_s2_conv_real_synthesis_workspace": (c_size_t, [c_int, c_int, c_int]),
+    "s2c_s2_conv_real_synthesis": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, c_size_t, _P]),
+    "s2c_s2_conv_real_relu_so3_rfft": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, c_size_t, _P]),
     "s2c_so3_ifft": (c_int, [_P, _P, c_long, c_int, c_int, c_int, _P, c_size_t, _P]),
     "s2c_s2_fft_workspace": (c_size_t, [c_long, c_int, c_int]),
     "s2c_s2_fft": (c_int, [_P, c_int, _P, c_long, c_int, c_int, c_int, _P, c_size_t, _P]),

@@ -194,14 +194,17 @@ static bool so3_prefers_cluster(ClKind kind, int N, long nbatch) {
 // 446 -> 214 us, b = 16 270 -> 198, b = 10, 5120 signals 215 -> 180 [154 -> 139]), the synthesis up to 1500 signals where
 // walking blocks take four betas at a time (b = 16: 193 -> 164 us, at 3200 signals 382 -> 428 [338 -> 302]; b = 12:
 // 77 -> 74, 136 -> 173) and everywhere else (b = 15, 3200 signals: 542 -> 361, b = 10, 5120: 161 -> 157 [134 -> 118]).
+// `product` 2, both factors spectra of real signals (s2_mirror; full -> half product): b = 16, six features, 3200 signals:
+// walking 440 -> 395, planes 442 -> 355; b = 14, three, 3840: 385 -> 372, 337 -> 301; b = 12, one, 4000: walking 150 -> 147,
+// planes 176 -> 165; the relay of b = 10, one, 5120: 148 -> 139.
 static bool so3_prefers_planes(ClKind kind, int N, int K, int nl, long nbatch, const void* ws, size_t ws_bytes,
-                               bool product = false) {
+                               int product = 0) {
   const int forced = g_cluster.load();
   if (g_force_general || !small_supported(N) || !ws || forced == 1 || forced == 2) return false;
   if (ws_bytes < so3_mid_v_per_z(N, K) * (size_t)std::min<long>(kWigZT, nbatch) || nl > kColMaxDegrees) return false;
   if (forced == 3) return true;
   const bool full = 3 * K > N, relay = kind == kClRelay;
-  if (product) return nbatch >= (N >= 22 ? 256 : 600) && (relay || N < 24 || N % 4 != 0 || nbatch <= 1500);
+  if (product) return nbatch >= (N >= 22 ? 256 : 600) && (relay || N < 24 || N % 4 != 0 || nbatch <= 1500 || (product == 2 && N > 24));
   if (N >= 26) return nbatch >= (full ? (relay ? 32 : 48) : 256);
   if (N == 24) return nbatch >= (full ? 64 : relay ? 512 : 256);
   return nbatch >= (N == 22 ? 256 : 600);
@@ -233,7 +236,7 @@ static So3Route analysis_route(int N, int K, int nl, long nbatch, const void* ws
   return big_route(N);
 }
 // `one_kernel`: a synthesis that writes no signal (its integral)
-static So3Route synthesis_route(int N, int K, long nbatch, const void* ws, size_t ws_bytes, bool product = false,
+static So3Route synthesis_route(int N, int K, long nbatch, const void* ws, size_t ws_bytes, int product = 0,
                                 bool one_kernel = false) {
   if (!one_kernel && so3_prefers_planes(kClSynthesis, N, K, K, nbatch, ws, ws_bytes, product)) return kPlanes;
   if (!g_force_general && N <= kFusedMaxN) {
@@ -242,7 +245,7 @@ static So3Route synthesis_route(int N, int K, long nbatch, const void* ws, size_
   }
   return big_route(N);
 }
-static bool relay_takes_planes(int N, int Kin, int Kout, long nbatch, const void* ws, size_t ws_bytes, bool product) {
+static bool relay_takes_planes(int N, int Kin, int Kout, long nbatch, const void* ws, size_t ws_bytes, int product) {
   return so3_prefers_planes(kClRelay, N, Kin, Kout, nbatch, ws, ws_bytes, product) &&
          ws_bytes >= (so3_mid_v_per_z(N, Kin) + so3_mid_v_per_z(N, Kout)) * (size_t)std::min<long>(kWigZT, nbatch);
 }
@@ -268,6 +271,8 @@ static int launch_fwd_wigner_col(FwdWignerParams w, stream_t st) {
 static int launch_inv_wigner_col(InvWignerParams w, stream_t st) {
   w.ZT = std::min(kColZT, (w.nbatch + 31) / 32 * 32);
   w.nzt = (w.nbatch + w.ZT - 1) / w.ZT;
+  if (w.xs && w.s2_real)
+    return S2C_LAUNCH(so3_inv_wigner_col_s2real, (long)w.pan.npairs * w.nzt, w.ZT, wigner_col_smem(w.N, w.pan.nl), st, w);
   if (w.xs)
     return S2C_LAUNCH(so3_inv_wigner_col_s2, (long)w.pan.npairs * w.nzt, w.ZT, wigner_col_smem(w.N, w.pan.nl), st, w);
   return S2C_LAUNCH(so3_inv_wigner_col, (long)w.pan.npairs * w.nzt, w.ZT, wigner_col_smem(w.N, w.pan.nl), st, w);
@@ -437,6 +442,7 @@ struct S2ProductArgs {
   const float2* xs = nullptr;
   const float2* ys = nullptr;
   int nb = 0, fin = 0, fout = 0;
+  int real = 0;      // spectra of real signals
 };
 
 static bool so3_synthesis_is_fused(int b_in, int b_out) {
@@ -455,14 +461,14 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
   PanelsDev pan;
   S2C_TRY(TableCache::get().fft(N, fft));
   S2C_TRY(TableCache::get().panels(b_out, K, K, weighted, false, pan));
-  const So3Route route = synthesis_route(N, K, nbatch, ws, ws_bytes, prod != nullptr, integral != nullptr);
+  const So3Route route = synthesis_route(N, K, nbatch, ws, ws_bytes, prod ? 1 + prod->real : 0, integral != nullptr);
   const bool small = route == kPlanes, mid = small || route == kMid;
   if (mask && (out_stride != 1 || out_off != 0))
     return fail(S2C_ERR_UNSUPPORTED, "masked synthesis: real output only");
   if (route == kCluster) {
     ClInvParams f;
     f.in.x = x; f.in.x_zstride = nbatch; f.in.mode = mode;
-    f.in.xs = f.in.ys = nullptr; f.in.s2_nb = f.in.s2_fin = f.in.s2_fout = 0;
+    f.in.xs = f.in.ys = nullptr; f.in.s2_nb = f.in.s2_fin = f.in.s2_fout = f.in.s2_real = 0;
     f.out = out; f.out_stride = out_stride; f.out_off = out_off;
     f.bias = bias; f.nfeat = nfeat > 0 ? nfeat : 1;
     S2C_TRY(TableCache::get().cluster(b_out, K, K, weighted, f.tab));
@@ -478,7 +484,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     if (prod) {
       f.in.mode = kS2Product;
       f.in.xs = prod->xs; f.in.ys = prod->ys;
-      f.in.s2_nb = prod->nb; f.in.s2_fin = prod->fin; f.in.s2_fout = prod->fout;
+      f.in.s2_nb = prod->nb; f.in.s2_fin = prod->fin; f.in.s2_fout = prod->fout; f.in.s2_real = prod->real;
     }
     int rc = S2C_OK;
     S2C_DISPATCH_N(N, rc = S2C_LAUNCH_CL(so3_inv_cl, kN, (nbatch + kFusedZG - 1) / kFusedZG,
@@ -493,7 +499,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     f.pan = pan; f.tw = fft.tw;
     f.nbatch = (int)nbatch; f.K = K; f.BG = fused_bg(N); f.KP = fused_kp(N); f.PS = fused_plane_stride(N, K);
     f.nrows = pan.nrows; f.mode = mode;
-    f.xs = nullptr; f.ys = nullptr; f.s2_nb = f.s2_fin = f.s2_fout = 0;
+    f.xs = nullptr; f.ys = nullptr; f.s2_nb = f.s2_fin = f.s2_fout = f.s2_real = 0;
     f.iw = nullptr; f.isum = nullptr;
     f.mask = mask;
     f.wide = out_stride == 1 && out_off == 0 && N % 4 == 0 && out && (uintptr_t)out % 32 == 0 &&
@@ -507,7 +513,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     if (prod) {
       f.mode = kS2Product;
       f.xs = prod->xs; f.ys = prod->ys;
-      f.s2_nb = prod->nb; f.s2_fin = prod->fin; f.s2_fout = prod->fout;
+      f.s2_nb = prod->nb; f.s2_fin = prod->fin; f.s2_fout = prod->fout; f.s2_real = prod->real;
     }
     int rc = S2C_OK;
     const long grid = (nbatch + kFusedZG - 1) / kFusedZG;
@@ -565,7 +571,7 @@ static int so3_synthesis(const float2* x, float* out, long out_stride, long out_
     w.mode = mode;
     if (prod) {
       w.xs = prod->xs; w.ys = prod->ys;
-      w.s2_nb = prod->nb; w.s2_fin = prod->fin; w.s2_fout = prod->fout;
+      w.s2_nb = prod->nb; w.s2_fin = prod->fin; w.s2_fout = prod->fout; w.s2_real = prod->real;
       w.z0 = z0;
     }
     if (small) {
@@ -938,7 +944,7 @@ static int relay_bg(int N, int Kin, int nrows_in, int nrows_out) {
 
 // relay kernel: synthesis at bandwidth b_mid of a spectrum of bandwidth b_in (plain, or the s2_mm
 // product of xs and ys when xs is set), + bias, ReLU, analysis to bandwidth b_next
-static int relay_launch(const float2* x, const float2* xs, const float2* ys, int s2_nb, int s2_fin,
+static int relay_launch(const float2* x, const float2* xs, const float2* ys, int s2_nb, int s2_fin, int s2_real,
                         float* out, long nz, int nfeat, int b_in, int b_mid, int b_next,
                         const float* bias, void* ws, size_t ws_bytes, stream_t st, const char* who) {
   const int N = 2 * b_mid;
@@ -946,7 +952,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
     return fail(S2C_ERR_UNSUPPORTED,
                 std::string(who) + ": needs 2 b <= 32, b_in <= b and b_next <= b");
   const size_t v1 = so3_mid_v_per_z(N, b_in), v2 = so3_mid_v_per_z(N, b_next);
-  if (relay_takes_planes(N, b_in, b_next, nz, ws, ws_bytes, xs != nullptr)) {
+  if (relay_takes_planes(N, b_in, b_next, nz, ws, ws_bytes, xs ? 1 + s2_real : 0)) {
     PanelsDev pin, pout;
     S2C_TRY(TableCache::get().panels(b_mid, b_in, b_in, false, false, pin));
     S2C_TRY(TableCache::get().panels(b_mid, b_next, b_next, true, false, pout));
@@ -958,7 +964,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
       InvWignerParams w;
       w.x = xs ? nullptr : x + z0; w.x_zstride = nz; w.s = v; w.pan = pin;
       w.nbatch = (int)zc; w.N = N; w.K = b_in; w.mode = kSo3Real;
-      w.xs = xs; w.ys = ys; w.s2_nb = s2_nb; w.s2_fin = s2_fin; w.s2_fout = nfeat; w.z0 = z0;
+      w.xs = xs; w.ys = ys; w.s2_nb = s2_nb; w.s2_fin = s2_fin; w.s2_fout = nfeat; w.s2_real = s2_real; w.z0 = z0;
       S2C_TRY(launch_inv_wigner_col(w, st));
       SmallParams g;
       g.x = nullptr; g.out = nullptr; g.stride = 1; g.off = 0; g.v = v; g.v2 = vo;
@@ -980,7 +986,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
     S2C_TRY(TableCache::get().cluster(b_mid, b_next, b_next, true, f.tout));
     f.in.x = x; f.in.x_zstride = nz; f.in.mode = xs ? kS2Product : kSo3Real;
     f.in.xs = xs; f.in.ys = ys;
-    f.in.s2_nb = s2_nb; f.in.s2_fin = s2_fin; f.in.s2_fout = nfeat;
+    f.in.s2_nb = s2_nb; f.in.s2_fin = s2_fin; f.in.s2_fout = nfeat; f.in.s2_real = s2_real;
     f.bias = bias; f.nfeat = nfeat > 0 ? nfeat : 1;
     f.out = (float2*)out; f.out_zstride = nz;
     f.nbatch = (int)nz; f.Kin = b_in; f.Kout = b_next;
@@ -1000,7 +1006,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
   S2C_TRY(TableCache::get().grouped(b_mid, b_next, b_next, true, f.BG, &f.wout_g, &f.wout_stride));
   f.x = x; f.x_zstride = nz;
   f.xs = xs; f.ys = ys;
-  f.s2_nb = s2_nb; f.s2_fin = s2_fin; f.s2_fout = nfeat;
+  f.s2_nb = s2_nb; f.s2_fin = s2_fin; f.s2_fout = nfeat; f.s2_real = s2_real;
   f.bias = bias; f.nfeat = nfeat > 0 ? nfeat : 1;
   f.out = (float2*)out; f.out_zstride = nz;
   f.tw = fft.tw;
@@ -1013,7 +1019,7 @@ static int relay_launch(const float2* x, const float2* xs, const float2* ys, int
   return rc;
 }
 
-static size_t relay_workspace(long nbatch, int b_in, int b_mid, int b_next, bool product) {
+static size_t relay_workspace(long nbatch, int b_in, int b_mid, int b_next, int product) {
   const int N = 2 * b_mid;
   if (nbatch < 1 || b_in < 1 || b_next < 1 || N > kFusedMaxN || b_in > b_mid || b_next > b_mid ||
       !relay_takes_planes(N, b_in, b_next, nbatch, kAnyWorkspace, kAnySize, product))
@@ -1022,23 +1028,31 @@ static size_t relay_workspace(long nbatch, int b_in, int b_mid, int b_next, bool
   return v * (size_t)chunk_signals(nbatch, v);
 }
 size_t s2c_so3_relay_workspace(long nbatch, int b_in, int b_mid, int b_next) {
-  return relay_workspace(nbatch, b_in, b_mid, b_next, false);
+  return relay_workspace(nbatch, b_in, b_mid, b_next, 0);
 }
 size_t s2c_s2_conv_relu_so3_rfft_workspace(int nbatch, int f_out, int b, int b_next) {
-  return relay_workspace((long)nbatch * f_out, b, b, b_next, true);
+  return relay_workspace((long)nbatch * f_out, b, b, b_next, 1);
+}
+
+static int s2_relay(int real, const float* xs, const float* ys, float* out, int nbatch, int f_in, int f_out, int b, int b_next,
+                    const float* bias, void* ws, size_t ws_bytes, void* stream) {
+  S2C_TRY(check_b(b, b_next));
+  if (!xs || !ys || !out || nbatch < 1 || f_in < 1 || f_out < 1)
+    return fail(S2C_ERR_BAD_ARG, "s2c_s2_conv_relu_so3_rfft: bad argument");
+  return relay_launch(nullptr, (const float2*)xs, (const float2*)ys, nbatch, f_in, real, out,
+                      (long)nbatch * f_out, f_out, b, b, b_next, bias, ws, ws_bytes, as_stream(stream),
+                      "s2c_s2_conv_relu_so3_rfft");
 }
 
 int s2c_s2_conv_relu_so3_rfft_ws(const float* xs, const float* ys, float* out, int nbatch, int f_in,
                                  int f_out, int b, int b_next, const float* bias, void* ws,
                                  size_t ws_bytes, void* stream) {
-  S2C_TRY(check_b(b, b_next));
-  if (!xs || !ys || !out || nbatch < 1 || f_in < 1 || f_out < 1)
-    return fail(S2C_ERR_BAD_ARG, "s2c_s2_conv_relu_so3_rfft: bad argument");
-  return relay_launch(nullptr, (const float2*)xs, (const float2*)ys, nbatch, f_in, out,
-                      (long)nbatch * f_out, f_out, b, b, b_next, bias, ws, ws_bytes, as_stream(stream),
-                      "s2c_s2_conv_relu_so3_rfft");
+  return s2_relay(0, xs, ys, out, nbatch, f_in, f_out, b, b_next, bias, ws, ws_bytes, stream);
 }
-
+int s2c_s2_conv_real_relu_so3_rfft(const float* xs, const float* ys, float* out, int nbatch, int f_in, int f_out, int b,
+                                   int b_next, const float* bias, void* ws, size_t ws_bytes, void* stream) {
+  return s2_relay(1, xs, ys, out, nbatch, f_in, f_out, b, b_next, bias, ws, ws_bytes, stream);
+}
 int s2c_s2_conv_relu_so3_rfft(const float* xs, const float* ys, float* out, int nbatch, int f_in,
                               int f_out, int b, int b_next, const float* bias, void* stream) {
   return s2c_s2_conv_relu_so3_rfft_ws(xs, ys, out, nbatch, f_in, f_out, b, b_next, bias, nullptr, 0, stream);
@@ -1051,7 +1065,7 @@ int s2c_so3_rifft_relu_rfft_ws(const float* x, float* out, long nbatch, int b_in
   if (!x || !out || nbatch < 1) return fail(S2C_ERR_BAD_ARG, "s2c_so3_rifft_relu_rfft: bad argument");
   if (bias && nfeature < 1)
     return fail(S2C_ERR_BAD_ARG, "s2c_so3_rifft_relu_rfft: nfeature must be >= 1 with a bias");
-  return relay_launch((const float2*)x, nullptr, nullptr, 0, 0, out, nbatch, bias ? nfeature : 0,
+  return relay_launch((const float2*)x, nullptr, nullptr, 0, 0, 0, out, nbatch, bias ? nfeature : 0,
                       b_in, b_mid, b_next, bias, ws, ws_bytes, as_stream(stream), "s2c_so3_rifft_relu_rfft");
 }
 
@@ -1066,17 +1080,18 @@ static bool s2_product_in_wigner(int b) {
   return use_mid_kernels(2 * b) && inv_wigner_t_smem(2 * b, b) <= (size_t)dev_smem_limit() - 1024;
 }
 
-size_t s2c_s2_conv_synthesis_workspace(int nbatch, int f_out, int b) {
+static size_t s2_synthesis_workspace(int real, int nbatch, int f_out, int b) {
   if (nbatch < 1 || f_out < 1 || b < 1) return 0;
   const long nz = (long)nbatch * f_out;
   const bool product = so3_synthesis_is_fused(b, b) || s2_product_in_wigner(b);
   const size_t z_bytes = product ? 0 : (size_t)so3_nspec(b) * nz * sizeof(float2);
-  return z_bytes + route_workspace(synthesis_route(2 * b, b, nz, kAnyWorkspace, kAnySize, product), 2 * b, b, nz);
+  return z_bytes + route_workspace(synthesis_route(2 * b, b, nz, kAnyWorkspace, kAnySize, product ? 1 + real : 0), 2 * b, b, nz);
 }
+size_t s2c_s2_conv_synthesis_workspace(int nbatch, int f_out, int b) { return s2_synthesis_workspace(0, nbatch, f_out, b); }
+size_t s2c_s2_conv_real_synthesis_workspace(int nbatch, int f_out, int b) { return s2_synthesis_workspace(1, nbatch, f_out, b); }
 
-int s2c_s2_conv_synthesis(const float* xs, const float* ys, float* out, int nbatch, int f_in,
-                          int f_out, int b, const float* bias, void* ws, size_t ws_bytes,
-                          void* stream) {
+static int s2_synthesis(int real, const float* xs, const float* ys, float* out, int nbatch, int f_in, int f_out, int b,
+                        const float* bias, void* ws, size_t ws_bytes, void* stream) {
   S2C_TRY(check_b(b, b));
   if (!xs || !ys || !out || nbatch < 1 || f_in < 1 || f_out < 1)
     return fail(S2C_ERR_BAD_ARG, "s2c_s2_conv_synthesis: bad argument");
@@ -1084,7 +1099,7 @@ int s2c_s2_conv_synthesis(const float* xs, const float* ys, float* out, int nbat
   if (so3_synthesis_is_fused(b, b)) {
     S2ProductArgs pr;
     pr.xs = (const float2*)xs; pr.ys = (const float2*)ys;
-    pr.nb = nbatch; pr.fin = f_in; pr.fout = f_out;
+    pr.nb = nbatch; pr.fin = f_in; pr.fout = f_out; pr.real = real;
     return so3_synthesis(nullptr, out, 1, 0, nz, b, b, false, kSo3Real, bias, f_out, ws, ws_bytes,
                          as_stream(stream), &pr);
   }
@@ -1092,7 +1107,7 @@ int s2c_s2_conv_synthesis(const float* xs, const float* ys, float* out, int nbat
   if (s2_product_in_wigner(b)) {
     S2ProductArgs pr;
     pr.xs = (const float2*)xs; pr.ys = (const float2*)ys;
-    pr.nb = nbatch; pr.fin = f_in; pr.fout = f_out;
+    pr.nb = nbatch; pr.fin = f_in; pr.fout = f_out; pr.real = real;
     return so3_synthesis(nullptr, out, 1, 0, nz, b, b, false, kSo3Real, bias, f_out, ws, ws_bytes,
                          as_stream(stream), &pr);
   }
@@ -1102,6 +1117,15 @@ int s2c_s2_conv_synthesis(const float* xs, const float* ys, float* out, int nbat
   S2C_TRY(mm_dispatch(false, kMmFwd, xs, ys, (float*)ws, b, nbatch, f_in, f_out, as_stream(stream)));
   return so3_synthesis((const float2*)ws, out, 1, 0, nz, b, b, false, kSo3Real, bias, f_out,
                        (unsigned char*)ws + z_bytes, ws_bytes - z_bytes, as_stream(stream));
+}
+int s2c_s2_conv_synthesis(const float* xs, const float* ys, float* out, int nbatch, int f_in,
+                          int f_out, int b, const float* bias, void* ws, size_t ws_bytes,
+                          void* stream) {
+  return s2_synthesis(0, xs, ys, out, nbatch, f_in, f_out, b, bias, ws, ws_bytes, stream);
+}
+int s2c_s2_conv_real_synthesis(const float* xs, const float* ys, float* out, int nbatch, int f_in, int f_out, int b,
+                               const float* bias, void* ws, size_t ws_bytes, void* stream) {
+  return s2_synthesis(1, xs, ys, out, nbatch, f_in, f_out, b, bias, ws, ws_bytes, stream);
 }
 
 int s2c_so3_ifft(const float* x, float* out, long nbatch, int b_in, int b_out, int for_grad,

@@ -67,6 +67,7 @@ struct ClSpectrumIn {
   const float2* xs;    // [K*K, s2_nb, s2_fin]
   const float2* ys;    // [K*K, s2_fin, s2_fout]
   int s2_nb, s2_fin, s2_fout;
+  int s2_real;         // (s2_mirror)
 };
 struct ClInvParams {
   ClSpectrumIn in;
@@ -167,26 +168,12 @@ struct Cl {
 #pragma unroll
         for (int z = 0; z < ZG; ++z) { av[z] = make_float2(0.f, 0.f); bv[z] = make_float2(0.f, 0.f); }
         for (int k = 0; k < p.s2_fin; ++k) {
-          const float2 xk = xa[k], xm = xb[k];
-          const float4 y01 = *reinterpret_cast<const float4*>(ya + (long)k * p.s2_fout);
-          const float4 y23 = *reinterpret_cast<const float4*>(ya + (long)k * p.s2_fout + 2);
-          const float4 w01 = *reinterpret_cast<const float4*>(yb + (long)k * p.s2_fout);
-          const float4 w23 = *reinterpret_cast<const float4*>(yb + (long)k * p.s2_fout + 2);
-          const float2 yv[ZG] = {make_float2(y01.x, y01.y), make_float2(y01.z, y01.w),
-                                 make_float2(y23.x, y23.y), make_float2(y23.z, y23.w)};
-          const float2 wv[ZG] = {make_float2(w01.x, w01.y), make_float2(w01.z, w01.w),
-                                 make_float2(w23.x, w23.y), make_float2(w23.z, w23.w)};
+          s2_multiply_add(xa[k], ya + (long)k * p.s2_fout, av);
+          if (!p.s2_real) s2_multiply_add(xb[k], yb + (long)k * p.s2_fout, bv);
+        }
+        if (p.s2_real) {
 #pragma unroll
-          for (int z = 0; z < ZG; ++z) {   // x * conj(y)
-            av[z].x = fmaf(xk.x, yv[z].x, av[z].x);
-            av[z].x = fmaf(xk.y, yv[z].y, av[z].x);
-            av[z].y = fmaf(xk.y, yv[z].x, av[z].y);
-            av[z].y = fmaf(-xk.x, yv[z].y, av[z].y);
-            bv[z].x = fmaf(xm.x, wv[z].x, bv[z].x);
-            bv[z].x = fmaf(xm.y, wv[z].y, bv[z].x);
-            bv[z].y = fmaf(xm.y, wv[z].x, bv[z].y);
-            bv[z].y = fmaf(-xm.x, wv[z].y, bv[z].y);
-          }
+          for (int z = 0; z < ZG; ++z) bv[z] = s2_mirror(av[z], m - n);
         }
 #pragma unroll
         for (int z = 0; z < ZG; ++z) Xs[row.y * ZG + z] = symmetrise(av[z], bv[z], m - n, p.mode);
@@ -218,7 +205,7 @@ struct Cl {
           if (prod) {
             const int z = (int)(b.z0 + zz), zi = z / p.s2_fout, zj = z - zi * p.s2_fout;
             a = s2_product_entry(p, l, m, n, zi, zj);
-            c = s2_product_entry(p, l, -m, -n, zi, zj);
+            c = p.s2_real ? s2_mirror(a, m - n) : s2_product_entry(p, l, -m, -n, zi, zj);
           } else {
             a = p.x[so3_row(l, m, n) * p.x_zstride + b.z0 + zz];
             c = p.x[so3_row(l, -m, -n) * p.x_zstride + b.z0 + zz];

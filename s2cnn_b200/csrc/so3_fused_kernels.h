@@ -48,6 +48,7 @@ struct InvFusedParams {
   const float2* xs;    // [K*K, s2_nb, s2_fin]
   const float2* ys;    // [K*K, s2_fin, s2_fout]
   int s2_nb, s2_fin, s2_fout;
+  int s2_real;         // (s2_mirror)
   // optional tail of a network: instead of writing the signal, integrate max(signal, 0) over SO(3)
   // (so3_integrate(relu(.)), s2cnn/soft/so3_integrate.py:7-29) and write one number per batch element
   const float* iw;     // quadrature weights [N] (null: write the signal)
@@ -148,26 +149,12 @@ struct so3_inv_fused_impl {
 #pragma unroll
           for (int z = 0; z < ZG; ++z) { av[z] = make_float2(0.f, 0.f); bv[z] = make_float2(0.f, 0.f); }
           for (int k = 0; k < p.s2_fin; ++k) {
-            const float2 xk = xa[k], xm = xb[k];
-            const float4 y01 = *reinterpret_cast<const float4*>(ya + (long)k * p.s2_fout);
-            const float4 y23 = *reinterpret_cast<const float4*>(ya + (long)k * p.s2_fout + 2);
-            const float4 w01 = *reinterpret_cast<const float4*>(yb + (long)k * p.s2_fout);
-            const float4 w23 = *reinterpret_cast<const float4*>(yb + (long)k * p.s2_fout + 2);
-            const float2 yv[ZG] = {make_float2(y01.x, y01.y), make_float2(y01.z, y01.w),
-                                   make_float2(y23.x, y23.y), make_float2(y23.z, y23.w)};
-            const float2 wv[ZG] = {make_float2(w01.x, w01.y), make_float2(w01.z, w01.w),
-                                   make_float2(w23.x, w23.y), make_float2(w23.z, w23.w)};
+            s2_multiply_add(xa[k], ya + (long)k * p.s2_fout, av);
+            if (!p.s2_real) s2_multiply_add(xb[k], yb + (long)k * p.s2_fout, bv);
+          }
+          if (p.s2_real) {
 #pragma unroll
-            for (int z = 0; z < ZG; ++z) {   // x * conj(y)
-              av[z].x = fmaf(xk.x, yv[z].x, av[z].x);
-              av[z].x = fmaf(xk.y, yv[z].y, av[z].x);
-              av[z].y = fmaf(xk.y, yv[z].x, av[z].y);
-              av[z].y = fmaf(-xk.x, yv[z].y, av[z].y);
-              bv[z].x = fmaf(xm.x, wv[z].x, bv[z].x);
-              bv[z].x = fmaf(xm.y, wv[z].y, bv[z].x);
-              bv[z].y = fmaf(xm.y, wv[z].x, bv[z].y);
-              bv[z].y = fmaf(-xm.x, wv[z].y, bv[z].y);
-            }
+            for (int z = 0; z < ZG; ++z) bv[z] = s2_mirror(av[z], m - n);
           }
         } else {
           const float2* qa = p.x + so3_row(l, m, n) * p.x_zstride + z0;
@@ -222,7 +209,7 @@ struct so3_inv_fused_impl {
             const int z = (int)(z0 + zz);
             const int i = z / p.s2_fout, j = z - i * p.s2_fout;
             a[u] = s2_product_entry(p, l, m, n, i, j);
-            b[u] = s2_product_entry(p, l, -m, -n, i, j);
+            b[u] = p.s2_real ? s2_mirror(a[u], m - n) : s2_product_entry(p, l, -m, -n, i, j);
           } else {
             a[u] = p.x[so3_row(l, m, n) * p.x_zstride + z0 + zz];
             b[u] = p.x[so3_row(l, -m, -n) * p.x_zstride + z0 + zz];

@@ -287,6 +287,28 @@ S2C_KERNEL(so3_fwd_wigner, FwdWignerParams) {
   }
 }
 
+// The S2 product evaluated inside a synthesis (kS2Product): z[l,m,n][i,j] = sum_k x[l,m][i,k] conj(y[l,n][k,j]).
+// One k for four neighbouring j: acc[j] += x conj(y[j]), 16-byte aligned.
+S2C_D void s2_multiply_add(float2 x, const float2* y, float2 (&acc)[4]) {
+  const float4 y01 = *reinterpret_cast<const float4*>(y), y23 = *reinterpret_cast<const float4*>(y + 2);
+  const float2 yv[4] = {make_float2(y01.x, y01.y), make_float2(y01.z, y01.w), make_float2(y23.x, y23.y),
+                        make_float2(y23.z, y23.w)};
+#pragma unroll
+  for (int z = 0; z < 4; ++z) {
+    acc[z].x = fmaf(x.x, yv[z].x, acc[z].x);
+    acc[z].x = fmaf(x.y, yv[z].y, acc[z].x);
+    acc[z].y = fmaf(x.y, yv[z].x, acc[z].y);
+    acc[z].y = fmaf(-x.x, yv[z].y, acc[z].y);
+  }
+}
+// `s2_real`: x and y are spectra of real signals, x[l,-m] = (-1)^m conj x[l,m], so that entry (-m, -n) is the mirror of
+// entry (m, n) - for factors that are mirrors to the last bit, as the transforms at 2b < 64 make them, to the last bit:
+// the same products in the same order with other signs - and half of the multiply-adds and loads suffice.
+S2C_D float2 s2_mirror(float2 a, int m_minus_n) {
+  const float s = (m_minus_n & 1) ? -1.f : 1.f;
+  return make_float2(s * a.x, -s * a.y);
+}
+
 // ---------------------------------------------------------------------------------------------
 // synthesis, pass 1: Wigner-d contraction over l
 // ---------------------------------------------------------------------------------------------
@@ -300,6 +322,7 @@ struct InvWignerParams {
   const float2* xs = nullptr;   // [l * m, s2_nb, s2_fin]
   const float2* ys = nullptr;   // [l * m, s2_fin, s2_fout]
   int s2_nb = 0, s2_fin = 0, s2_fout = 0;
+  int s2_real = 0;              // (s2_mirror)
   long z0 = 0;
 };
 

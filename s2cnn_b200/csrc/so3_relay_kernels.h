@@ -28,6 +28,7 @@ struct RelayParams {
   const float2* xs;    // [Kin^2, s2_nb, s2_fin]
   const float2* ys;    // [Kin^2, s2_fin, s2_fout]
   int s2_nb, s2_fin, s2_fout;
+  int s2_real;         // (s2_mirror)
   const float* bias;   // optional [nfeat]
   int nfeat;
   PanelsDev pin;       // beta grid of b, nl = Kin (unweighted)
@@ -134,26 +135,12 @@ struct so3_relay_fused_impl {
 #pragma unroll
         for (int z = 0; z < ZG; ++z) { av[z] = make_float2(0.f, 0.f); bv[z] = make_float2(0.f, 0.f); }
         for (int k = 0; k < p.s2_fin; ++k) {
-          const float2 xk = xa[k], xm = xb[k];
-          const float4 y01 = *reinterpret_cast<const float4*>(ya + (long)k * p.s2_fout);
-          const float4 y23 = *reinterpret_cast<const float4*>(ya + (long)k * p.s2_fout + 2);
-          const float4 w01 = *reinterpret_cast<const float4*>(yb + (long)k * p.s2_fout);
-          const float4 w23 = *reinterpret_cast<const float4*>(yb + (long)k * p.s2_fout + 2);
-          const float2 yv[ZG] = {make_float2(y01.x, y01.y), make_float2(y01.z, y01.w),
-                                 make_float2(y23.x, y23.y), make_float2(y23.z, y23.w)};
-          const float2 wv[ZG] = {make_float2(w01.x, w01.y), make_float2(w01.z, w01.w),
-                                 make_float2(w23.x, w23.y), make_float2(w23.z, w23.w)};
+          s2_multiply_add(xa[k], ya + (long)k * p.s2_fout, av);
+          if (!p.s2_real) s2_multiply_add(xb[k], yb + (long)k * p.s2_fout, bv);
+        }
+        if (p.s2_real) {
 #pragma unroll
-          for (int z = 0; z < ZG; ++z) {   // x * conj(y)
-            av[z].x = fmaf(xk.x, yv[z].x, av[z].x);
-            av[z].x = fmaf(xk.y, yv[z].y, av[z].x);
-            av[z].y = fmaf(xk.y, yv[z].x, av[z].y);
-            av[z].y = fmaf(-xk.x, yv[z].y, av[z].y);
-            bv[z].x = fmaf(xm.x, wv[z].x, bv[z].x);
-            bv[z].x = fmaf(xm.y, wv[z].y, bv[z].x);
-            bv[z].y = fmaf(xm.y, wv[z].x, bv[z].y);
-            bv[z].y = fmaf(-xm.x, wv[z].y, bv[z].y);
-          }
+          for (int z = 0; z < ZG; ++z) bv[z] = s2_mirror(av[z], m - n);
         }
         const float fudge = ((m - n) & 1) ? -1.f : 1.f;
 #pragma unroll
@@ -174,13 +161,15 @@ struct so3_relay_fused_impl {
         const float2* ya = p.ys + (long)(l * l + l + n) * p.s2_fin * p.s2_fout + j;
         const float2* yb = p.ys + (long)(l * l + l - n) * p.s2_fin * p.s2_fout + j;
         for (int k = 0; k < p.s2_fin; ++k) {
-          const float2 xk = xa[k], xm = xb[k];
-          const float2 yk = ya[(long)k * p.s2_fout], ym = yb[(long)k * p.s2_fout];
+          const float2 xk = xa[k], yk = ya[(long)k * p.s2_fout];
           a.x = fmaf(xk.x, yk.x, a.x); a.x = fmaf(xk.y, yk.y, a.x);
           a.y = fmaf(xk.y, yk.x, a.y); a.y = fmaf(-xk.x, yk.y, a.y);
+          if (p.s2_real) continue;
+          const float2 xm = xb[k], ym = yb[(long)k * p.s2_fout];
           b.x = fmaf(xm.x, ym.x, b.x); b.x = fmaf(xm.y, ym.y, b.x);
           b.y = fmaf(xm.y, ym.x, b.y); b.y = fmaf(-xm.x, ym.y, b.y);
         }
+        if (p.s2_real) b = s2_mirror(a, m - n);
       }
       const float fudge = ((m - n) & 1) ? -1.f : 1.f;
       xh_at(r, zz) = make_float2(0.5f * (a.x + fudge * b.x), 0.5f * (a.y - fudge * b.y));

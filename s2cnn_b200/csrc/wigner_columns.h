@@ -117,7 +117,8 @@ S2C_KERNEL_BOUNDS(so3_fwd_wigner_col, FwdWignerParams, kColZT, 6) {
 }
 
 // S[beta][z] = sum_l W[l][beta] Xs[l][z],  Xs = symmetrised spectrum (or S2 product); table as [l][beta]
-template <bool kProduct>
+enum ColProduct { kColPlain, kColProduct, kColRealProduct };     // (kColRealProduct: s2_mirror)
+template <ColProduct kProduct>
 S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned char* smem) {
   const int N = p.N, NP = col_nb(N);
   const int pair = ctx.bid / p.nzt, zt = ctx.bid - pair * p.nzt;
@@ -137,7 +138,7 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
   auto degrees = [&](auto tiles) {
     constexpr int T = decltype(tiles)::value;
     float2 x[4 * T];
-    if constexpr (kProduct) {
+    if constexpr (kProduct != kColPlain) {
       // the loads of four degrees are in flight together (one product after the other: 101 us at b = 10, 5120
       // signals; all degrees at once do not fit the registers); multiply-adds in the order of the single-kernel transforms
       const unsigned zz = (unsigned)(p.z0 + z), i = zz / (unsigned)p.s2_fout, j = zz - i * (unsigned)p.s2_fout;
@@ -157,8 +158,9 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               if (4 * t + q < L) {
-                u[q] = xr[m * xs]; u2[q] = xr[-m * xs];
-                v[q] = yr[n * ys]; v2[q] = yr[-n * ys];
+                u[q] = xr[m * xs];
+                v[q] = yr[n * ys];
+                if constexpr (kProduct == kColProduct) { u2[q] = xr[-m * xs]; v2[q] = yr[-n * ys]; }
               }
               xr += 2L * (l + q + 1) * xs;
               yr += 2L * (l + q + 1) * ys;
@@ -173,13 +175,15 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
             for (int q = 0; q < 4; ++q) {
               if (4 * t + q >= L) continue;
               mul(u[q], v[q], a[q]);
-              mul(u2[q], v2[q], b[q]);
+              if constexpr (kProduct == kColProduct) mul(u2[q], v2[q], b[q]);
             }
           }
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          x[4 * t + q] = make_float2(0.5f * (a[q].x + fudge * b[q].x), 0.5f * (a[q].y - fudge * b[q].y));
+        for (int q = 0; q < 4; ++q) {
+          if constexpr (kProduct == kColRealProduct) x[4 * t + q] = a[q];
+          else x[4 * t + q] = make_float2(0.5f * (a[q].x + fudge * b[q].x), 0.5f * (a[q].y - fudge * b[q].y));
+        }
         // rows (l, 0) -> (l + 4, 0): l (l + 1) grows by 8 l + 20
         x0 += (8L * l + 20) * xs;
         y0 += (8L * l + 20) * ys;
@@ -233,7 +237,8 @@ S2C_D void inv_wigner_col(const Ctx& ctx, const InvWignerParams& p, unsigned cha
   else if (LT == 3) degrees(std::integral_constant<int, 3>{});
   else degrees(std::integral_constant<int, 4>{});
 }
-S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) { inv_wigner_col<false>(ctx, p, smem); }
-S2C_KERNEL_BOUNDS(so3_inv_wigner_col_s2, InvWignerParams, kColZT, 6) { inv_wigner_col<true>(ctx, p, smem); }
+S2C_KERNEL_BOUNDS(so3_inv_wigner_col, InvWignerParams, kColZT, 6) { inv_wigner_col<kColPlain>(ctx, p, smem); }
+S2C_KERNEL_BOUNDS(so3_inv_wigner_col_s2, InvWignerParams, kColZT, 6) { inv_wigner_col<kColProduct>(ctx, p, smem); }
+S2C_KERNEL_BOUNDS(so3_inv_wigner_col_s2real, InvWignerParams, kColZT, 6) { inv_wigner_col<kColRealProduct>(ctx, p, smem); }
 
 }  // namespace s2c

@@ -283,7 +283,8 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
     } else if (zz < zc && p.xs) {
       const int l = lmin + li;
       const int z = (int)(p.z0 + z0 + zz), i = z / p.s2_fout, j = z - i * p.s2_fout;
-      const float2 a = wig_s2_product(p, l, m, n, i, j), b = wig_s2_product(p, l, -m, -n, i, j);
+      const float2 a = wig_s2_product(p, l, m, n, i, j);
+      const float2 b = p.s2_real ? s2_mirror(a, m - n) : wig_s2_product(p, l, -m, -n, i, j);
       v = make_float2(0.5f * (a.x + fudge * b.x), 0.5f * (a.y - fudge * b.y));
     } else if (zz < zc) {
       const int l = lmin + li;

@@ -79,7 +79,7 @@ long s2_bandwidth(long nspec) {
   X(last_error) X(is_cuda_build) X(tables_computed) X(so3_analysis_workspace) X(so3_synthesis_workspace) X(so3_rfft)               \
   X(so3_rfft_relu) X(so3_rfft_sums_ws) X(so3_relay_workspace) X(s2_conv_relu_so3_rfft_workspace) X(s2_conv_relu_so3_rfft_ws) X(so3_rifft_relu_rfft_ws) X(so3_rifft_relu_grad_ws) X(so3_fft) X(so3_rifft)                 \
   X(so3_rifft_relu_integrate)                      \
-  X(s2_conv_synthesis_workspace) X(s2_conv_synthesis) X(so3_ifft) X(s2_fft_workspace) X(s2_fft)    \
+  X(s2_conv_synthesis_workspace) X(s2_conv_synthesis) X(s2_conv_real_synthesis_workspace) X(s2_conv_real_synthesis) X(s2_conv_real_relu_so3_rfft) X(so3_ifft) X(s2_fft_workspace) X(s2_fft)    \
   X(s2_ifft) X(so3_mm) X(so3_mm_gradx_ws) X(so3_mm_gradx_workspace) X(so3_mm_grady_ws) X(so3_mm_grady_workspace) X(so3_mm_real) X(so3_mm_real_workspace) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
   X(s2_mm_grady) X(rft_forward) X(rft_forward_t) X(rft_forward_scaled) X(rft_backward_scaled) X(rft_backward_workspace) X(so3_integrate)                  \
   X(so3_integrate_backward) X(so3_rotate_spectrum) X(project_on_sphere)
@@ -331,7 +331,8 @@ struct Ops {
     return d;
   }
 
-  Tensor s2_conv_relu_so3_rfft(const Tensor& xs_, const Tensor& ys_, const OptTensor& bias, int64_t b_next) {
+  // `real`: the factors are spectra of real signals
+  Tensor s2_conv_relu_so3_rfft(const Tensor& xs_, const Tensor& ys_, const OptTensor& bias, int64_t b_next, bool real) {
     prep(xs_); prep(ys_); prep(bias);
     const S2Product d = s2_product_dims(xs_, ys_);
     const Tensor xs = xs_.contiguous(), ys = ys_.contiguous();
@@ -342,7 +343,10 @@ struct Ops {
     Tensor out = empty_like_shape(xs, {so3_nspec(b_next), d.nb, d.fo, 2});
     Ctx c(*this, xs);
     const Scratch ws(s2_conv_relu_so3_rfft_workspace_((int)d.nb, (int)d.fo, (int)d.b, (int)b_next), xs);
-    S2C_CALL(s2_conv_relu_so3_rfft_ws, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, (int)b_next, bp, ws.p, ws.n, c.stream);
+    if (real)
+      S2C_CALL(s2_conv_real_relu_so3_rfft, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, (int)b_next, bp, ws.p, ws.n, c.stream);
+    else
+      S2C_CALL(s2_conv_relu_so3_rfft_ws, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, (int)b_next, bp, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -365,7 +369,7 @@ struct Ops {
     return out;
   }
 
-  Tensor s2_conv_synthesis(const Tensor& xs_, const Tensor& ys_, const OptTensor& bias) {
+  Tensor s2_conv_synthesis(const Tensor& xs_, const Tensor& ys_, const OptTensor& bias, bool real) {
     prep(xs_); prep(ys_); prep(bias);
     const S2Product d = s2_product_dims(xs_, ys_);
     const Tensor xs = xs_.contiguous(), ys = ys_.contiguous();
@@ -376,8 +380,11 @@ struct Ops {
     const long n = 2 * d.b;
     Tensor out = empty_like_shape(xs, {d.nb, d.fo, n, n, n});
     Ctx c(*this, xs);
-    const Scratch ws(s2_conv_synthesis_workspace_((int)d.nb, (int)d.fo, (int)d.b), xs);
-    S2C_CALL(s2_conv_synthesis, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, bp, ws.p, ws.n, c.stream);
+    const Scratch ws((real ? s2_conv_real_synthesis_workspace_ : s2_conv_synthesis_workspace_)((int)d.nb, (int)d.fo, (int)d.b), xs);
+    if (real)
+      S2C_CALL(s2_conv_real_synthesis, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, bp, ws.p, ws.n, c.stream);
+    else
+      S2C_CALL(s2_conv_synthesis, cptr(xs), cptr(ys), ptr(out), (int)d.nb, (int)d.fi, (int)d.fo, (int)d.b, bp, ws.p, ws.n, c.stream);
     return out;
   }
 
@@ -724,7 +731,8 @@ struct S2ProductSynthesis : torch::autograd::Function<S2ProductSynthesis> {
     keep_ops(ctx, ops);
     ctx->save_for_backward({x, y});
     ctx->saved_data["bias_shape"] = bias.sizes().vec();
-    return reinterpret_cast<Ops*>(ops)->s2_conv_synthesis(x, y, bias);
+    // (the full product, as in SpectralMm: a kernel spectrum is a mirror of itself but for single last bits)
+    return reinterpret_cast<Ops*>(ops)->s2_conv_synthesis(x, y, bias, false);
   }
   static tensor_list backward(AutogradContext* ctx, tensor_list g) {
     const auto saved = ctx->get_saved_variables();
@@ -854,9 +862,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("so3_rifft", &Ops::so3_rifft, "x"_a, "for_grad"_a = false, "b_out"_a = none, "bias"_a = none, nogil)
       .def("so3_rifft_relu_grad", &Ops::so3_rifft_relu_grad, "x"_a, "act"_a, nogil)
       .def("so3_rifft_relu_integrate", &Ops::so3_rifft_relu_integrate, "x"_a, "bias"_a = none, "b_out"_a = none, nogil)
-      .def("s2_conv_relu_so3_rfft", &Ops::s2_conv_relu_so3_rfft, "xs"_a, "ys"_a, "bias"_a, "b_next"_a, nogil)
+      .def("s2_conv_relu_so3_rfft", &Ops::s2_conv_relu_so3_rfft, "xs"_a, "ys"_a, "bias"_a, "b_next"_a, "real"_a = false, nogil)
       .def("so3_rifft_relu_rfft", &Ops::so3_rifft_relu_rfft, "x"_a, "bias"_a, "b_mid"_a, "b_next"_a, nogil)
-      .def("s2_conv_synthesis", &Ops::s2_conv_synthesis, "xs"_a, "ys"_a, "bias"_a = none, nogil)
+      .def("s2_conv_synthesis", &Ops::s2_conv_synthesis, "xs"_a, "ys"_a, "bias"_a = none, "real"_a = false, nogil)
       .def("so3_ifft", &Ops::so3_ifft, "x"_a, "for_grad"_a = false, "b_out"_a = none, nogil)
       .def("s2_fft", &Ops::s2_fft, "x"_a, "for_grad"_a = false, "b_out"_a = none, "x_is_real"_a = false, nogil)
       .def("s2_ifft", &Ops::s2_ifft, "x"_a, "for_grad"_a = false, "b_out"_a = none, "out_is_real"_a = false, nogil)
@@ -900,7 +908,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           }, "x"_a, "bias"_a, nogil)
       .def("ag_s2_product_synthesis", [](Ops& o, const Tensor& x, const Tensor& y, const Tensor& bias) {
             S2C_TRACED("ag_s2_product_synthesis", x, y, bias);
-            return wants_grad(x, y, bias) ? S2ProductSynthesis::apply(id(o), x, y, bias) : o.s2_conv_synthesis(x, y, bias);
+            return wants_grad(x, y, bias) ? S2ProductSynthesis::apply(id(o), x, y, bias) : o.s2_conv_synthesis(x, y, bias, true);
           }, "x"_a, "y"_a, "bias"_a, nogil)
       .def("ag_so3_mm", [](Ops& o, const Tensor& x, const Tensor& y) {
             S2C_TRACED("ag_so3_mm", x, y);

@@ -16,7 +16,8 @@ from ._recompute import fused_or_recompute
 def _product_synthesis(x, y, bias):
     """``SO3_ifft_real(s2_mm(x, y)) + bias`` (s2_conv.py:42-45) as one differentiable op: for small
     bandwidths the product is evaluated inside the synthesis kernel and the SO(3) spectrum never
-    reaches memory."""
+    reaches memory.  ``x`` and ``y`` are spectra of real signals (half products
+    where no gradient is recorded)."""
     return cuda_ops().ag_s2_product_synthesis(x, y, bias)
 
 
@@ -77,7 +78,7 @@ class S2Convolution(Module):
             else:
                 plain = lambda xx, yy, bb: SO3_fft_real.apply(torch.relu(_product_synthesis(xx, yy, bb)), b_next)  # noqa: E731
             if 2 * self.b_out <= 32 and b_next <= self.b_out:
-                fused = lambda xx, yy, bb: cuda_ops().s2_conv_relu_so3_rfft(xx, yy, bb, b_next)  # noqa: E731
+                fused = lambda xx, yy, bb: cuda_ops().s2_conv_relu_so3_rfft(xx, yy, bb, b_next, real=True)  # noqa: E731
                 grad = torch.is_grad_enabled() and (x.requires_grad or y.requires_grad or own_bias.requires_grad)
                 return fused_or_recompute(fused, plain, (x, y, own_bias), grad,
                                           getattr(self, "fused_training", False))
