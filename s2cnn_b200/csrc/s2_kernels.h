@@ -271,19 +271,25 @@ template <int N>
 __global__ void __launch_bounds__(256) s2_fwd_fused(const S2FwdFusedParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   s2_fwd_fused_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 template <int N>
 __global__ void __launch_bounds__(256) s2_fwd_rows(const S2RowsParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   s2_fwd_rows_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 template <int N>
 __global__ void __launch_bounds__(256) s2_inv_rows(const S2RowsParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   s2_inv_rows_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 S2C_LAUNCHER_N(s2_fwd_fused, S2FwdFusedParams)
 S2C_LAUNCHER_N(s2_fwd_rows, S2RowsParams)

@@ -760,7 +760,9 @@ struct so3_relay_cl_impl {
     extern __shared__ float4 s2c_dyn_smem[];                                                             \
     constexpr int C = cl_size(N);                                                                        \
     ClCtx ctx{(int)threadIdx.x, (int)blockDim.x, (int)(blockIdx.x / C), (int)(blockIdx.x % C)};          \
+    stream_order_wait();                                                                                 \
     name##_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));                         \
+    stream_order_next();  \
   }
 S2C_CLUSTER_KERNEL(so3_inv_cl, ClInvParams)
 S2C_CLUSTER_KERNEL(so3_fwd_cl, ClFwdParams)

@@ -732,13 +732,17 @@ template <int N>
 __global__ void __launch_bounds__(kFusedMaxThreads) so3_inv_fused(const InvFusedParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_inv_fused_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 template <int N>
 __global__ void __launch_bounds__(kFusedMaxThreads) so3_fwd_fused(const FwdFusedParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_fwd_fused_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 // Launcher of a kernel family with a compile-time length, launch_<name><N>; the launch records carry the
 // instantiation's name, e.g. "so3_inv_fused<20>".  In the split build (build.py) only parts.cu defines

@@ -327,13 +327,17 @@ template <int N>
 __global__ void __launch_bounds__(kMidThreads, 3) so3_fwd_mid(const MidParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_fwd_mid_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 template <int N>
 __global__ void __launch_bounds__(kMidThreads, 3) so3_inv_mid(const MidParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_inv_mid_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 S2C_LAUNCHER_N(so3_fwd_mid, MidParams)
 S2C_LAUNCHER_N(so3_inv_mid, MidParams)

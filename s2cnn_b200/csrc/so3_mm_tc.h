@@ -375,6 +375,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  stream_order_wait();     // (what is above touches no memory of another kernel; no other CTA of these fits beside this one)
+  stream_order_next();     // (CTAs of 150 KB: none of these beside a waiting one of the next kernel, whose set-up is the longest)
 
   bool ok = true;
   // a wait that gives up tells every role to leave its loop

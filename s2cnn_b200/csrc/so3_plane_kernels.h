@@ -380,13 +380,17 @@ template <int N>
 __global__ void __launch_bounds__(plane_threads(kPlaneRW), 2) so3_fwd_plane(const FwdPlaneParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_fwd_plane_impl<N, kPlaneRW>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 template <int N>
 __global__ void __launch_bounds__(plane_threads(kPlaneRW), 2) so3_inv_plane(const InvPlaneParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_inv_plane_impl<N, kPlaneRW>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 #define S2C_LAUNCH_PLANE(name, N, grid, stream, params)                                       \
   s2c::launch_impl<name<N>>(#name, (long)(grid), s2c::plane_threads(s2c::kPlaneRW),           \

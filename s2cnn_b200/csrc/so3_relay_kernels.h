@@ -384,7 +384,9 @@ template <int N>
 __global__ void __launch_bounds__(256, 3) so3_relay_fused(const RelayParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_relay_fused_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 S2C_LAUNCHER_N(so3_relay_fused, RelayParams)
 #endif

@@ -296,7 +296,9 @@ struct so3_relay_small_impl {
   __global__ void __launch_bounds__(small_threads(N), N == 32 ? 5 : 768 / small_threads(N)) name(const SmallParams p) {                \
     extern __shared__ float4 s2c_dyn_smem[];                                                     \
     Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};                 \
+    stream_order_wait();                                                                           \
     name##_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));                 \
+    stream_order_next();  \
   }                                                                                              \
   S2C_LAUNCHER_N(name, SmallParams)
 S2C_SMALL_KERNEL(so3_fwd_small)

@@ -620,13 +620,17 @@ template <int N>
 __global__ void __launch_bounds__(kRowsThreads, 1) so3_fwd_wigner_r(const FwdRowsParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_fwd_wigner_r_impl<N>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 template <int N, int ZQ>
 __global__ void __launch_bounds__(kRowsThreadsI, 2) so3_inv_wigner_r(const InvRowsParams p) {
   extern __shared__ float4 s2c_dyn_smem[];
   Ctx ctx{(int)threadIdx.x, (int)blockDim.x, (int)blockIdx.x, (int)gridDim.x};
+  stream_order_wait();
   so3_inv_wigner_r_impl<N, ZQ>::run(ctx, p, reinterpret_cast<unsigned char*>(s2c_dyn_smem));
+  stream_order_next();
 }
 #define S2C_LAUNCH_FWD_ROWS(N, grid, stream, params)                                                             \
   s2c::launch_impl<so3_fwd_wigner_r<N>>("so3_fwd_wigner_r", (long)(grid), s2c::kRowsThreads, s2c::rows_fwd_smem(N), \
