@@ -258,6 +258,9 @@ int s2c_s2_mm_gradx(const float* gz, const float* y, float* gx, int nl, int nbat
 /* Replaces _cuda_S2_mm.backward grad-y, s2cnn/s2_mm.py:94-99 (+ s2mm_grady.cu :258-312). */
 int s2c_s2_mm_grady(const float* gz, const float* x, float* gy, int nl, int nbatch, int f_in,
                     int f_out, void* stream);
+/* The same two for spectra of real signals, as s2c_so3_mm_real. */
+int s2c_s2_mm_real_gradx(const float* gz, const float* y, float* gx, int nl, int nbatch, int f_in, int f_out, void* stream);
+int s2c_s2_mm_real_grady(const float* gz, const float* x, float* gy, int nl, int nbatch, int f_in, int f_out, void* stream);
 
 /* ---- kernel-grid -> spectrum transforms ----------------------------------------------------- */
 /* out[s, f, :] = sum_a x[f, a] F[a, s, :];  x [nf, n_grid], F [n_grid, nspec, 2] (device),

@@ -83,6 +83,8 @@ _SIGNATURES = {
     "s2c_s2_mm": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_s2_mm_gradx": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_s2_mm_grady": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
+    "s2c_s2_mm_real_gradx": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
+    "s2c_s2_mm_real_grady": (c_int, [_P, _P, _P, c_int, c_int, c_int, c_int, _P]),
     "s2c_rft_forward": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P]),
     "s2c_rft_forward_t": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P]),
     "s2c_rft_forward_scaled": (c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_float, _P]),

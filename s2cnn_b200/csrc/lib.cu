@@ -1341,11 +1341,15 @@ static int so3_mm_tc_launch(int op, int half, const float* a, const float* b, fl
   const long tiles = so3_mm_tc_tiles(op, half, nl, nb, fi, fo);
   p.csize = p.groups = 1;
   p.part = nullptr; p.count = nullptr;
-  // The forward product always runs one CTA per tile: its rounding is then the same whatever the batch.
+  // The rounding of a forward product is the same whatever the batch: one CTA per tile, or segments
   if (op != kTcFwd) S2C_TRY(tc_share(p, op, tiles, ws, ws_bytes, st));
+  const int blocks = (2 * nl - 1) * p.nblk;
+  p.segs = op == kTcFwd && half ? tc_segments(nl, fi, fo, blocks) : 0;
+  if (p.segs > 1 && tiles <= kTcSlots[p.segs]) p.csize = p.segs;
   const int ns = p.csize * p.groups;
   const long ctas = tiles * ns;
-  const bool flush = tc_flush(p, (2L * nl - 1) * p.nblk, ns);
+  const bool flush = p.segs > 1 ? ns == 1 : tc_flush(p, blocks, ns);
+  p.two = half && p.segs <= 1;
   const bool vec = so3_mm_tc_vec16(op, nb, fi, fo);
   if (op == kTcFwd) return launch_so3_mm_tc<kTcFwd>("so3_mm_tc_kernel", ctas, flush, vec, st, p);
   if (op == kTcGradX) return launch_so3_mm_tc<kTcGradX>("so3_mm_tc_gradx", ctas, flush, vec, st, p);
@@ -1359,7 +1363,7 @@ static int plain_tc_launch(bool a_strided, const float* a, const float* b, float
                            float scale, void* ws, size_t ws_bytes, stream_t st) {
   MmTcParams p;
   p.a = a; p.b = b; p.c = c;
-  p.nl = 1; p.nb = (int)M; p.fi = (int)(K / 2); p.fo = (int)(N / 2); p.half = 0;
+  p.nl = 1; p.nb = (int)M; p.fi = (int)(K / 2); p.fo = (int)(N / 2); p.half = p.two = p.segs = 0;
   p.run = (int)K;
   tc_blocks(p);
   p.a_rs = a_rs; p.a_ps = a_ps; p.b_rs = b_rs; p.b_ps = b_ps; p.c_rs = c_rs; p.c_ps = c_ps;
@@ -1477,32 +1481,45 @@ int s2c_s2_mm(const float* x, const float* y, float* z, int nl, int nb, int fi, 
   if (!x || !y || !z) return fail(S2C_ERR_BAD_ARG, "s2c_s2_mm: null pointer");
   return mm_dispatch(false, kMmFwd, x, y, z, nl, nb, fi, fo, as_stream(st));
 }
-int s2c_s2_mm_gradx(const float* gz, const float* y, float* gx, int nl, int nb, int fi, int fo,
-                    void* st) {
+static int s2_mm_gradx_any(int real, const float* gz, const float* y, float* gx, int nl, int nb, int fi, int fo, void* st) {
   if (!gz || !y || !gx) return fail(S2C_ERR_BAD_ARG, "s2c_s2_mm_gradx: null pointer");
   if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
   if (!g_force_general && s2_mm_thin_supported(nl, fi, fo)) {
     S2ThinParams p;
     p.gz = (const float2*)gz; p.other = (const float2*)y; p.out = (float2*)gx;
-    p.nl = nl; p.nb = nb; p.fi = fi; p.fo = fo;
-    const long blocks = (long)nl * nl * ((nb + kThinRows - 1) / kThinRows);
+    p.nl = nl; p.nb = nb; p.fi = fi; p.fo = fo; p.real = real;
+    const long blocks = (long)thin_rows(nl, real) * ((nb + kThinRows - 1) / kThinRows);
     return S2C_LAUNCH(s2_mm_gradx_thin, blocks, kThinRows * kThinSlices,
                       s2_gradx_thin_smem(nl, fi, fo), as_stream(st), p);
   }
   return mm_dispatch(false, kMmGradX, gz, y, gx, nl, nb, fi, fo, as_stream(st));
 }
-int s2c_s2_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo,
-                    void* st) {
+static int s2_mm_grady_any(int real, const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo, void* st) {
   if (!gz || !x || !gy) return fail(S2C_ERR_BAD_ARG, "s2c_s2_mm_grady: null pointer");
   if (nl < 1 || nb < 1 || fi < 1 || fo < 1) return fail(S2C_ERR_BAD_ARG, "sizes must be >= 1");
   if (!g_force_general && s2_mm_thin_supported(nl, fi, fo)) {
     S2ThinParams p;
     p.gz = (const float2*)gz; p.other = (const float2*)x; p.out = (float2*)gy;
-    p.nl = nl; p.nb = nb; p.fi = fi; p.fo = fo;
-    return S2C_LAUNCH(s2_mm_grady_thin, (long)nl * nl, s2_grady_thin_threads(fo),
+    p.nl = nl; p.nb = nb; p.fi = fi; p.fo = fo; p.real = real;
+    return S2C_LAUNCH(s2_mm_grady_thin, (long)thin_rows(nl, real), s2_grady_thin_threads(fo),
                       s2_grady_thin_smem(fo), as_stream(st), p);
   }
   return mm_dispatch(false, kMmGradY, x, gz, gy, nl, nb, fi, fo, as_stream(st));
+}
+int s2c_s2_mm_gradx(const float* gz, const float* y, float* gx, int nl, int nb, int fi, int fo, void* st) {
+  return s2_mm_gradx_any(0, gz, y, gx, nl, nb, fi, fo, st);
+}
+int s2c_s2_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo, void* st) {
+  return s2_mm_grady_any(0, gz, x, gy, nl, nb, fi, fo, st);
+}
+// Spectra of real signals: half of the result's rows, the others mirrored, and half of gz read.  Gradient of y, 6 -> 100
+// channels, nl = 16, batch 32: 103 -> 72 us (with eight rows in flight for four); 1 -> 8, nl = 30, batch 32: 69 -> 41; of x:
+// 333 -> 176, 50 -> 38.
+int s2c_s2_mm_real_gradx(const float* gz, const float* y, float* gx, int nl, int nb, int fi, int fo, void* st) {
+  return s2_mm_gradx_any(1, gz, y, gx, nl, nb, fi, fo, st);
+}
+int s2c_s2_mm_real_grady(const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo, void* st) {
+  return s2_mm_grady_any(1, gz, x, gy, nl, nb, fi, fo, st);
 }
 
 // ---- kernel-grid -> spectrum -----------------------------------------------------------------------

@@ -22,12 +22,33 @@ struct S2ThinParams {
   const float2* other;  // grad x: y [nl^2][fi][fo];  grad y: x [nl^2][nb][fi]
   float2* out;          // grad x: gx [nl^2][nb][fi]; grad y: gy [nl^2][fi][fo]
   int nl, nb, fi, fo;
+  int real;             // gz and other are spectra of real signals: rows (l, m >= 0) of out, the others are their mirrors
 };
+
+// row (l, m) of block t of a tile: all rows l^2 + m, or those of m >= 0 (index l .. 2l) in order of l
+struct ThinRow {
+  int l, m;
+};
+S2C_D ThinRow thin_row(int t, int real);
+S2C_HD int thin_rows(int nl, int real) { return real ? nl * (nl + 1) / 2 : nl * nl; }
+// the mirror of a row's value: out[l, -m] = (-1)^m conj out[l, m]
+S2C_D float2 thin_mirror(float2 v, int l, int m) { return ((m - l) & 1) ? make_float2(-v.x, v.y) : make_float2(v.x, -v.y); }
 
 S2C_D int thin_isqrt(int v) {   // floor(sqrt(v)) for the small row indices used here
   int r = (int)sqrtf((float)v);
   while (r * r > v) --r;
   while ((r + 1) * (r + 1) <= v) ++r;
+  return r;
+}
+S2C_D ThinRow thin_row(int t, int real) {
+  ThinRow r;
+  if (real) {
+    r.l = (thin_isqrt(8 * t + 1) - 1) / 2;
+    r.m = r.l + t - r.l * (r.l + 1) / 2;
+  } else {
+    r.l = thin_isqrt(t);
+    r.m = t - r.l * r.l;
+  }
   return r;
 }
 
@@ -44,7 +65,8 @@ S2C_KERNEL(s2_mm_gradx_thin, S2ThinParams) {
   // be the short ones
   const int rbid = ctx.nblk - 1 - ctx.bid;
   const int lm = rbid / tiles_i, itile = rbid - lm * tiles_i;
-  const int l = thin_isqrt(lm), m = lm - l * l;
+  const ThinRow tr = thin_row(lm, p.real);
+  const int l = tr.l, m = tr.m;
   const int L = 2 * l + 1;
   float2* ys = reinterpret_cast<float2*>(smem);                     // [L][fi][fo]
   float2* red = ys + (size_t)(2 * p.nl - 1) * p.fi * p.fo;          // [slices][rows][kThinFi]
@@ -93,6 +115,7 @@ S2C_KERNEL(s2_mm_gradx_thin, S2ThinParams) {
           s.y += t.y;
         }
         dst[k] = s;
+        if (p.real && m > l) p.out[((long)(l * l + 2 * l - m) * p.nb + i) * p.fi + k] = thin_mirror(s, l, m);
       }
     }
   }
@@ -109,7 +132,8 @@ inline size_t s2_grady_thin_smem(int fo) {
 // block = (l, n); thread = (slice of the batch rows, j); all of (m, i) is summed inside the block
 S2C_KERNEL_BOUNDS(s2_mm_grady_thin, S2ThinParams, 1024, 1) {
   const int rbid = ctx.nblk - 1 - ctx.bid;     // largest degrees (the long blocks) first
-  const int l = thin_isqrt(rbid), n = rbid - l * l;
+  const ThinRow tr = thin_row(rbid, p.real);
+  const int l = tr.l, n = tr.m;
   const int L = 2 * l + 1;
   const int nsl = ctx.nthr / p.fo;
   const int j = ctx.tid % p.fo, sl = ctx.tid / p.fo;
@@ -117,7 +141,7 @@ S2C_KERNEL_BOUNDS(s2_mm_grady_thin, S2ThinParams, 1024, 1) {
   float2 acc[kThinFi];
 #pragma unroll
   for (int k = 0; k < kThinFi; ++k) acc[k] = make_float2(0.f, 0.f);
-  // the rows (m, i) in one run over the slices, four in flight: with a loop over m around one over i a batch
+  // the rows (m, i) in one run over the slices, eight in flight: with a loop over m around one over i a batch
   // smaller than the slices left most threads idle and every m waited for its own loads (f_out = 8, batch 32,
   // b = 30: 168 us)
   if (sl < nsl) {
@@ -126,11 +150,11 @@ S2C_KERNEL_BOUNDS(s2_mm_grady_thin, S2ThinParams, 1024, 1) {
     const long gm = (long)L * p.nb * p.fo;                  // from m to m + 1
     const int rows = L * p.nb, dm = nsl / p.nb, di = nsl - dm * p.nb;
     int m = sl / p.nb, i = sl - m * p.nb;
-    for (int q = sl; q < rows; q += 4 * nsl) {
-      float2 gv[4];
-      int rq[4];
+    for (int q = sl; q < rows; q += 8 * nsl) {
+      float2 gv[8];
+      int rq[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 8; ++u) {
         rq[u] = q + u * nsl;
         gv[u] = make_float2(0.f, 0.f);
         if (rq[u] < rows) gv[u] = g0[m * gm + (long)i * p.fo];
@@ -139,7 +163,7 @@ S2C_KERNEL_BOUNDS(s2_mm_grady_thin, S2ThinParams, 1024, 1) {
         if (i >= p.nb) { i -= p.nb; ++m; }
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 8; ++u) {
         if (rq[u] >= rows) break;
         const float2* xr = x0 + (long)rq[u] * p.fi;         // rows of x are contiguous in (m, i)
 #pragma unroll
@@ -168,6 +192,7 @@ S2C_KERNEL_BOUNDS(s2_mm_grady_thin, S2ThinParams, 1024, 1) {
       s.y += t.y;
     }
     p.out[((long)(l * l + n) * p.fi + k) * p.fo + jj] = s;
+    if (p.real && n > l) p.out[((long)(l * l + 2 * l - n) * p.fi + k) * p.fo + jj] = thin_mirror(s, l, n);
   }
 }
 

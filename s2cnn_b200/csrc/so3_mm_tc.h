@@ -86,6 +86,8 @@ struct MmTcParams {
   float* c;         // output
   int nl, nb, fi, fo;
   int half;         // spectra of real signals: rows of outer index l .. 2l only, the others are their mirrors
+  int two;          // without partial sums: the products with a lo part go into the second accumulator
+  int segs;         // > 1: a tile's K blocks are summed in this many segments, in one CTA or one to a CTA of a cluster (tc_segments)
   int run;          // floats per outer contraction index: 2 fi (fwd), 2 fo (grad x), 2 nb (grad y)
   int kblk;         // floats per K block (multiple of 8, <= kTcKMax)
   int nblk;         // K blocks per run
@@ -345,10 +347,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   const long spec0 = (long)l * (4L * l * l - 1) / 3;
   const int fi2 = 2 * p.fi, fo2 = 2 * p.fo;
   const int nit = it_hi - it_lo;                          // K blocks of this CTA (a shared tile: possibly none)
-  const bool two_accs = !FLUSH && p.half;
+  const bool two_accs = !FLUSH && p.two;
   // accumulator groups (one when the whole chain stays in the tensor core's accumulator)
   const int flush_blocks = p.half ? kTcFlushBlocks - 1 : kTcFlushBlocks;
-  const int ngroups = FLUSH ? (nit + flush_blocks - 1) / flush_blocks : 1;
+  const bool segmented = p.segs > 1;
+  const int ngroups = !FLUSH ? 1 : segmented ? min(p.segs, nit) : (nit + flush_blocks - 1) / flush_blocks;
+  // first block beyond the group that begins at block `it` (segments: floor(r nit / segs), empty ones left out)
+  auto group_end = [&](int it) {
+    if (!segmented) return it + flush_blocks;
+    int r = (it + 1) * p.segs / nit;
+    while (r * nit / p.segs <= it) ++r;
+    return r * nit / p.segs;
+  };
 
   // ---- set-up: barriers, tensor memory ------------------------------------------------------
   if (tid == 0) {
@@ -401,6 +411,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     const int steps_full = (p.kblk + 7) / 8;
     const int steps_tail = (p.run - (p.nblk - 1) * p.kblk + 7) / 8;
     int kb = kb_lo, s = 0, g = 0, ing = 0;           // block within its run, stage, group, block within its group
+    int g_end = FLUSH && nit > 0 ? group_end(0) : 0;
     uint32_t full_par = 0;                        // parity of the `full` phase of the current round of stages
     for (int it = 0; it < nit; ++it) {
       if (__any_sync(0xffffffffu, *abort_flag)) break;
@@ -426,12 +437,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
           }
         }
         tc_commit(&empty[s]);     // arrives when these MMAs have read the stage
-        if ((FLUSH && ing + 1 == flush_blocks) || it + 1 == nit) tc_commit(&accdone[g & 1]);
+        if ((FLUSH && it + 1 == g_end) || it + 1 == nit) tc_commit(&accdone[g & 1]);
       }
       __syncwarp();
       if (++kb == p.nblk) kb = 0;
       if (++s == kTcStages) { s = 0; full_par ^= 1u; }
-      if (FLUSH && ++ing == flush_blocks) { ing = 0; ++g; }
+      ++ing;
+      if (FLUSH && it + 1 == g_end) {
+        ing = 0;
+        ++g;
+        if (it + 1 < nit) g_end = group_end(it + 1);
+      }
     }
   } else if (warp <= kTcCollectorWarps) {
     // ================================ collectors ================================================
@@ -698,7 +714,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
       store2(gcol + 2, o.z, o.w);
     }
   };
-  constexpr bool kShares = OP == kTcGradX || OP == kTcGradY || OP == kTcPlainSC;
+  constexpr bool kShares = OP != kTcPlainCC;
   if (kShares && nsplit > 1) {
     // ---- a shared tile.  16-byte chunk c4 of a thread's 32 columns lies at [c4][warp][lane]; rank r of the cluster
     // takes the chunks 8 r / csize .. of every thread.  (All threads of all CTAs pass the barriers, also after a
@@ -817,20 +833,32 @@ inline size_t tc_share_bytes(long tiles, int groups) {
 struct TcShare {
   int csize = 1, groups = 1;
 };
+// clusters resident on the chip, by size (cudaOccupancyMaxActiveClusters)
+constexpr int kTcSlots[kTcMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+// The half forward product of layers whose longest contraction, of `blocks` K blocks, takes up to eight segments of 7.5 on
+// average: each segment is one chain of the tensor core, and the segments are added in their order, rounded - in one CTA (as
+// groups of partial sums) or, where the tiles are too few for the chip, by a cluster with one segment to a CTA.  The
+// number follows from the layer alone, so that a result does not depend on the batch it was computed in.  Whole chain in
+// one CTA -> cluster: 20 -> 40, nl = 6, batch 1: 13.7 -> 10.1 us, batch 32: 15.5 -> 12.1; 13 -> 9, nl = 7, batch 5: 17.1 ->
+// 9.9; segments in one CTA, for more tiles than clusters: 16 -> 24, nl = 7, batch 32: 17.8 -> 18.6.  0: a layer with too many
+// tiles for clusters even at batch 1, or longer contractions: one CTA, the whole chain or groups of seven.
+inline int tc_segments(int nl, int fi, int fo, int blocks) {
+  const int s = (2 * blocks + 14) / 15;
+  return s <= kTcMaxCluster && so3_mm_tc_tiles(kTcFwd, 1, nl, 1, fi, fo) <= kTcSlots[s] ? s : 0;
+}
+
 // CTAs per tile.  One CTA fits on an SM; a product with few output tiles and a long contraction (the
 // transposed kernel transform of a layer with few channels: one or two tiles of several hundred K
 // blocks; the gradients of small batches) leaves most of the 148 SMs idle for the length of the longest
 // tile.  Estimate of the makespan in K blocks: where all clusters are resident at once the longest one, else at
 // least their average load and a last, short one (the grid starts with the highest degrees).  A CTA costs kCta
 // blocks on top of its own (set-up, pipeline fill, epilogue: about 6 us against 0.6 us a block), sharing within a
-// cluster another kShare and between clusters another kGather.  kSlots: clusters resident on the chip, by size
-// (cudaOccupancyMaxActiveClusters).  The split is taken only where the estimate drops by a tenth, so that large
+// cluster another kShare and between clusters another kGather.  The split is taken only where the estimate drops by a tenth, so that large
 // products keep one CTA per tile.  One CTA per tile -> shared (us): 100 -> 255 channels, nl 5, batch 32, grad-x 123 -> 86;
 // 20 -> 40, nl 6, batch 32, grad-x 29 -> 14, grad-y 22 -> 14; 13 -> 9, nl 7, batch 5, grad-x 14 -> 9; kernel gradients
 // (rows x grid x spectrum) 800 x 192 x 286 26 -> 11, 10000 x 192 x 1330 137 -> 115, 128 x 36 x 4495 (15 clusters) 189 -> 16.
 inline TcShare tc_pick_share(int op, int half, int nl, int nb, int fi, int fo, int nblk, bool several_clusters) {
   constexpr double kCta = 8, kShare = 4, kGather = 6;
-  constexpr int kSlots[kTcMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
   const long tiles = so3_mm_tc_tiles(op, half, nl, nb, fi, fo);
   auto estimate = [&](int c, int groups) {
     const int ns = c * groups;
@@ -841,13 +869,13 @@ inline TcShare tc_pick_share(int op, int half, int nl, int nb, int fi, int fo, i
       longest = std::max(longest, shortest);
       load += (double)tc_tiles_for(op, half, nb, fi, fo, l) * groups * shortest;
     }
-    return tiles * groups <= kSlots[c] ? longest : std::max(longest, load / kSlots[c] + shortest);
+    return tiles * groups <= kTcSlots[c] ? longest : std::max(longest, load / kTcSlots[c] + shortest);
   };
   TcShare best;
   double t = 0.9 * estimate(1, 1);
   for (int c = 2; c <= kTcMaxCluster; ++c)
     if (const double e = estimate(c, 1); e < t) { t = e; best.csize = c; }
-  for (int g = 2; several_clusters && tiles * g <= kSlots[kTcMaxCluster]; ++g)
+  for (int g = 2; several_clusters && tiles * g <= kTcSlots[kTcMaxCluster]; ++g)
     if (const double e = estimate(kTcMaxCluster, g); e < t) { t = e; best.csize = kTcMaxCluster; best.groups = g; }
   return best;
 }

@@ -81,7 +81,7 @@ long s2_bandwidth(long nspec) {
   X(so3_rifft_relu_integrate)                      \
   X(s2_conv_synthesis_workspace) X(s2_conv_synthesis) X(s2_conv_real_synthesis_workspace) X(s2_conv_real_synthesis) X(s2_conv_real_relu_so3_rfft) X(so3_ifft) X(s2_fft_workspace) X(s2_fft)    \
   X(s2_ifft) X(so3_mm) X(so3_mm_gradx_ws) X(so3_mm_gradx_workspace) X(so3_mm_grady_ws) X(so3_mm_grady_workspace) X(so3_mm_real) X(so3_mm_real_workspace) X(so3_mm_tc_status) X(s2_mm) X(s2_mm_gradx) \
-  X(s2_mm_grady) X(rft_forward) X(rft_forward_t) X(rft_forward_scaled) X(rft_backward_scaled) X(rft_backward_workspace) X(so3_integrate)                  \
+  X(s2_mm_grady) X(s2_mm_real_gradx) X(s2_mm_real_grady) X(rft_forward) X(rft_forward_t) X(rft_forward_scaled) X(rft_backward_scaled) X(rft_backward_workspace) X(so3_integrate)                  \
   X(so3_integrate_backward) X(so3_rotate_spectrum) X(project_on_sphere)
 
 struct Ops {
@@ -513,13 +513,13 @@ struct Ops {
     const S2Product d = s2_product_dims(x, y);
     return mm("s2c_s2_mm", s2_mm_, x, y, {so3_nspec(d.b), d.nb, d.fo, 2}, d.b, d.nb, d.fi, d.fo);
   }
-  Tensor s2_mm_gradx(const Tensor& gz, const Tensor& y, int64_t nb, int64_t fi) {
+  Tensor s2_mm_gradx(const Tensor& gz, const Tensor& y, int64_t nb, int64_t fi, bool real) {
     const long nl = s2_bandwidth(y.size(0)), fo = y.size(2);
-    return mm("s2c_s2_mm_gradx", s2_mm_gradx_, gz, y, {nl * nl, nb, fi, 2}, nl, nb, fi, fo);
+    return mm("s2c_s2_mm_gradx", real ? s2_mm_real_gradx_ : s2_mm_gradx_, gz, y, {nl * nl, nb, fi, 2}, nl, nb, fi, fo);
   }
-  Tensor s2_mm_grady(const Tensor& gz, const Tensor& x, int64_t fo) {
+  Tensor s2_mm_grady(const Tensor& gz, const Tensor& x, int64_t fo, bool real) {
     const long nl = s2_bandwidth(x.size(0)), nb = x.size(1), fi = x.size(2);
-    return mm("s2c_s2_mm_grady", s2_mm_grady_, gz, x, {nl * nl, fi, fo, 2}, nl, nb, fi, fo);
+    return mm("s2c_s2_mm_grady", real ? s2_mm_real_grady_ : s2_mm_grady_, gz, x, {nl * nl, fi, fo, 2}, nl, nb, fi, fo);
   }
 
   // -- kernel-grid -> spectrum ----------------------------------------------------------------------
@@ -742,8 +742,8 @@ struct S2ProductSynthesis : torch::autograd::Function<S2ProductSynthesis> {
     const bool wx = ctx->needs_input_grad(0), wy = ctx->needs_input_grad(1);
     std::tie(gz, gb) = spectrum_and_bias_grad(o, g[0].contiguous(), wx || wy, ctx->needs_input_grad(2),
                                               s2_bandwidth(x.size(0)), ctx->saved_data["bias_shape"].toIntVector());
-    if (wx) gx = o->s2_mm_gradx(gz, y, x.size(1), x.size(2));
-    if (wy) gy = o->s2_mm_grady(gz, x, y.size(2));
+    if (wx) gx = o->s2_mm_gradx(gz, y, x.size(1), x.size(2), true);
+    if (wy) gy = o->s2_mm_grady(gz, x, y.size(2), true);
     return {Variable(), gx, gy, gb};
   }
 };
@@ -767,9 +767,9 @@ struct SpectralMm : torch::autograd::Function<SpectralMm<KIND>> {
     const Tensor gz = g[0].contiguous();
     const long nb = x.size(1), fi = x.size(2), fo = y.size(2);
     if (ctx->needs_input_grad(0))
-      gx = KIND == kSo3Mm ? o->so3_mm_gradx(gz, y, nb, fi) : KIND == kSo3MmReal ? o->so3_mm_real_gradx(gz, y, nb, fi) : o->s2_mm_gradx(gz, y, nb, fi);
+      gx = KIND == kSo3Mm ? o->so3_mm_gradx(gz, y, nb, fi) : KIND == kSo3MmReal ? o->so3_mm_real_gradx(gz, y, nb, fi) : o->s2_mm_gradx(gz, y, nb, fi, false);
     if (ctx->needs_input_grad(1))
-      gy = KIND == kSo3Mm ? o->so3_mm_grady(gz, x, fo) : KIND == kSo3MmReal ? o->so3_mm_real_grady(gz, x, fo) : o->s2_mm_grady(gz, x, fo);
+      gy = KIND == kSo3Mm ? o->so3_mm_grady(gz, x, fo) : KIND == kSo3MmReal ? o->so3_mm_real_grady(gz, x, fo) : o->s2_mm_grady(gz, x, fo, false);
     return {Variable(), gx, gy};
   }
 };
@@ -876,8 +876,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("so3_mm_real_gradx", &Ops::so3_mm_real_gradx, "gz"_a, "y"_a, "nb"_a, "fi"_a, nogil)
       .def("so3_mm_real_grady", &Ops::so3_mm_real_grady, "gz"_a, "x"_a, "fo"_a, nogil)
       .def("s2_mm", &Ops::s2_mm, "x"_a, "y"_a, nogil)
-      .def("s2_mm_gradx", &Ops::s2_mm_gradx, "gz"_a, "y"_a, "nb"_a, "fi"_a, nogil)
-      .def("s2_mm_grady", &Ops::s2_mm_grady, "gz"_a, "x"_a, "fo"_a, nogil)
+      .def("s2_mm_gradx", &Ops::s2_mm_gradx, "gz"_a, "y"_a, "nb"_a, "fi"_a, "real"_a = false, nogil)
+      .def("s2_mm_grady", &Ops::s2_mm_grady, "gz"_a, "x"_a, "fo"_a, "real"_a = false, nogil)
       .def("rft_forward", &Ops::rft_forward, "x"_a, "F"_a, nogil)
       .def("rft_forward_t", &Ops::rft_forward_t, "x"_a, "Ft"_a, nogil)
       .def("rft_backward", &Ops::rft_backward, "g"_a, "F"_a, "scale"_a = 1.0, nogil)

@@ -70,6 +70,37 @@ def test_half_products_match_the_full_ones(backend, nl, nb, fi, fo):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nl,fi,fo", [(6, 20, 40), (3, 32, 64), (7, 13, 9), (2, 4, 4), (7, 16, 24), (12, 24, 3)])
+def test_forward_does_not_depend_on_the_batch(nl, fi, fo):
+    """A tile's segments, one to a block of a cluster (few signals) or one after the other, give the same bits."""
+    ops, dev = backends.get("cuda")
+    gen = torch.Generator().manual_seed(fo)
+    x, y = real_spectrum(nl, 300, fi, gen=gen).to(dev), real_spectrum(nl, fi, fo, gen=gen).to(dev)
+    z = ops.so3_mm_real(x, y)
+    for n in (1, 3, 17, 32, 129):
+        assert torch.equal(ops.so3_mm_real(x[:, :n].contiguous(), y), z[:, :n]), n
+
+
+def real_s2_spectrum(b, *shape, gen):
+    out = real_spectrum(b, *shape, gen=gen)
+    return torch.cat([out[n3(l) + l * (2 * l + 1):n3(l) + (l + 1) * (2 * l + 1)] for l in range(b)]).contiguous()  # m = 0
+
+
+@pytest.mark.parametrize("backend", backends.BACKENDS)
+@pytest.mark.parametrize("nl,nb,fi,fo", [(1, 1, 1, 1), (4, 65, 1, 3), (7, 3, 8, 5), (5, 2, 9, 4), (12, 20, 6, 33)])
+def test_half_s2_gradients_match_the_full_ones(backend, nl, nb, fi, fo):
+    """f_in above 8 takes the general product."""
+    ops, dev = backends.get(backend)
+    gen = torch.Generator().manual_seed(nl + fo)
+    gz = real_spectrum(nl, nb, fo, gen=gen).to(dev)
+    x, y = real_s2_spectrum(nl, nb, fi, gen=gen).to(dev), real_s2_spectrum(nl, fi, fo, gen=gen).to(dev)
+    for name, a, b in (("gx", ops.s2_mm_gradx(gz, y, nb, fi, real=True), ops.s2_mm_gradx(gz, y, nb, fi)),
+                       ("gy", ops.s2_mm_grady(gz, x, fo, real=True), ops.s2_mm_grady(gz, x, fo))):
+        # both are sums of at most (2 nl - 1) * max(nb, fo) terms in float32, in other orders
+        assert ((a - b).norm() / b.norm()).item() < 5e-6, name
+
+
+@pytest.mark.gpu
 def test_a_given_spectrum_keeps_the_full_product():
     torch.manual_seed(3)
     conv = S.SO3Convolution(3, 4, 5, 4, S.so3_near_identity_grid()).cuda()
