@@ -1175,8 +1175,15 @@ int s2c_s2_fft(const float* x, int x_is_real, float* out, long nbatch, int b_in,
   const int G = fft_group(N, N), Gg = fft_group(N, N / 2);  // alpha passes, gamma passes
   for (long z0 = 0; z0 < nbatch; z0 += chunk) {
     const long zc = std::min(chunk, nbatch - z0);
+    // A real signal's coefficients of m < 0 mirror those of m > 0.  (Up to 32 degrees both are computed: those spectra
+    // feed the layers, whose recorded passes keep their bits, see SpectralMm in host_ops.cpp.)  192 signals, b = 64,
+    // analysis and synthesis: 48 -> 35 us and 43 -> 34; 512: 101 -> 65 and 81 -> 62.
+    const int ht = wig_s2_zt(K, zc);
+    const bool half = x_is_real && K > 32 && !g_force_general && s2_length(N) &&
+                      fwd_wigner_t_fits(N, b_out, ht, dev_smem_limit());
     if (!g_force_general && s2_length(N)) {
       S2RowsParams r;
+      r.half = half;
       r.x = x + (size_t)z0 * N * N * (x_is_real ? 1 : 2); r.out = nullptr;
       r.complex = !x_is_real; r.v = (float2*)ws; r.tw = fft.tw;
       r.nbatch = (int)zc; r.K = K;
@@ -1203,10 +1210,11 @@ int s2c_s2_fft(const float* x, int x_is_real, float* out, long nbatch, int b_in,
     w.ZT = (int)std::min<long>(32, zc);
     w.nzt = (int)((zc + w.ZT - 1) / w.ZT);
     w.mode = kS2;
-    if (const int zt = wig_s2_zt(pan.npairs, zc); fwd_wigner_t_fits(N, b_out, zt, dev_smem_limit())) {
+    if (const int zt = half ? ht : wig_s2_zt(pan.npairs, zc); fwd_wigner_t_fits(N, b_out, zt, dev_smem_limit())) {
       w.ZT = zt;
       w.nzt = (int)((zc + zt - 1) / zt);
-      S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)pan.npairs * w.nzt, kThreads,
+      w.s2_half = half;
+      S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)(half ? K : pan.npairs) * w.nzt, kThreads,
                          fwd_wigner_t_smem(N, b_out, zt), st, w));
       continue;
     }
@@ -1243,10 +1251,14 @@ int s2c_s2_ifft(const float* x, float* out, int out_is_real, long nbatch, int b_
     w.ZT = (int)std::min<long>(32, zc);
     w.nzt = (int)((zc + w.ZT - 1) / w.ZT);
     w.mode = kS2;
-    if (const int zt = wig_s2_zt(pan.npairs, zc); inv_wigner_t_smem(N, K, zt) <= (size_t)dev_smem_limit() - 1024) {
+    // the real part alone: the spectrum is symmetrised while it is staged, and V[-m] = conj V[m]
+    const int ht = wig_s2_zt(K, zc);
+    const bool half = out_is_real && !g_force_general && s2_length(N) && inv_wigner_t_smem(N, K, ht) <= (size_t)dev_smem_limit() - 1024;
+    if (const int zt = half ? ht : wig_s2_zt(pan.npairs, zc); inv_wigner_t_smem(N, K, zt) <= (size_t)dev_smem_limit() - 1024) {
       w.ZT = zt;
       w.nzt = (int)((zc + zt - 1) / zt);
-      S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)pan.npairs * w.nzt, kThreads,
+      w.s2_half = half;
+      S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)(half ? K : pan.npairs) * w.nzt, kThreads,
                          inv_wigner_t_smem(N, K, zt), st, w));
     } else {
       const size_t wsm = align_up((size_t)K * N * sizeof(float), 16) + (size_t)K * w.ZT * sizeof(float2);
@@ -1254,6 +1266,7 @@ int s2c_s2_ifft(const float* x, float* out, int out_is_real, long nbatch, int b_
     }
     if (!g_force_general && s2_length(N)) {
       S2RowsParams r;
+      r.half = half;
       r.x = nullptr; r.out = out + (size_t)z0 * N * N * (out_is_real ? 1 : 2);
       r.complex = !out_is_real; r.v = (float2*)ws; r.tw = fft.tw;
       r.nbatch = (int)zc; r.K = K;

@@ -162,6 +162,7 @@ struct S2RowsParams {
   float2* v;           // [m + K - 1][z][beta]
   const float2* tw;
   int nbatch, K;
+  int half;            // only m >= 0 is written / read: real signals, V[-m] = conj V[m]
 };
 S2C_HD constexpr int s2_rows_groups(int N) { return (N + kS2Rows - 1) / kS2Rows; }
 inline size_t s2_fwd_rows_smem(int N) { return ((size_t)N + (size_t)kS2Rows * (N + 1)) * sizeof(float2); }
@@ -209,7 +210,7 @@ struct s2_fwd_rows_impl {
       float2* o = p.v + z * N + beta0 + row;
       F::template tail<-1>(v, tw, [&](int q, float2 val) {
         const int f = f0 + R1 * q, m = f < H ? f : f - N;
-        if (m < K && m > -K) o[(long)(m + K - 1) * p.nbatch * N] = val;
+        if (m < K && m > (p.half ? -1 : -K)) o[(long)(m + K - 1) * p.nbatch * N] = val;
       });
     }
   }
@@ -237,7 +238,9 @@ struct s2_inv_rows_impl {
 #pragma unroll
       for (int k = 0; k < R1; ++k) {
         const int f = j + k * R2, m = f < H ? f : f - N;
-        v[k] = (m < K && m > -K) ? s[(long)(m + K - 1) * p.nbatch * N] : make_float2(0.f, 0.f);
+        const bool other = p.half && m < 0;
+        v[k] = (m < K && m > -K) ? s[(long)((other ? -m : m) + K - 1) * p.nbatch * N] : make_float2(0.f, 0.f);
+        if (other) v[k].y = -v[k].y;
       }
       F::template head<+1>(v, j, tw);
       float2* a = A + row * LD + j;

@@ -42,7 +42,7 @@ inline int wig_s2_zt(int npairs, long nbatch) {
 // different bank groups).  S2 transforms (kS2) are the n = 0 column without mirror rows.
 S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
   const int N = p.N, NH = wig_np(N);
-  const int pair = ctx.bid / p.nzt, zt = ctx.bid - pair * p.nzt;
+  const int bt0 = ctx.bid / p.nzt, zt = ctx.bid - bt0 * p.nzt, pair = bt0 + (p.s2_half ? p.K - 1 : 0);
   int m, n;
   if (p.mode == kS2) { m = pair - (p.K - 1); n = 0; } else so3_pair_decode(pair, p.K, m, n);
   const int am = m < 0 ? -m : m;
@@ -179,7 +179,9 @@ S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) {
     if (li >= L || zz >= zc) return;
     const int l = lmin + li;
     if (p.mode == kS2) {
-      p.out[((long)l * l + l + m) * p.out_zstride + z0 + zz] = make_float2(re, im);
+      float2* o = p.out + ((long)l * l + l) * p.out_zstride + z0 + zz;
+      o[m * p.out_zstride] = make_float2(re, im);
+      if (p.s2_half && m > 0) o[-m * p.out_zstride] = make_float2(fudge * re, -fudge * im);
       return;
     }
     float2* o1 = p.out + so3_row(l, m, n) * p.out_zstride + z0 + zz;
@@ -237,7 +239,7 @@ S2C_D float2 wig_s2_product(const InvWignerParams& p, int l, int m, int n, int i
 // S[z][beta] = sum_l W[l][beta] Xs[l][z],  Xs = symmetrised spectrum
 S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
   const int N = p.N, NP = wig_np(N);
-  const int pair = ctx.bid / p.nzt, zt = ctx.bid - pair * p.nzt;
+  const int bt0 = ctx.bid / p.nzt, zt = ctx.bid - bt0 * p.nzt, pair = bt0 + (p.s2_half ? p.K - 1 : 0);
   int m, n;
   if (p.mode == kS2) { m = pair - (p.K - 1); n = 0; } else so3_pair_decode(pair, p.K, m, n);
   const int am = m < 0 ? -m : m;
@@ -280,6 +282,10 @@ S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) {
     if (zz < zc && p.mode == kS2) {
       const long l = lmin + li;
       v = p.x[(l * l + l + m) * p.x_zstride + z0 + zz];
+      if (p.s2_half) {
+        const float2 w = p.x[(l * l + l - m) * p.x_zstride + z0 + zz];
+        v = make_float2(0.5f * (v.x + fudge * w.x), 0.5f * (v.y - fudge * w.y));
+      }
     } else if (zz < zc && p.xs) {
       const int l = lmin + li;
       const int z = (int)(p.z0 + z0 + zz), i = z / p.s2_fout, j = z - i * p.s2_fout;
