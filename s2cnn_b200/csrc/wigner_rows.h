@@ -294,7 +294,7 @@ struct so3_fwd_wigner_r_impl {
     float* xch = reinterpret_cast<float*>(bar + 4) + warp * 32 * 17;
     const int K = p.K, zc = p.zc, items = rows_items(K, zc);
     const RowsLane ln(lane);
-    auto next = [&](int round) { return round * ctx.nblk + (round & 1 ? ctx.nblk - 1 - ctx.bid : ctx.bid); };
+    auto next = [&](int turn) { return turn * ctx.nblk + (turn & 1 ? ctx.nblk - 1 - ctx.bid : ctx.bid); };
 
     // the item's part of V, one copy per sign; issued by one thread once every warp has the part before in registers
     auto fetch = [&](int item) {
@@ -312,9 +312,9 @@ struct so3_fwd_wigner_r_impl {
     }
     ctx.sync();
 
-    for (int round = 0; next(round) < items; ++round) {
-      const RowsGeom g = rows_geom(p.order, next(round), zc);
-      const unsigned phase = round & 1;
+    for (int turn = 0; next(turn) < items; ++turn) {
+      const RowsGeom g = rows_geom(p.order, next(turn), zc);
+      const unsigned phase = turn & 1;
       const int n = g.n, m = g.m0 + warp;
       const int lmin = m > n ? m : n;
       const int L = (m < K) ? p.nl - lmin : 0;
@@ -366,13 +366,13 @@ struct so3_fwd_wigner_r_impl {
         if (atomicAdd(readers, 1) == kRowsMG - 1) {
           *readers = 0;
           __threadfence_block();
-          fetch(next(round + 1));
+          fetch(next(turn + 1));
         }
       }
       __syncwarp();
 #else
       ctx.sync();
-      if (ctx.tid == 0) fetch(next(round + 1));
+      if (ctx.tid == 0) fetch(next(turn + 1));
 #endif
 
       // output: row li + b % 4 (lanes b < 4) or its mirror (b >= 4), frequency +-m, batch elements from zp

@@ -48,3 +48,20 @@ def test_workspace_aligned_to_16_bytes():
     lib.call("s2c_so3_rfft", p(want.data_ptr()), p(spec.data_ptr()), 6, 32, 32, 0, p(at), n, stream)
     torch.cuda.synchronize()
     assert torch.equal(out, want) and torch.equal(spec, ops.so3_rfft(want))
+
+
+@pytest.mark.gpu
+def test_long_chunks_equal_short_ones():
+    """300 signals at b = 32: two chunks of 152 and 148, against chunks of 8; equal to the last bit."""
+    ops, dev = backends.get("cuda")
+    gen = torch.Generator(device=dev).manual_seed(4)
+    x = torch.randn(300, 64, 64, 64, generator=gen, device=dev)
+    res = []
+    try:
+        for width in (0, 8):
+            ops.lib.s2c_debug_plane_chunk(width)
+            spec = ops.so3_rfft(x, b_out=13)
+            res.append((spec, ops.so3_rifft(spec, b_out=32)))
+    finally:
+        ops.lib.s2c_debug_plane_chunk(0)
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
