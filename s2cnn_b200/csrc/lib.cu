@@ -1464,14 +1464,16 @@ int s2c_so3_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb,
   return s2c_so3_mm_grady_ws(gz, x, gy, nl, nb, fi, fo, nullptr, 0, st);
 }
 // Products of spectra of real signals.  X[l,-m,-n] = (-1)^(m-n) conj X[l,m,n] holds for the operands and so for the
-// result: the tensor cores compute the rows of outer index l .. 2l (m >= 0; the kernel index for the gradient of y), half
+// result: the tensor cores compute the columns (z) or rows (gradients) of outer index l .. 2l, half
 // of the multiply-adds, and write each coefficient and its mirror.  us on one B200, all rows -> half, for z, gx
-// and gy: 100 -> 100 channels, nl = 10, batch 32: 314, 325, 314 -> 205, 211, 203; 16 -> 16, nl = 15, batch 32: 77, 80, 65 -> 50,
-// 52, 51; 20 -> 40, nl = 6, batch 256: 46, 50, 52 -> 33, 33, 36.  Calls of one tile row (batch 1) take the time they took.
+// and gy: 100 -> 100 channels, nl = 10, batch 32: 314, 325, 314 -> 199, 211, 203; 16 -> 16, nl = 15, batch 32: 77, 80, 65 -> 49,
+// 52, 51; 20 -> 40, nl = 6, batch 256: 42, 50, 52 -> 32, 33, 36; 8 -> 16, nl = 15, batch 32: z 41 -> 28 (half of the rows: 32).
+// Calls whose tiles all run at once take the time they took, or 1 - 2 us more (16 -> 24, nl = 7, batch 32: 16.5 -> 19.2,
+// segments in one CTA).
 size_t s2c_so3_mm_real_workspace(int op, int nl, int nb, int fi, int fo) {
 #ifndef S2C_EMUL
   if ((op == kTcGradX || op == kTcGradY) && nl >= 1 && nb >= 1 && fi >= 1 && fo >= 1)
-    return tc_share_workspace(op, 1, nl, nb, fi, fo, tc_run(op, nb, fi, fo));
+    return tc_share_workspace(op, kTcHalfRows, nl, nb, fi, fo, tc_run(op, nb, fi, fo));
 #endif
   return 0;
 }
@@ -1484,7 +1486,7 @@ int s2c_so3_mm_real(int op, const float* u, const float* v, float* out, int nl, 
 #ifndef S2C_EMUL
   static_assert((int)kTcFwd == 0 && (int)kTcGradX == 1 && (int)kTcGradY == 2, "op codes");
   bool handled = false;
-  S2C_TRY(so3_mm_tc_launch(op, 1, a, b, out, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
+  S2C_TRY(so3_mm_tc_launch(op, op == kTcFwd ? kTcHalfColumns : kTcHalfRows, a, b, out, nl, nb, fi, fo, ws, ws_bytes, as_stream(st), &handled));
   if (handled) return S2C_OK;
 #endif
   static_assert(kMmFwd == 0 && kMmGradX == 1 && kMmGradY == 2, "op codes");

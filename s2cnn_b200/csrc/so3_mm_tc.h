@@ -80,12 +80,18 @@ namespace s2c {
 //   SC: the row operand holds k as pairs `a_ps` floats apart.
 enum TcOp : int { kTcFwd = 0, kTcGradX = 1, kTcGradY = 2, kTcPlainCC = 3, kTcPlainSC = 4 };
 
+// The forward product takes half of the columns: their number does not shrink with the batch, so that small batches gain, too
+// (two signals, 46 -> 93 channels, nl = 10: 150 tiles, one wave and a rest -> 80), and which half is computed - and so the
+// rounding - does not depend on it.
+enum TcHalf : int { kTcWhole = 0, kTcHalfRows = 1, kTcHalfColumns = 2 };
+
 struct MmTcParams {
   const float* a;   // operand read along the output rows
   const float* b;   // operand read along the output columns
   float* c;         // output
   int nl, nb, fi, fo;
-  int half;         // spectra of real signals: rows of outer index l .. 2l only, the others are their mirrors
+  int half;         // spectra of real signals: rows (kTcHalfRows) or columns (kTcHalfColumns) of outer index l .. 2l only,
+                    // the others are their mirrors
   int two;          // without partial sums: the products with a lo part go into the second accumulator
   int segs;         // > 1: a tile's K blocks are summed in this many segments, in one CTA or one to a CTA of a cluster (tc_segments)
   int run;          // floats per outer contraction index: 2 fi (fwd), 2 fo (grad x), 2 nb (grad y)
@@ -301,7 +307,7 @@ __device__ __forceinline__ float tc_hi(float v) { return __uint_as_float(__float
 __host__ __device__ __forceinline__ long tc_tiles_for(int op, int half, int nb, int fi, int fo, int l) {
   const TcGeom g = tc_geom(op, nb, fi, fo);
   const long L = 2 * l + 1;
-  const long M = (half ? l + 1 : L) * g.RI, N = L * g.CW;
+  const long M = (half == kTcHalfRows ? l + 1 : L) * g.RI, N = (half == kTcHalfColumns ? l + 1 : L) * g.CW;
   return ((M + kTcBM - 1) / kTcBM) * ((N + kTcBN - 1) / kTcBN);
 }
 
@@ -340,8 +346,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   const int o_lo = it_lo / p.nblk, kb_lo = it_lo - o_lo * p.nblk;
   const TcGeom geo = tc_geom(OP, p.nb, p.fi, p.fo);
   const int RI = geo.RI, CW = geo.CW;
-  const int ro0 = p.half ? l : 0;                         // outer index of the first row
-  const int M = (L - ro0) * RI, Np = L * CW;
+  // outer indices of the first row and column
+  const int ro0 = p.half == kTcHalfRows ? l : 0, co0 = p.half == kTcHalfColumns ? l : 0;
+  const int M = (L - ro0) * RI, Np = (L - co0) * CW;
   const int tiles_n = (Np + kTcBN - 1) / kTcBN;
   const int row0 = (int)(t / tiles_n) * kTcBM, col0 = (int)(t % tiles_n) * kTcBN;
   const long spec0 = (long)l * (4L * l * l - 1) / 3;
@@ -511,7 +518,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     const float* gB = nullptr;
     {
       const int gcol = col0 + (plain ? bcol : 2 * bcol);
-      const int co = gcol / CW, in = (gcol - co * CW) >> 1;
+      const int cq = gcol / CW, in = (gcol - cq * CW) >> 1, co = co0 + cq;
       long base;
       if (OP == kTcFwd)        base = ((spec0 + (long)co * L) * p.fi * p.fo + in) * 2;
       else if (OP == kTcGradX) base = ((spec0 + co) * p.fi + in) * fo2;
@@ -685,7 +692,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   // mirror (-m, -n) is coefficient L * L - 1 - q, (-1)^(m - n) = (-1)^q times the conjugate (L is odd)
   constexpr bool kPlain = OP == kTcPlainCC || OP == kTcPlainSC;
   const int sro = OP == kTcGradY ? 1 : L, sco = OP == kTcGradY ? L : 1;
-  const bool mirror = !kPlain && p.half && rq > 0;
+  const bool row_mirror = !kPlain && p.half == kTcHalfRows && rq > 0, col_half = !kPlain && p.half == kTcHalfColumns;
   auto at_coefficient = [&](int q, int rem) { return p.c + ((spec0 + q) * RI + ri) * CW + rem; };
   auto mirrored = [](float4 o, float s) { return make_float4(s * o.x, -s * o.y, s * o.z, -s * o.w); };
   // two columns (one complex number: never straddles an outer column index), four with VEC
@@ -695,9 +702,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
       if (OP == kTcPlainSC) { a *= p.scale; b *= p.scale; }
       *reinterpret_cast<float2*>(p.c + (long)r * p.c_rs + (long)(gcol >> 1) * p.c_ps) = make_float2(a, b);
     } else {
-      const int co = gcol / CW, rem = gcol - co * CW, q = ro * sro + co * sco;
+      const int cq = gcol / CW, rem = gcol - cq * CW, q = ro * sro + (co0 + cq) * sco;
       *reinterpret_cast<float2*>(at_coefficient(q, rem)) = make_float2(a, b);
-      if (mirror) {
+      if (row_mirror || (col_half && cq > 0)) {
         const float s = (q & 1) ? -1.f : 1.f;
         *reinterpret_cast<float2*>(at_coefficient(L * L - 1 - q, rem)) = make_float2(s * a, -s * b);
       }
@@ -706,9 +713,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   auto store4 = [&](int gcol, float4 o) {
     if constexpr (VEC && !kPlain) {
       if (gcol >= Np) return;     // CW is a multiple of 4, so a group of 4 is all in or all out
-      const int co = gcol / CW, rem = gcol - co * CW, q = ro * sro + co * sco;
+      const int cq = gcol / CW, rem = gcol - cq * CW, q = ro * sro + (co0 + cq) * sco;
       *reinterpret_cast<float4*>(at_coefficient(q, rem)) = o;
-      if (mirror) *reinterpret_cast<float4*>(at_coefficient(L * L - 1 - q, rem)) = mirrored(o, (q & 1) ? -1.f : 1.f);
+      if (row_mirror || (col_half && cq > 0)) *reinterpret_cast<float4*>(at_coefficient(L * L - 1 - q, rem)) = mirrored(o, (q & 1) ? -1.f : 1.f);
     } else {
       store2(gcol, o.x, o.y);
       store2(gcol + 2, o.z, o.w);
@@ -766,12 +773,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
       for (int c8 = 0; c8 < 4; ++c8) {
         const int gcol = col0 + cbase + 8 * c8;
         if (gcol < Np) {
-          const int co = gcol / CW, rem = gcol - co * CW, q = ro * sro + co * sco;
+          const int cq = gcol / CW, rem = gcol - cq * CW, q = ro * sro + (co0 + cq) * sco;
           float8 o;
           o.lo = make_float4(v[8 * c8], v[8 * c8 + 1], v[8 * c8 + 2], v[8 * c8 + 3]);
           o.hi = make_float4(v[8 * c8 + 4], v[8 * c8 + 5], v[8 * c8 + 6], v[8 * c8 + 7]);
           st_global_256(at_coefficient(q, rem), o);
-          if (mirror) {
+          if (row_mirror || (col_half && cq > 0)) {
             const float s = (q & 1) ? -1.f : 1.f;
             o.lo = mirrored(o.lo, s);
             o.hi = mirrored(o.hi, s);
@@ -844,7 +851,7 @@ constexpr int kTcSlots[kTcMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15}
 // tiles for clusters even at batch 1, or longer contractions: one CTA, the whole chain or groups of seven.
 inline int tc_segments(int nl, int fi, int fo, int blocks) {
   const int s = (2 * blocks + 14) / 15;
-  return s <= kTcMaxCluster && so3_mm_tc_tiles(kTcFwd, 1, nl, 1, fi, fo) <= kTcSlots[s] ? s : 0;
+  return s <= kTcMaxCluster && so3_mm_tc_tiles(kTcFwd, kTcHalfColumns, nl, 1, fi, fo) <= kTcSlots[s] ? s : 0;
 }
 
 // CTAs per tile.  One CTA fits on an SM; a product with few output tiles and a long contraction (the

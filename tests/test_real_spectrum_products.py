@@ -60,8 +60,8 @@ def test_half_products_match_the_full_ones(backend, nl, nb, fi, fo):
         err = [((t.double() - w).norm() / w.norm()).item() for t in (g, f)]
         assert err[0] < 1e-5, (name, err)
         assert_close(g, f, name)
-        if backend == "cuda":     # the halves mirror each other exactly (m = 0 is its own half: computed as a whole)
-            m0 = torch.cat([(torch.arange((2 * l + 1) ** 2) // (2 * l + 1) == l) if name != "gy" else
+        if backend == "cuda":     # the halves mirror each other exactly (index 0 is its own half: computed as a whole)
+            m0 = torch.cat([(torch.arange((2 * l + 1) ** 2) // (2 * l + 1) == l) if name == "gx" else
                             (torch.arange((2 * l + 1) ** 2) % (2 * l + 1) == l) for l in range(nl)])
             assert torch.equal(g[~m0], mirrored(g, nl)[~m0]), name
     if backend == "cuda":
