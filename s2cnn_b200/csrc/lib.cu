@@ -817,11 +817,12 @@ size_t s2c_so3_fft_workspace(long nbatch, int b_in, int b_out) {
   const size_t per_z = s2c_so3_fft_workspace_min(b_in, b_out);
   if (!per_z) return 0;
   if (plane_supported(2 * b_in) && plane_supported(2 * b_out)) {
-    // large-bandwidth path: one chunk of the scratch array V (sized to stay in L2); never less than
-    // one signal of the three-pass organisation, which the test switches can select instead
+    // large-bandwidth path: one chunk of the scratch array V of whichever direction wants more (a chunk's signals and a
+    // signal's V go by the length of the grid, b_in's or b_out's); never less than one signal of the three-pass
+    // organisation, which the test switches can select instead
     const int K = std::min(b_in, b_out);
-    const size_t v = std::max(so3_v_per_z(2 * b_in, K), so3_v_per_z(2 * b_out, K));
-    return std::max(per_z, v * (size_t)std::min<long>(rows_zc(2 * b_in), std::max(1L, nbatch)));
+    auto v = [&](int N) { return so3_v_per_z(N, K) * (size_t)std::min<long>(rows_zc(N), std::max(1L, nbatch)); };
+    return std::max(per_z, std::max(v(2 * b_in), v(2 * b_out)));
   }
   const size_t target = (size_t)256 << 20;
   long chunk = (long)std::max<size_t>(32, target / per_z);

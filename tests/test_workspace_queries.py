@@ -33,6 +33,15 @@ def test_single_kernel_paths_need_no_workspace(backend):
 
 
 @pytest.mark.parametrize("backend", backends.BACKENDS)
+@pytest.mark.parametrize("b_in,b_out", [(32, 32), (64, 64), (32, 64), (64, 32)])
+def test_query_for_both_directions_takes_the_larger_one(backend, b_in, b_out):
+    lib = backends.get(backend)[0].lib
+    for nb in (1, 8, 31, 64, 256, 300):
+        both = max(lib.s2c_so3_analysis_workspace(nb, b_in, b_out), lib.s2c_so3_synthesis_workspace(nb, b_in, b_out))
+        assert lib.s2c_so3_fft_workspace(nb, b_in, b_out) == max(both, lib.s2c_so3_fft_workspace_min(b_in, b_out)) <= 256 * MB, nb
+
+
+@pytest.mark.parametrize("backend", backends.BACKENDS)
 def test_queries_answer_nonsense_with_nothing(backend):
     lib = backends.get(backend)[0].lib
     for name in ("so3_fft", "so3_analysis", "so3_synthesis", "s2_fft"):
