@@ -78,8 +78,9 @@ class S2Convolution(Module):
             else:
                 plain = lambda xx, yy, bb: SO3_fft_real.apply(torch.relu(_product_synthesis(xx, yy, bb)), b_next)  # noqa: E731
             if 2 * self.b_out <= 32 and b_next <= self.b_out:
-                fused = lambda xx, yy, bb: cuda_ops().s2_conv_relu_so3_rfft(xx, yy, bb, b_next, real=True)  # noqa: E731
                 grad = torch.is_grad_enabled() and (x.requires_grad or y.requires_grad or own_bias.requires_grad)
+                # a recorded pass computes whole products: its backward recomputes them through the unfused chain
+                fused = lambda xx, yy, bb: cuda_ops().s2_conv_relu_so3_rfft(xx, yy, bb, b_next, real=not grad)  # noqa: E731
                 return fused_or_recompute(fused, plain, (x, y, own_bias), grad,
                                           getattr(self, "fused_training", False))
             return plain(x, y, own_bias)

@@ -194,3 +194,25 @@ def test_fused_training_recompute_rule_gives_the_same_gradients(backend):
         n0 = ops.lib.s2c_launch_count()
         fused(x)
         assert n_fwd < ops.lib.s2c_launch_count() - n0     # the training forward really was the fused one
+
+
+@pytest.mark.parametrize("backend", backends.BACKENDS)
+@pytest.mark.parametrize("b_in,b,b_next,f", [(8, 5, 4, 3), (8, 7, 7, 4), (12, 10, 6, 4)])
+def test_recorded_fused_pass_keeps_the_full_product(monkeypatch, backend, b_in, b, b_next, f):
+    """A recorded pass computes whole products whether its kernels are fused or not (a kernel spectrum is its own mirror but
+    for single last bits), so that backward recomputes the very values of the forward: equal to the last bit."""
+    import s2cnn_b200 as S
+    with backends.active(backend) as (_, dev):
+        torch.manual_seed(b)
+        conv = S.S2Convolution(2, f, b_in, b, S.s2_near_identity_grid(max_beta=0.7, n_alpha=5, n_beta=3)).to(dev)
+        x = torch.randn(3, 2, 2 * b_in, 2 * b_in, device=dev)
+        want = conv(x, relu_so3_fft=b_next)
+        conv.fused_training = True
+        got = conv(x, relu_so3_fft=b_next)
+        assert got.requires_grad and torch.equal(got, want)
+        calls, fused = [], S.ops.cuda_ops().s2_conv_relu_so3_rfft
+        monkeypatch.setattr(S.ops.cuda_ops(), "s2_conv_relu_so3_rfft", lambda *a, **k: calls.append(k.get("real", False)) or fused(*a, **k))
+        conv(x, relu_so3_fft=b_next)
+        with torch.no_grad():
+            conv(x, relu_so3_fft=b_next)
+        assert calls == [False, True]
