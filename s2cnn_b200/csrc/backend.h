@@ -235,8 +235,10 @@ inline int launch_impl(const char* kname, long grid, int block, size_t smem, str
 namespace s2c {
 // ---- asynchronous bulk copy global -> shared (TMA, 1-D) completing on an mbarrier -------------
 // dst, src and bytes must be multiples of 16.  One thread initialises the barrier and issues the
-// copies; every thread waits with bulk_wait (bounded: returns false if the copy never lands, in
-// which case the caller reads the data from global memory instead).
+// copies; every thread waits with bulk_wait (bounded: returns false if the copy has not landed by then, in
+// which case the caller reads the data from global memory instead).  A further copy may only be issued into a phase
+// that is over, and while a phase is not over the parity of the next one reads as landed: who issues looks at it
+// (bulk_over) first, and once a copy has been given up none is issued or trusted any more.
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
@@ -254,15 +256,6 @@ __device__ __forceinline__ void bulk_load_issue(void* dst, const void* src, unsi
           smem_u32(dst)),
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
-}
-// Shared -> global by the same engine, issued by one thread after bulk_store_fence() of every thread that wrote the
-// shared memory and a block barrier; bulk_store_wait() before the shared memory is given up.  16-byte aligned.
-__device__ __forceinline__ void bulk_store_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void bulk_store_issue(void* dst, const void* src, unsigned bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_store_wait() {
-  asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 // two independent single-precision operations in one instruction, each rounded as the scalar one
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -334,22 +327,27 @@ __device__ __forceinline__ void cl_store_float(cl_addr base, int off, float v) {
 }
 
 
+// is the phase of this parity over?  (one try, of bounded length)
+__device__ __forceinline__ bool bulk_over(unsigned long long* bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return done;
+}
 __device__ __forceinline__ bool bulk_wait(const Ctx&, unsigned long long* bar, unsigned parity) {
-  const unsigned addr = smem_u32(bar);
   for (int spin = 0; spin < (1 << 20); ++spin) {
-    unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (bulk_over(bar, parity)) return true;
     if (spin > 32) __nanosleep(32);
   }
   return false;
 }
+// for results that are known to be wrong
+__device__ __forceinline__ float bulk_nan() { return __int_as_float(0x7fffffff); }
 }  // namespace s2c
 
 #else
@@ -467,6 +465,7 @@ inline int dev_smem_limit() { return 227 * 1024; }
 inline int dev_sm_count() { return 3; }
 
 extern thread_local long g_launch_count;
+void emu_bulk_block_end();     // (see EmuBulk)
 
 template <class Impl, class P>
 struct EmuLaunch {
@@ -495,6 +494,7 @@ inline int emu_launch(const char* kname, long grid, int block, size_t smem, cons
   for (long b = 0; b < grid; ++b) {
     L.bid = (int)b;
     emu_run_block(block, &EmuLaunch<Impl, P>::entry, &L);
+    emu_bulk_block_end();
   }
   ++g_launch_count;
   return S2C_OK;
@@ -511,15 +511,41 @@ inline int emu_launch(const char* kname, long grid, int block, size_t smem, cons
 #define S2C_KERNEL_BOUNDS(name, P, MAXT, MINB) S2C_KERNEL(name, P)
 
 namespace s2c {
-// Host stand-ins of the bulk-copy helpers: the copy happens at issue time, the wait is a block
-// barrier (every thread of the block calls it at the same point).
-inline void bulk_barrier_init(unsigned long long*) {}
-inline void bulk_load_issue(void* dst, const void* src, unsigned bytes, unsigned long long*) {
+// Host stand-ins of the bulk-copy helpers.  The wait is a block barrier (every thread of the block calls it at the same
+// point).  The copy happens at issue time and ends the barrier's phase (bit 0 of the barrier: its parity), except for one
+// that a test holds back: that one lands when one thread asks for it by itself (bulk_over), or never.
+struct EmuBulk {
+  long hold = 0, issued = 0;                  // hold: the number of the copy to hold back, from 1 (0: none)
+  int never = 0;
+  long faults = 0;                            // copies into a phase that is not over, and past the end of their block
+  void* dst = nullptr;
+  const void* src = nullptr;
+  unsigned bytes = 0;
+  unsigned long long* bar = nullptr;          // the held copy's barrier, until it lands
+};
+extern EmuBulk g_emu_bulk;
+inline void bulk_barrier_init(unsigned long long* bar) { *bar = 0; }
+inline void bulk_load_issue(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
+  EmuBulk& e = g_emu_bulk;
+  if (e.bar == bar) ++e.faults;
+  if (++e.issued == e.hold) {
+    e.dst = dst; e.src = src; e.bytes = bytes; e.bar = bar;
+    return;
+  }
   std::memcpy(dst, src, bytes);
+  *bar ^= 1;
 }
-inline void bulk_store_fence() {}
-inline void bulk_store_issue(void* dst, const void* src, unsigned bytes) { std::memcpy(dst, src, bytes); }
-inline void bulk_store_wait() {}
+// (a thread's own try, behind the waits: the held copy lands now, or never)
+inline bool bulk_over(unsigned long long* bar, unsigned parity) {
+  EmuBulk& e = g_emu_bulk;
+  if (e.bar == bar && !e.never) {
+    std::memcpy(e.dst, e.src, e.bytes);
+    e.bar = nullptr;
+    *bar ^= 1;
+  }
+  return (*bar & 1) != parity;
+}
+inline float bulk_nan() { return std::nanf(""); }
 inline float2 fma2(float2 a, float2 b, float2 c) { return make_float2(std::fma(a.x, b.x, c.x), std::fma(a.y, b.y, c.y)); }
 inline float relu(float v) { return v <= 0.f ? 0.f : v; }
 struct float8 {
@@ -595,9 +621,9 @@ inline int emu_launch_cluster(const char* kname, long nclusters, int c, int bloc
   ++g_launch_count;
   return S2C_OK;
 }
-inline bool bulk_wait(const Ctx& ctx, unsigned long long*, unsigned) {
+inline bool bulk_wait(const Ctx& ctx, unsigned long long* bar, unsigned parity) {
   ctx.sync();
-  return true;
+  return (*bar & 1) != parity;
 }
 }  // namespace s2c
 

@@ -35,6 +35,13 @@
 
 namespace s2c {
 thread_local long g_launch_count = 0;
+#ifdef S2C_EMUL
+EmuBulk g_emu_bulk;
+void emu_bulk_block_end() {
+  if (g_emu_bulk.bar && !g_emu_bulk.never) ++g_emu_bulk.faults;
+  g_emu_bulk.bar = nullptr;
+}
+#endif
 // test switches (process-wide, race-free; see the "test hooks" section of the header)
 static std::atomic<int> g_force_general{0};   // 1 = no single-kernel path, 2 = also no plane kernels
 static std::atomic<int> g_cluster{0};         // 2b <= 32: 0 by batch size, 1 cluster, 2 walking, 3 plane kernels
@@ -666,6 +673,17 @@ int s2c_is_cuda_build(void) {
   return 1;
 #endif
 }
+
+#ifdef S2C_EMUL
+// test of late bulk copies: holds back the nth copy from now (0: none), for good if `never`; returns the faults so far
+long s2c_emul_hold_copy(long nth, int never) {
+  const long faults = g_emu_bulk.faults;
+  g_emu_bulk = EmuBulk{};
+  g_emu_bulk.hold = nth;
+  g_emu_bulk.never = never;
+  return faults;
+}
+#endif
 
 void s2c_timing_begin(void) {
 #ifndef S2C_EMUL

@@ -73,6 +73,23 @@ S2C_D float2 s2_product_entry(const InvFusedParams& p, int l, int m, int n, int 
   return make_float2(re, im);
 }
 
+// A copy of a table slice that has been given up (backend.h): the next phase's parity would read as landed and the slice
+// at hand be taken for the next one.  No number of the rest may then look right: coefficient (0, 0, 0), which every sample
+// sums, becomes NaN in all batch elements of the block, which is also how the issuing thread knows it later.  (NaNs that
+// came with all four spectra spoil the same samples by themselves; a flag beside the barrier cost registers: 64 -> 106 at N = 16.)
+template <class XhAt>
+S2C_D bool fused_spoiled(XhAt xh_at) {
+  bool all = true;
+#pragma unroll
+  for (int z = 0; z < kFusedZG; ++z) all = all && xh_at(0, z).x != xh_at(0, z).x;
+  return all;
+}
+template <class XhAt>
+S2C_D void fused_spoil(XhAt xh_at) {
+#pragma unroll
+  for (int z = 0; z < kFusedZG; ++z) xh_at(0, z).x = bulk_nan();
+}
+
 template <int N>
 struct so3_inv_fused_impl {
   static S2C_D void run(const Ctx& ctx, const InvFusedParams& p, unsigned char* smem) {
@@ -308,8 +325,15 @@ struct so3_inv_fused_impl {
         }
       }
       ctx.sync();
-      if (ctx.tid == 0 && bg0 + p.BG < N)   // every thread is done with this slice: fetch the next
-        bulk_load_issue(Wg, p.pan.data_g + (size_t)(grp + 1) * p.pan.g_stride, wbytes, wbar);
+      if (ctx.tid == 0) {   // every thread is done with this slice: fetch the next
+        const bool over = bulk_over(wbar, (unsigned)(grp & 1));
+        if (bg0 + p.BG >= N) {
+        } else if (over && !fused_spoiled(xh_at)) {
+          bulk_load_issue(Wg, p.pan.data_g + (size_t)(grp + 1) * p.pan.g_stride, wbytes, wbar);
+        } else {
+          fused_spoil(xh_at);
+        }
+      }
       // ---- column FFTs m -> alpha: one thread per (z, beta, n) ------------------------------
       for (int it = ctx.tid; it < ZG * bc * K; it += ctx.nthr) {
         const int n = it % K, zb = it / K;

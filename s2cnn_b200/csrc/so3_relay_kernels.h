@@ -248,8 +248,15 @@ struct so3_relay_fused_impl {
         }
       }
       ctx.sync();
-      if (ctx.tid == 0 && bg0 + p.BG < N)   // every thread is done with this slice: fetch the next
-        bulk_load_issue(Wg, p.win_g + (size_t)(grp + 1) * p.win_stride, wbytes, wbar);
+      if (ctx.tid == 0) {   // every thread is done with this slice: fetch the next
+        const bool over = bulk_over(wbar, (unsigned)(grp & 1));
+        if (bg0 + p.BG >= N) {
+        } else if (over && !fused_spoiled(xh_at)) {
+          bulk_load_issue(Wg, p.win_g + (size_t)(grp + 1) * p.win_stride, wbytes, wbar);
+        } else {
+          fused_spoil(xh_at);
+        }
+      }
       // ---- synthesis: column FFTs m -> alpha, one thread per (z, beta, n) ----------------------
       for (int it = ctx.tid; it < ZG * bc * Kin; it += ctx.nthr) {
         const int n = it % Kin, zb = it / Kin;
