@@ -380,6 +380,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // What is above touches no memory of another kernel.  Tensor memory is taken behind the wait: a kernel ahead that lets
+  // these CTAs in before it has taken its own could never get it from a CTA that holds all of it and waits.
+  stream_order_wait();
   if (warp == 0) {
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -392,7 +395,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  stream_order_wait();     // (what is above touches no memory of another kernel; no other CTA of these fits beside this one)
   stream_order_next();     // (CTAs of 150 KB: none of these beside a waiting one of the next kernel, whose set-up is the longest)
 
   bool ok = true;

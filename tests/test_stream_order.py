@@ -1,5 +1,8 @@
 """Kernels are launched before the ones ahead of them in the stream have finished (``stream_order_wait`` in backend.h): a
 chain of calls that read and overwrite the same few buffers gives what it gives with a wait after every call."""
+import os
+import re
+
 import pytest
 import torch
 
@@ -50,3 +53,20 @@ def test_two_streams_with_chains_of_their_own():
     for res in got:
         for a, b in zip(res, want):
             assert torch.equal(a, b)
+
+
+def test_kernels_wait_before_they_touch_what_others_do():
+    """Every kernel waits, and the tensor-core one takes tensor memory behind the wait, not while a kernel ahead may
+    still want its own."""
+    csrc = os.path.join(os.path.dirname(S.__file__), "csrc")
+    kernels = 0
+    for name in sorted(os.listdir(csrc)):
+        text = open(os.path.join(csrc, name)).read()
+        text = re.sub(r"//.*", "", text)
+        for part in re.split(r"__global__\s+void", text)[1:]:
+            kernels += 1
+            head, wait = part.find("run("), part.find("stream_order_wait()")
+            alloc = part.find("tcgen05.alloc")
+            first = min(p for p in (head, alloc) if p >= 0)
+            assert 0 <= wait < first, (name, part[:60])
+    assert kernels >= 15
