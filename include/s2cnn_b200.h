@@ -327,7 +327,7 @@ int s2c_project_on_sphere(const float* verts, int nv, const int* faces, int nf, 
  *     32 < 2b <= 64 and 2b = 128 (both row transforms of a (z, beta) plane in one kernel) by the three
  *     separate passes every other size uses; 0 restores the defaults.
  *   s2c_debug_plane_chunk(signals): signals per chunk of the large-bandwidth path (1 .. 32 at b = 64, 256 at b = 32); 0
- *     restores the default (8, or what the workspace holds).
+ *     restores the default: equal chunks of at most 32 / 256, or of what the workspace holds.
  *   s2c_debug_cluster(mode): 2b <= 32: 1 the cluster kernels, 2 the kernels whose blocks walk beta, 3 the
  *     plane kernels (where they exist and a workspace is given); 0 restores the choice by batch size. */
 void s2c_debug_force_general_path(int level);

@@ -1194,8 +1194,9 @@ int s2c_s2_fft(const float* x, int x_is_real, float* out, long nbatch, int b_in,
   const int G = fft_group(N, N), Gg = fft_group(N, N / 2);  // alpha passes, gamma passes
   for (long z0 = 0; z0 < nbatch; z0 += chunk) {
     const long zc = std::min(chunk, nbatch - z0);
-    // A real signal's coefficients of m < 0 mirror those of m > 0.  (Up to 32 degrees both are computed: those spectra
-    // feed the layers, whose recorded passes keep their bits, see SpectralMm in host_ops.cpp.)  192 signals, b = 64,
+    // A real signal's coefficients of m < 0 mirror those of m > 0.  Up to 32 degrees both are computed, also in calls that
+    // would gain from the half: not by speed but because a change of bits there reaches the recorded passes of nearly all
+    // layers (see SpectralMm in host_ops.cpp), and this call does not know whether it is recorded.  192 signals, b = 64,
     // analysis and synthesis: 48 -> 35 us and 43 -> 34; 512: 101 -> 65 and 81 -> 62.
     const int ht = wig_s2_zt(K, zc);
     const bool half = x_is_real && K > 32 && !g_force_general && s2_length(N) &&

@@ -55,7 +55,8 @@ class S2Convolution(Module):
         :x:      [batch, feature_in,  beta, alpha]
         :relu_so3_fft: (extension) bandwidth b_next of the SO3Convolution that follows: return
                  SO3_fft_real(relu(conv(x)), b_next) - that layer's input spectrum
-                 [l * m * n, batch, feature_out, complex] (pass it on with ``input_spectrum=True``).
+                 [l * m * n, batch, feature_out, complex] (pass it on with ``input_spectrum=True,
+                 real_spectrum=True``; without the latter the layer computes whole products).
                  Without autograd and for 2 b_out <= 32 the signal between the layers is never written.
         :channel_scale, bias: (extension, used by ``s2cnn_b200.fuse`` to fold an eval-mode BatchNorm3d
                  into the layer) multiply output channel j by channel_scale[j] - applied to the

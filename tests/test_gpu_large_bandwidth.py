@@ -1,5 +1,5 @@
-"""Bandwidth 64 (the standalone-FFT benchmark size, 2b = 128: plane kernels + lanes-over-beta
-Wigner kernels in L2-sized batch chunks, checked against the three separate passes with the two-step
+"""Bandwidth 64 (the standalone-FFT benchmark size, 2b = 128: plane kernels + Wigner kernels with eight
+beta slices per warp, in batch chunks of up to 32, checked against the three separate passes with the two-step
 8 x 16 register FFT) on the GPU: spectrum parity against the oracle for one batch element, the reference's idempotence
 property of the round trip (tests/so3_fft.py:34-44) and linearity at a larger batch."""
 import pytest
@@ -24,8 +24,8 @@ def test_b64_spectrum_matches_oracle():
 @pytest.mark.gpu
 @pytest.mark.parametrize("b_out", [64, 20])
 def test_b64_plane_kernels_match_three_pass_path(b_out):
-    """Every way the library can run 2b = 128 gives the same spectrum and signal (batch 11: a full
-    chunk of 8 and a ragged one of 3; chunks of 2: five full and one of a single signal; b_out <
+    """Every way the library can run 2b = 128 gives the same spectrum and signal (batch 11: one chunk by
+    default, whose last eight and four are ragged; chunks of 2: five full and one of a single signal; b_out <
     b_in keeps a subset of columns)."""
     from s2cnn_b200.ops import cuda_ops
     ops = cuda_ops()

@@ -69,8 +69,20 @@ def test_half_products_match_the_full_ones(backend, nl, nb, fi, fo):
         assert _lib.cuda_lib().s2c_so3_mm_tc_status() == 0
 
 
+# layers whose forward products are not segmented: contractions too long for eight segments (partial sums every seven
+# blocks), or too many tiles for clusters (one chain, the products with a lo part in an accumulator of their own)
+WIDE = [(10, 2, 100, 100), (5, 3, 100, 255), (15, 2, 16, 16), (15, 2, 8, 16)]
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("nl,fi,fo", [(6, 20, 40), (3, 32, 64), (7, 13, 9), (2, 4, 4), (7, 16, 24), (12, 24, 3)])
+@pytest.mark.parametrize("nl,nb,fi,fo", WIDE)
+def test_wide_half_products_match_the_full_ones(nl, nb, fi, fo):
+    test_half_products_match_the_full_ones("cuda", nl, nb, fi, fo)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nl,fi,fo", [(6, 20, 40), (3, 32, 64), (7, 13, 9), (2, 4, 4), (7, 16, 24), (12, 24, 3)] +
+                         [(nl, fi, fo) for nl, _, fi, fo in WIDE])
 def test_forward_does_not_depend_on_the_batch(nl, fi, fo):
     """A tile's segments, one to a block of a cluster (few signals) or one after the other, give the same bits."""
     ops, dev = backends.get("cuda")
@@ -113,6 +125,18 @@ def test_a_given_spectrum_keeps_the_full_product():
         a = conv(xs.cuda(), input_spectrum=True)
         b = conv(xs.cuda(), input_spectrum=True, real_spectrum=True)
     assert_close(b, a, "real spectrum")
+
+
+@pytest.mark.gpu
+def test_wide_layer_without_gradients():
+    """40 -> 60 channels at ten degrees, the half product with partial sums, through the module (no gradient recorded)."""
+    torch.manual_seed(5)
+    grid = S.so3_near_identity_grid(n_alpha=4, n_beta=2, n_gamma=3)
+    conv = S.SO3Convolution(40, 60, 10, 10, grid)
+    x = torch.randn(2, 40, 20, 20, 20)
+    want = O.so3_convolution(x, conv.kernel.detach(), conv.bias.detach(), 10, 10, grid)
+    with torch.no_grad():
+        assert_close(conv.cuda()(x.cuda()), want, "y")
 
 
 @pytest.mark.gpu

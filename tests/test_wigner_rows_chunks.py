@@ -51,17 +51,18 @@ def test_workspace_aligned_to_16_bytes():
 
 
 @pytest.mark.gpu
-def test_long_chunks_equal_short_ones():
-    """300 signals at b = 32: two chunks of 152 and 148, against chunks of 8; equal to the last bit."""
+@pytest.mark.parametrize("b,width,k", [(32, 300, 13), (64, 35, 9)])
+def test_long_chunks_equal_short_ones(b, width, k):
+    """300 signals at b = 32: two chunks of 152 and 148, 35 at b = 64: of 24 and 11, against chunks of 8; equal to the last bit."""
     ops, dev = backends.get("cuda")
     gen = torch.Generator(device=dev).manual_seed(4)
-    x = torch.randn(300, 64, 64, 64, generator=gen, device=dev)
+    x = torch.randn(width, 2 * b, 2 * b, 2 * b, generator=gen, device=dev)
     res = []
     try:
         for width in (0, 8):
             ops.lib.s2c_debug_plane_chunk(width)
-            spec = ops.so3_rfft(x, b_out=13)
-            res.append((spec, ops.so3_rifft(spec, b_out=32)))
+            spec = ops.so3_rfft(x, b_out=k)
+            res.append((spec, ops.so3_rifft(spec, b_out=b)))
     finally:
         ops.lib.s2c_debug_plane_chunk(0)
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
