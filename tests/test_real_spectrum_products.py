@@ -112,6 +112,38 @@ def test_half_s2_gradients_match_the_full_ones(backend, nl, nb, fi, fo):
         assert ((a - b).norm() / b.norm()).item() < 5e-6, name
 
 
+# Relative error of the symmetric part, which is what the transforms behind a gradient read, of gx and gy when every row was
+# computed (float32 against float64, mean of four draws): mirrored rows have no two independent roundings to average and
+# must not be further off
+WHOLE_ERROR = [((6, 16, 1, 10), 0.98e-7, 1.53e-7), ((10, 4, 1, 32), 2.02e-7, 0.87e-7), ((12, 5, 3, 60), 3.05e-7, 0.72e-7)]
+WHOLE_ERROR_GPU = [((10, 32, 1, 20), 1.62e-7, 1.10e-7), ((30, 32, 1, 8), 1.77e-7, 1.74e-7), ((30, 7, 1, 8), 1.79e-7, 1.55e-7),
+                   ((16, 32, 6, 100), 4.49e-7, 1.66e-7), ((16, 30, 3, 40), 2.87e-7, 1.19e-7), ((14, 64, 1, 16), 1.72e-7, 1.49e-7)]
+
+
+@pytest.mark.parametrize("backend,sizes,gx,gy", [pytest.param("emul", *c) for c in WHOLE_ERROR] +
+                         [pytest.param("cuda", *c, marks=pytest.mark.gpu) for c in WHOLE_ERROR + WHOLE_ERROR_GPU])
+def test_half_s2_gradients_are_no_less_precise(backend, sizes, gx, gy):
+    ops, dev = backends.get(backend)
+    nl, nb, fi, fo = sizes
+    off = {"gx": [], "gy": []}
+    for seed in range(4):
+        gen = torch.Generator().manual_seed(seed)
+        gz = real_spectrum(nl, nb, fo, gen=gen)
+        x, y = real_s2_spectrum(nl, nb, fi, gen=gen), real_s2_spectrum(nl, fi, fo, gen=gen)
+        gc, xc, yc = (torch.view_as_complex(t.double()) for t in (gz, x, y))
+        want = {"gx": torch.zeros_like(xc), "gy": torch.zeros_like(yc)}
+        for l in range(nl):
+            L, s = 2 * l + 1, slice(l * l, (l + 1) ** 2)
+            gl = gc[n3(l):n3(l + 1)].reshape(L, L, nb, fo)
+            want["gx"][s] = torch.einsum("mnij,nkj->mik", gl, yc[s])
+            want["gy"][s] = torch.einsum("mnij,mik->nkj", gl.conj(), xc[s])
+        gd, xd, yd = gz.to(dev), x.to(dev), y.to(dev)
+        for name, got in (("gx", ops.s2_mm_gradx(gd, yd, nb, fi, real=True)), ("gy", ops.s2_mm_grady(gd, xd, fo, real=True))):
+            w = torch.view_as_real(want[name])     # (mirrored itself, as got is: the difference is the symmetric part's)
+            off[name].append(((got.cpu().double() - w).norm() / w.norm()).item())
+    assert sum(off["gx"]) / 4 <= gx and sum(off["gy"]) / 4 <= gy, off
+
+
 @pytest.mark.gpu
 def test_a_given_spectrum_keeps_the_full_product():
     torch.manual_seed(3)
