@@ -1233,9 +1233,9 @@ int s2c_s2_fft(const float* x, int x_is_real, float* out, long nbatch, int b_in,
     if (const int zt = half ? ht : wig_s2_zt(pan.npairs, zc); fwd_wigner_t_fits(N, b_out, zt, dev_smem_limit())) {
       w.ZT = zt;
       w.nzt = (int)((zc + zt - 1) / zt);
-      w.s2_half = half;
-      S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)(half ? K : pan.npairs) * w.nzt, kThreads,
-                         fwd_wigner_t_smem(N, b_out, zt), st, w));
+      const size_t wsm = fwd_wigner_t_smem(N, b_out, zt);
+      if (half) S2C_TRY(S2C_LAUNCH(s2_fwd_wigner_t_half, (long)K * w.nzt, kThreads, wsm, st, w));
+      else S2C_TRY(S2C_LAUNCH(so3_fwd_wigner_t, (long)pan.npairs * w.nzt, kThreads, wsm, st, w));
       continue;
     }
     const size_t wsm = align_up((size_t)b_out * (N + 1) * sizeof(float), 16) +
@@ -1277,9 +1277,9 @@ int s2c_s2_ifft(const float* x, float* out, int out_is_real, long nbatch, int b_
     if (const int zt = half ? ht : wig_s2_zt(pan.npairs, zc); inv_wigner_t_smem(N, K, zt) <= (size_t)dev_smem_limit() - 1024) {
       w.ZT = zt;
       w.nzt = (int)((zc + zt - 1) / zt);
-      w.s2_half = half;
-      S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)(half ? K : pan.npairs) * w.nzt, kThreads,
-                         inv_wigner_t_smem(N, K, zt), st, w));
+      const size_t wsm = inv_wigner_t_smem(N, K, zt);
+      if (half) S2C_TRY(S2C_LAUNCH(s2_inv_wigner_t_half, (long)K * w.nzt, kThreads, wsm, st, w));
+      else S2C_TRY(S2C_LAUNCH(so3_inv_wigner_t, (long)pan.npairs * w.nzt, kThreads, wsm, st, w));
     } else {
       const size_t wsm = align_up((size_t)K * N * sizeof(float), 16) + (size_t)K * w.ZT * sizeof(float2);
       S2C_TRY(S2C_LAUNCH(so3_inv_wigner, (long)pan.npairs * w.nzt, kThreads, wsm, st, w));

@@ -226,7 +226,6 @@ struct FwdWignerParams {
   long out_zstride;
   PanelsDev pan;
   int nbatch, N, K, nl, ZT, nzt, mode;
-  int s2_half = 0;   // so3_fwd_wigner_t, S2 transform of real signals: m >= 0 only, the other rows are their mirrors
 };
 
 S2C_KERNEL(so3_fwd_wigner, FwdWignerParams) {
@@ -325,7 +324,6 @@ struct InvWignerParams {
   int s2_nb = 0, s2_fin = 0, s2_fout = 0;
   int s2_real = 0;              // (s2_mirror)
   long z0 = 0;
-  int s2_half = 0;   // so3_inv_wigner_t, S2 transform whose real part is wanted: m >= 0 only, of the symmetrised spectrum
 };
 
 S2C_KERNEL(so3_inv_wigner, InvWignerParams) {
