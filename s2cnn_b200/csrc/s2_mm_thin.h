@@ -91,27 +91,26 @@ S2C_KERNEL(s2_mm_gradx_thin, S2ThinParams) {
       const float2* g = p.gz + ((row0 + n) * p.nb + i) * p.fo;
       const float2* yn = ys + (size_t)n * p.fi * p.fo;
       for (int j0 = 0; j0 < p.fo; j0 += kThinChain) {
-        float2 part[kThinFi];
+        float2 gv[kThinChain];
 #pragma unroll
-        for (int k = 0; k < kThinFi; ++k) part[k] = make_float2(0.f, 0.f);
+        for (int u = 0; u < kThinChain; ++u) gv[u] = j0 + u < p.fo ? g[j0 + u] : make_float2(0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < kThinChain; ++u) {
-          const int j = j0 + u;
-          if (j >= p.fo) break;
-          const float2 gv = g[j];
+        for (int k = 0; k < kThinFi; ++k) {
+          if (k < p.fi) {
+            float2 part = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int k = 0; k < kThinFi; ++k) {
-            if (k < p.fi) {
-              const float2 yv = yn[k * p.fo + j];
-              part[k].x = fmaf(gv.x, yv.x, part[k].x);
-              part[k].x = fmaf(-gv.y, yv.y, part[k].x);
-              part[k].y = fmaf(gv.x, yv.y, part[k].y);
-              part[k].y = fmaf(gv.y, yv.x, part[k].y);
+            for (int u = 0; u < kThinChain; ++u) {
+              if (j0 + u < p.fo) {
+                const float2 yv = yn[k * p.fo + j0 + u];
+                part.x = fmaf(gv[u].x, yv.x, part.x);
+                part.x = fmaf(-gv[u].y, yv.y, part.x);
+                part.y = fmaf(gv[u].x, yv.y, part.y);
+                part.y = fmaf(gv[u].y, yv.x, part.y);
+              }
             }
+            acc[k] = cadd(acc[k], part);
           }
         }
-#pragma unroll
-        for (int k = 0; k < kThinFi; ++k) acc[k] = cadd(acc[k], part[k]);
       }
     }
   }
@@ -167,39 +166,35 @@ S2C_KERNEL_BOUNDS(s2_mm_grady_thin, S2ThinParams, 1024, 1) {
     int m = sl / p.nb, i = sl - m * p.nb;
     for (int q = sl; q < rows; q += 8 * nsl) {
       float2 gv[8];
-      int rq[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        rq[u] = q + u * nsl;
         gv[u] = make_float2(0.f, 0.f);
-        if (rq[u] < rows) gv[u] = g0[m * gm + (long)i * p.fo];
+        if (q + u * nsl < rows) gv[u] = g0[m * gm + (long)i * p.fo];
         m += dm;
         i += di;
         if (i >= p.nb) { i -= p.nb; ++m; }
       }
 #pragma unroll
       for (int u0 = 0; u0 < 8; u0 += kThinChain) {
-        if (rq[u0] >= rows) break;
-        float2 part[kThinFi];
+        // (one feature's chain at a time: the chains of all would not fit the 64 registers)
 #pragma unroll
-        for (int k = 0; k < kThinFi; ++k) part[k] = make_float2(0.f, 0.f);
+        for (int k = 0; k < kThinFi; ++k) {
+          if (k < p.fi) {
+            float2 part = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int u = u0; u < u0 + kThinChain; ++u) {
-          if (rq[u] >= rows) break;
-          const float2* xr = x0 + (long)rq[u] * p.fi;         // rows of x are contiguous in (m, i)
-#pragma unroll
-          for (int k = 0; k < kThinFi; ++k) {
-            if (k < p.fi) {
-              const float2 xv = xr[k];   // conj(gv) * xv
-              part[k].x = fmaf(gv[u].x, xv.x, part[k].x);
-              part[k].x = fmaf(gv[u].y, xv.y, part[k].x);
-              part[k].y = fmaf(gv[u].x, xv.y, part[k].y);
-              part[k].y = fmaf(-gv[u].y, xv.x, part[k].y);
+            for (int u = u0; u < u0 + kThinChain; ++u) {
+              const int r = q + u * nsl;
+              if (r < rows) {
+                const float2 xv = x0[(long)r * p.fi + k];   // rows of x are contiguous in (m, i);  conj(gv) * xv
+                part.x = fmaf(gv[u].x, xv.x, part.x);
+                part.x = fmaf(gv[u].y, xv.y, part.x);
+                part.y = fmaf(gv[u].x, xv.y, part.y);
+                part.y = fmaf(-gv[u].y, xv.x, part.y);
+              }
             }
+            acc[k] = cadd(acc[k], part);
           }
         }
-#pragma unroll
-        for (int k = 0; k < kThinFi; ++k) acc[k] = cadd(acc[k], part[k]);
       }
     }
   }
