@@ -113,7 +113,7 @@ static void rows_order(int nl, int K, RowsOrder* out) {
 }
 static int launch_fwd_rows(int N, stream_t st, FwdRowsParams& f) {
   rows_order(f.nl, f.K, &f.order);
-  const long grid = std::min<long>(rows_items(f.K, f.zc), (N == 128 ? 1 : 2) * (long)dev_sm_count());
+  const long grid = std::min<long>(rows_items(f.K, f.zc), (long)dev_sm_count());
   if (N == 128) return S2C_LAUNCH_FWD_ROWS(128, grid, st, f);
   return S2C_LAUNCH_FWD_ROWS(64, grid, st, f);
 }
@@ -1380,7 +1380,8 @@ static int so3_mm_tc_launch(int op, int half, const float* a, const float* b, fl
   p.segs = op == kTcFwd && half ? tc_segments(nl, fi, fo, blocks) : 0;
   if (p.segs > 1 && tiles <= kTcSlots[p.segs]) p.csize = p.segs;
   const int ns = p.csize * p.groups;
-  const long ctas = tiles * ns;
+  p.twins = tc_twins(half, tiles, ns);
+  const long ctas = tiles * (p.twins ? 2 : ns);
   const bool flush = p.segs > 1 ? ns == 1 : tc_flush(p, blocks, ns);
   p.two = half && p.segs <= 1;
   const bool vec = so3_mm_tc_vec16(op, nb, fi, fo);
@@ -1396,7 +1397,7 @@ static int plain_tc_launch(bool a_strided, const float* a, const float* b, float
                            float scale, void* ws, size_t ws_bytes, stream_t st) {
   MmTcParams p;
   p.a = a; p.b = b; p.c = c;
-  p.nl = 1; p.nb = (int)M; p.fi = (int)(K / 2); p.fo = (int)(N / 2); p.half = p.two = p.segs = 0;
+  p.nl = 1; p.nb = (int)M; p.fi = (int)(K / 2); p.fo = (int)(N / 2); p.half = p.two = p.segs = p.twins = 0;
   p.run = (int)K;
   tc_blocks(p);
   p.a_rs = a_rs; p.a_ps = a_ps; p.b_rs = b_rs; p.b_ps = b_ps; p.c_rs = c_rs; p.c_ps = c_ps;

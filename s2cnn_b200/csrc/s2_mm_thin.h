@@ -139,6 +139,10 @@ inline int s2_grady_thin_threads(int fo) {
   int t = (1024 / fo) * fo;          // whole slices of fo threads
   return t < fo ? fo : t;
 }
+S2C_HD int s2_grady_sharers(int nthr, int outputs) {
+  const int s = nthr / outputs;
+  return s < 1 ? 1 : s > 16 ? 16 : s;
+}
 inline size_t s2_grady_thin_smem(int fo) {
   return (size_t)s2_grady_thin_threads(fo) * kThinFi * sizeof(float2);
 }
@@ -201,18 +205,44 @@ S2C_KERNEL_BOUNDS(s2_mm_grady_thin, S2ThinParams, 1024, 1) {
 #pragma unroll
   for (int k = 0; k < kThinFi; ++k) red[ctx.tid * kThinFi + k] = acc[k];
   ctx.sync();
-  // fixed summation order over the slices
-  for (int e = ctx.tid; e < p.fo * p.fi; e += ctx.nthr) {
+  // The sum over the slices, in a fixed order and rounded once: it is the longest chain of all (128 slices at f_out = 8).  With
+  // few outputs up to 16 threads share one (one thread each, 1 -> 8 channels, nl = 30, batch 7: 26.6 us; SHAREFIG).
+  const int outputs = p.fo * p.fi, sharers = s2_grady_sharers(ctx.nthr, outputs);
+  struct Sum {
+    double re = 0, im = 0;
+  };
+  auto write = [&](int e, const Sum& t) {
     const int k = e / p.fo, jj = e - k * p.fo;
-    double re = 0, im = 0;     // (up to 1024 slices: the longest chain of all, rounded once)
-    for (int s2 = 0; s2 < nsl; ++s2) {
-      const float2 t = red[(s2 * p.fo + jj) * kThinFi + k];
-      re += t.x;
-      im += t.y;
-    }
-    const float2 s = make_float2((float)re, (float)im);
+    const float2 s = make_float2((float)t.re, (float)t.im);
     p.out[((long)(l * l + n) * p.fi + k) * p.fo + jj] = s;
     if (p.real && n > l) p.out[((long)(l * l + 2 * l - n) * p.fi + k) * p.fo + jj] = thin_mirror(s, l, n);
+  };
+  auto slices = [&](int e, int first) {
+    const int k = e / p.fo, jj = e - k * p.fo;
+    Sum t;
+    for (int s2 = first; s2 < nsl; s2 += sharers) {
+      const float2 v = red[(s2 * p.fo + jj) * kThinFi + k];
+      t.re += v.x;
+      t.im += v.y;
+    }
+    return t;
+  };
+  if (sharers == 1) {
+    for (int e = ctx.tid; e < outputs; e += ctx.nthr) write(e, slices(e, 0));
+  } else {
+    Sum t;
+    if (ctx.tid < outputs * sharers) t = slices(ctx.tid % outputs, ctx.tid / outputs);
+    ctx.sync();                  // (the parts take the place of what they were made from)
+    Sum* parts = reinterpret_cast<Sum*>(smem);
+    if (ctx.tid < outputs * sharers) parts[ctx.tid] = t;
+    ctx.sync();
+    if (ctx.tid < outputs) {
+      for (int g = 1; g < sharers; ++g) {
+        t.re += parts[g * outputs + ctx.tid].re;
+        t.im += parts[g * outputs + ctx.tid].im;
+      }
+      write(ctx.tid, t);
+    }
   }
 }
 

@@ -93,6 +93,7 @@ struct MmTcParams {
   int half;         // spectra of real signals: rows (kTcHalfRows) or columns (kTcHalfColumns) of outer index l .. 2l only,
                     // the others are their mirrors
   int two;          // without partial sums: the products with a lo part go into the second accumulator
+  int twins;        // half products, one CTA per tile: two CTAs compute it, one writes the tile and one its mirror (tc_twins)
   int segs;         // > 1: a tile's K blocks are summed in this many segments, in one CTA or one to a CTA of a cluster (tc_segments)
   int run;          // floats per outer contraction index: 2 fi (fwd), 2 fo (grad x), 2 nb (grad y)
   int kblk;         // floats per K block (multiple of 8, <= kTcKMax)
@@ -330,18 +331,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
   // ---- which tile ---------------------------------------------------------------------------
-  const int nsplit = p.csize * p.groups;
+  const int nsplit = p.csize * p.groups, per_tile = p.twins ? 2 : nsplit;
   int l = p.nl - 1;
   long t = blockIdx.x;
   for (;; --l) {
-    const long c = tc_tiles_for(OP, p.half, p.nb, p.fi, p.fo, l) * nsplit;
+    const long c = tc_tiles_for(OP, p.half, p.nb, p.fi, p.fo, l) * per_tile;
     if (t < c) break;
     t -= c;
   }
   const int L = 2 * l + 1;
   // K blocks handled by this CTA: [it_lo, it_hi) of the L * nblk blocks (outer index, block of its run)
-  const int split = (int)(t % nsplit);
-  t /= nsplit;
+  const bool second = p.twins && t % 2 == 1;      // of a pair: writes the mirror
+  const int split = p.twins ? 0 : (int)(t % nsplit);
+  t /= per_tile;
   const int it_lo = (int)((long)split * L * p.nblk / nsplit), it_hi = (int)((long)(split + 1) * L * p.nblk / nsplit);
   const int o_lo = it_lo / p.nblk, kb_lo = it_lo - o_lo * p.nblk;
   const TcGeom geo = tc_geom(OP, p.nb, p.fi, p.fo);
@@ -694,7 +696,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   // mirror (-m, -n) is coefficient L * L - 1 - q, (-1)^(m - n) = (-1)^q times the conjugate (L is odd)
   constexpr bool kPlain = OP == kTcPlainCC || OP == kTcPlainSC;
   const int sro = OP == kTcGradY ? 1 : L, sco = OP == kTcGradY ? L : 1;
-  const bool row_mirror = !kPlain && p.half == kTcHalfRows && rq > 0, col_half = !kPlain && p.half == kTcHalfColumns;
+  const bool mirrors = !kPlain && (second || !p.twins);
+  const bool row_mirror = mirrors && p.half == kTcHalfRows && rq > 0, col_half = mirrors && p.half == kTcHalfColumns;
   auto at_coefficient = [&](int q, int rem) { return p.c + ((spec0 + q) * RI + ri) * CW + rem; };
   auto mirrored = [](float4 o, float s) { return make_float4(s * o.x, -s * o.y, s * o.z, -s * o.w); };
   // two columns (one complex number: never straddles an outer column index), four with VEC
@@ -705,7 +708,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
       *reinterpret_cast<float2*>(p.c + (long)r * p.c_rs + (long)(gcol >> 1) * p.c_ps) = make_float2(a, b);
     } else {
       const int cq = gcol / CW, rem = gcol - cq * CW, q = ro * sro + (co0 + cq) * sco;
-      *reinterpret_cast<float2*>(at_coefficient(q, rem)) = make_float2(a, b);
+      if (!second) *reinterpret_cast<float2*>(at_coefficient(q, rem)) = make_float2(a, b);
       if (row_mirror || (col_half && cq > 0)) {
         const float s = (q & 1) ? -1.f : 1.f;
         *reinterpret_cast<float2*>(at_coefficient(L * L - 1 - q, rem)) = make_float2(s * a, -s * b);
@@ -716,7 +719,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
     if constexpr (VEC && !kPlain) {
       if (gcol >= Np) return;     // CW is a multiple of 4, so a group of 4 is all in or all out
       const int cq = gcol / CW, rem = gcol - cq * CW, q = ro * sro + (co0 + cq) * sco;
-      *reinterpret_cast<float4*>(at_coefficient(q, rem)) = o;
+      if (!second) *reinterpret_cast<float4*>(at_coefficient(q, rem)) = o;
       if (row_mirror || (col_half && cq > 0)) *reinterpret_cast<float4*>(at_coefficient(L * L - 1 - q, rem)) = mirrored(o, (q & 1) ? -1.f : 1.f);
     } else {
       store2(gcol, o.x, o.y);
@@ -779,7 +782,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
           float8 o;
           o.lo = make_float4(v[8 * c8], v[8 * c8 + 1], v[8 * c8 + 2], v[8 * c8 + 3]);
           o.hi = make_float4(v[8 * c8 + 4], v[8 * c8 + 5], v[8 * c8 + 6], v[8 * c8 + 7]);
-          st_global_256(at_coefficient(q, rem), o);
+          if (!second) st_global_256(at_coefficient(q, rem), o);
           if (row_mirror || (col_half && cq > 0)) {
             const float s = (q & 1) ? -1.f : 1.f;
             o.lo = mirrored(o.lo, s);
@@ -853,8 +856,13 @@ constexpr int kTcSlots[kTcMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15}
 // tiles for clusters even at batch 1, or longer contractions: one CTA, the whole chain or groups of seven.
 inline int tc_segments(int nl, int fi, int fo, int blocks) {
   const int s = (2 * blocks + 14) / 15;
-  return s <= kTcMaxCluster && so3_mm_tc_tiles(kTcFwd, kTcHalfColumns, nl, 1, fi, fo) <= kTcSlots[s] ? s : 0;
+  return blocks >= 12 && s <= kTcMaxCluster && so3_mm_tc_tiles(kTcFwd, kTcHalfColumns, nl, 1, fi, fo) <= kTcSlots[s] ? s : 0;
 }
+
+// A half product whose tiles leave half of the chip idle: each is computed twice, by one CTA that writes the tile and one
+// that writes its mirror, since a CTA's 64 KB of output take 1 - 2 us on one SM.  The results are the same.  All
+// columns -> half in one CTA -> pairs: TWINFIGS
+inline bool tc_twins(int half, long tiles, int ns) { return half && ns == 1 && 2 * tiles <= kTcSlots[1]; }
 
 // CTAs per tile.  One CTA fits on an SM; a product with few output tiles and a long contraction (the
 // transposed kernel transform of a layer with few channels: one or two tiles of several hundred K

@@ -21,7 +21,7 @@ constexpr int kWigZT = 64;  // batch elements per block tile (even): SO(3), and 
 // 64 degrees 1.96e-7 / 2.1e-7 / 1.23e-7, there and back 2.47e-7 / 2.67e-7 / 1.74e-7, the signal of a random spectrum of 20
 // degrees 1.03e-7 / 1.1e-7 / 0.97e-7.  (Not below it: the signal of 20 degrees that a whole analysis made, 0.92e-7 / 1.05e-7 /
 // 1.0e-7, where the row transforms are most of the error.)
-constexpr int kWigChain = 8;
+constexpr int kWigChain = 8, kWigChainBeta = 32;     // degrees (synthesis), betas (analysis)
 
 // Rows of N mod 4 = 2 betas are staged with two columns of zeros.
 S2C_HD constexpr int wig_np(int N) { return (N + 3) / 4 * 4; }
@@ -161,7 +161,7 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
         const float* wp = Ws + 4 * tl * LDW;
         const float2* vp = Vs + zz * LDV;
         for (int bt = 0; bt < NH; bt += 4) {
-          if (kHalf && bt % kWigChain == 0) next_chain(t);
+          if (kHalf && bt % kWigChainBeta == 0) next_chain(t);
           const float4 va = *reinterpret_cast<const float4*>(vp + bt);
           const float4 vb = *reinterpret_cast<const float4*>(vp + bt + 2);
 #pragma unroll
@@ -179,7 +179,7 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
         const float2* v0 = Vs + tz * LDV;
         const float2* v1 = Vs + (tz + ZH) * LDV;
         for (int bt = 0; bt < NH; bt += 4) {
-          if (kHalf && bt % kWigChain == 0) next_chain(t);
+          if (kHalf && bt % kWigChainBeta == 0) next_chain(t);
           float4 w4[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) w4[i] = *reinterpret_cast<const float4*>(wp + i * LDW + bt);
