@@ -120,6 +120,9 @@ inline int dev_smem_limit() {
 // another kernel touches; that returns when the kernel ahead has finished, its writes included.  So the order of the stream
 // stands; what goes away is 1 - 2 us between the end of a kernel and the first instruction of the next (two launches at
 // b = 22, 45 signals: 24.6 -> 20.8 us; 135 at b = 30, a training step: 2672 -> 2515; five, a rotation: 50.7 -> 39.5).
+// Those are calls one after another, whose first kernel also meets the last one of the call before.  Calls that are waited for
+// keep the gaps between their own kernels: analysis, synthesis and rotation of 200 signals at b = 12 24.6 -> 22.1, 26.1 -> 24.2
+// and 58 -> 49 us, of 2000 at b = 16, many waves each, 192 -> 189, 211 -> 204, 526 -> 515.  None at b = 9 - 64 got slower either way.
 // stream_order_next lets the next kernel's blocks in once every block has called it: at a block's end.  Called at the
 // beginning, the next kernel's blocks crowd on the SMs that are done first (rotation 46.9 us, S2 transforms of 192 signals
 // 77.6 instead of 67.4); the tensor-core products, one block per SM whatever comes next, call it there.

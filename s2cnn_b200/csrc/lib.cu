@@ -86,7 +86,8 @@ static int launch_inv_plane(int N, long zc, stream_t st, const InvPlaneParams& f
   if (N == 128) return S2C_LAUNCH_PLANE(so3_inv_plane, 128, grid, st, f);
   return S2C_LAUNCH_PLANE(so3_inv_plane, 64, grid, st, f);
 }
-// The order in which the analysis' Wigner kernel takes its items, one block per SM (two at N = 64) walking its share:
+// The order in which the analysis' Wigner kernel takes its items, one block per SM (no second one fits, at either length:
+// with two to an SM in the grid of N = 64, 64 signals took 63.2 us for 61.4, 512 485 for 482) walking its share:
 // sorted by their table rows and dealt out forwards and backwards in turn, so that the shares are equal to a few percent.
 // (In the order of n and m a quarter of the SM time was idle at b = 64: 48 us per 8 signals instead of 39.)
 static void rows_order(int nl, int K, RowsOrder* out) {

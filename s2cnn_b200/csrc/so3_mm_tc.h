@@ -341,18 +341,28 @@ __global__ void __launch_bounds__(kTcThreads, 1) so3_mm_tc_kernel(const MmTcPara
   }
   const int L = 2 * l + 1;
   // K blocks handled by this CTA: [it_lo, it_hi) of the L * nblk blocks (outer index, block of its run)
-  const bool second = p.twins && t % 2 == 1;      // of a pair: writes the mirror
-  const int split = p.twins ? 0 : (int)(t % nsplit);
-  t /= per_tile;
-  const int it_lo = (int)((long)split * L * p.nblk / nsplit), it_hi = (int)((long)(split + 1) * L * p.nblk / nsplit);
-  const int o_lo = it_lo / p.nblk, kb_lo = it_lo - o_lo * p.nblk;
+  // (few divisions, of 32 bits: every CTA waits for this)
+  int tile_no = (int)t, split = 0, it_lo = 0, it_hi = L * p.nblk, o_lo = 0;
+  bool second = false;      // of a pair: writes the mirror
+  if (p.twins) {
+    second = tile_no & 1;
+    tile_no >>= 1;
+  } else if (nsplit > 1) {
+    const int whole = tile_no / nsplit;
+    split = tile_no - whole * nsplit;
+    tile_no = whole;
+    it_lo = (int)((long)split * L * p.nblk / nsplit);
+    it_hi = (int)((long)(split + 1) * L * p.nblk / nsplit);
+    o_lo = it_lo / p.nblk;
+  }
+  const int kb_lo = it_lo - o_lo * p.nblk;
   const TcGeom geo = tc_geom(OP, p.nb, p.fi, p.fo);
   const int RI = geo.RI, CW = geo.CW;
   // outer indices of the first row and column
   const int ro0 = p.half == kTcHalfRows ? l : 0, co0 = p.half == kTcHalfColumns ? l : 0;
   const int M = (L - ro0) * RI, Np = (L - co0) * CW;
   const int tiles_n = (Np + kTcBN - 1) / kTcBN;
-  const int row0 = (int)(t / tiles_n) * kTcBM, col0 = (int)(t % tiles_n) * kTcBN;
+  const int row0 = tile_no / tiles_n * kTcBM, col0 = tile_no % tiles_n * kTcBN;
   const long spec0 = (long)l * (4L * l * l - 1) / 3;
   const int fi2 = 2 * p.fi, fo2 = 2 * p.fo;
   const int nit = it_hi - it_lo;                          // K blocks of this CTA (a shared tile: possibly none)

@@ -17,10 +17,10 @@ namespace s2c {
 constexpr int kWigZT = 64;  // batch elements per block tile (even): SO(3), and the most for S2
 // kHalf, S2 transforms of real signals: the frequencies m >= 0 alone.  The two signs are then one sum, no longer two with
 // independent roundings, of which whatever reads them takes the mean: terms are summed in chains of this many, which join
-// the sum.  Relative errors at b = 64 with all frequencies / half in one chain / half in these: symmetric part of a spectrum of
-// 64 degrees 1.96e-7 / 2.1e-7 / 1.23e-7, there and back 2.47e-7 / 2.67e-7 / 1.74e-7, the signal of a random spectrum of 20
-// degrees 1.03e-7 / 1.1e-7 / 0.97e-7.  (Not below it: the signal of 20 degrees that a whole analysis made, 0.92e-7 / 1.05e-7 /
-// 1.0e-7, where the row transforms are most of the error.)
+// the sum.  Relative errors at b = 64 with all frequencies / half in one chain / half in these, in 1e-7: symmetric part of a
+// spectrum of 64 degrees 1.94 / 2.08 / 1.39, there and back 2.45 / 2.68 / 1.87, the signal of such a spectrum 1.28 / 1.45 /
+// 1.10.  (Not quite for few degrees of a long grid, where the row transforms are most of the error: 20 degrees 0.92 / 1.05 /
+// 1.00.)
 constexpr int kWigChain = 8, kWigChainBeta = 32;     // degrees (synthesis), betas (analysis)
 
 // Rows of N mod 4 = 2 betas are staged with two columns of zeros.
@@ -79,6 +79,7 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
 
   // kHalf: what is in the accumulators joins the sums of the chains before
   float sr[kHalf ? 2 : 1][4][2], si[kHalf ? 2 : 1][4][2];
+  const int chain = kHalf ? kWigChainBeta : NH;
   auto next_chain = [&](int t) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -160,44 +161,50 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
         const int tl = tile / zc, zz = tile - tl * zc;
         const float* wp = Ws + 4 * tl * LDW;
         const float2* vp = Vs + zz * LDV;
-        for (int bt = 0; bt < NH; bt += 4) {
-          if (kHalf && bt % kWigChainBeta == 0) next_chain(t);
-          const float4 va = *reinterpret_cast<const float4*>(vp + bt);
-          const float4 vb = *reinterpret_cast<const float4*>(vp + bt + 2);
+        for (int first = 0; first < NH; first += chain) {
+          const int end = NH - first < chain ? NH : first + chain;
+          for (int bt = first; bt < end; bt += 4) {
+            const float4 va = *reinterpret_cast<const float4*>(vp + bt);
+            const float4 vb = *reinterpret_cast<const float4*>(vp + bt + 2);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 w4 = *reinterpret_cast<const float4*>(wp + i * LDW + bt);
-            ar[t][i][0] = fmaf(w4.x, va.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4.x, va.y, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4.y, va.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4.y, va.w, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4.z, vb.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4.z, vb.y, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4.w, vb.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4.w, vb.w, ai[t][i][0]);
+            for (int i = 0; i < 4; ++i) {
+              const float4 w4 = *reinterpret_cast<const float4*>(wp + i * LDW + bt);
+              ar[t][i][0] = fmaf(w4.x, va.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4.x, va.y, ai[t][i][0]);
+              ar[t][i][0] = fmaf(w4.y, va.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4.y, va.w, ai[t][i][0]);
+              ar[t][i][0] = fmaf(w4.z, vb.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4.z, vb.y, ai[t][i][0]);
+              ar[t][i][0] = fmaf(w4.w, vb.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4.w, vb.w, ai[t][i][0]);
+            }
           }
+          if (kHalf) next_chain(t);
         }
       } else {
         const int tl = tile / ZH, tz = tile - tl * ZH;
         const float* wp = Ws + 4 * tl * LDW;
         const float2* v0 = Vs + tz * LDV;
         const float2* v1 = Vs + (tz + ZH) * LDV;
-        for (int bt = 0; bt < NH; bt += 4) {
-          if (kHalf && bt % kWigChainBeta == 0) next_chain(t);
-          float4 w4[4];
+        for (int first = 0; first < NH; first += chain) {
+          const int end = NH - first < chain ? NH : first + chain;
+          for (int bt = first; bt < end; bt += 4) {
+            float4 w4[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) w4[i] = *reinterpret_cast<const float4*>(wp + i * LDW + bt);
-          const float4 a0 = *reinterpret_cast<const float4*>(v0 + bt);       // beta, beta+1 of z = tz
-          const float4 b0 = *reinterpret_cast<const float4*>(v0 + bt + 2);   // beta+2, beta+3
-          const float4 a1 = *reinterpret_cast<const float4*>(v1 + bt);       // z = tz + ZH
-          const float4 b1 = *reinterpret_cast<const float4*>(v1 + bt + 2);
+            for (int i = 0; i < 4; ++i) w4[i] = *reinterpret_cast<const float4*>(wp + i * LDW + bt);
+            const float4 a0 = *reinterpret_cast<const float4*>(v0 + bt);       // beta, beta+1 of z = tz
+            const float4 b0 = *reinterpret_cast<const float4*>(v0 + bt + 2);   // beta+2, beta+3
+            const float4 a1 = *reinterpret_cast<const float4*>(v1 + bt);       // z = tz + ZH
+            const float4 b1 = *reinterpret_cast<const float4*>(v1 + bt + 2);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            ar[t][i][0] = fmaf(w4[i].x, a0.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].x, a0.y, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4[i].y, a0.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].y, a0.w, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4[i].z, b0.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].z, b0.y, ai[t][i][0]);
-            ar[t][i][0] = fmaf(w4[i].w, b0.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].w, b0.w, ai[t][i][0]);
-            ar[t][i][1] = fmaf(w4[i].x, a1.x, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].x, a1.y, ai[t][i][1]);
-            ar[t][i][1] = fmaf(w4[i].y, a1.z, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].y, a1.w, ai[t][i][1]);
-            ar[t][i][1] = fmaf(w4[i].z, b1.x, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].z, b1.y, ai[t][i][1]);
-            ar[t][i][1] = fmaf(w4[i].w, b1.z, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].w, b1.w, ai[t][i][1]);
+            for (int i = 0; i < 4; ++i) {
+              ar[t][i][0] = fmaf(w4[i].x, a0.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].x, a0.y, ai[t][i][0]);
+              ar[t][i][0] = fmaf(w4[i].y, a0.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].y, a0.w, ai[t][i][0]);
+              ar[t][i][0] = fmaf(w4[i].z, b0.x, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].z, b0.y, ai[t][i][0]);
+              ar[t][i][0] = fmaf(w4[i].w, b0.z, ar[t][i][0]); ai[t][i][0] = fmaf(w4[i].w, b0.w, ai[t][i][0]);
+              ar[t][i][1] = fmaf(w4[i].x, a1.x, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].x, a1.y, ai[t][i][1]);
+              ar[t][i][1] = fmaf(w4[i].y, a1.z, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].y, a1.w, ai[t][i][1]);
+              ar[t][i][1] = fmaf(w4[i].z, b1.x, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].z, b1.y, ai[t][i][1]);
+              ar[t][i][1] = fmaf(w4[i].w, b1.z, ar[t][i][1]); ai[t][i][1] = fmaf(w4[i].w, b1.w, ai[t][i][1]);
+            }
           }
+          if (kHalf) next_chain(t);
         }
       }
     }
@@ -206,7 +213,6 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
   if constexpr (kHalf) {
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-      next_chain(t);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
