@@ -1490,8 +1490,8 @@ int s2c_so3_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb,
 // of the multiply-adds, and write each coefficient and its mirror.  us on one B200, all rows -> half, for z, gx
 // and gy: 100 -> 100 channels, nl = 10, batch 32: 314, 325, 314 -> 199, 211, 203; 16 -> 16, nl = 15, batch 32: 77, 80, 65 -> 49,
 // 52, 51; 20 -> 40, nl = 6, batch 256: 42, 50, 52 -> 32, 33, 36; 8 -> 16, nl = 15, batch 32: z 41 -> 28 (half of the rows: 32).
-// Calls whose tiles all run at once take the time they took, or 1 - 2 us more (16 -> 24, nl = 7, batch 32: 16.5 -> 19.2,
-// segments in one CTA).
+// Calls whose tiles all run at once take the time they took, or up to 3 us more (tc_twins); so do kernel gradients of one to four
+// signals (24 -> 46, nl = 8: 13.2 -> 16.5).
 size_t s2c_so3_mm_real_workspace(int op, int nl, int nb, int fi, int fo) {
 #ifndef S2C_EMUL
   if ((op == kTcGradX || op == kTcGradY) && nl >= 1 && nb >= 1 && fi >= 1 && fo >= 1)
@@ -1549,9 +1549,8 @@ int s2c_s2_mm_gradx(const float* gz, const float* y, float* gx, int nl, int nb, 
 int s2c_s2_mm_grady(const float* gz, const float* x, float* gy, int nl, int nb, int fi, int fo, void* st) {
   return s2_mm_grady_any(0, gz, x, gy, nl, nb, fi, fo, st);
 }
-// Spectra of real signals: half of the result's rows, the others mirrored, and half of gz read.  Gradient of y, 6 -> 100
-// channels, nl = 16, batch 32: 103 -> 72 us (with eight rows in flight for four); 1 -> 8, nl = 30, batch 32: 69 -> 41; of x:
-// 333 -> 176, 50 -> 38.
+// Spectra of real signals: half of the result's rows, the others mirrored, and half of gz read.  Gradient of y, all rows ->
+// half, 6 -> 100 channels, nl = 16, batch 32: 77 -> 52 us; 1 -> 8, nl = 30, batch 32: 48 -> 27; of x: 278 -> 179, 25 -> 17.
 int s2c_s2_mm_real_gradx(const float* gz, const float* y, float* gx, int nl, int nb, int fi, int fo, void* st) {
   return s2_mm_gradx_any(1, gz, y, gx, nl, nb, fi, fo, st);
 }

@@ -863,15 +863,21 @@ constexpr int kTcSlots[kTcMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15}
 // number follows from the layer alone, so that a result does not depend on the batch it was computed in.  Whole chain in
 // one CTA -> cluster: 20 -> 40, nl = 6, batch 1: 13.7 -> 10.1 us, batch 32: 15.5 -> 12.1; 13 -> 9, nl = 7, batch 5: 17.1 ->
 // 9.9; segments in one CTA, for more tiles than clusters: 16 -> 24, nl = 7, batch 32: 17.8 -> 18.6.  0: a layer with too many
-// tiles for clusters even at batch 1, or longer contractions: one CTA, the whole chain or groups of seven.
+// tiles for clusters even at batch 1, or longer contractions: one CTA, the whole chain or groups of seven; or shorter ones,
+// whose chain is worth less than a cluster's meeting (24 -> 32, nl = 3, ten blocks, batch 1 and 32: 8.7 and 10.5 in two segments,
+// 8.4 and 9.9 in one CTA and its twin; with 14 blocks, 24 -> 24, nl = 4, the clusters are half a microsecond ahead).
 inline int tc_segments(int nl, int fi, int fo, int blocks) {
   const int s = (2 * blocks + 14) / 15;
   return blocks >= 12 && s <= kTcMaxCluster && so3_mm_tc_tiles(kTcFwd, kTcHalfColumns, nl, 1, fi, fo) <= kTcSlots[s] ? s : 0;
 }
 
 // A half product whose tiles leave half of the chip idle: each is computed twice, by one CTA that writes the tile and one
-// that writes its mirror, since a CTA's 64 KB of output take 1 - 2 us on one SM.  The results are the same.  All
-// columns -> half in one CTA -> pairs: TWINFIGS
+// that writes its mirror, since a CTA's 64 KB of output take about 1 us on one SM.  The results are the same.  All
+// columns / half, one CTA per tile / pairs: 16 -> 24, nl = 7, batch 32: 15.9 / 18.8 / 17.4 us; 24 -> 46, nl = 8, batch 16:
+// 22.3 / 25.6 / 23.0; 8 -> 16, nl = 15, batch 7: 15.5 / 17.1 / 15.7.  What is left above the whole product is the adding of
+// segments in one CTA (up to 1.9 us), and up to 3 where the pairs no longer run at once (24 -> 46, nl = 8, batch 32: 22.9 /
+// 25.7): the price of half of the columns at 49 - 100 tiles, while fewer take clusters (batch 7: 21.5 / 11.4) and more take
+// several waves (batch 256: 139.7 / 101.2); the choice may not depend on the batch.
 inline bool tc_twins(int half, long tiles, int ns) { return half && ns == 1 && 2 * tiles <= kTcSlots[1]; }
 
 // CTAs per tile.  One CTA fits on an SM; a product with few output tiles and a long contraction (the

@@ -40,9 +40,10 @@
 
 namespace s2c {
 
-// Batch elements per chunk, 256 MB of V.  That is more than L2 holds: long launches weigh more than keeping V in L2 (64
-// signals at b = 64, analysis / synthesis: 651 / 699 us in chunks of 8 (67 MB), 603 / 637 of 16, 589 / 615 of 32, 581 / 602
-// of 64; 512 signals at b = 32: 1190 / 1188 us of 8, 632 / 666 of 32, 576 / 617 of 64, 525 / 602 of 128, 500 / 574 of 256).
+// Batch elements per chunk, 256 MB of V.  That is more than L2 holds: long launches weigh more than keeping V in L2, also
+// with programmatic launches (64 signals at b = 64, analysis / synthesis: 719 / 789 us in chunks of 4, 597 / 659 of 8 (67 MB),
+// 558 / 612 of 16, 561 / 598 of 32; 512 signals at b = 32: 901 / 937 us of 8, 552 / 607 of 32, 508 / 575 of 64, 490 / 574 of
+// 128, 490 / 555 of 256).
 S2C_HD constexpr int rows_zc(int N) { return N == 128 ? 32 : 256; }
 constexpr int kRowsZQ = 4;      // batch elements per item
 constexpr int kRowsMG = 16;     // values of |m| per item = warps per block

@@ -72,17 +72,19 @@ def test_half_products_match_the_full_ones(backend, nl, nb, fi, fo):
 # layers whose forward products are not segmented: contractions too long for eight segments (partial sums every seven
 # blocks), or too many tiles for clusters (one chain, the products with a lo part in an accumulator of their own)
 WIDE = [(10, 2, 100, 100), (5, 3, 100, 255), (15, 2, 16, 16), (15, 2, 8, 16)]
+# ... too short for segments; pairs of CTAs per tile, with segments and without; one CTA per tile where pairs do not fit
+PAIRS = [(2, 16, 32, 64), (7, 32, 16, 24), (15, 7, 8, 16), (6, 64, 8, 46), (8, 32, 24, 46), (5, 20, 9, 7)]
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nl,nb,fi,fo", WIDE)
+@pytest.mark.parametrize("nl,nb,fi,fo", WIDE + PAIRS)
 def test_wide_half_products_match_the_full_ones(nl, nb, fi, fo):
     test_half_products_match_the_full_ones("cuda", nl, nb, fi, fo)
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nl,fi,fo", [(6, 20, 40), (3, 32, 64), (7, 13, 9), (2, 4, 4), (7, 16, 24), (12, 24, 3)] +
-                         [(nl, fi, fo) for nl, _, fi, fo in WIDE])
+                         [(nl, fi, fo) for nl, _, fi, fo in WIDE + PAIRS])
 def test_forward_does_not_depend_on_the_batch(nl, fi, fo):
     """A tile's segments, one to a block of a cluster (few signals) or one after the other, give the same bits."""
     ops, dev = backends.get("cuda")
