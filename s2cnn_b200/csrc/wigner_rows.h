@@ -292,8 +292,10 @@ struct so3_fwd_wigner_r_impl {
     float* rings = reinterpret_cast<float*>(smem) + rows_tile_floats(N);
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(rings + kRowsMG * kRing);     // [sign]
     int* readers = reinterpret_cast<int*>(bar + 2);
-    // set by the lanes whose wait has given up: no copy is issued or trusted any more, V is read from global memory
-    volatile int* late = readers + 1;
+    // bit 16 of `readers` is set by the lanes whose wait has given up: no copy is issued or trusted any more (the count is
+    // never 15 again), V is read from global memory
+    constexpr int kLate = 1 << 16;
+    auto late = [&] { return *reinterpret_cast<const volatile int*>(readers) >= kLate; };
     float* xch = reinterpret_cast<float*>(bar + 4) + warp * 32 * 17;
     const int K = p.K, zc = p.zc, items = rows_items(K, zc);
     const RowsLane ln(lane);
@@ -311,7 +313,6 @@ struct so3_fwd_wigner_r_impl {
       bulk_barrier_init(bar);
       bulk_barrier_init(bar + 1);
       *readers = 0;
-      *late = 0;
       fetch(next(0));
     }
     ctx.sync();
@@ -340,8 +341,12 @@ struct so3_fwd_wigner_r_impl {
       // s = (-1)^(l+n).  Index [2 z + re/im][pair of neighbouring betas].
       float2 v1[4][2 * NP], v2[4][2 * NP];
       {
-        const bool landed = !*late && bulk_wait(ctx, bar, phase) && bulk_wait(ctx, bar + 1, phase);
-        if (!landed) *late = 1;
+        const bool landed = !late() && bulk_wait(ctx, bar, phase) && bulk_wait(ctx, bar + 1, phase);
+#ifndef S2C_EMUL
+        if (!landed) atomicOr(readers, kLate);
+#else
+        if (!landed) *readers |= kLate;
+#endif
         const float2* col = landed ? tile + ln.s * kRowsZQ * N * kRowsMG : p.v + rows_part(N, zc, g, ln.s);
 #pragma unroll
         for (int z = 0; z < 2; ++z) {
@@ -369,13 +374,13 @@ struct so3_fwd_wigner_r_impl {
         if (atomicAdd(readers, 1) == kRowsMG - 1) {
           *readers = 0;
           __threadfence_block();
-          if (!*late) fetch(next(turn + 1));
+          fetch(next(turn + 1));
         }
       }
       __syncwarp();
 #else
       ctx.sync();
-      if (ctx.tid == 0 && !*late) fetch(next(turn + 1));
+      if (ctx.tid == 0 && !late()) fetch(next(turn + 1));
 #endif
 
       // output: row li + b % 4 (lanes b < 4) or its mirror (b >= 4), frequency +-m, batch elements from zp
@@ -443,7 +448,7 @@ struct so3_fwd_wigner_r_impl {
       }
       ctx.sync_warp();                // the ring is free for the next item
     }
-    if (*late) {     // what is still under way gets its time, before the block's shared memory goes to another
+    if (late()) {     // what is still under way gets its time, before the block's shared memory goes to another
       for (int k = 0; k < 4; ++k) {
 #ifndef S2C_EMUL
         bulk_wait(ctx, bar + k / 2, k & 1);

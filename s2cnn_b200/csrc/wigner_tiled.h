@@ -78,24 +78,18 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
     for (int i = 0; i < 4; ++i) { ar[t][i][0] = ar[t][i][1] = ai[t][i][0] = ai[t][i][1] = 0.f; }
 
   // kHalf: what is in the accumulators joins the sums of the chains before
-  float sr[kHalf ? 2 : 1][4][2], si[kHalf ? 2 : 1][4][2];
+  float sr[4][2], si[4][2];
   const int chain = kHalf ? kWigChainBeta : NH;
   auto next_chain = [&](int t) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        sr[t][i][j] += ar[t][i][j];
-        si[t][i][j] += ai[t][i][j];
+        sr[i][j] += ar[t][i][j];
+        si[i][j] += ai[t][i][j];
         ar[t][i][j] = ai[t][i][j] = 0.f;
       }
   };
-  if constexpr (kHalf) {
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) { sr[t][i][0] = sr[t][i][1] = si[t][i][0] = si[t][i][1] = 0.f; }
-  }
 
   {
     if (N % 4 == 0) {
@@ -157,6 +151,10 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
     for (int t = 0; t < 2; ++t) {
       const int tile = ctx.tid + t * ctx.nthr;
       if (tile >= ntiles) continue;
+      if constexpr (kHalf) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sr[i][0] = sr[i][1] = si[i][0] = si[i][1] = 0.f;
+      }
       if (narrow) {
         const int tl = tile / zc, zz = tile - tl * zc;
         const float* wp = Ws + 4 * tl * LDW;
@@ -207,18 +205,15 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
           if (kHalf) next_chain(t);
         }
       }
+      if constexpr (kHalf) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) { ar[t][i][j] = sr[i][j]; ai[t][i][j] = si[i][j]; }
+      }
     }
   }
 
-  if constexpr (kHalf) {
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) { ar[t][i][j] = sr[t][i][j]; ai[t][i][j] = si[t][i][j]; }
-    }
-  }
   const float fudge = ((m - n) & 1) ? -1.f : 1.f;
   const bool self = (m == 0 && n == 0);
   auto emit = [&](int li, int zz, float re, float im) {
@@ -264,7 +259,7 @@ S2C_D void fwd_wigner_tiled(const Ctx& ctx, const FwdWignerParams& p, unsigned c
 }
 
 S2C_KERNEL(so3_fwd_wigner_t, FwdWignerParams) { fwd_wigner_tiled<false>(ctx, p, smem); }
-S2C_KERNEL(s2_fwd_wigner_t_half, FwdWignerParams) { fwd_wigner_tiled<true>(ctx, p, smem); }
+S2C_KERNEL_BOUNDS(s2_fwd_wigner_t_half, FwdWignerParams, kThreads, 3) { fwd_wigner_tiled<true>(ctx, p, smem); }
 
 inline size_t inv_wigner_t_smem(int N, int K, int zt = kWigZT) {
   return (size_t)K * wig_np(N) * sizeof(float) + (size_t)K * (zt + 2) * sizeof(float2);
@@ -367,7 +362,8 @@ S2C_D void inv_wigner_tiled(const Ctx& ctx, const InvWignerParams& p, unsigned c
       for (int i = 0; i < 4; ++i) acc[j][i] = make_float2(0.f, 0.f);
     const float* wp = Ws + 4 * tb;
     const float2* xp = Xs + 2 * tz;
-    float2 sum[kHalf ? 2 : 1][4];
+    float2 sum[2][4];
+    const int chain = kHalf ? kWigChain : L;
     auto next_chain = [&]() {
 #pragma unroll
       for (int j = 0; j < 2; ++j)
@@ -383,19 +379,21 @@ S2C_D void inv_wigner_tiled(const Ctx& ctx, const InvWignerParams& p, unsigned c
 #pragma unroll
         for (int i = 0; i < 4; ++i) sum[j][i] = make_float2(0.f, 0.f);
     }
-    for (int li = 0; li < L; ++li) {
-      if (kHalf && li % kWigChain == 0) next_chain();
-      const float4 w4 = *reinterpret_cast<const float4*>(wp + li * NP);
-      const float4 x4 = *reinterpret_cast<const float4*>(xp + li * ZP);  // (re0, im0, re1, im1)
-      const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+    for (int first = 0; first < L; first += chain) {
+      const int end = L - first < chain ? L : first + chain;
+      for (int li = first; li < end; ++li) {
+        const float4 w4 = *reinterpret_cast<const float4*>(wp + li * NP);
+        const float4 x4 = *reinterpret_cast<const float4*>(xp + li * ZP);  // (re0, im0, re1, im1)
+        const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        acc[0][i] = fma2(make_float2(w[i], w[i]), make_float2(x4.x, x4.y), acc[0][i]);
-        acc[1][i] = fma2(make_float2(w[i], w[i]), make_float2(x4.z, x4.w), acc[1][i]);
+        for (int i = 0; i < 4; ++i) {
+          acc[0][i] = fma2(make_float2(w[i], w[i]), make_float2(x4.x, x4.y), acc[0][i]);
+          acc[1][i] = fma2(make_float2(w[i], w[i]), make_float2(x4.z, x4.w), acc[1][i]);
+        }
       }
+      if (kHalf) next_chain();
     }
     if constexpr (kHalf) {
-      next_chain();
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -413,6 +411,6 @@ S2C_D void inv_wigner_tiled(const Ctx& ctx, const InvWignerParams& p, unsigned c
 }
 
 S2C_KERNEL(so3_inv_wigner_t, InvWignerParams) { inv_wigner_tiled<false>(ctx, p, smem); }
-S2C_KERNEL(s2_inv_wigner_t_half, InvWignerParams) { inv_wigner_tiled<true>(ctx, p, smem); }
+S2C_KERNEL_BOUNDS(s2_inv_wigner_t_half, InvWignerParams, kThreads, 4) { inv_wigner_tiled<true>(ctx, p, smem); }
 
 }  // namespace s2c
